@@ -18,19 +18,14 @@
 //                 the factored diagonal blocks into the fronts;
 //   k_syrk        one CTA per 64x64 tile of every front's trailing lower
 //                 triangle: register-blocked rank-32 update.
-//   k_inverse     one warp per 32 columns of each diagonal block: L_JJ^{-1},
-//                 stored row-major, so the solves are matrix-vector products.
+//   k_diag_inv, k_offdiag_inv, k_w  X = L_JJ^{-1} and W = L_RJ X of every
+//                 front, stored as one column-major matrix M = [X; W], so the
+//                 solves are matrix-vector products.
 //
-// Solve H0 v (3 right-hand sides interleaved per node), per level and in
-// tiles of 32 rows (or columns) of a front, so that large fronts spread over
-// many CTAs:
-//   forward   k_fwd_y: y_J = L_JJ^{-1} f_J, f = b_J + children's updates
-//             k_fwd_g: g = f_R - L_RJ y_J (the update passed to the parent)
-//   backward  k_bwd_t: t_J = y_J - L_RJ^T x_R (x_R from the ancestors)
-//             k_bwd_x: x_J = L_JJ^{-T} t_J
-// Every sum is formed in a fixed order (no atomics): results are deterministic.
-// The whole solve (gather, 4 launches per level, scatter) is replayed as one
-// CUDA graph per input vector.
+// Solve H0 v (3 right-hand sides interleaved per node): one persistent launch,
+// k_solve below.  Every sum is formed in a fixed order (no atomics): results
+// are deterministic.  An application by itself is replayed as one CUDA graph
+// per input vector.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,16 +43,16 @@ namespace {
 constexpr int kFT = 256;  // factor threads
 constexpr int kNB = 32;   // factor panel width
 constexpr int kTS = 64;   // SYRK tile
-constexpr int kST = 256;  // solve threads: one warp per output row / column
+constexpr int kST = 256;  // solve threads
 constexpr int kRT = 32;   // columns per CTA of the inverse / transpose kernels
-constexpr int kStageBudget = 4096;        // staged doubles per solve tile (rows of a tile x row length)
-constexpr long long kWholeBudget = 4096;  // staged doubles up to which one CTA solves a whole front
 
-// one work item of the persistent triangular solve
-struct SolveItem {
-    int kind, s, r0, r1;  // kind, front, rows [r0, r1) of the tile
-    int cbeg, cend;       // contributions assembled for the front's own rows (or the tile's)
-    int cbeg2, cend2;     // update tiles: contributions of the tile's below-diagonal rows
+// one work item of the persistent triangular solve: a tile of a front, with
+// all that a CTA has to know of the front, so that one load starts its work
+struct alignas(16) SolveItem {
+    int kind, s, r0, r1;    // front, rows (forward) or columns (backward) [r0, r1)
+    int parent, r, c, f0;   // the front's parent, rows, columns, first column
+    int nk, target, ptarget, pad;  // children; counts to wait for: own (children's updates, or own y), parent's x
+    long long xw, rows, slot, upd; // offsets of M, of the row list, of the slot table, of the update vector
 };
 
 struct Tile {
@@ -97,7 +92,8 @@ struct Precond {
     std::vector<int> h_item_front;  // the front of every item (host)
     int* d_item_group = nullptr;    // batch unions: member of every item
     const int* d_frozen = nullptr;  // batch unions: per-member flag, 1 = skip its items
-    int *d_tgt = nullptr, *d_parent = nullptr, *d_cnt = nullptr, *d_prow = nullptr;
+    int *d_parent = nullptr, *d_cnt = nullptr, *d_prow = nullptr;
+    int* d_slot = nullptr;  // the fronts' slot tables (see SolveArgs)
     // subtree solves below the cut level (sub_levels levels of the tree)
     int sub_levels = 0, n_subs = 0;
     int sub_max_r = 0, sub_max_cols = 0, sub_max_depth = 0, sub_max_m = 0, sub_max_c = 0, sub_max_mroot = 0;
@@ -105,7 +101,6 @@ struct Precond {
     SubTree* d_subs = nullptr;
     SubChunk* d_chunks = nullptr;
     int *d_depth = nullptr, *d_xidx = nullptr;
-    int stage_d = 0, work_d = 0;
     // factor schedule: per (level, step) the fronts with a panel at that step and the SYRK tiles
     struct Step {
         int level, k0, panel_off, panel_cnt, syrk_off, syrk_cnt, panel_chunks;
@@ -116,21 +111,20 @@ struct Precond {
     int *d_first = nullptr, *d_ncol = nullptr, *d_nrow = nullptr, *d_rows = nullptr, *d_child_ptr = nullptr,
         *d_child_list = nullptr, *d_relind = nullptr, *d_level_list = nullptr, *d_perm = nullptr, *d_fail = nullptr,
         *d_panel_list = nullptr;
-    long long *d_front_off = nullptr, *d_rows_off = nullptr, *d_relind_off = nullptr, *d_dinv_off = nullptr,
+    long long *d_front_off = nullptr, *d_rows_off = nullptr, *d_relind_off = nullptr, *d_xw_off = nullptr,
               *d_upd_off = nullptr, *d_a_pos = nullptr, *d_a_src = nullptr;
     Tile* d_inv = nullptr;
     int *d_contrib_ptr = nullptr, *d_contrib_idx = nullptr, *d_below_front = nullptr;
     Tile *d_ea = nullptr, *d_oinv = nullptr;  // extend-add column tiles, off-diagonal inverse column groups
     std::vector<int> ea_off;                  // nlev + 1
     int n_oinv = 0;
-    long long* d_lt_off = nullptr;
-    double *d_dinvT = nullptr, *d_w = nullptr, *d_wt = nullptr;
+    double* d_xw = nullptr;                   // every front's M = [X; W]
     int4* d_wtiles = nullptr;  // (front, 64-row tile, 64-column tile) of every W
     int n_wtiles = 0;
     int4* d_syrk = nullptr;
     double* d_diag_tmp = nullptr;  // factored diagonal blocks of one panel step, [fronts in step][kNB][kNB]
     int max_panel_cnt = 0;
-    double *d_front = nullptr, *d_dinv = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
+    double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
            *d_vals = nullptr;
     // graph replay of the numeric factorisation (the same launches every solve)
     cudaGraphExec_t factor_exec = nullptr;
@@ -145,14 +139,16 @@ namespace {
 struct FrontArgs {
     const int *first, *ncol, *nrow, *rows, *child_ptr, *child_list, *relind, *level_list, *contrib_ptr, *contrib_idx,
         *below_front;
-    const long long *front_off, *rows_off, *relind_off, *dinv_off, *upd_off, *lt_off;
+    const long long *front_off, *rows_off, *relind_off, *xw_off, *upd_off;
     double* front;
-    double* dinv;   // L_JJ^{-1}, row-major
-    double* dinvT;  // its transpose, row-major
-    double* w;      // W = L_RJ L_JJ^{-1}, row-major (r - c) x c
-    double* wt;     // W^T, row-major c x (r - c)
+    double* xw;  // per front M = [X; W], X = L_JJ^{-1} (c x c, zeros above the diagonal), W = L_RJ X ((r - c) x c):
+                 // r x c column-major, leading dimension ld_of(r)
     int* fail;
 };
+
+// leading dimension of a front's M: r rounded up to even, so that every
+// column starts on a 16-byte boundary (the pad row holds zeros)
+__host__ __device__ __forceinline__ long long ld_of(int r) { return (r + 1) & ~1; }
 
 
 // ------------------------------------------------------------------ factorisation
@@ -325,8 +321,6 @@ __global__ void __launch_bounds__(kFT) k_syrk(FrontArgs a, const int4* __restric
         }
 }
 
-// Inverse of the diagonal block, row-major: X = L_JJ^{-1}.  One warp per 32
-// columns; lane j owns column j and reads only its own earlier entries.
 // L_JJ^{-1} in two passes.  Pass 1: the inverse of every 32x32 diagonal tile,
 // one warp per tile, column j of the inverse by forward substitution in
 // shared memory; the tile's upper triangle is written as zeros because pass 2
@@ -356,12 +350,9 @@ __global__ void __launch_bounds__(32) k_diag_inv(FrontArgs a, const Tile* __rest
     }
     __syncwarp();
     if (j >= kb) return;
-    double* Xg = a.dinv + a.dinv_off[s];
-    double* XTg = a.dinvT + a.dinv_off[s];
-    for (int i = 0; i < kb; i++) {
-        Xg[static_cast<long long>(j0 + i) * c + j0 + j] = X[i][j];
-        XTg[static_cast<long long>(j0 + i) * c + j0 + j] = X[j][i];
-    }
+    double* M = a.xw + a.xw_off[s];
+    const long long ld = ld_of(r);
+    for (int i = 0; i < kb; i++) M[(j0 + i) * ld + j0 + j] = X[j][i];
 }
 
 // Pass 2: the tiles below the diagonal, for 8 columns [j0, j0+8) per CTA.
@@ -379,8 +370,8 @@ __global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __
     const int jb0 = (j0 / kRT) * kRT;
     if (jb0 + kRT >= c) return;  // no tile below the diagonal one
     const double* F = a.front + a.front_off[s];
-    double* X = a.dinv + a.dinv_off[s];
-    double* XT = a.dinvT + a.dinv_off[s];
+    double* X = a.xw + a.xw_off[s];
+    const long long ld = ld_of(r);
     __shared__ double As[kRT][kRT + 1];
     __shared__ double Bs[kRT][kIC + 1];
     const int tid = threadIdx.x, jj = tid & (kIC - 1), ii = tid >> 3;  // rows ii and ii + 16
@@ -394,8 +385,8 @@ __global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __
         }
 #pragma unroll
         for (int q = 0; q < kRT * kIC / kIT; q++) {
-            const int idx = tid + q * kIT, kk = idx >> 3, cc = idx & 7;
-            pb[q] = cc < ncols ? X[static_cast<long long>(k0 + kk) * c + j0 + cc] : 0.0;
+            const int idx = tid + q * kIT, kk = idx & 31, cc = idx >> 5;
+            pb[q] = cc < ncols ? X[(j0 + cc) * ld + k0 + kk] : 0.0;
         }
     };
     for (int i0 = jb0 + kRT; i0 < c; i0 += kRT) {
@@ -411,7 +402,7 @@ __global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __
 #pragma unroll
             for (int q = 0; q < kRT * kIC / kIT; q++) {
                 const int idx = tid + q * kIT;
-                Bs[idx >> 3][idx & 7] = pb[q];
+                Bs[idx & 31][idx >> 5] = pb[q];
             }
             __syncthreads();
             if (k0 + kRT < i0) fetch(i0, ib, k0 + kRT);
@@ -427,8 +418,8 @@ __global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __
         Bs[ii][jj] = acc0;
         Bs[ii + 16][jj] = acc1;
         for (int idx = tid; idx < kRT * kRT; idx += kIT) {
-            const int rr = idx >> 5, kk = idx & 31;
-            As[rr][kk] = (rr < ib && kk < ib) ? X[static_cast<long long>(i0 + rr) * c + i0 + kk] : 0.0;
+            const int rr = idx & 31, kk = idx >> 5;
+            As[rr][kk] = (rr < ib && kk < ib) ? X[(i0 + kk) * ld + i0 + rr] : 0.0;
         }
         __syncthreads();
         double x0 = 0.0, x1 = 0.0;
@@ -439,14 +430,8 @@ __global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __
             x1 += As[ii + 16][kk] * t;
         }
         if (jj < ncols) {
-            if (ii < ib) {
-                X[static_cast<long long>(i0 + ii) * c + j0 + jj] = -x0;
-                XT[static_cast<long long>(j0 + jj) * c + i0 + ii] = -x0;
-            }
-            if (ii + 16 < ib) {
-                X[static_cast<long long>(i0 + ii + 16) * c + j0 + jj] = -x1;
-                XT[static_cast<long long>(j0 + jj) * c + i0 + ii + 16] = -x1;
-            }
+            if (ii < ib) X[(j0 + jj) * ld + i0 + ii] = -x0;
+            if (ii + 16 < ib) X[(j0 + jj) * ld + i0 + ii + 16] = -x1;
         }
         __syncthreads();
     }
@@ -467,34 +452,56 @@ __global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __
 // bounded, and a wait that runs out sets the error flag and makes every later
 // wait give up.
 //
-// Before it waits, a CTA stages everything of its item that does not depend
-// on other items -- the factor rows it multiplies with (odd row stride in
-// shared memory, so lanes on different rows hit different banks) and the
-// index lists of the assembly -- with cp.async, so only the dependent vectors
-// are fetched after the wait.
-//
-// Item kinds.  A small front is one item per sweep; a large one is split into
-// tiles of rows sized so that a tile's factor rows fill about kStageBudget
-// doubles.  Every output row is a dot product computed by a group of g lanes
-// (g = 32 for a handful of long rows, down to one thread per row for many
-// short ones).  With W = L_RJ L_JJ^{-1} from the factorisation, each sweep has
-// one dependent step per tree level:
-//   kFwdFront  y_J = L_JJ^{-1} f_J and g = f_R - W f_J for a whole front
-//   kFwdY      y rows of one tile         (waits: children's g)
-//   kFwdG      update rows of one tile    (waits: children's g)
-//   kBwdFront  x_J = L_JJ^{-T} y_J - W^T x_R for a whole front
-//   kBwdX      x rows of one tile         (waits: own y, parent's x)
-enum ItemKind { kFwdFront = 0, kFwdY = 1, kFwdG = 2, kBwdFront = 3, kBwdX = 5 };
+// Both sweeps read the same matrix M = [X; W] of a front (X = L_JJ^{-1},
+// W = L_RJ X, r x c column-major):
+//   forward   M f_J:  y_J = X f_J and the update g = f_R - W f_J; f = b + the
+//             children's updates
+//   backward  x_J = M^T [y_J; -x_R]
+// so an application reads nnz(L) doubles twice and holds them once: the
+// backward sweep finds in L2 what the forward sweep read last, and a factor
+// of up to about 100 MB stays there between applications.
+//   * Forward tiles are rows of M.  A lane owns two consecutive rows (16-byte
+//     loads; a warp reads up to 512 consecutive bytes of a column) and keeps
+//     their sums in registers; what the rows leave of the CTA splits the
+//     columns, and the partial sums meet in shared memory.
+//   * Backward tiles are groups of four columns, one per warp (or several
+//     warps splitting the rows of one): a lane takes two consecutive rows of
+//     the four columns, so the vector in shared memory is read once for four
+//     columns; one 12-value reduction over the lanes at the end.
+//   * The matrix goes from memory to registers; only the vectors pass through
+//     shared memory, in chunks of kVC entries, so the kernel's shared memory
+//     does not depend on the fronts and every model runs 3 CTAs per SM.
+//   * All that can be had before the wait is loaded before it: the item's
+//     record, the first columns of a forward tile, the index of every row to
+//     be assembled (a dense table per front and child: consecutive threads
+//     read consecutive entries), and the backward tile's part over y.
+// What bounds it: the chain of dependent fronts (11-13 per sweep, about 5 us
+// each: notice, gather, product, publish), then the factor's bytes.  One
+// application (inside a solve, with both matrices and their transposes staged
+// through shared memory before): C3D8 beam 124 -> 113 us, C3D20R cap 330 ->
+// 192 us (281 MB, 1.5 TB/s), C3D10 finger 439 -> 241 us (340 MB, 1.4 TB/s).
+// Every sum has a fixed order (no atomics on data): results repeat bitwise.
+enum ItemKind { kFwdTile = 0, kBwdTile = 1 };
+
+constexpr int kVC = 1024;      // vector entries (nodes) of a chunk in shared memory
+constexpr int kMaxR = 256;     // most rows of a forward tile
+constexpr int kFU = 4;         // columns a forward lane loads at a time
+// doubles of M per tile (see precond_setup).  One application, beam / cap /
+// finger, with kTileMin 1024, 2048, 4096: 115 / 192 / 242, 113 / 193 / 241,
+// 119 / 192 / 238 us; with kTileMax 4096, 6144, 10240: 114 / 196 / 243,
+// 113 / 193 / 241, 114 / 193 / 241 us.
+constexpr int kTileMin = 2048, kTileMax = 6144;
+constexpr int kRed = 8 * 64 * 3;  // doubles of the partial sums of a tile
+constexpr size_t kSolveSmem = sizeof(double) * (3 * (kVC + kMaxR) + kRed);
 
 // device counters, one int array: [cY ns][cGin ns][exits, ns - 1 unused][cX ns][ticket][error]
 struct SolveArgs {
     FrontArgs a;
-    const int* parent;
-    const int* prow;          // per front row (rows_off[s] + t): the node's index in v
+    const int* prow;          // per front row: the node's index in v
     const SolveItem* items;
-    const int* tgt;           // targets of the four counter groups
+    const int* slot;          // per front, child q, row t (item.slot + q r + t): the update entry of that child
+                              // landing on the row, or -1
     int n_items, ns;
-    int stage_d, work_d;      // shared-memory layout: staged doubles, work doubles, then ints
     double* v;
     double* y;
     double* t;
@@ -517,7 +524,7 @@ __device__ __forceinline__ int ld_acquire(const int* p)
     return v;
 }
 
-// thread 0 only: wait until *c >= target; false after `limit` polls (the
+// one thread: wait until *c >= target; false after `limit` polls (the
 // error flag is then set) or when another wait has already given up
 __device__ bool wait_ge(const int* c, int target, int* err, int limit)
 {
@@ -539,31 +546,389 @@ __device__ __forceinline__ void ld3(const double* p, double& a, double& b, doubl
     c = __ldcg(p + 2);
 }
 
+// The index of one row's assembly: the node of an own column (or -1) and the
+// update entries of the first two children (or -1); loaded before the wait.
+struct RowIdx {
+    int v, g, h;
+};
+__device__ __forceinline__ RowIdx row_idx(const SolveArgs& A, const SolveItem& d, int t, bool valid)
+{
+    RowIdx x { -1, -1, -1 };
+    if (!valid) return x;
+    if (t < d.c) x.v = __ldg(A.prow + d.rows + t);
+    if (d.nk > 0) x.g = __ldg(A.slot + d.slot + t);
+    if (d.nk > 1) x.h = __ldg(A.slot + d.slot + d.r + t);
+    return x;
+}
+
+// f on n1 front rows from t1 on and n2 rows from t2 on into dst (3 per row):
+// the right-hand side on own columns (t < c) plus the children's update
+// entries landing on the row, children in order.  The loads of two rows per
+// thread (right-hand side and two children; more children follow) are issued
+// before they are added; `ix` holds the first two rows' indices.
+__device__ __forceinline__ void assemble(const SolveArgs& A, const SolveItem& d, int t1, int n1, int t2, int n2,
+    double* dst, RowIdx (&ix)[2])
+{
+    const int n = n1 + n2;
+    for (int i0 = threadIdx.x; i0 < n; i0 += 2 * kST) {
+        double b[2][3], g[2][3], h[2][3];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) b[u][k] = g[u][k] = h[u][k] = 0.0;
+            if (ix[u].v >= 0) ld3(A.v + 3LL * ix[u].v, b[u][0], b[u][1], b[u][2]);
+            if (ix[u].g >= 0) ld3(A.upd + 3LL * ix[u].g, g[u][0], g[u][1], g[u][2]);
+            if (ix[u].h >= 0) ld3(A.upd + 3LL * ix[u].h, h[u][0], h[u][1], h[u][2]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {  // the next two rows' indices
+            const int i = i0 + (u + 2) * kST;
+            ix[u] = row_idx(A, d, i < n1 ? t1 + i : t2 + i - n1, i < n);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int i = i0 + u * kST, t = i < n1 ? t1 + i : t2 + i - n1;
+            if (i >= n) break;
+#pragma unroll
+            for (int k = 0; k < 3; k++) b[u][k] = b[u][k] + g[u][k] + h[u][k];
+            for (int q = 2; q < d.nk; q++) {
+                const int e = __ldg(A.slot + d.slot + static_cast<long long>(q) * d.r + t);
+                if (e < 0) continue;
+                double x0, x1, x2;
+                ld3(A.upd + 3LL * e, x0, x1, x2);
+                b[u][0] += x0;
+                b[u][1] += x1;
+                b[u][2] += x2;
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++) dst[3 * i + k] = b[u][k];
+        }
+    }
+}
+
+// the indices of the first two rows per thread of a following assemble
+__device__ __forceinline__ void first_idx(const SolveArgs& A, const SolveItem& d, int t1, int n1, int t2, int n2,
+    RowIdx (&ix)[2])
+{
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int i = threadIdx.x + u * kST;
+        ix[u] = row_idx(A, d, i < n1 ? t1 + i : t2 + i - n1, i < n1 + n2);
+    }
+}
+
+__device__ __forceinline__ double2 ldm2(const double* p) { return __ldg(reinterpret_cast<const double2*>(p)); }
+
+__device__ __forceinline__ void fma6(double* acc, double2 m, const double* f)
+{
+    const double f0 = f[0], f1 = f[1], f2 = f[2];
+    acc[0] += m.x * f0;
+    acc[1] += m.x * f1;
+    acc[2] += m.x * f2;
+    acc[3] += m.y * f0;
+    acc[4] += m.y * f1;
+    acc[5] += m.y * f2;
+}
+
+// twelve column sums (four columns x three components) over rows [i0, i1) of
+// the chunk that starts at row zb (even), each lane two rows every `step`
+__device__ __forceinline__ void cols_acc(double (&acc)[4][3], const double* const (&Mc)[4], const double* z, int zb,
+    int i0, int i1, int step)
+{
+#pragma unroll 2
+    for (int i = i0; i < i1; i += step) {
+        double2 m[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) m[q] = ldm2(Mc[q] + i);
+        const double2* zp = reinterpret_cast<const double2*>(z + 3 * (i - zb));
+        const double2 za = zp[0], zc = zp[1], ze = zp[2];  // (z0 z1) (z2 z0') (z1' z2')
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            acc[q][0] += m[q].x * za.x;
+            acc[q][1] += m[q].x * za.y;
+            acc[q][2] += m[q].x * zc.x;
+            acc[q][0] += m[q].y * zc.y;
+            acc[q][1] += m[q].y * ze.x;
+            acc[q][2] += m[q].y * ze.y;
+        }
+    }
+}
+
+// the twelve sums over a warp: on return lane l holds the three components of
+// column l >> 3 in acc[0]
+__device__ __forceinline__ void cols_reduce(double (&acc)[4][3])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const double keep = lane & 16 ? acc[q + 2][k] : acc[q][k], send = lane & 16 ? acc[q][k] : acc[q + 2][k];
+            acc[q][k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double keep = lane & 8 ? acc[1][k] : acc[0][k], send = lane & 8 ? acc[0][k] : acc[1][k];
+        double x = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        x += __shfl_xor_sync(0xffffffffu, x, 4);
+        x += __shfl_xor_sync(0xffffffffu, x, 2);
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        acc[0][k] = x;
+    }
+}
+
+__global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
+{
+    griddep_wait();
+    extern __shared__ __align__(16) double sm[];
+    double* vec = sm;                      // [kVC + kMaxR][3] chunk of the vector, and f on a tile's own below rows
+    double* red = sm + 3 * (kVC + kMaxR);  // partial sums
+    __shared__ int item_sh, ok_sh, ok2_sh;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    int* ticket = A.cnt + 4 * A.ns;
+    int* err = ticket + 1;
+    if (tid == 0) {
+        const int next = atomicAdd(ticket, 1);
+        if (next == 0 && A.stamp) {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            *A.stamp = t;
+        }
+        item_sh = next;
+    }
+    __syncthreads();
+    for (;;) {
+        const int it = item_sh;
+        if (it >= A.n_items) {
+            griddep_launch();  // no more items for this CTA
+            break;
+        }
+        if (A.frozen && A.frozen[A.item_group[it]]) {
+            // a batch member that stopped iterating: its tree of fronts (no
+            // other member's items depend on it) is skipped whole
+            __syncthreads();
+            if (tid == 0) item_sh = atomicAdd(ticket, 1);
+            __syncthreads();
+            continue;
+        }
+        const int bump = A.test_wait && it == A.n_items - 1 ? 1 : 0;
+        const SolveItem d = A.items[it];
+        const long long ld = ld_of(d.r);
+        const double* M = A.a.xw + d.xw;
+        const int r0 = d.r0, r1 = d.r1, c = d.c;
+        // The next ticket is drawn once this item's dependencies are in (a
+        // few microseconds before the CTA is free), not when the item starts:
+        // a CTA whose item waits on a long chain would otherwise hold up the
+        // item of the ticket it drew.
+        int next = 0;
+        if (d.kind == kFwdTile) {
+            // rows [r0, r1): 2^lsh row pairs per warp, 2^bsh blocks of 64 rows,
+            // the rest of the CTA splits the columns
+            const int R = r1 - r0, kend = min(c, r1);
+            const int lsh = R <= 8 ? 2 : R <= 16 ? 3 : R <= 32 ? 4 : 5;
+            const int bsh = R <= 64 ? 0 : R <= 128 ? 1 : 2;
+            const int nw = 8 >> bsh, KS = nw << (5 - lsh);  // warps per block, column split
+            const int lrow = ((w & ((1 << bsh) - 1)) << 6) + 2 * (lane & ((1 << lsh) - 1));
+            const int wk = w >> bsh, ks = (wk << (5 - lsh)) + (lane >> lsh);
+            const bool act = lrow < R;
+            const double* Mr = M + r0 + lrow;
+            double2 buf[kFU];
+#pragma unroll
+            for (int u = 0; u < kFU; u++)
+                buf[u] = act && ks + u * KS < kend ? ldm2(Mr + (ks + u * KS) * ld) : make_double2(0.0, 0.0);
+            const int b0 = max(r0, c), nb = r1 - b0;  // the tile's below rows (nb <= 0: none)
+            RowIdx ix[2];
+            first_idx(A, d, 0, min(kend, kVC), b0, max(nb, 0), ix);
+            if (tid == 0) {
+                ok_sh = wait_ge(A.cnt + A.ns + d.s, d.target + bump, err, A.spin_limit);
+                next = atomicAdd(ticket, 1);
+            }
+            __syncthreads();
+            if (ok_sh) {
+                double acc[6] = { 0, 0, 0, 0, 0, 0 };
+                int k = ks;
+                for (int kb = 0; kb < kend; kb += kVC) {
+                    const int ke = min(kend, kb + kVC);
+                    // own columns to vec; with the first chunk, the tile's below rows after them
+                    if (kb > 0) {
+                        __syncthreads();
+                        first_idx(A, d, kb, ke - kb, 0, 0, ix);
+                        assemble(A, d, kb, ke - kb, 0, 0, vec, ix);
+                    } else {
+                        assemble(A, d, 0, ke, b0, max(nb, 0), vec, ix);
+                    }
+                    __syncthreads();
+                    if (act)
+                        while (k < ke) {
+                            if (k != ks) {
+#pragma unroll
+                                for (int u = 0; u < kFU; u++)
+                                    buf[u] = k + u * KS < ke ? ldm2(Mr + (k + u * KS) * ld) : make_double2(0.0, 0.0);
+                            }
+#pragma unroll
+                            for (int u = 0; u < kFU; u++)
+                                if (k + u * KS < ke) fma6(acc, buf[u], vec + 3 * (k + u * KS - kb));
+                            k += kFU * KS;
+                            if (k >= ke) {  // the first column of the next chunk
+                                k = ke + ((ks - ke) % KS + KS) % KS;
+                                break;
+                            }
+                        }
+                }
+                for (int o = 1 << lsh; o < 32; o <<= 1)
+#pragma unroll
+                    for (int q = 0; q < 6; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+                if (act && (lane >> lsh) == 0) {
+                    double* o = red + (wk * (64 << bsh) + lrow) * 3;
+#pragma unroll
+                    for (int q = 0; q < 6; q++) o[q] = acc[q];
+                }
+                __syncthreads();
+                const double* fr = vec + 3 * min(kend, kVC);
+                for (int i = tid; i < 3 * R; i += kST) {
+                    double sum = 0.0;
+                    for (int h = 0; h < nw; h++) sum += red[h * (192 << bsh) + i];
+                    if (i < 3 * (c - r0))
+                        A.y[3LL * (d.f0 + r0) + i] = sum;
+                    else
+                        A.upd[d.upd + 3LL * (r0 - c) + i] = fr[i - 3 * (b0 - r0)] - sum;
+                }
+            }
+            if (tid == 0) item_sh = next;
+            __syncthreads();  // the item's results are written
+            if (tid == 0) {
+                __threadfence();
+                if (r0 < c) atomicAdd(A.cnt + d.s, 1);
+                if (r1 > c && d.parent >= 0) atomicAdd(A.cnt + A.ns + d.parent, 1);
+            }
+        } else {
+            // columns [r0, r1), at most 32: one quad of columns per warp, or
+            // (fewer than 8 quads) several warps splitting the quad's rows
+            const int nq = (r1 - r0 + 3) >> 2;
+            const int qsh = nq <= 1 ? 0 : nq <= 2 ? 1 : nq <= 4 ? 2 : 3;
+            const int quad = w & ((1 << qsh) - 1), h = w >> qsh, wk = 8 >> qsh, step = 64 * wk;
+            const bool act = quad < nq;
+            const int* pr = A.prow + d.rows;
+            const double* Mc[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) Mc[q] = M + min(r0 + 4 * quad + q, r1 - 1) * ld;
+            if (tid == 0) {
+                ok_sh = wait_ge(A.cnt + d.s, d.target + bump, err, A.spin_limit);
+                if (!ok_sh) next = atomicAdd(ticket, 1);
+            }
+            __syncthreads();
+            if (ok_sh) {
+                double acc[4][3] = {};
+                // own columns: y, this front's forward result
+                for (int zb = r0 & ~1; zb < c; zb += kVC) {
+                    const int ze = min(c, zb + kVC), zl = (ze + 1) & ~1, n = 3 * (ze - zb);
+                    if (zb > r0) __syncthreads();
+                    const double* y = A.y + 3LL * (d.f0 + zb);
+#pragma unroll 4
+                    for (int i = tid; i < 3 * (zl - zb); i += kST) vec[i] = i < n ? __ldcg(y + i) : 0.0;
+                    __syncthreads();
+                    if (act) cols_acc(acc, Mc, vec, zb, zb + 64 * h + 2 * lane, ze, step);
+                }
+                // below rows: -x of the ancestors, complete with the parent's
+                const int zc = c & ~1;
+                int ip[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int t = zc + tid + u * kST;
+                    ip[u] = t >= c && t < d.r ? __ldg(pr + t) : -1;
+                }
+                if (tid == 0) {
+                    ok2_sh = d.parent < 0 || wait_ge(A.cnt + 3 * A.ns + d.parent, d.ptarget, err, A.spin_limit);
+                    next = atomicAdd(ticket, 1);
+                }
+                __syncthreads();
+                if (ok2_sh) {
+                    for (int zb = zc; zb < d.r; zb += kVC) {
+                        const int ze = min(d.r, zb + kVC), zl = (ze + 1) & ~1;
+                        if (zb > zc) {
+                            __syncthreads();
+#pragma unroll
+                            for (int u = 0; u < 4; u++) {
+                                const int t = zb + tid + u * kST;
+                                ip[u] = t < d.r ? __ldg(pr + t) : -1;
+                            }
+                        }
+                        double x[4][3];
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            x[u][0] = x[u][1] = x[u][2] = 0.0;
+                            if (ip[u] >= 0) ld3(A.v + 3LL * ip[u], x[u][0], x[u][1], x[u][2]);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const int i = tid + u * kST;
+                            if (zb + i >= zl) break;
+#pragma unroll
+                            for (int k = 0; k < 3; k++) vec[3 * i + k] = -x[u][k];
+                        }
+                        __syncthreads();
+                        if (act) cols_acc(acc, Mc, vec, zb, zb + 64 * h + 2 * lane, ze, step);
+                    }
+                    cols_reduce(acc);
+                    if ((lane & 7) == 0) {
+                        double* o = red + ((h << qsh) + quad) * 12 + 3 * (lane >> 3);
+#pragma unroll
+                        for (int k = 0; k < 3; k++) o[k] = acc[0][k];
+                    }
+                    __syncthreads();
+                    if (tid < 3 * (r1 - r0)) {
+                        double x = 0.0;
+                        for (int q = 0; q < wk; q++) x += red[(q << qsh) * 12 + tid];
+                        A.v[3LL * __ldg(pr + r0 + tid / 3) + tid % 3] = x;
+                    }
+                }
+            }
+            if (tid == 0) item_sh = next;
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();
+                atomicAdd(A.cnt + 3 * A.ns + d.s, 1);
+            }
+        }
+    }
+    // A solve that gave up leaves v partly overwritten: the last CTA to
+    // leave fills it with NaN, so that a caller who cannot read the error
+    // flag (a replayed graph) still sees that the result is not valid.
+    if (tid == 0) {
+        __threadfence();
+        ok_sh = atomicAdd(A.cnt + 2 * A.ns, 1) == static_cast<int>(gridDim.x) - 1 && *reinterpret_cast<volatile int*>(err);
+    }
+    __syncthreads();
+    if (ok_sh) {
+        __threadfence();
+        for (int i = tid; i < A.n3; i += kST) A.v[i] = __longlong_as_double(0x7ff8000000000000LL);
+    }
+}
+
+// ------------------------------------------------- staged row products (subtree solves)
 __device__ __forceinline__ void cp8(double* dst, const double* src)
 {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
 }
-__device__ __forceinline__ void stage_i(int* dst, const int* src, int n)
-{
-    for (int i = threadIdx.x; i < n; i += kST) {
-        const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst + i));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src + i) : "memory");
-    }
-}
-// rows [0, R) of a matrix with leading dimension ld, entries k in [lo(row), hi(row)),
-// into dst with row stride lp; lo / hi: 0 = 0 / L, 1 = 0 / row0 + row + 1 (lower
-// triangle), 2 = row0 + row / L (upper triangle); one warp per row
-__device__ __forceinline__ void stage_rows(double* dst, int lp, const double* src, long long ld, int R, int L, int tri,
-    int row0)
+// rows [0, R) at src + row * ld, entries k in [max(lo0 + row, 0), L), into dst
+// with row stride lp; one warp per row
+__device__ __forceinline__ void stage_rows(double* dst, int lp, const double* src, long long ld, int R, int L, int lo0)
 {
     const int lane = threadIdx.x & 31;
     for (int rr = threadIdx.x >> 5; rr < R; rr += kST / 32) {
-        const int lo = tri == 2 ? row0 + rr : 0;
-        const int hi = tri == 1 ? row0 + rr + 1 : L;
         const double* sr = src + rr * ld;
         double* dr = dst + rr * lp;
-        for (int k = lo + lane; k < hi; k += 32) cp8(dr + k, sr + k);
+        for (int k = max(lo0 + rr, 0) + lane; k < L; k += 32) cp8(dr + k, sr + k);
+    }
+}
+// rows [0, R) of a column-major matrix (row q, column k at src[k ld + q]),
+// entries k in [0, min(L, hi0 + row + 1)), into dst with row stride lp
+__device__ __forceinline__ void stage_cols(double* dst, int lp, const double* src, long long ld, int R, int L, int hi0)
+{
+    for (int idx = threadIdx.x; idx < R * L; idx += kST) {
+        const int k = idx / R, rr = idx - k * R;
+        if (k < hi0 + rr + 1) cp8(dst + rr * lp + k, src + k * ld + rr);
     }
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -580,7 +945,7 @@ __device__ __forceinline__ int lanes_per_row(int R)
 
 // Dot products of staged rows [0, R) (row stride lp) with a 3-component vector
 // v in shared memory (entry k at v[3 (k - vbase)]), over k in [lo, hi) with
-// lo / hi as in stage_rows.  Each row gets a group of g threads (g = kST / R
+// lo / hi for tri 0: 0 / L, 1: 0 / row0 + row + 1 (lower triangle), 2: row0 + row / L.  Each row gets a group of g threads (g = kST / R
 // rounded to a power of two: a whole CTA for one row, one thread per row for
 // kST rows); a group wider than a warp adds its warps' partial sums through
 // shared memory.  Every sum has a fixed order.  out is called with
@@ -651,345 +1016,6 @@ __device__ __forceinline__ void rows_dot(const double* M, int lp, const double* 
     }
 }
 
-// f_t for front rows [t0, t1) into f (3 per row): the right-hand side for own
-// columns (t < c) plus the children's update entries landing on the row, from
-// the staged contribution pointers cp (row t0 first) and indices ci (starting
-// at contribution cbeg) and the staged node indices pr (row t0 first).  Each
-// thread first issues the loads of up to kBatch rows (right-hand side and the
-// first two contributions of each) and only then adds them, so the rows cost
-// one memory latency instead of one each; further contributions (rows with
-// more than two children behind them) follow in order.
-constexpr int kBatch = 2;
-__device__ __forceinline__ void assemble(const SolveArgs& A, int t0, int t1, int c, const int* cp, const int* ci,
-    int cbeg, const int* pr, double* f)
-{
-    for (int base = t0; base < t1; base += kST * kBatch) {
-        double b[kBatch][3], g[kBatch][2][3];
-#pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-            const int t = base + static_cast<int>(threadIdx.x) + u * kST;
-            const bool valid = t < t1;
-            const int q0 = valid ? cp[t - t0] : 0, q1 = valid ? cp[t - t0 + 1] : 0;
-            b[u][0] = b[u][1] = b[u][2] = 0.0;
-            if (valid && t < c) ld3(A.v + 3LL * pr[t - t0], b[u][0], b[u][1], b[u][2]);
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                g[u][e][0] = g[u][e][1] = g[u][e][2] = 0.0;
-                if (q0 + e < q1) ld3(A.upd + 3LL * ci[q0 + e - cbeg], g[u][e][0], g[u][e][1], g[u][e][2]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-            const int t = base + static_cast<int>(threadIdx.x) + u * kST;
-            if (t >= t1) continue;
-            double x0 = b[u][0] + g[u][0][0] + g[u][1][0];
-            double x1 = b[u][1] + g[u][0][1] + g[u][1][1];
-            double x2 = b[u][2] + g[u][0][2] + g[u][1][2];
-            for (int q = cp[t - t0] + 2; q < cp[t - t0 + 1]; q++) {
-                double h0, h1, h2;
-                ld3(A.upd + 3LL * ci[q - cbeg], h0, h1, h2);
-                x0 += h0;
-                x1 += h1;
-                x2 += h2;
-            }
-            double* o = f + 3 * (t - t0);
-            o[0] = x0;
-            o[1] = x1;
-            o[2] = x2;
-        }
-    }
-}
-
-// n doubles from global memory written by other CTAs of this launch into
-// shared memory, loads batched ahead of the stores
-__device__ __forceinline__ void copy_cg(double* dst, const double* src, int n)
-{
-    for (int base = 0; base < n; base += kST * 8) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int i = base + static_cast<int>(threadIdx.x) + u * kST;
-            v[u] = i < n ? __ldcg(src + i) : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int i = base + static_cast<int>(threadIdx.x) + u * kST;
-            if (i < n) dst[i] = v[u];
-        }
-    }
-}
-
-// x_R: the solution on n front rows whose node indices are pr[0..n), gathered
-// from v (3 per node) into shared memory, loads batched ahead of the stores
-__device__ __forceinline__ void gather3(double* dst, const double* v, const int* pr, int n)
-{
-    for (int base = 0; base < n; base += kST * kBatch) {
-        double x[kBatch][3];
-#pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-            const int k = base + static_cast<int>(threadIdx.x) + u * kST;
-            x[u][0] = x[u][1] = x[u][2] = 0.0;
-            if (k < n) ld3(v + 3LL * pr[k], x[u][0], x[u][1], x[u][2]);
-        }
-#pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-            const int k = base + static_cast<int>(threadIdx.x) + u * kST;
-            if (k < n) {
-                dst[3 * k] = x[u][0];
-                dst[3 * k + 1] = x[u][1];
-                dst[3 * k + 2] = x[u][2];
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kST) k_solve(SolveArgs A)
-{
-    griddep_wait();
-    extern __shared__ double sm[];
-    double* st = sm;                                  // staged factor rows
-    double* wk = sm + A.stage_d;                      // work vectors
-    int* si = reinterpret_cast<int*>(wk + A.work_d);  // staged index lists
-    __shared__ int item_sh, ok_sh, ok2_sh;
-    const int ns = A.ns;
-    int* cY = A.cnt;
-    int* cGin = A.cnt + ns;
-    int* cX = A.cnt + 3 * ns;
-    int* ticket = A.cnt + 4 * ns;
-    int* err = ticket + 1;
-    const int* tY = A.tgt;
-    const int* tGin = A.tgt + ns;
-    const int* tX = A.tgt + 3 * ns;
-    int* exits = A.cnt + 2 * ns;
-    const int tid = threadIdx.x;
-    const FrontArgs& a = A.a;
-    int next = 0;  // thread 0: the ticket taken ahead
-    if (tid == 0) {
-        next = atomicAdd(ticket, 1);
-        if (next == 0 && A.stamp) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            *A.stamp = t;
-        }
-    }
-    for (;;) {
-        if (tid == 0) item_sh = next;
-        __syncthreads();
-        const int it = item_sh;
-        if (it >= A.n_items) {
-            griddep_launch();  // no more items for this CTA
-            break;
-        }
-        if (A.frozen && A.frozen[A.item_group[it]]) {
-            // a batch member that stopped iterating: its tree of fronts (no
-            // other member's items depend on it) is skipped whole
-            if (tid == 0) next = atomicAdd(ticket, 1);
-            __syncthreads();
-            continue;
-        }
-        const int bump = A.test_wait && it == A.n_items - 1 ? 1 : 0;
-        const SolveItem d = A.items[it];
-        const int kind = d.kind, s = d.s, r0 = d.r0, r1 = d.r1, R = r1 - r0, cbeg = d.cbeg, cend = d.cend;
-        const int p = A.parent[s];
-        const int r = a.nrow[s], c = a.ncol[s], m = r - c, f0 = a.first[s];
-        const long long ro = a.rows_off[s];
-        const double* X = a.dinv + a.dinv_off[s];
-        const double* XT = a.dinvT + a.dinv_off[s];
-        const double* W = a.w + a.lt_off[s];
-        const double* WT = a.wt + a.lt_off[s];
-        const int lc = odd(c), lm = odd(m);
-        const int nci = cend - cbeg, nci2 = d.cend2 - d.cbeg2;
-        // stage what does not depend on other items
-        switch (kind) {
-        case kFwdFront:
-            stage_rows(st, lc, X, c, c, c, 1, 0);           // L_JJ^{-1} rows (lower)
-            stage_rows(st + c * lc, lc, W, c, m, c, 0, 0);  // W rows
-            stage_i(si, a.contrib_ptr + ro, r + 1);
-            stage_i(si + r + 1, a.contrib_idx + cbeg, nci);
-            stage_i(si + r + 1 + nci, A.prow + ro, c);
-            break;
-        case kFwdY:
-            stage_rows(st, lc, X + static_cast<long long>(r0) * c, c, R, c, 1, r0);
-            stage_i(si, a.contrib_ptr + ro, r1 + 1);
-            stage_i(si + r1 + 1, a.contrib_idx + cbeg, nci);
-            stage_i(si + r1 + 1 + nci, A.prow + ro, r1);
-            break;
-        case kFwdG: {
-            stage_rows(st, lc, W + static_cast<long long>(r0) * c, c, R, c, 0, 0);
-            int* q = si;
-            stage_i(q, a.contrib_ptr + ro, c + 1);
-            stage_i(q + c + 1, a.contrib_idx + cbeg, nci);
-            stage_i(q + c + 1 + nci, A.prow + ro, c);
-            q += 2 * c + 1 + nci;
-            stage_i(q, a.contrib_ptr + ro + c + r0, R + 1);
-            stage_i(q + R + 1, a.contrib_idx + d.cbeg2, nci2);
-            break;
-        }
-        case kBwdFront:
-            stage_rows(st, lc, XT, c, c, c, 2, 0);             // L_JJ^{-T} rows (upper)
-            stage_rows(st + c * lc, lm, WT, m, c, m, 0, 0);  // W^T rows
-            stage_i(si, A.prow + ro, r);
-            break;
-        default:  // kBwdX
-            stage_rows(st, lc, XT + static_cast<long long>(r0) * c, c, R, c, 2, r0);
-            stage_rows(st + R * lc, lm, WT + static_cast<long long>(r0) * m, m, R, m, 0, 0);
-            stage_i(si, A.prow + ro, r);
-            break;
-        }
-        stage_commit();
-        // The next ticket is drawn once this item's dependencies are in (a
-        // few microseconds before the CTA is free), not when the item starts:
-        // a CTA whose item waits on a long chain would otherwise hold up the
-        // item of the ticket it drew.  Backward items wait in two steps: their
-        // own front's forward result first, the parent's solution last.
-        const bool bwd = kind == kBwdFront || kind == kBwdX;
-        if (tid == 0) {
-            const bool ok = bwd ? wait_ge(cY + s, tY[s] + bump, err, A.spin_limit)
-                                : wait_ge(cGin + s, tGin[s] + bump, err, A.spin_limit);
-            ok_sh = ok;
-            if (!bwd || !ok) next = atomicAdd(ticket, 1);
-        }
-        // backward items: thread 0 waits for the parent's x, then draws the next ticket
-        auto parent_wait = [&]() {
-            if (tid == 0) {
-                ok2_sh = p < 0 || wait_ge(cX + p, tX[p], err, A.spin_limit);
-                next = atomicAdd(ticket, 1);
-            }
-            __syncthreads();
-        };
-        stage_wait();
-        __syncthreads();
-        if (ok_sh) {
-            switch (kind) {
-            case kFwdFront: {
-                double* f = wk;  // [r][3]
-                const int* ci = si + r + 1;
-                assemble(A, 0, r, c, si, ci, cbeg, ci + nci, f);
-                __syncthreads();
-                rows_dot(st, lc, f, 0, c, c, 1, 0, [&](int i, double y0, double y1, double y2) {
-                    double* yg = A.y + 3LL * (f0 + i);
-                    yg[0] = y0;
-                    yg[1] = y1;
-                    yg[2] = y2;
-                });
-                double* g = A.upd + a.upd_off[s];
-                rows_dot(st + c * lc, lc, f, 0, m, c, 0, 0, [&](int k, double d0, double d1, double d2) {
-                    const double* fk = f + 3 * (c + k);
-                    g[3 * k] = fk[0] - d0;
-                    g[3 * k + 1] = fk[1] - d1;
-                    g[3 * k + 2] = fk[2] - d2;
-                });
-                break;
-            }
-            case kFwdY: {
-                double* f = wk;  // [r1][3]
-                const int* ci = si + r1 + 1;
-                assemble(A, 0, r1, c, si, ci, cbeg, ci + nci, f);
-                __syncthreads();
-                rows_dot(st, lc, f, 0, R, c, 1, r0, [&](int i, double y0, double y1, double y2) {
-                    double* yg = A.y + 3LL * (f0 + r0 + i);
-                    yg[0] = y0;
-                    yg[1] = y1;
-                    yg[2] = y2;
-                });
-                break;
-            }
-            case kFwdG: {
-                double* fj = wk;          // [c][3]
-                double* fr = wk + 3 * c;  // [R][3]
-                const int* q = si;
-                const int* ci = q + c + 1;
-                assemble(A, 0, c, c, q, ci, cbeg, ci + nci, fj);
-                q += 2 * c + 1 + nci;
-                assemble(A, c + r0, c + r1, c, q, q + R + 1, d.cbeg2, nullptr, fr);
-                __syncthreads();
-                double* g = A.upd + a.upd_off[s] + 3LL * r0;
-                rows_dot(st, lc, fj, 0, R, c, 0, 0, [&](int k, double d0, double d1, double d2) {
-                    g[3 * k] = fr[3 * k] - d0;
-                    g[3 * k + 1] = fr[3 * k + 1] - d1;
-                    g[3 * k + 2] = fr[3 * k + 2] - d2;
-                });
-                break;
-            }
-            case kBwdFront: {
-                double* yj = wk;               // [c][3]
-                double* xr = wk + 3 * c;       // [m][3]
-                double* xs = wk + 3 * r;       // [c][3]
-                copy_cg(yj, A.y + 3LL * f0, 3 * c);
-                __syncthreads();
-                // L_JJ^{-T} y_J needs only this front's forward result
-                rows_dot(st, lc, yj, 0, c, c, 2, 0, [&](int i, double x0, double x1, double x2) {
-                    xs[3 * i] = x0;
-                    xs[3 * i + 1] = x1;
-                    xs[3 * i + 2] = x2;
-                });
-                parent_wait();
-                if (!ok2_sh) break;
-                gather3(xr, A.v, si + c, m);
-                __syncthreads();
-                rows_dot(st + c * lc, lm, xr, 0, c, m, 0, 0, [&](int i, double s0, double s1, double s2) {
-                    double* o = A.v + 3LL * si[i];
-                    o[0] = xs[3 * i] - s0;
-                    o[1] = xs[3 * i + 1] - s1;
-                    o[2] = xs[3 * i + 2] - s2;
-                });
-                break;
-            }
-            default: {  // kBwdX
-                double* yj = wk;                      // [c - r0][3]
-                double* xr = wk + 3 * (c - r0);       // [m][3]
-                double* xs = xr + 3 * m;              // [R][3]
-                copy_cg(yj, A.y + 3LL * (f0 + r0), 3 * (c - r0));
-                __syncthreads();
-                rows_dot(st, lc, yj, r0, R, c, 2, r0, [&](int i, double x0, double x1, double x2) {
-                    xs[3 * i] = x0;
-                    xs[3 * i + 1] = x1;
-                    xs[3 * i + 2] = x2;
-                });
-                parent_wait();
-                if (!ok2_sh) break;
-                gather3(xr, A.v, si + c, m);
-                __syncthreads();
-                rows_dot(st + R * lc, lm, xr, 0, R, m, 0, 0, [&](int i, double s0, double s1, double s2) {
-                    double* o = A.v + 3LL * si[r0 + i];
-                    o[0] = xs[3 * i] - s0;
-                    o[1] = xs[3 * i + 1] - s1;
-                    o[2] = xs[3 * i + 2] - s2;
-                });
-                break;
-            }
-            }
-        }
-        __syncthreads();  // the item's results are written
-        if (tid == 0) {
-            __threadfence();
-            switch (kind) {
-            case kFwdFront:
-                atomicAdd(cY + s, 1);
-                if (p >= 0) atomicAdd(cGin + p, 1);
-                break;
-            case kFwdY: atomicAdd(cY + s, 1); break;
-            case kFwdG:
-                if (p >= 0) atomicAdd(cGin + p, 1);
-                break;
-            default: atomicAdd(cX + s, 1); break;  // kBwdFront, kBwdX
-            }
-        }
-    }
-    // A solve that gave up leaves v partly overwritten: the last CTA to
-    // leave fills it with NaN, so that a caller who cannot read the error
-    // flag (a replayed graph) still sees that the result is not valid.
-    if (tid == 0) {
-        __threadfence();
-        ok_sh = atomicAdd(exits, 1) == static_cast<int>(gridDim.x) - 1 && *reinterpret_cast<volatile int*>(err);
-    }
-    __syncthreads();
-    if (ok_sh) {
-        __threadfence();
-        for (int i = tid; i < A.n3; i += kST) A.v[i] = __longlong_as_double(0x7ff8000000000000LL);
-    }
-}
-
 // ---------------------------------------------------------------- subtree solves
 // Below a cut level the elimination tree has many small fronts, and in the
 // dataflow solve above every one of its levels costs an inter-CTA
@@ -1026,15 +1052,17 @@ struct SubArgs {
 __device__ __forceinline__ void sub_stage(const SubArgs& A, const SubChunk& ch, double* dst)
 {
     const FrontArgs& a = A.a;
-    const int s = ch.s, c = a.ncol[s], m = a.nrow[s] - c, R = ch.b - ch.a;
+    const int s = ch.s, c = a.ncol[s], r = a.nrow[s], m = r - c, R = ch.b - ch.a;
     const int lc = odd(c), lm = odd(m);
+    const double* M = a.xw + a.xw_off[s];
+    const long long ld = ld_of(r);
     if (ch.kind == 0) {
-        stage_rows(dst, lc, a.dinv + a.dinv_off[s] + static_cast<long long>(ch.a) * c, c, R, c, 1, ch.a);
+        stage_cols(dst, lc, M + ch.a, ld, R, c, ch.a);
     } else if (ch.kind == 1) {
-        stage_rows(dst, lc, a.w + a.lt_off[s] + static_cast<long long>(ch.a) * c, c, R, c, 0, 0);
+        stage_cols(dst, lc, M + c + ch.a, ld, R, c, c);
     } else {
-        stage_rows(dst, lc, a.dinvT + a.dinv_off[s] + static_cast<long long>(ch.a) * c, c, R, c, 2, ch.a);
-        stage_rows(dst + R * lc, lm, a.wt + a.lt_off[s] + static_cast<long long>(ch.a) * m, m, R, m, 0, 0);
+        stage_rows(dst, lc, M + ch.a * ld, ld, R, c, ch.a);
+        stage_rows(dst + R * lc, lm, M + ch.a * ld + c, ld, R, m, -R);
     }
     stage_commit();
 }
@@ -1204,8 +1232,8 @@ __global__ void __launch_bounds__(kST) k_sub_bwd(SubArgs A)
 
 // W = L_RJ L_JJ^{-1} for every front, one 64 x 64 tile of W per CTA (4 x 4
 // per thread), L_RJ from the front's panel and L_JJ^{-1} (lower triangular,
-// entries above the diagonal masked) in blocks of 32; written row-major as W
-// and as its transpose.  With W the forward sweep forms a front's update
+// entries above the diagonal masked) in blocks of 32, written into the rows
+// below X in M.  With W the forward sweep forms a front's update
 // g = f_R - W f_J without waiting for y_J, and the backward sweep forms
 // x_J = L_JJ^{-T} y_J - W^T x_R in one step.
 __global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__ tiles)
@@ -1214,7 +1242,8 @@ __global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__
     const int s = tl.x, k0 = tl.y * 64, j0 = tl.z * 64;
     const int r = a.nrow[s], c = a.ncol[s], m = r - c;
     const double* F = a.front + a.front_off[s];
-    const double* X = a.dinv + a.dinv_off[s];
+    double* M = a.xw + a.xw_off[s];
+    const long long ld = ld_of(r);
     __shared__ double As[32][64 + 1];  // As[i][k] = L_RJ[k0 + k][i0 + i]
     __shared__ double Bs[32][64 + 1];  // Bs[i][j] = X[i0 + i][j0 + j]
     const int tid = threadIdx.x, tk = (tid & 15) * 4, tj = (tid >> 4) * 4;
@@ -1222,9 +1251,11 @@ __global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__
     for (int i0 = (j0 / 32) * 32; i0 < c; i0 += 32) {
         for (int idx = tid; idx < 32 * 64; idx += 256) {
             const int i = idx >> 6, kk = idx & 63;
-            const int gi = i0 + i, gk = k0 + kk, gj = j0 + kk;
+            const int gi = i0 + i, gk = k0 + kk;
             As[i][kk] = (gi < c && gk < m) ? F[static_cast<long long>(gi) * r + c + gk] : 0.0;
-            Bs[i][kk] = (gi < c && gj < c && gi >= gj) ? X[static_cast<long long>(gi) * c + gj] : 0.0;
+            const int bi = idx & 31, bj = idx >> 5;  // consecutive threads on consecutive rows of X
+            const int hi = i0 + bi, hj = j0 + bj;
+            Bs[bi][bj] = (hi < c && hj < c && hi >= hj) ? M[hj * ld + hi] : 0.0;
         }
         __syncthreads();
 #pragma unroll 8
@@ -1242,17 +1273,12 @@ __global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__
         }
         __syncthreads();
     }
-    double* W = a.w + a.lt_off[s];
-    double* WT = a.wt + a.lt_off[s];
 #pragma unroll
-    for (int x = 0; x < 4; x++)
+    for (int y = 0; y < 4; y++)
 #pragma unroll
-        for (int y = 0; y < 4; y++) {
+        for (int x = 0; x < 4; x++) {
             const int gk = k0 + tk + x, gj = j0 + tj + y;
-            if (gk < m && gj < c) {
-                W[static_cast<long long>(gk) * c + gj] = acc[x][y];
-                WT[static_cast<long long>(gj) * m + gk] = acc[x][y];
-            }
+            if (gk < m && gj < c) M[gj * ld + c + gk] = acc[x][y];
         }
 }
 
@@ -1260,7 +1286,7 @@ FrontArgs args_of(Precond& P)
 {
     return FrontArgs { P.d_first, P.d_ncol, P.d_nrow, P.d_rows, P.d_child_ptr, P.d_child_list, P.d_relind,
         P.d_level_list, P.d_contrib_ptr, P.d_contrib_idx, P.d_below_front, P.d_front_off, P.d_rows_off,
-        P.d_relind_off, P.d_dinv_off, P.d_upd_off, P.d_lt_off, P.d_front, P.d_dinv, P.d_dinvT, P.d_w, P.d_wt, P.d_fail };
+        P.d_relind_off, P.d_xw_off, P.d_upd_off, P.d_front, P.d_xw, P.d_fail };
 }
 
 // the work buffers of one solve
@@ -1290,8 +1316,7 @@ efem_status enqueue_solve(const Precond& P, const FrontArgs& a, const SolveBufs&
     const SubArgs B { a, P.d_parent, P.d_prow, P.d_perm, P.d_subs, P.d_chunks, P.d_depth, P.d_xidx, P.sub_max_r,
         P.sub_max_cols, P.sub_max_depth, P.sub_max_m, P.sub_max_c, P.sub_max_mroot, d_v, b.y, b.upd, stamp };
     if (P.n_subs > 0) k_sub_fwd<<<P.n_subs, kST, P.sub_smem_f, st>>>(B);
-    SolveArgs A { a, P.d_parent, P.d_prow, P.d_items, P.d_tgt, P.n_items, ns, P.stage_d, P.work_d, d_v, b.y, b.t,
-        b.upd, b.cnt, P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, P.d_item_group,
+    SolveArgs A { a, P.d_prow, P.d_items, P.d_slot, P.n_items, ns, d_v, b.y, b.t, b.upd, b.cnt, P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, P.d_item_group,
         P.d_item_group ? P.d_frozen : nullptr };
     if (P.n_items > 0) launch_k(k_solve, P.solve_grid, kST, P.solve_smem, st, A);
     if (P.n_subs > 0) k_sub_bwd<<<P.n_subs, kST, P.sub_smem_b, st>>>(B);
@@ -1310,10 +1335,10 @@ void free_precond(Model& m)
     if (P.factor_exec) cudaGraphExecDestroy(P.factor_exec);
     if (P.capture) cudaStreamDestroy(P.capture);
     for (int** p : { &P.d_first, &P.d_ncol, &P.d_nrow, &P.d_rows, &P.d_child_ptr, &P.d_child_list, &P.d_relind,
-             &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_panel_list, &P.d_contrib_ptr, &P.d_contrib_idx, &P.d_below_front, &P.d_tgt, &P.d_parent, &P.d_cnt, &P.d_prow, &P.d_depth, &P.d_xidx })
+             &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_panel_list, &P.d_contrib_ptr, &P.d_contrib_idx, &P.d_below_front, &P.d_parent, &P.d_cnt, &P.d_prow, &P.d_depth, &P.d_xidx, &P.d_slot })
         dev_free(*p);
-    for (long long** p : { &P.d_front_off, &P.d_rows_off, &P.d_relind_off, &P.d_dinv_off, &P.d_upd_off, &P.d_a_pos,
-             &P.d_a_src, &P.d_lt_off })
+    for (long long** p : { &P.d_front_off, &P.d_rows_off, &P.d_relind_off, &P.d_xw_off, &P.d_upd_off, &P.d_a_pos,
+             &P.d_a_src })
         dev_free(*p);
     for (Tile** p : { &P.d_inv, &P.d_ea, &P.d_oinv }) dev_free(*p);
     dev_free(P.d_items);
@@ -1322,7 +1347,7 @@ void free_precond(Model& m)
     dev_free(P.d_chunks);
     dev_free(P.d_syrk);
     dev_free(P.d_wtiles);
-    for (double** p : { &P.d_front, &P.d_dinv, &P.d_dinvT, &P.d_w, &P.d_wt, &P.d_upd, &P.d_y, &P.d_t, &P.d_vals,
+    for (double** p : { &P.d_front, &P.d_xw, &P.d_upd, &P.d_y, &P.d_t, &P.d_vals,
              &P.d_diag_tmp })
         dev_free(*p);
     delete m.precond;
@@ -1545,122 +1570,74 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     P.sub_max_mroot = sp.max_mroot;
     P.sub_smem_f = sp.smem_f;
     P.sub_smem_b = sp.smem_b;
-    // solve items above the cut: forward sweep by level (leaves first),
-    // backward sweep by level (root first).  Each item records the ranges of
-    // contributions its rows assemble, and the shared memory it stages is
-    // sized here.
-    // Tiles take a multiple of 4 rows, at least 4.  A front with rows longer
-    // than kStageBudget / 4 then stages more than the budget, and on a mesh
-    // like the C3D20 cap that halves the CTAs per SM for every item of the
-    // solve; so the schedule is also built with tiles of 1-3 rows for such
-    // fronts (more items, more repeated assembly), and the one with more CTAs
-    // per SM is kept (the 4-row one on a tie).
-    struct Schedule {
-        std::vector<SolveItem> items;
-        std::vector<int> tgt;
-        size_t stage_d = 1, work_d = 1, ints = 1;
-        size_t smem() const { return sizeof(double) * (stage_d + work_d) + sizeof(int) * ints; }
+    // Storage of the fronts' M = [X; W] and the slot tables of the assembly.
+    std::vector<long long> xw_off(S.ns + 1, 0), slot_off(S.ns + 1, 0);
+    for (int s = 0; s < S.ns; s++) {
+        xw_off[s + 1] = xw_off[s] + ld_of(S.nrow[s]) * S.ncol[s];
+        slot_off[s + 1] = slot_off[s] + static_cast<long long>(S.child_ptr[s + 1] - S.child_ptr[s]) * S.nrow[s];
+    }
+    const long long xw_size = xw_off[S.ns];
+    std::vector<int> slot(static_cast<size_t>(slot_off[S.ns]), -1);
+    for (int s = 0; s < S.ns; s++)
+        for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; q++) {
+            const int ch = S.child_list[q];
+            int* sl = slot.data() + slot_off[s] + static_cast<long long>(q - S.child_ptr[s]) * S.nrow[s];
+            for (long long j = S.relind_off[ch]; j < S.relind_off[ch + 1]; j++)
+                sl[S.relind[j]] = static_cast<int>(S.upd_off[ch] / 3 + (j - S.relind_off[ch]));
+        }
+    // Solve items above the cut: forward sweep by level (leaves first),
+    // backward sweep by level (root first).  A tile holds about lev_td doubles
+    // of M: a level's share per resident CTA, so that levels with little work
+    // still spread over the chip, within [kTileMin, kTileMax] (below it the
+    // tiles' repeated assembly of f costs more than the spread gives, above it
+    // a level's last tiles run alone).
+    EFEM_CUDA(cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSolveSmem)));
+    int per_sm = 0, sms = 0;
+    EFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve, kST, kSolveSmem));
+    EFEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device));
+    P.slots = std::max(1, per_sm) * std::max(1, sms);
+    std::vector<int> lev_td(nlev, 0);
+    auto area = [&](int s) { return static_cast<long long>(S.nrow[s]) * S.ncol[s]; };
+    for (int l = 0; l < nlev; l++) {
+        long long sum = 0;
+        for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) sum += area(S.level_list[q]);
+        lev_td[l] = static_cast<int>(std::min<long long>(kTileMax, std::max<long long>(kTileMin, sum / P.slots)));
+    }
+    auto fwd_rows = [&](int s) {  // rows of a forward tile: equal tiles of about lev_td doubles, a multiple of 8
+        const int r = S.nrow[s], td = lev_td[lev[s]];
+        const long long nt = std::max<long long>(std::max<long long>(1, (area(s) + td / 2) / td), (r + kMaxR - 1) / kMaxR);
+        return std::min(kMaxR, std::max(8, static_cast<int>(((r + nt - 1) / nt + 7) / 8 * 8)));
     };
-    std::vector<char> whole(S.ns, 0);
-    auto schedule = [&](int min_rows, Schedule& sch) {
-        std::vector<SolveItem>& items = sch.items;
-        std::vector<int>& tgt = sch.tgt;
-        tgt.assign(4 * static_cast<size_t>(S.ns), 0);
-        size_t& stage_d = sch.stage_d;
-        size_t& work_d = sch.work_d;
-        size_t& ints = sch.ints;
-        auto need = [&](size_t sd, size_t wd, size_t ni) {
-            stage_d = std::max(stage_d, sd);
-            work_d = std::max(work_d, wd);
-            ints = std::max(ints, ni);
-        };
-        auto tile = [&](int per_row) {  // rows per tile when a row stages per_row doubles
-            const int t = kStageBudget / per_row;
-            return t >= 4 ? std::min(256, t / 4 * 4) : std::max(min_rows, t);
-        };
-        auto ntiles = [&](int n, int per_row) { const int t = tile(per_row); return (n + t - 1) / t; };
-        auto crange = [&](int s, int t0, int t1) {  // contributions of front rows [t0, t1)
-            const long long ro = S.rows_off[s];
-            return t1 > t0 ? std::make_pair(S.contrib_ptr[ro + t0], S.contrib_ptr[ro + t1]) : std::make_pair(0, 0);
-        };
-        for (int s = 0; s < S.ns; s++) {
-            const int c = S.ncol[s], mm = S.nrow[s] - c, r = S.nrow[s];
-            const int lc = odd_h(c), lm = odd_h(mm);
-            whole[s] = static_cast<long long>(r) * lc <= kWholeBudget && static_cast<long long>(c) * (lc + lm) <= kWholeBudget;
-            tgt[s] = whole[s] ? 1 : ntiles(c, lc);  // y of s complete
-            if (S.parent[s] >= 0 && !in_sub[s])     // children's g complete (subtree roots finish before k_solve)
-                tgt[S.ns + S.parent[s]] += whole[s] ? 1 : ntiles(mm, lc);
-            tgt[3 * S.ns + s] = whole[s] ? 1 : ntiles(c, lc + lm);                              // x of s complete
-        }
-        for (int l = K; l < nlev; l++) {
-            for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
-                const int s = S.level_list[q];
-                const int c = S.ncol[s], r = S.nrow[s], mm = r - c, lc = odd_h(c);
-                if (whole[s]) {
-                    const auto cr = crange(s, 0, r);
-                    items.push_back(SolveItem { kFwdFront, s, 0, c, cr.first, cr.second, 0, 0 });
-                    need(static_cast<size_t>(r) * lc, 3 * static_cast<size_t>(r), r + 1 + (cr.second - cr.first) + c);
-                    continue;
-                }
-                const int ty = tile(lc);
-                for (int o = 0; o < c; o += ty) {
-                    const int i1 = std::min(c, o + ty);
-                    const auto cr = crange(s, 0, i1);
-                    items.push_back(SolveItem { kFwdY, s, o, i1, cr.first, cr.second, 0, 0 });
-                    need(static_cast<size_t>(i1 - o) * lc, 3 * static_cast<size_t>(i1), i1 + 1 + (cr.second - cr.first) + i1);
-                }
-                const auto cj = crange(s, 0, c);
-                for (int o = 0; o < mm; o += ty) {
-                    const int k1 = std::min(mm, o + ty);
-                    const auto cr = crange(s, c + o, c + k1);
-                    items.push_back(SolveItem { kFwdG, s, o, k1, cj.first, cj.second, cr.first, cr.second });
-                    need(static_cast<size_t>(k1 - o) * lc, 3 * static_cast<size_t>(c + k1 - o),
-                        2 * static_cast<size_t>(c) + 1 + (cj.second - cj.first) + (k1 - o + 1) + (cr.second - cr.first));
-                }
-            }
-        }
-        for (int l = nlev - 1; l >= K; l--) {
-            for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
-                const int s = S.level_list[q];
-                const int c = S.ncol[s], r = S.nrow[s], mm = r - c, lc = odd_h(c), lm = odd_h(mm);
-                if (whole[s]) {
-                    items.push_back(SolveItem { kBwdFront, s, 0, c, 0, 0, 0, 0 });
-                    need(static_cast<size_t>(c) * (lc + lm), 3 * static_cast<size_t>(r + c), r);
-                    continue;
-                }
-                const int tx = tile(lc + lm);
-                for (int o = 0; o < c; o += tx) {
-                    const int i1 = std::min(c, o + tx);
-                    items.push_back(SolveItem { kBwdX, s, o, i1, 0, 0, 0, 0 });
-                    need(static_cast<size_t>(i1 - o) * (lc + lm), 3 * static_cast<size_t>(c - o + mm + i1 - o), r);
-                }
-            }
+    auto bwd_cols = [&](int s) {  // columns of a backward tile, a multiple of 4
+        const int c = S.ncol[s], td = lev_td[lev[s]];
+        const long long nt = std::max<long long>(1, (area(s) + td / 2) / td);
+        return std::min(32, std::max(4, static_cast<int>(((c + nt - 1) / nt + 3) / 4 * 4)));
+    };
+    std::vector<int> tY(S.ns, 0), tG(S.ns, 0), tX(S.ns, 0);  // tiles that complete y, the children's g, x of a front
+    for (int s = 0; s < S.ns; s++) {
+        const int c = S.ncol[s], r = S.nrow[s], fr = fwd_rows(s), bc = bwd_cols(s);
+        tY[s] = (c + fr - 1) / fr;
+        tX[s] = (c + bc - 1) / bc;
+        if (S.parent[s] >= 0 && !in_sub[s])  // (subtree roots finish before k_solve)
+            tG[S.parent[s]] += (r + fr - 1) / fr - c / fr;
+    }
+    std::vector<SolveItem> items;
+    auto sweep = [&](int l, bool fwd) {
+        for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
+            const int s = S.level_list[q], p = S.parent[s];
+            const int n = fwd ? S.nrow[s] : S.ncol[s], step = fwd ? fwd_rows(s) : bwd_cols(s);
+            for (int o = 0; o < n; o += step)
+                items.push_back(SolveItem { fwd ? kFwdTile : kBwdTile, s, o, std::min(n, o + step), p, S.nrow[s], S.ncol[s],
+                    S.first[s], S.child_ptr[s + 1] - S.child_ptr[s], fwd ? tG[s] : tY[s], !fwd && p >= 0 ? tX[p] : 0, 0,
+                    xw_off[s], S.rows_off[s], slot_off[s], S.upd_off[s] });
         }
     };
-    Schedule sch4, sch1;
-    schedule(4, sch4);
-    schedule(1, sch1);
-    EFEM_CUDA(cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    int per4 = 0, per1 = 0;
-    if (sch4.smem() <= 200 * 1024)
-        EFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per4, k_solve, kST, sch4.smem()));
-    if (sch1.smem() <= 200 * 1024)
-        EFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, k_solve, kST, sch1.smem()));
-    Schedule& sch = per1 > per4 ? sch1 : sch4;
-    std::vector<SolveItem>& items = sch.items;
-    std::vector<int>& tgt = sch.tgt;
-    const size_t stage_d = sch.stage_d, work_d = sch.work_d, ints = sch.ints;
+    for (int l = K; l < nlev; l++) sweep(l, true);
+    for (int l = nlev - 1; l >= K; l--) sweep(l, false);
     P.n_items = static_cast<int>(items.size());
     P.h_item_front.resize(items.size());
     for (size_t i = 0; i < items.size(); i++) P.h_item_front[i] = items[i].s;
-    P.stage_d = static_cast<int>(stage_d);
-    P.work_d = static_cast<int>(work_d);
-    P.solve_smem = sizeof(double) * (stage_d + work_d) + sizeof(int) * ints;
-    if (P.solve_smem > 200 * 1024) {
-        set_error("a front of the approximate-Jacobian factor is too large for the solve kernel ("
-            + std::to_string(P.max_r) + " rows)");
-        return EFEM_ERR_UNSUPPORTED;
-    }
+    P.solve_smem = kSolveSmem;
     // node index in v of every front row
     std::vector<int> prow(S.rows.size());
     for (size_t q = 0; q < S.rows.size(); q++) prow[q] = S.perm[S.rows[q]];
@@ -1680,9 +1657,9 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     UP(P.d_front_off, S.front_off);
     UP(P.d_rows_off, S.rows_off);
     UP(P.d_relind_off, S.relind_off);
-    UP(P.d_dinv_off, S.dinv_off);
+    UP(P.d_xw_off, xw_off);
+    UP(P.d_slot, slot);
     UP(P.d_upd_off, S.upd_off);
-    UP(P.d_lt_off, S.lt_off);
     UP(P.d_contrib_ptr, S.contrib_ptr);
     UP(P.d_contrib_idx, S.contrib_idx);
     UP(P.d_a_pos, S.a_pos);
@@ -1691,7 +1668,6 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     UP(P.d_parent, S.parent);
     UP(P.d_prow, prow);
     UP(P.d_items, items);
-    UP(P.d_tgt, tgt);
     if (P.n_subs > 0) {
         UP(P.d_subs, subs);
         UP(P.d_chunks, chunks);
@@ -1708,10 +1684,8 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
 #undef UP
     const size_t n3 = 3 * static_cast<size_t>(std::max(S.n, 1));
     if ((st = dev_alloc(&P.d_front, static_cast<size_t>(S.front_size))) != EFEM_OK) return st;
-    if ((st = dev_alloc(&P.d_dinv, static_cast<size_t>(std::max<long long>(S.dinv_size, 1)))) != EFEM_OK) return st;
-    if ((st = dev_alloc(&P.d_dinvT, static_cast<size_t>(std::max<long long>(S.dinv_size, 1)))) != EFEM_OK) return st;
-    if ((st = dev_alloc(&P.d_w, static_cast<size_t>(std::max<long long>(S.lt_size, 1)))) != EFEM_OK) return st;
-    if ((st = dev_alloc(&P.d_wt, static_cast<size_t>(std::max<long long>(S.lt_size, 1)))) != EFEM_OK) return st;
+    if ((st = dev_alloc(&P.d_xw, static_cast<size_t>(std::max<long long>(xw_size, 1)))) != EFEM_OK) return st;
+    EFEM_CUDA(cudaMemsetAsync(P.d_xw, 0, sizeof(double) * std::max<long long>(xw_size, 1), m.stream));  // above X's diagonal, pad rows
     if ((st = dev_alloc(&P.d_upd, static_cast<size_t>(std::max<long long>(S.upd_size, 1)))) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_y, n3)) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_t, n3)) != EFEM_OK) return st;
@@ -1720,11 +1694,6 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     if ((st = dev_alloc(&P.d_diag_tmp, static_cast<size_t>(std::max(P.max_panel_cnt, 1)) * kNB * kNB)) != EFEM_OK)
         return st;
     // persistent solve: as many CTAs as fit on the device at once
-    EFEM_CUDA(cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    int per_sm = 0, sms = 0;
-    EFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve, kST, P.solve_smem));
-    EFEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device));
-    P.slots = std::max(1, per_sm) * std::max(1, sms);
     P.solve_grid_full = std::max(1, std::min(P.n_items, P.slots));
     P.solve_grid = solve_grid_for(P);
     if (P.n_subs > 0) {

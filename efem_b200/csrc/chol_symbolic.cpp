@@ -293,25 +293,19 @@ void symbolic_analysis(int n, const std::vector<int>& rowptr, const std::vector<
     }
     // storage offsets and flop count
     S.front_off.resize(ns + 1);
-    S.dinv_off.resize(ns + 1);
     S.upd_off.resize(ns + 1);
-    S.lt_off.resize(ns + 1);
-    S.front_off[0] = S.dinv_off[0] = S.upd_off[0] = S.lt_off[0] = 0;
+    S.front_off[0] = S.upd_off[0] = 0;
     S.nnz_L = 0;
     S.flops = 0;
     for (int k = 0; k < ns; k++) {
         const long long r = S.nrow[k], c = S.ncol[k];
         S.front_off[k + 1] = S.front_off[k] + r * r;
-        S.dinv_off[k + 1] = S.dinv_off[k] + c * c;
         S.upd_off[k + 1] = S.upd_off[k] + 3 * (r - c);
-        S.lt_off[k + 1] = S.lt_off[k] + (r - c) * c;
         S.nnz_L += c * r - c * (c - 1) / 2;
         S.flops += c * c * c / 3.0 + static_cast<double>(r - c) * c * c + static_cast<double>(r - c) * (r - c) * c;
     }
     S.front_size = S.front_off[ns];
-    S.dinv_size = S.dinv_off[ns];
     S.upd_size = S.upd_off[ns];
-    S.lt_size = S.lt_off[ns];
     // children's update-vector entries per parent row, in child order
     {
         std::vector<int> cnt(S.rows.size() + 1, 0);
