@@ -579,6 +579,7 @@ struct AdjointWS {
     double* hcol = nullptr;    // device: the Hessenberg column being formed
     double* h_hcol = nullptr;  // pinned host copy
     MatParams<Dual>* mats = nullptr;
+    int mats_seed = -2;  // the seed `mats` holds: 5 slot + k, -1 none, -2 not uploaded
     double* dscale = nullptr;
     std::vector<double> h_part;
     // stored tangents at u, used while blocks_ready is set (inside one adjoint
@@ -635,6 +636,10 @@ efem_status alloc_aws(Model& m)
 // k (0 C10, 1 C01, 2 C20, 3 C30, 4 D1) of material slot `slot` (-1: none)
 efem_status upload_dual_mats(Model& m, int slot, int k)
 {
+    // the table depends on the seed alone (a model's materials are fixed)
+    const int seed = slot < 0 ? -1 : 5 * slot + k;
+    if (m.aws->mats_seed == seed) return EFEM_OK;
+    m.aws->mats_seed = -2;
     std::vector<MatParams<Dual>> h(std::max<size_t>(m.materials_used.size(), 1));
     for (size_t i = 0; i < m.materials_used.size(); i++) {
         const HostMaterial& hm = m.materials_used[i];
@@ -647,6 +652,7 @@ efem_status upload_dual_mats(Model& m, int slot, int k)
         h[i].D1 = Dual(hm.D1, s && k == 4 ? 1.0 : 0.0);
     }
     EFEM_CUDA(cudaMemcpyAsync(m.aws->mats, h.data(), sizeof(MatParams<Dual>) * h.size(), cudaMemcpyHostToDevice, m.stream));
+    m.aws->mats_seed = seed;
     return EFEM_OK;
 }
 

@@ -124,6 +124,7 @@ struct Precond {
     int4* d_syrk = nullptr;
     double* d_diag_tmp = nullptr;  // factored diagonal blocks of one panel step, [fronts in step][kNB][kNB]
     int max_panel_cnt = 0;
+    int* h_flag = nullptr;  // pinned: the error flag read back after an application
     double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
            *d_vals = nullptr;
     // graph replay of the numeric factorisation (the same launches every solve)
@@ -1334,6 +1335,7 @@ void free_precond(Model& m)
     P.graphs.clear();
     if (P.factor_exec) cudaGraphExecDestroy(P.factor_exec);
     if (P.capture) cudaStreamDestroy(P.capture);
+    if (P.h_flag) cudaFreeHost(P.h_flag);
     for (int** p : { &P.d_first, &P.d_ncol, &P.d_nrow, &P.d_rows, &P.d_child_ptr, &P.d_child_list, &P.d_relind,
              &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_panel_list, &P.d_contrib_ptr, &P.d_contrib_idx, &P.d_below_front, &P.d_parent, &P.d_cnt, &P.d_prow, &P.d_depth, &P.d_xidx, &P.d_slot })
         dev_free(*p);
@@ -1701,6 +1703,7 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
         EFEM_CUDA(cudaFuncSetAttribute(k_sub_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
     EFEM_CUDA(cudaStreamCreateWithFlags(&P.capture, cudaStreamNonBlocking));
+    EFEM_CUDA(cudaMallocHost(&P.h_flag, sizeof(int)));
     P.ready = true;  // analysed; the numeric factor follows
     return precond_factor(m, ok, ms_factor);
 }
@@ -1920,12 +1923,12 @@ const int* precond_error_flag(const Model& m)
     return m.precond && m.precond->d_cnt ? m.precond->d_cnt + 4LL * m.precond->S.ns + 1 : nullptr;
 }
 
-static efem_status check_solve_flag(const int* d_flag, cudaStream_t st)
+// h_flag: where the flag is read back to (pinned memory spares the copy's staging)
+static efem_status check_solve_flag(const int* d_flag, cudaStream_t st, int* h_flag)
 {
-    int flag = 0;
-    EFEM_CUDA(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    EFEM_CUDA(cudaMemcpyAsync(h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     EFEM_CUDA(cudaStreamSynchronize(st));
-    if (flag) {
+    if (*h_flag) {
         set_error("the triangular solve of the preconditioner gave up waiting for a front");
         return EFEM_ERR_TIMEOUT;
     }
@@ -1935,7 +1938,7 @@ static efem_status check_solve_flag(const int* d_flag, cudaStream_t st)
 efem_status precond_check(Model& m)
 {
     const int* f = precond_error_flag(m);
-    return f ? check_solve_flag(f, m.stream) : EFEM_OK;
+    return f ? check_solve_flag(f, m.stream, m.precond->h_flag) : EFEM_OK;
 }
 
 // ============================================================================
@@ -2066,5 +2069,5 @@ extern "C" efem_status efem_precond_apply_noalloc(void* model, double* d_v)
     if (st != EFEM_OK) return st;
     EFEM_CUDA(cudaGetLastError());
     if (capturing) return EFEM_OK;  // recorded into the caller's graph; a give-up shows as NaN in d_v
-    return check_solve_flag(counters + 4LL * S.ns + 1, m.stream);
+    return check_solve_flag(counters + 4LL * S.ns + 1, m.stream, P.h_flag);
 }

@@ -607,11 +607,13 @@ efem_status ensure_device(Model& m)
         if (s != EFEM_OK) return s;           \
     }
     for (auto& b : m.blocks) {
-        std::vector<int> soa(b.h_conn.size());
-        for (int e = 0; e < b.n; e++)
-            for (int a = 0; a < b.nen; a++)
-                soa[static_cast<size_t>(a) * b.n + e] = b.h_conn[static_cast<size_t>(e) * b.nen + a];
-        UP(b.conn, soa);
+        if (!b.conn) {  // every call comes through here: transpose only for the upload itself
+            std::vector<int> soa(b.h_conn.size());
+            for (int e = 0; e < b.n; e++)
+                for (int a = 0; a < b.nen; a++)
+                    soa[static_cast<size_t>(a) * b.n + e] = b.h_conn[static_cast<size_t>(e) * b.nen + a];
+            UP(b.conn, soa);
+        }
         UP(b.mat, b.h_mat);
         UP(b.vol, b.h_vol);
         UP(b.vol_f, to_f32(b.h_vol));
