@@ -723,7 +723,7 @@ efem_status setup_union(Union& U)
     }
     M.d_frozen_groups = U.d_frozen;
     for (auto& c : U.cap) EFEM_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
-    U.per_res = 1 + static_cast<long long>(M.blocks.size() + M.faces.size());
+    U.per_res = residual_launches(M);
     return EFEM_OK;
 }
 

@@ -64,23 +64,218 @@ struct Scatter {
 template <int NGP, int BLK>
 constexpr int elems_per_cta() { return (BLK / NGP) < 1 ? 1 : ((BLK / NGP) > 128 ? 128 : BLK / NGP); }
 
-// MT: the block's one material law, or -1 when its elements mix laws
-template <int NEN, int NGP, typename T, int BLK, int MT>
-__global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a)
+template <typename T>
+struct FaceArgs {
+    int n, n_free;
+    int gmax;                         // most points of a face in the set
+    const int* __restrict__ conn;     // [NEN][n]
+    const int* __restrict__ table;    // [n]
+    const double* __restrict__ A0;    // [n][3]
+    const T* __restrict__ J0inv;      // [n][MAX_FGP][9]
+    const double* __restrict__ load;  // [n][4]
+    const int* __restrict__ t_ngp;
+    const T* __restrict__ t_w;        // [t][MAX_FGP]
+    const T* __restrict__ t_N;        // [t][MAX_FGP][NEN]
+    const T* __restrict__ t_dN;       // [t][MAX_FGP][NEN][3]
+    const double* __restrict__ u;
+    double* __restrict__ r;
+    double* __restrict__ contrib;     // deterministic scatter: [3][n_slots], or null for atomics
+    size_t n_slots, slot0;
+};
+
+// Pressure faces, EPB per tile, in the element kernel's phases: (face, node)
+// threads stage u, (face, point) threads form cof(F_g) A0, and (face, node)
+// threads add up and scatter the nodal forces.  A face is a few hundred
+// dependent FP64 operations, so latency bounds it and not its work: with one
+// thread per face, all in that thread's local memory, the 2 752 faces of the
+// C3D20R cap took 34.8 us (22 CTAs), more than twice its elements; in phases
+// 11.4 us by themselves.  The element kernel's launch carries them as its
+// first CTAs (k_elem_residual), where they overlap with the elements.
+template <int NEN, int BLK>
+constexpr int face_epb() { return (NEN >= 20 ? 8 : NEN >= 8 ? 16 : 32) * BLK / 128; }
+
+template <int NEN, typename T, int EPB>
+struct FaceSmem {
+    T u[EPB][(NEN * 3) | 1];       // displacements relative to the parent's first node, as in the element kernel
+    T cA[EPB][(MAX_FGP * 3) | 1];  // cof(F_g) A0 (directed loads: its norm) at every face point
+    int node[EPB][NEN];
+    int table[EPB], ngp[EPB];
+};
+
+template <int NEN, typename T, int BLK>
+__device__ void face_tile(const FaceArgs<T>& a, int tile, FaceSmem<NEN, T, face_epb<NEN, BLK>()>& sm)
+{
+    constexpr int EPB = face_epb<NEN, BLK>();
+    const int tid = threadIdx.x, fb = tile * EPB;
+    // the (face, point) pair of phase 2: its inputs are on their way while u is staged
+    const int el1 = tid / a.gmax, g1 = tid - el1 * a.gmax, f1 = fb + el1;
+    const bool on1 = tid < EPB * a.gmax && f1 < a.n;
+    T Ji1[9], A01[3];
+#pragma unroll
+    for (int k = 0; k < 9; k++) Ji1[k] = on1 ? __ldg(a.J0inv + (static_cast<size_t>(f1) * MAX_FGP + g1) * 9 + k) : T(0);
+#pragma unroll
+    for (int k = 0; k < 3; k++) A01[k] = on1 ? static_cast<T>(__ldg(a.A0 + 3 * f1 + k)) : T(0);
+    const double directed1 = on1 ? __ldg(a.load + 4 * f1) : 0.0;
+    if (tid < EPB) {
+        const int t = fb + tid < a.n ? __ldg(a.table + fb + tid) : 0;
+        sm.table[tid] = t;
+        sm.ngp[tid] = __ldg(a.t_ngp + t);
+    }
+    for (int i = tid; i < EPB * NEN; i += BLK) {
+        const int el = i % EPB, q = i / EPB, f = fb + el;
+        int node = a.n_free;
+        double u0 = 0.0, u1 = 0.0, u2 = 0.0;
+        if (f < a.n) {
+            node = __ldg(a.conn + static_cast<size_t>(q) * a.n + f);
+            const int n0 = __ldg(a.conn + f);
+            double z0 = 0.0, z1 = 0.0, z2 = 0.0;
+            if (node < a.n_free) {
+                u0 = __ldg(a.u + 3 * node);
+                u1 = __ldg(a.u + 3 * node + 1);
+                u2 = __ldg(a.u + 3 * node + 2);
+            }
+            if (n0 < a.n_free) {
+                z0 = __ldg(a.u + 3 * n0);
+                z1 = __ldg(a.u + 3 * n0 + 1);
+                z2 = __ldg(a.u + 3 * n0 + 2);
+            }
+            u0 -= z0;
+            u1 -= z1;
+            u2 -= z2;
+        }
+        sm.node[el][q] = node;
+        sm.u[el][3 * q] = static_cast<T>(u0);
+        sm.u[el][3 * q + 1] = static_cast<T>(u1);
+        sm.u[el][3 * q + 2] = static_cast<T>(u2);
+    }
+    __syncthreads();
+    for (int i = tid; i < EPB * a.gmax; i += BLK) {
+        const int el = i / a.gmax, g = i - el * a.gmax, f = fb + el;
+        if (f >= a.n) break;
+        if (g >= sm.ngp[el]) continue;
+        const T* dN = a.t_dN + (static_cast<size_t>(sm.table[el]) * MAX_FGP + g) * NEN * 3;
+        T Ji[9], A0[3];
+        double directed = directed1;
+#pragma unroll
+        for (int k = 0; k < 9; k++) Ji[k] = Ji1[k];
+#pragma unroll
+        for (int k = 0; k < 3; k++) A0[k] = A01[k];
+        if (i != tid) {  // more (face, point) pairs than threads
+#pragma unroll
+            for (int k = 0; k < 9; k++) Ji[k] = __ldg(a.J0inv + (static_cast<size_t>(f) * MAX_FGP + g) * 9 + k);
+#pragma unroll
+            for (int k = 0; k < 3; k++) A0[k] = static_cast<T>(__ldg(a.A0 + 3 * f + k));
+            directed = __ldg(a.load + 4 * f);
+        }
+        T A[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
+#pragma unroll(NEN == 4 ? 4 : 5)
+        for (int q = 0; q < NEN; q++)
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) A[3 * c + k] += sm.u[el][3 * q + c] * __ldg(dN + 3 * q + k);
+        T H[9];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) H[3 * c + j] = A[3 * c] * Ji[j] + A[3 * c + 1] * Ji[3 + j] + A[3 * c + 2] * Ji[6 + j];
+        Kin<T> k;
+        kinematics(H, k);
+        // cof F A0 = (I + B) A0
+        T cA[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) cA[c] = A0[c] + k.B[3 * c] * A0[0] + k.B[3 * c + 1] * A0[1] + k.B[3 * c + 2] * A0[2];
+        if (directed != 0.0) cA[0] = sqrt(cA[0] * cA[0] + cA[1] * cA[1] + cA[2] * cA[2]);
+#pragma unroll
+        for (int c = 0; c < 3; c++) sm.cA[el][3 * g + c] = cA[c];
+    }
+    __syncthreads();
+    for (int i = tid; i < EPB * NEN; i += BLK) {
+        const int el = i % EPB, q = i / EPB, f = fb + el;
+        if (f >= a.n) continue;
+        const int node = sm.node[el][q];
+        if (node >= a.n_free) continue;
+        const int t = sm.table[el], ngp = sm.ngp[el];
+        const T* tw = a.t_w + t * MAX_FGP;
+        const T* tN = a.t_N + static_cast<size_t>(t) * MAX_FGP * NEN + q;
+        const double* L = a.load + 4 * f;
+        const double l0 = __ldg(L), l1 = __ldg(L + 1), l2 = __ldg(L + 2), l3 = __ldg(L + 3);
+        T v0 = 0, v1 = 0, v2 = 0;
+#pragma unroll 3
+        for (int g = 0; g < ngp; g++) {
+            const T wn = __ldg(tw + g) * __ldg(tN + g * NEN);
+            v0 += wn * sm.cA[el][3 * g];
+            v1 += wn * sm.cA[el][3 * g + 1];
+            v2 += wn * sm.cA[el][3 * g + 2];
+        }
+        double f0, f1, f2;
+        if (l0 != 0.0) {
+            f0 = l1 * static_cast<double>(v0);
+            f1 = l2 * static_cast<double>(v0);
+            f2 = l3 * static_cast<double>(v0);
+        } else {
+            f0 = l1 * static_cast<double>(v0);
+            f1 = l1 * static_cast<double>(v1);
+            f2 = l1 * static_cast<double>(v2);
+        }
+        if (a.contrib) {
+            const size_t sl = a.slot0 + static_cast<size_t>(q) * a.n + f;
+            a.contrib[sl] = -f0;
+            a.contrib[a.n_slots + sl] = -f1;
+            a.contrib[2 * a.n_slots + sl] = -f2;
+        } else {
+            atomicAdd(a.r + 3 * node, -f0);
+            atomicAdd(a.r + 3 * node + 1, -f1);
+            atomicAdd(a.r + 3 * node + 2, -f2);
+        }
+    }
+}
+
+// faces without an element block of their kind to go with
+template <int NEN, typename T>
+__global__ void __launch_bounds__(kBlock) k_face_residual(FaceArgs<T> a)
 {
     griddep_wait();
-    constexpr int EPB = elems_per_cta<NGP, BLK>();
+    __shared__ FaceSmem<NEN, T, face_epb<NEN, kBlock>()> sm;
+    face_tile<NEN, T, kBlock>(a, blockIdx.x, sm);
+    griddep_launch();
+}
+
+template <int NEN, int NGP, typename T, int EPB>
+struct ElemSmem {
     // per-element rows padded to an odd length, so that threads on
     // consecutive elements (phases 1 and 3) or Gauss points (phase 2) read
     // different shared-memory banks
-    constexpr int SU = (NEN * 3) | 1, SS = (NGP * 9) | 1, SD = (NEN * 3) | 1, SN = NEN | 1;
-    __shared__ T s_u[EPB][SU];     // [element][node * 3 + component]
-    __shared__ T s_S[EPB][SS];     // [element][gp * 9 + 3 i + j]
-    __shared__ T s_dN[NGP][SD];    // [gp][node * 3 + k]
-    __shared__ int s_node[EPB][SN];
+    T u[EPB][(NEN * 3) | 1];   // [element][node * 3 + component]
+    T S[EPB][(NGP * 9) | 1];   // [element][gp * 9 + 3 i + j]
+    T dN[NGP][(NEN * 3) | 1];  // [gp][node * 3 + k]
+    int node[EPB][NEN | 1];
+};
+
+// MT: the block's one material law, or -1 when its elements mix laws.  The
+// first n_face_tiles CTAs take the pressure faces of the block's kind.
+template <int NEN, int NGP, typename T, int BLK, int MT>
+__global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a, FaceArgs<T> fa, int n_face_tiles)
+{
+    griddep_wait();
+    constexpr int EPB = elems_per_cta<NGP, BLK>();
+    __shared__ union Smem {
+        ElemSmem<NEN, NGP, T, EPB> e;
+        FaceSmem<NEN, T, face_epb<NEN, BLK>()> f;
+        __device__ Smem() {}
+    } smem;
+    if (static_cast<int>(blockIdx.x) < n_face_tiles) {
+        face_tile<NEN, T, BLK>(fa, blockIdx.x, smem.f);
+        griddep_launch();
+        return;
+    }
+    auto& s_u = smem.e.u;
+    auto& s_S = smem.e.S;
+    auto& s_dN = smem.e.dN;
+    auto& s_node = smem.e.node;
 
     const int tid = threadIdx.x;
-    const int e0 = blockIdx.x * EPB;
+    const int e0 = (static_cast<int>(blockIdx.x) - n_face_tiles) * EPB;
     if (a.frozen) {  // a batch union: skip the CTA when every member it covers has stopped iterating
         const int e1 = min(a.n, e0 + EPB) - 1;
         bool act = false;
@@ -196,115 +391,6 @@ __global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a)
     griddep_launch();
 }
 
-template <typename T>
-struct FaceArgs {
-    int n, n_free;
-    const int* __restrict__ conn;     // [NEN][n]
-    const int* __restrict__ table;    // [n]
-    const double* __restrict__ A0;    // [n][3]
-    const T* __restrict__ J0inv;      // [n][MAX_FGP][9]
-    const double* __restrict__ load;  // [n][4]
-    const int* __restrict__ t_ngp;
-    const T* __restrict__ t_w;        // [t][MAX_FGP]
-    const T* __restrict__ t_N;        // [t][MAX_FGP][NEN]
-    const T* __restrict__ t_dN;       // [t][MAX_FGP][NEN][3]
-    const double* __restrict__ u;
-    double* __restrict__ r;
-    double* __restrict__ contrib;     // deterministic scatter: [3][n_slots], or null for atomics
-    size_t n_slots, slot0;
-};
-
-// One thread per face: cof(F_g) A0 at every face point, then the nodal forces
-// of all element nodes.
-template <int NEN, typename T>
-__global__ void __launch_bounds__(kBlock) k_face_residual(FaceArgs<T> a)
-{
-    griddep_wait();
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= a.n) return;
-    const int t = a.table[f];
-    const int ngp = a.t_ngp[t];
-    int node[NEN];
-    T uu[NEN][3];
-    double u0[3] = { 0.0, 0.0, 0.0 };  // displacements relative to the parent's first node, as in the element kernel
-    {
-        const int n0 = a.conn[f];
-        if (n0 < a.n_free)
-            for (int c = 0; c < 3; c++) u0[c] = a.u[3 * n0 + c];
-    }
-#pragma unroll
-    for (int q = 0; q < NEN; q++) {
-        node[q] = a.conn[static_cast<size_t>(q) * a.n + f];
-        const bool fr = node[q] < a.n_free;
-        uu[q][0] = static_cast<T>((fr ? a.u[3 * node[q]] : 0.0) - u0[0]);
-        uu[q][1] = static_cast<T>((fr ? a.u[3 * node[q] + 1] : 0.0) - u0[1]);
-        uu[q][2] = static_cast<T>((fr ? a.u[3 * node[q] + 2] : 0.0) - u0[2]);
-    }
-    const T A0[3] = { static_cast<T>(a.A0[3 * f]), static_cast<T>(a.A0[3 * f + 1]), static_cast<T>(a.A0[3 * f + 2]) };
-    const bool directed = a.load[4 * f] != 0.0;
-    T cA[MAX_FGP][3];
-    for (int g = 0; g < ngp; g++) {
-        const T* dN = a.t_dN + (static_cast<size_t>(t) * MAX_FGP + g) * NEN * 3;
-        T A[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
-        for (int q = 0; q < NEN; q++)
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int k = 0; k < 3; k++) A[3 * i + k] += uu[q][i] * dN[3 * q + k];
-        const T* Ji = a.J0inv + (static_cast<size_t>(f) * MAX_FGP + g) * 9;
-        T H[9];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) H[3 * i + j] = A[3 * i] * Ji[j] + A[3 * i + 1] * Ji[3 + j] + A[3 * i + 2] * Ji[6 + j];
-        Kin<T> k;
-        kinematics(H, k);
-        // cof F A0 = (I + B) A0
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-            cA[g][i] = A0[i] + k.B[3 * i] * A0[0] + k.B[3 * i + 1] * A0[1] + k.B[3 * i + 2] * A0[2];
-        if (directed) {
-            const T nrm = sqrt(cA[g][0] * cA[g][0] + cA[g][1] * cA[g][1] + cA[g][2] * cA[g][2]);
-            cA[g][0] = nrm;
-        }
-    }
-    const double* L = a.load + 4 * f;
-    for (int q = 0; q < NEN; q++) {
-        if (node[q] >= a.n_free) continue;
-        T v0 = 0, v1 = 0, v2 = 0;
-        for (int g = 0; g < ngp; g++) {
-            const T wn = a.t_w[t * MAX_FGP + g] * a.t_N[(static_cast<size_t>(t) * MAX_FGP + g) * NEN + q];
-            if (directed) {
-                v0 += wn * cA[g][0];
-            } else {
-                v0 += wn * cA[g][0];
-                v1 += wn * cA[g][1];
-                v2 += wn * cA[g][2];
-            }
-        }
-        double f0, f1, f2;
-        if (directed) {
-            f0 = L[1] * static_cast<double>(v0);
-            f1 = L[2] * static_cast<double>(v0);
-            f2 = L[3] * static_cast<double>(v0);
-        } else {
-            f0 = L[1] * static_cast<double>(v0);
-            f1 = L[1] * static_cast<double>(v1);
-            f2 = L[1] * static_cast<double>(v2);
-        }
-        if (a.contrib) {
-            const size_t sl = a.slot0 + static_cast<size_t>(q) * a.n + f;
-            a.contrib[sl] = -f0;
-            a.contrib[a.n_slots + sl] = -f1;
-            a.contrib[2 * a.n_slots + sl] = -f2;
-        } else {
-            atomicAdd(a.r + 3 * node[q], -f0);
-            atomicAdd(a.r + 3 * node[q] + 1, -f1);
-            atomicAdd(a.r + 3 * node[q] + 2, -f2);
-        }
-    }
-}
-
 // Deterministic scatter, second half: free node i adds its contributions in
 // ascending slot order, r_i += sum_k contrib[gidx[k]], one thread per node
 __global__ void __launch_bounds__(kBlock) k_gather(int n_free, const int* __restrict__ gptr,
@@ -326,38 +412,40 @@ __global__ void __launch_bounds__(kBlock) k_gather(int n_free, const int* __rest
 }
 
 template <int NEN, int NGP, typename T, int BLK>
-void launch_elem_blk(const ElemArgs<T>& a, int mt, cudaStream_t st)
+void launch_elem_blk(const ElemArgs<T>& a, const FaceArgs<T>& fa, int mt, cudaStream_t st)
 {
-    constexpr int EPB = elems_per_cta<NGP, BLK>();
-    const int grid = (a.n + EPB - 1) / EPB;
+    constexpr int EPB = elems_per_cta<NGP, BLK>(), FPB = face_epb<NEN, BLK>();
+    const int ft = (fa.n + FPB - 1) / FPB, grid = ft + (a.n + EPB - 1) / EPB;
     switch (mt) {
-    case EFEM_NEO_HOOKEAN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_NEO_HOOKEAN>, grid, BLK, 0, st, a); break;
-    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_MOONEY_RIVLIN>, grid, BLK, 0, st, a); break;
-    case EFEM_YEOH: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_YEOH>, grid, BLK, 0, st, a); break;
-    default: launch_k(k_elem_residual<NEN, NGP, T, BLK, -1>, grid, BLK, 0, st, a); break;
+    case EFEM_NEO_HOOKEAN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_NEO_HOOKEAN>, grid, BLK, 0, st, a, fa, ft); break;
+    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_MOONEY_RIVLIN>, grid, BLK, 0, st, a, fa, ft); break;
+    case EFEM_YEOH: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_YEOH>, grid, BLK, 0, st, a, fa, ft); break;
+    default: launch_k(k_elem_residual<NEN, NGP, T, BLK, -1>, grid, BLK, 0, st, a, fa, ft); break;
     }
 }
 
 template <int NEN, int NGP, typename T>
 void launch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, const T* J0, const T* dN, const T* gw,
-    int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc, const int* frozen)
+    int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc, const int* frozen,
+    const FaceArgs<T>& fa)
 {
     ElemArgs<T> a { b.n, n_free, b.conn, b.mat, vol, J0, dN, gw, mats, u, r, sc.contrib, sc.n_slots, sc.slot0,
         b.egroup, b.egroup ? frozen : nullptr };
-    if (threads == 64) launch_elem_blk<NEN, NGP, T, 64>(a, b.mat_type, st);
-    else if (threads == 256) launch_elem_blk<NEN, NGP, T, 256>(a, b.mat_type, st);
-    else launch_elem_blk<NEN, NGP, T, 128>(a, b.mat_type, st);
+    if (threads == 64) launch_elem_blk<NEN, NGP, T, 64>(a, fa, b.mat_type, st);
+    else if (threads == 256) launch_elem_blk<NEN, NGP, T, 256>(a, fa, b.mat_type, st);
+    else launch_elem_blk<NEN, NGP, T, 128>(a, fa, b.mat_type, st);
 }
 
+// the element forces of block b and, with fa.n > 0, the pressure faces of its kind
 template <typename T>
 void dispatch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, const T* J0, const T* dN, const T* gw,
     int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc = Scatter(),
-    const int* frozen = nullptr)
+    const int* frozen = nullptr, const FaceArgs<T>& fa = FaceArgs<T> {})
 {
-#define CASE(NEN, NGP)                                                                             \
-    if (b.nen == NEN && b.ngp == NGP) {                                                            \
-        launch_elem<NEN, NGP, T>(b, mats, vol, J0, dN, gw, n_free, u, r, st, threads, sc, frozen); \
-        return;                                                                                    \
+#define CASE(NEN, NGP)                                                                                 \
+    if (b.nen == NEN && b.ngp == NGP) {                                                                \
+        launch_elem<NEN, NGP, T>(b, mats, vol, J0, dN, gw, n_free, u, r, st, threads, sc, frozen, fa); \
+        return;                                                                                        \
     }
     CASE(4, 1)
     CASE(10, 4)
@@ -370,18 +458,33 @@ void dispatch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, co
 }
 
 template <typename T>
-void dispatch_face(const DevFaces& f, const T* J0, const T* tw, const T* tN, const T* tdN, int n_free, const double* u,
-    double* r, cudaStream_t st, const Scatter& sc)
+FaceArgs<T> face_args(const DevFaces& f, const T* J0, const T* tw, const T* tN, const T* tdN, int n_free,
+    const double* u, double* r, const Scatter& sc)
 {
-    FaceArgs<T> a { f.n, n_free, f.conn, f.table, f.A0, J0, f.load, f.t_ngp, tw, tN, tdN, u, r, sc.contrib, sc.n_slots,
-        sc.slot0 };
-    const int grid = (f.n + kBlock - 1) / kBlock;
-    switch (f.nen) {
-    case 4: launch_k(k_face_residual<4, T>, grid, kBlock, 0, st, a); break;
-    case 8: launch_k(k_face_residual<8, T>, grid, kBlock, 0, st, a); break;
-    case 10: launch_k(k_face_residual<10, T>, grid, kBlock, 0, st, a); break;
-    case 20: launch_k(k_face_residual<20, T>, grid, kBlock, 0, st, a); break;
+    const int gmax = *std::max_element(f.h_ngp.begin(), f.h_ngp.end());
+    return FaceArgs<T> { f.n, n_free, gmax, f.conn, f.table, f.A0, J0, f.load, f.t_ngp, tw, tN, tdN, u, r, sc.contrib,
+        sc.n_slots, sc.slot0 };
+}
+
+template <typename T>
+void dispatch_face(int nen, const FaceArgs<T>& a, cudaStream_t st)
+{
+    auto grid_of = [&](int epb) { return (a.n + epb - 1) / epb; };
+    switch (nen) {
+    case 4: launch_k(k_face_residual<4, T>, grid_of(face_epb<4, kBlock>()), kBlock, 0, st, a); break;
+    case 8: launch_k(k_face_residual<8, T>, grid_of(face_epb<8, kBlock>()), kBlock, 0, st, a); break;
+    case 10: launch_k(k_face_residual<10, T>, grid_of(face_epb<10, kBlock>()), kBlock, 0, st, a); break;
+    case 20: launch_k(k_face_residual<20, T>, grid_of(face_epb<20, kBlock>()), kBlock, 0, st, a); break;
     }
+}
+
+// The element block whose launch carries face set f: the first one with
+// elements of the same kind (-1: none, all of that kind lack a material)
+int block_of_faces(const Model& m, const DevFaces& f)
+{
+    for (size_t b = 0; b < m.blocks.size(); b++)
+        if (m.blocks[b].n > 0 && m.blocks[b].nen == f.nen) return static_cast<int>(b);
+    return -1;
 }
 
 }  // namespace
@@ -441,6 +544,15 @@ efem_status tune_element_blocks(Model& m)
     return EFEM_OK;
 }
 
+// kernels of one residual evaluation
+int residual_launches(const Model& m)
+{
+    int n = 1 + (m.opts.deterministic ? 1 : 0);
+    for (auto& b : m.blocks) n += b.n > 0;
+    for (auto& f : m.faces) n += f.n > 0 && block_of_faces(m, f) < 0;
+    return n;
+}
+
 efem_status launch_residual(Model& m, const double* d_u, double* d_r)
 {
     return launch_residual_on(m, d_u, d_r, m.stream);
@@ -463,27 +575,38 @@ efem_status launch_residual_on(Model& m, const double* d_u, double* d_r, cudaStr
         set_error("deterministic scatter requested but its tables are not built");
         return EFEM_ERR_ARG;
     }
-    for (auto& b : m.blocks) {
+    auto faces_of = [&](const DevFaces& f, auto tag) {
+        using T = decltype(tag);
+        Scatter sc;
+        if (det) sc = Scatter { m.d_contrib, m.n_slots, f.slot0 };
+        if constexpr (sizeof(T) == 4)
+            return face_args<float>(f, f.J0inv_f, f.t_w_f, f.t_N_f, f.t_dN_f, m.n_free, d_u, d_r, sc);
+        else
+            return face_args<double>(f, f.J0inv, f.t_w, f.t_N, f.t_dN, m.n_free, d_u, d_r, sc);
+    };
+    for (size_t bi = 0; bi < m.blocks.size(); bi++) {
+        const DevBlock& b = m.blocks[bi];
         if (b.n == 0) continue;
         m.launches++;
         Scatter sc;
         if (det) sc = Scatter { m.d_contrib, m.n_slots, b.slot0 };
+        const DevFaces* with = nullptr;
+        for (auto& f : m.faces)
+            if (f.n > 0 && block_of_faces(m, f) == static_cast<int>(bi)) with = &f;
         if (mixed)
             dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, d_u, d_r, stream,
-                b.threads[1], sc, m.d_frozen_groups);
+                b.threads[1], sc, m.d_frozen_groups, with ? faces_of(*with, 0.0f) : FaceArgs<float> {});
         else
             dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, d_u, d_r, stream, b.threads[0], sc,
-                m.d_frozen_groups);
+                m.d_frozen_groups, with ? faces_of(*with, 0.0) : FaceArgs<double> {});
     }
     for (auto& f : m.faces) {
-        if (f.n == 0) continue;
+        if (f.n == 0 || block_of_faces(m, f) >= 0) continue;
         m.launches++;
-        Scatter sc;
-        if (det) sc = Scatter { m.d_contrib, m.n_slots, f.slot0 };
         if (mixed)
-            dispatch_face<float>(f, f.J0inv_f, f.t_w_f, f.t_N_f, f.t_dN_f, m.n_free, d_u, d_r, stream, sc);
+            dispatch_face<float>(f.nen, faces_of(f, 0.0f), stream);
         else
-            dispatch_face<double>(f, f.J0inv, f.t_w, f.t_N, f.t_dN, m.n_free, d_u, d_r, stream, sc);
+            dispatch_face<double>(f.nen, faces_of(f, 0.0), stream);
     }
     if (det) {
         launch_k(k_gather, (m.n_free + kBlock - 1) / kBlock, kBlock, 0, stream, m.n_free, m.d_gptr, m.d_gidx,

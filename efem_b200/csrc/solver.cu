@@ -1125,7 +1125,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
     const double eps = m.opts.residual_criterion;
     std::memset(info, 0, sizeof(*info));
     const long long launches0 = m.launches;
-    const long long per_res = 1 + static_cast<long long>(m.blocks.size() + m.faces.size()) + (m.opts.deterministic ? 1 : 0);
+    const long long per_res = residual_launches(m);
     double ms_pc = 0.0;
     double rinf = 0.0, xinf = 0.0;
     int k = 1;
