@@ -11,16 +11,12 @@
 //   k_extend_add  one CTA per front: add the children's update blocks through
 //                 the precomputed relative indices, children in a fixed order
 //                 (the factor is bitwise repeatable);
-//   per 32-column panel step of the level's fronts:
-//   k_panel       per front and chunk of rows: Cholesky of the 32x32
-//                 diagonal block in shared memory (one warp), then the
-//                 panel TRSM on the chunk's rows; k_panel_store then writes
-//                 the factored diagonal blocks into the fronts;
-//   k_syrk        one CTA per 64x64 tile of every front's trailing lower
-//                 triangle: register-blocked rank-32 update.
-//   k_diag_inv, k_offdiag_inv, k_w  X = L_JJ^{-1} and W = L_RJ X of every
-//                 front, stored as one column-major matrix M = [X; W], so the
-//                 solves are matrix-vector products.
+//   k_diag, k_step  the inverse of the first 32 x 32 diagonal block's factor;
+//                 then per 32-column step the panel, the update of the
+//                 trailing triangle and the next block's inverse;
+//   k_inverse     X = L_JJ^{-1} by doubling;
+//   k_w           W = L_RJ X.  [X; W] is stored as one column-major matrix M
+//                 per front, so the solves are matrix-vector products.
 //
 // Solve H0 v (3 right-hand sides interleaved per node): one persistent launch,
 // k_solve below.  Every sum is formed in a fixed order (no atomics): results
@@ -42,9 +38,9 @@ namespace efem {
 namespace {
 constexpr int kFT = 256;  // factor threads
 constexpr int kNB = 32;   // factor panel width
-constexpr int kTS = 64;   // SYRK tile
+constexpr int kTS = 64;   // update tile
+constexpr int kInvBatch = 8;  // steps between the inverse's launches
 constexpr int kST = 256;  // solve threads
-constexpr int kRT = 32;   // columns per CTA of the inverse / transpose kernels
 
 // one work item of the persistent triangular solve: a tile of a front, with
 // all that a CTA has to know of the front, so that one load starts its work
@@ -53,11 +49,6 @@ struct alignas(16) SolveItem {
     int parent, r, c, f0;   // the front's parent, rows, columns, first column
     int nk, target, ptarget, pad;  // children; counts to wait for: own (children's updates, or own y), parent's x
     long long xw, rows, slot, upd; // offsets of M, of the row list, of the slot table, of the update vector
-};
-
-struct Tile {
-    int s;    // front
-    int off;  // first row / column of the tile (multiple of kRT)
 };
 
 // a subtree solved by one CTA (see k_sub_fwd) and its chunks of factor rows
@@ -101,29 +92,30 @@ struct Precond {
     SubTree* d_subs = nullptr;
     SubChunk* d_chunks = nullptr;
     int *d_depth = nullptr, *d_xidx = nullptr;
-    // factor schedule: per (level, step) the fronts with a panel at that step and the SYRK tiles
+    // factor schedule: per level the tiles of every 32-column step, and of the
+    // products of the inverse's doublings (block size h) that follow step `after`
     struct Step {
-        int level, k0, panel_off, panel_cnt, syrk_off, syrk_cnt, panel_chunks;
+        int k0, off, cnt;
+    };
+    struct Inv {
+        int after, h, second, off, cnt;
     };
     std::vector<Step> steps;
-    std::vector<int> lev_first_step;  // index into steps, nlev + 1
-    int n_inv_tiles = 0;
-    int *d_first = nullptr, *d_ncol = nullptr, *d_nrow = nullptr, *d_rows = nullptr, *d_child_ptr = nullptr,
-        *d_child_list = nullptr, *d_relind = nullptr, *d_level_list = nullptr, *d_perm = nullptr, *d_fail = nullptr,
-        *d_panel_list = nullptr;
-    long long *d_front_off = nullptr, *d_rows_off = nullptr, *d_relind_off = nullptr, *d_xw_off = nullptr,
+    std::vector<Inv> invs;
+    std::vector<int> lev_first_step, lev_first_inv;  // indices into steps and invs, nlev + 1
+    int *d_first = nullptr, *d_ncol = nullptr, *d_nrow = nullptr, *d_child_ptr = nullptr,
+        *d_child_list = nullptr, *d_relind = nullptr, *d_level_list = nullptr, *d_perm = nullptr, *d_fail = nullptr;
+    long long *d_slot_off = nullptr, *d_front_off = nullptr, *d_rows_off = nullptr, *d_relind_off = nullptr, *d_xw_off = nullptr,
               *d_upd_off = nullptr, *d_a_pos = nullptr, *d_a_src = nullptr;
-    Tile* d_inv = nullptr;
-    int *d_contrib_ptr = nullptr, *d_contrib_idx = nullptr, *d_below_front = nullptr;
-    Tile *d_ea = nullptr, *d_oinv = nullptr;  // extend-add column tiles, off-diagonal inverse column groups
-    std::vector<int> ea_off;                  // nlev + 1
-    int n_oinv = 0;
-    double* d_xw = nullptr;                   // every front's M = [X; W]
+    int4* d_ea = nullptr;     // extend-add tiles (front, first row, first column)
+    longlong2* d_zero = nullptr;  // spans of the fronts' own columns
+    int n_zero = 0;
+    std::vector<int> ea_off;  // nlev + 1
+    double *d_xw = nullptr, *d_lp = nullptr;  // every front's M = [X; W], and its panels of L
     int4* d_wtiles = nullptr;  // (front, 64-row tile, 64-column tile) of every W
-    int n_wtiles = 0;
-    int4* d_syrk = nullptr;
-    double* d_diag_tmp = nullptr;  // factored diagonal blocks of one panel step, [fronts in step][kNB][kNB]
-    int max_panel_cnt = 0;
+    std::vector<int> w_off;    // nlev + 1
+    int4 *d_steps = nullptr, *d_invs = nullptr;  // tiles of k_step and k_inverse
+    cudaStream_t capture2 = nullptr;  // second branch of the factorisation's graph
     int* h_flag = nullptr;  // pinned: the error flag read back after an application
     double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
            *d_vals = nullptr;
@@ -138,12 +130,13 @@ struct Precond {
 namespace {
 
 struct FrontArgs {
-    const int *first, *ncol, *nrow, *rows, *child_ptr, *child_list, *relind, *level_list, *contrib_ptr, *contrib_idx,
-        *below_front;
-    const long long *front_off, *rows_off, *relind_off, *xw_off, *upd_off;
+    const int *first, *ncol, *nrow, *child_ptr, *child_list, *relind;
+    const int* slot;  // per front, child q, row t (slot_off[s] + q r + t): the update entry of that child landing on the row, or -1
+    const long long *front_off, *rows_off, *relind_off, *xw_off, *upd_off, *slot_off;
     double* front;
     double* xw;  // per front M = [X; W], X = L_JJ^{-1} (c x c, zeros above the diagonal), W = L_RJ X ((r - c) x c):
                  // r x c column-major, leading dimension ld_of(r)
+    double* lp;  // the panels L below the 32 x 32 diagonal blocks, laid out as M
     int* fail;
 };
 
@@ -160,282 +153,389 @@ __global__ void k_scatter_a(double* __restrict__ front, const long long* __restr
         front[pos[k]] = vals[src[k]];
 }
 
-// Children's update blocks into the fronts of one level, one warp per front
-// column p (8 per CTA): the contributions landing on column p are added in
-// child order, each one a column j of a child's update block whose rows
-// i >= j go to the parent rows relind[i].  No two warps touch the same entry,
-// so the sums need no atomics and are bitwise repeatable.
-__global__ void __launch_bounds__(kFT) k_extend_add(FrontArgs a, const Tile* __restrict__ tiles)
+// zeros in the fronts' own columns (the trailing parts are written before they
+// are read); span = first double, count
+__global__ void __launch_bounds__(kFT) k_zero(double* __restrict__ front, const longlong2* __restrict__ spans)
 {
-    const Tile tl = tiles[blockIdx.x];
-    const int s = tl.s;
-    const int p = tl.off + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int r = a.nrow[s];
-    if (p >= r) return;
-    double* Fp = a.front + a.front_off[s] + static_cast<long long>(p) * r;
-    const long long row = a.rows_off[s] + p;
-    for (int q = a.contrib_ptr[row]; q < a.contrib_ptr[row + 1]; q++) {
-        const int idx = a.contrib_idx[q];
-        const int ch = a.below_front[idx];
-        const int j = idx - static_cast<int>(a.upd_off[ch] / 3);
-        const int rc = a.nrow[ch], cc = a.ncol[ch], m = rc - cc;
-        const int* ri = a.relind + a.relind_off[ch];
-        const double* U = a.front + a.front_off[ch] + static_cast<long long>(cc + j) * rc + cc;
-        for (int i = j + lane; i < m; i += 32) Fp[ri[i]] += U[i];
-        __syncwarp();
-    }
+    const longlong2 sp = spans[blockIdx.x];
+    for (long long i = threadIdx.x; i < sp.y; i += kFT) front[sp.x + i] = 0.0;
 }
 
-// Diagonal block and panel of step k0 for the fronts in the step's list.
-// Grid (fronts, row chunks): every CTA factors the panel's kb x kb diagonal
-// block (one warp, left-looking, with the reciprocals of the pivots so that
-// no division sits on a dependent chain; every CTA computes the same block,
-// so the factor does not depend on the grid) and solves up to kFT of the rows
-// below it, one per thread.  Chunk 0 leaves the factored block in tmp, and
-// k_panel_store copies it into the front afterwards: written in place, it
-// could reach a chunk CTA of a later wave before that CTA has read the
-// unfactored block.
-__global__ void __launch_bounds__(kFT) k_panel(FrontArgs a, const int* __restrict__ list, int k0,
-    double* __restrict__ tmp)
-{
-    const int s = list[blockIdx.x];
-    const int r = a.nrow[s], c = a.ncol[s];
-    const int kb = min(kNB, c - k0);
-    const int row0 = k0 + kb + static_cast<int>(blockIdx.y) * kFT;
-    if (blockIdx.y > 0 && row0 >= r) return;  // uniform over the CTA
-    double* F = a.front + a.front_off[s];
-    const int tid = threadIdx.x;
-    __shared__ double D[kNB][kNB + 1];
-    __shared__ double Dinv[kNB];  // 1 / L_jj: the divisions leave the dependent chains
-    for (int idx = tid; idx < kb * kb; idx += kFT) {
-        const int i = idx % kb, j = idx / kb;
-        D[i][j] = (i >= j) ? F[(k0 + i) + static_cast<long long>(k0 + j) * r] : 0.0;
-    }
-    __syncthreads();
-    if (tid < 32) {
-        const int i = tid;
-        for (int j = 0; j < kb; j++) {
-            if (i == j) {
-                double d = D[j][j];
-                for (int k = 0; k < j; k++) d -= D[j][k] * D[j][k];
-                if (!(d > 0.0)) {
-                    if (blockIdx.y == 0) *a.fail = 1;
-                    d = 1.0;
-                }
-                const double sd = sqrt(d);
-                D[j][j] = sd;
-                Dinv[j] = 1.0 / sd;
-            }
-            __syncwarp();
-            if (i > j && i < kb) {
-                double t = D[i][j];
-                for (int k = 0; k < j; k++) t -= D[i][k] * D[j][k];
-                D[i][j] = t * Dinv[j];
-            }
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    if (blockIdx.y == 0)
-        for (int idx = tid; idx < kb * kb; idx += kFT) {
-            const int i = idx % kb, j = idx / kb;
-            if (i >= j) tmp[static_cast<size_t>(blockIdx.x) * kNB * kNB + idx] = D[i][j];
-        }
-    // rows below the block: x L^T = f
-    for (int i = row0 + tid; i < min(r, row0 + kFT); i += kFT) {
-        double x[kNB];
-#pragma unroll
-        for (int j = 0; j < kNB; j++) x[j] = j < kb ? F[i + static_cast<long long>(k0 + j) * r] : 0.0;
-#pragma unroll
-        for (int j = 0; j < kNB; j++) {
-            if (j < kb) {
-                double sum = x[j];
-#pragma unroll
-                for (int k = 0; k < kNB; k++)
-                    if (k < j) sum -= x[k] * D[j][k];
-                x[j] = sum * Dinv[j];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kNB; j++)
-            if (j < kb) F[i + static_cast<long long>(k0 + j) * r] = x[j];
-    }
-}
-
-// the factored diagonal blocks of a panel step, from k_panel's tmp into the fronts
-__global__ void __launch_bounds__(kFT) k_panel_store(FrontArgs a, const int* __restrict__ list, int k0,
-    const double* __restrict__ tmp)
-{
-    const int s = list[blockIdx.x];
-    const int r = a.nrow[s], c = a.ncol[s];
-    const int kb = min(kNB, c - k0);
-    double* F = a.front + a.front_off[s];
-    for (int idx = threadIdx.x; idx < kb * kb; idx += kFT) {
-        const int i = idx % kb, j = idx / kb;
-        if (i >= j) F[(k0 + i) + static_cast<long long>(k0 + j) * r] = tmp[static_cast<size_t>(blockIdx.x) * kNB * kNB + idx];
-    }
-}
-
-// trailing lower triangle -= P P^T for one 64x64 tile; tile = (front, ti, tj)
-__global__ void __launch_bounds__(kFT) k_syrk(FrontArgs a, const int4* __restrict__ tiles, int k0)
+// Children's update blocks into the fronts of one level: one CTA per 64 rows x
+// 32 columns of a front's lower triangle, every entry the sum over the
+// children in order (no atomics: the factor is bitwise repeatable), read
+// through the slot tables of the solve's assembly (entry of child q landing on
+// row t, or -1).  Own columns hold L's entries and are added to; the trailing
+// part is written, so nothing has to clear it.  Bound by memory once the
+// chain slots -> children's entries is short: 12-47 us per level of the cap,
+// with 165 MB cleared beforehand (own columns) instead of 836; one warp per
+// column following the children's index lists took 32-48 us and needed all of
+// the front cleared.
+constexpr int kER = 64, kEC = 32;
+__global__ void __launch_bounds__(kFT) k_extend_add(FrontArgs a, const int4* __restrict__ tiles)
 {
     const int4 tl = tiles[blockIdx.x];
-    const int s = tl.x, ti = tl.y, tj = tl.z;
-    const int r = a.nrow[s], c = a.ncol[s];
-    const int kb = min(kNB, c - k0);
-    const int base = k0 + kb;
+    const int s = tl.x, p0 = tl.y, q0 = tl.z;  // first row, first column
+    const int r = a.nrow[s], c = a.ncol[s], k1 = a.child_ptr[s], k2 = a.child_ptr[s + 1];
+    const int i = p0 + (threadIdx.x & (kER - 1)), jl = threadIdx.x >> 6;  // columns jl + 4 e
     double* F = a.front + a.front_off[s];
-    const int tid = threadIdx.x;
-    __shared__ double Pi[kTS][kNB + 1];
-    __shared__ double Pj[kTS][kNB + 1];
-    for (int idx = tid; idx < kTS * kNB; idx += kFT) {
-        const int p = idx % kTS, k = idx / kTS;
-        const int gi = base + ti * kTS + p, gj = base + tj * kTS + p;
-        Pi[p][k] = (k < kb && gi < r) ? F[gi + static_cast<long long>(k0 + k) * r] : 0.0;
-        Pj[p][k] = (k < kb && gj < r) ? F[gj + static_cast<long long>(k0 + k) * r] : 0.0;
+    griddep_wait();
+    griddep_launch();
+    double sum[kEC / 4];
+#pragma unroll
+    for (int e = 0; e < kEC / 4; e++) {
+        const int j = q0 + jl + 4 * e;
+        sum[e] = i < r && j < c && i >= j ? F[i + static_cast<long long>(j) * r] : 0.0;
     }
-    __syncthreads();
-    const int a0 = (tid % 16) * 4, b0 = (tid / 16) * 4;
+    for (int k = k1; k < k2; k++) {
+        const int ch = a.child_list[k], rc = a.nrow[ch], cc = a.ncol[ch];
+        const int* sl = a.slot + a.slot_off[s] + static_cast<long long>(k - k1) * r;
+        const int b0 = static_cast<int>(a.upd_off[ch] / 3);
+        const int si = i < r ? sl[i] : -1;
+        const double* U = a.front + a.front_off[ch] + static_cast<long long>(cc) * rc + cc;
+#pragma unroll
+        for (int e = 0; e < kEC / 4; e++) {
+            const int j = q0 + jl + 4 * e;
+            const int sj = j <= i && j < r ? sl[j] : -1;
+            if (si >= 0 && sj >= 0) sum[e] += U[static_cast<long long>(sj - b0) * rc + si - b0];
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < kEC / 4; e++) {
+        const int j = q0 + jl + 4 * e;
+        if (i < r && j <= i) F[i + static_cast<long long>(j) * r] = sum[e];
+    }
+}
+
+// ---- the 32-column steps of a level's fronts
+//
+// k_step, one launch per step k0: update tiles (ti, tj) form L = A X_kk^T on
+// their two 64-row blocks of the step's columns -- a product with the inverse
+// of the factored diagonal block, no substitution -- and subtract L_i L_j^T
+// from their 64 x 64 tile of the trailing lower triangle.  The first tile of a
+// row block keeps its L in the panel array; the front itself is only read in
+// the step's columns, so no CTA can overtake another.  The tile that holds the
+// next diagonal block then factors it and leaves its inverse for the next step
+// (k_diag does so for the first), so the 32 pivots are done once per front and
+// no launch waits for them alone.
+//
+// What bounds it: the chain of one step (load, product, update, 32 pivots of
+// about 200 cycles) times the steps on the way to the root.  As three kernels,
+// with a one-warp left-looking 32 x 32 Cholesky and one substitution per row, a
+// step took 34 + 4 + 20 us (cold), now 13-20 us on the upper levels.  Whole
+// factorisations: C3D8 beam 3.87 -> 1.37 ms, C3D20R cap 9.8 -> 3.85 ms, C3D10
+// finger 10.4 -> 4.3 ms.  Every CTA repeating the block's elimination instead
+// of taking the inverse from the step before: cap 4.6 ms; four pivots per
+// exchange, for fewer barriers: slower (360 cycles per pivot).
+constexpr int kStoreL = 1, kNextDiag = 2;        // tile.w
+constexpr int kPS = kNB + 1, kXS = kNB + 2;      // shared-memory strides
+
+__device__ __forceinline__ void cp8z(double* dst, const double* src, bool on)
+{
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(on ? 8 : 0) : "memory");
+}
+
+// The inverse of the Cholesky factor of a kb x kb block (lower triangle in A:
+// lane = row, columns w + 8 q of warp w; the identity past kb) into M.  The row
+// operations that take the block to D^{1/2} L^T take the identity to L^{-1}, up
+// to the rows' scaling.  The pivot column and the pivot row of X pass through
+// shared memory; unrolled in full (200 cycles per pivot, 310 as a loop; one warp
+// with the block in its registers needs 200 for the factor alone).
+struct DiagSmem {
+    double col[2][kNB], xrow[2][kNB];
+};
+__device__ __forceinline__ void diag_inverse(double (&A)[4], int kb, double* M, long long ld, int* fail, DiagSmem& sm)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double X[4], dl = 1.0;
+    bool bad = false;
+#pragma unroll
+    for (int q = 0; q < 4; q++) X[q] = lane == w + 8 * q ? 1.0 : 0.0;
+#pragma unroll
+    for (int j = 0; j < kNB; j++) {
+        const int jq = j >> 3, p = j & 1;
+        if (w == (j & 7)) sm.col[p][lane] = A[jq];
+        if (lane == j) {
+#pragma unroll
+            for (int q = 0; q <= jq; q++) sm.xrow[p][w + 8 * q] = X[q];
+        }
+        __syncthreads();
+        double d = sm.col[p][j];
+        if (!(d > 0.0)) {
+            bad = true;
+            d = 1.0;
+        }
+        const double f = lane > j ? sm.col[p][lane] * __drcp_rn(d) : 0.0;
+        if (lane == j) dl = d;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (q >= jq) A[q] -= f * sm.col[p][w + 8 * q];
+            if (q <= jq) X[q] -= f * sm.xrow[p][w + 8 * q];
+        }
+    }
+    if (bad && threadIdx.x == 0) *fail = 1;
+    const double sc = 1.0 / sqrt(dl);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (lane < kb && w + 8 * q < kb) M[(w + 8 * q) * ld + lane] = X[q] * sc;
+}
+
+// the first diagonal block of every front of a level
+__global__ void __launch_bounds__(kFT) k_diag(FrontArgs a, const int* __restrict__ list)
+{
+    __shared__ DiagSmem sm;
+    const int s = list[blockIdx.x], r = a.nrow[s], kb = min(kNB, a.ncol[s]);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double* F = a.front + a.front_off[s];
+    double* M = a.xw + a.xw_off[s];
+    griddep_wait();
+    griddep_launch();
+    double A[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int cc = w + 8 * q;
+        A[q] = lane < kb && cc < kb ? (lane >= cc ? F[lane + static_cast<long long>(cc) * r] : 0.0) : (lane == cc ? 1.0 : 0.0);
+    }
+    diag_inverse(A, kb, M, ld_of(r), a.fail, sm);
+}
+
+// Rows [0, 64) of a panel (in P, row stride kPS) times X_kk^T: rows lane and
+// lane + 32, columns 4 w + q (X_kk lower triangular: k <= 4 w + 3)
+__device__ __forceinline__ void panel_times(const double* P, const double* XT, double (&o)[2][4])
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 4; q++) o[0][q] = o[1][q] = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < 4 * w + 4; k++) {
+        const double p0 = P[lane * kPS + k], p1 = P[(lane + 32) * kPS + k];
+        const double2 xa = *reinterpret_cast<const double2*>(XT + k * kXS + 4 * w);
+        const double2 xb = *reinterpret_cast<const double2*>(XT + k * kXS + 4 * w + 2);
+        o[0][0] += p0 * xa.x;
+        o[0][1] += p0 * xa.y;
+        o[0][2] += p0 * xb.x;
+        o[0][3] += p0 * xb.y;
+        o[1][0] += p1 * xa.x;
+        o[1][1] += p1 * xa.y;
+        o[1][2] += p1 * xb.x;
+        o[1][3] += p1 * xb.y;
+    }
+}
+
+__global__ void __launch_bounds__(kFT, 3) k_step(FrontArgs a, const int4* __restrict__ tiles, int k0)
+{
+    __shared__ __align__(16) double XT[kNB * kXS];  // X_kk transposed: XT[k][j] = X_kk[j][k]
+    __shared__ double buf[2 * kTS * kPS];           // panels Pi, Pj, then L of both
+    __shared__ DiagSmem dsm;
+    const int4 tl = tiles[blockIdx.x];
+    const int s = tl.x;
+    const int r = a.nrow[s], c = a.ncol[s], kb = min(kNB, c - k0), base = k0 + kb;
+    // the trailing part of a front without children holds nothing before its first step
+    const bool fresh = k0 == 0 && a.child_ptr[s] == a.child_ptr[s + 1];
+    double* F = a.front + a.front_off[s];
+    const long long mo = a.xw_off[s], ld = ld_of(r);
+    double* M = a.xw + mo;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const bool two = tl.y != tl.z;  // off the diagonal: two row blocks
+    const int i0 = base + tl.y * kTS, j0 = base + tl.z * kTS;
+    double* Pi = buf;
+    double* Pj = two ? buf + kTS * kPS : buf;
+    griddep_wait();
+    griddep_launch();
+#pragma unroll
+    for (int it = 0; it < kNB * kNB / kFT; it++) {
+        const int idx = tid + it * kFT, j = idx & 31, k = idx >> 5;
+        cp8z(XT + k * kXS + j, M + (k0 + min(k, kb - 1)) * ld + k0 + min(j, kb - 1), k < kb && j < kb);
+    }
+#pragma unroll
+    for (int it = 0; it < kTS * kNB / kFT; it++) {
+        const int idx = tid + it * kFT, p = idx & (kTS - 1), k = idx >> 6;
+        const double* Fk = F + static_cast<long long>(k0 + min(k, kb - 1)) * r;
+        cp8z(Pi + p * kPS + k, Fk + min(i0 + p, r - 1), k < kb && i0 + p < r);
+        if (two) cp8z(Pj + p * kPS + k, Fk + min(j0 + p, r - 1), k < kb && j0 + p < r);
+    }
+    // tile rows (tid & 15) + 16 x, columns (tid >> 4) + 16 y
+    const int ra = tid & 15, ca = tid >> 4;
     double acc[4][4];
 #pragma unroll
-    for (int x = 0; x < 4; x++)
+    for (int y = 0; y < 4; y++)
 #pragma unroll
-        for (int y = 0; y < 4; y++) acc[x][y] = 0.0;
+        for (int x = 0; x < 4; x++) {
+            const int gi = i0 + ra + 16 * x, gj = j0 + ca + 16 * y;
+            acc[x][y] = gi < r && gi >= gj && !(fresh && gj >= c) ? F[gi + static_cast<long long>(gj) * r] : 0.0;
+        }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    {
+        double o[2][4], oj[2][4];
+        panel_times(Pi, XT, o);
+        if (two) panel_times(Pj, XT, oj);
+        __syncthreads();
+        double* Lp = a.lp + mo;
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int row = lane + 32 * x, k = 4 * w + q;
+                Pi[row * kPS + k] = o[x][q];
+                if (two) Pj[row * kPS + k] = oj[x][q];
+                if ((tl.w & kStoreL) && i0 + row < r && k < kb) Lp[(k0 + k) * ld + i0 + row] = o[x][q];
+            }
+    }
+    __syncthreads();
+#pragma unroll 2
     for (int k = 0; k < kb; k++) {
         double pa[4], pb[4];
 #pragma unroll
         for (int x = 0; x < 4; x++) {
-            pa[x] = Pi[a0 + x][k];
-            pb[x] = Pj[b0 + x][k];
+            pa[x] = Pi[(ra + 16 * x) * kPS + k];
+            pb[x] = Pj[(ca + 16 * x) * kPS + k];
         }
 #pragma unroll
         for (int x = 0; x < 4; x++)
 #pragma unroll
-            for (int y = 0; y < 4; y++) acc[x][y] += pa[x] * pb[y];
+            for (int y = 0; y < 4; y++) acc[x][y] -= pa[x] * pb[y];
     }
 #pragma unroll
-    for (int x = 0; x < 4; x++)
+    for (int y = 0; y < 4; y++)
 #pragma unroll
-        for (int y = 0; y < 4; y++) {
-            const int gi = base + ti * kTS + a0 + x, gj = base + tj * kTS + b0 + y;
-            if (gi < r && gj < r && gi >= gj) F[gi + static_cast<long long>(gj) * r] -= acc[x][y];
+        for (int x = 0; x < 4; x++) {
+            const int gi = i0 + ra + 16 * x, gj = j0 + ca + 16 * y;
+            if (gi < r && gi >= gj) F[gi + static_cast<long long>(gj) * r] = acc[x][y];
         }
-}
-
-// L_JJ^{-1} in two passes.  Pass 1: the inverse of every 32x32 diagonal tile,
-// one warp per tile, column j of the inverse by forward substitution in
-// shared memory; the tile's upper triangle is written as zeros because pass 2
-// reads whole tiles.
-__global__ void __launch_bounds__(32) k_diag_inv(FrontArgs a, const Tile* __restrict__ tiles)
-{
-    const Tile tl = tiles[blockIdx.x];
-    const int s = tl.s, j0 = tl.off;
-    const int r = a.nrow[s], c = a.ncol[s];
-    const int kb = min(kRT, c - j0);
-    const double* F = a.front + a.front_off[s];
-    __shared__ double D[kRT][kRT + 1];
-    __shared__ double X[kRT][kRT + 1];
-    const int j = threadIdx.x;
-    for (int k = 0; k < kb; k++) D[j][k] = j < kb ? F[static_cast<long long>(j0 + k) * r + j0 + j] : 0.0;
-    __syncwarp();
-    for (int i = 0; i < kb; i++) {  // thread j owns column j of X
-        double v = 0.0;
-        if (i == j) {
-            v = 1.0 / D[i][i];
-        } else if (i > j) {
-            double acc = 0.0;
-            for (int k = j; k < i; k++) acc += D[i][k] * X[k][j];
-            v = -acc / D[i][i];
-        }
-        X[i][j] = v;
+    if (!(tl.w & kNextDiag)) return;
+    // the next step's diagonal block, rows and columns [0, 32) of this tile
+    const int kn = min(kNB, c - base);
+    __syncthreads();
+#pragma unroll
+    for (int y = 0; y < 2; y++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) buf[(ra + 16 * x) * kPS + ca + 16 * y] = acc[x][y];
+    __syncthreads();
+    double A[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int cc = w + 8 * q;
+        A[q] = lane < kn && cc < kn ? (lane >= cc ? buf[lane * kPS + cc] : 0.0) : (lane == cc ? 1.0 : 0.0);
     }
-    __syncwarp();
-    if (j >= kb) return;
-    double* M = a.xw + a.xw_off[s];
-    const long long ld = ld_of(r);
-    for (int i = 0; i < kb; i++) M[(j0 + i) * ld + j0 + j] = X[j][i];
+    diag_inverse(A, kn, M + base * ld + base, ld, a.fail, dsm);
 }
 
-// Pass 2: the tiles below the diagonal, for 8 columns [j0, j0+8) per CTA.
-// With J the diagonal tile holding the columns, block row I > J of the
-// inverse is X_IJ = -X_II sum_{K=J}^{I-1} L_IK X_KJ (left-looking, the
-// columns are independent).  The next L_IK / X_KJ tiles are fetched into
-// registers while the current ones are multiplied.
-constexpr int kIC = 8;     // columns per CTA
-constexpr int kIT = 128;   // threads per CTA
-__global__ void __launch_bounds__(kIT) k_offdiag_inv(FrontArgs a, const Tile* __restrict__ tiles)
+// acc(64 x 64) += A(64 rows, k) B(k, 64 columns) over k in [k0, k1), 256
+// threads, rows (tid & 15) + 16 x and columns (tid >> 4) + 16 y per thread
+// (consecutive lanes on consecutive rows: no bank conflicts), in blocks of 16
+// with the next block's operands fetched into registers while one is used.
+// la(i, k) and lb(k, j) read an entry (0 outside).
+constexpr int kGK = 16;
+struct GemmSmem {
+    double A[kGK][65], B[kGK][65];
+};
+template <typename LA, typename LB>
+__device__ __forceinline__ void gemm64(GemmSmem& sm, double (&acc)[4][4], int k0, int k1, LA la, LB lb)
 {
-    const Tile tl = tiles[blockIdx.x];
-    const int s = tl.s, j0 = tl.off;
-    const int r = a.nrow[s], c = a.ncol[s];
-    const int jb0 = (j0 / kRT) * kRT;
-    if (jb0 + kRT >= c) return;  // no tile below the diagonal one
-    const double* F = a.front + a.front_off[s];
-    double* X = a.xw + a.xw_off[s];
-    const long long ld = ld_of(r);
-    __shared__ double As[kRT][kRT + 1];
-    __shared__ double Bs[kRT][kIC + 1];
-    const int tid = threadIdx.x, jj = tid & (kIC - 1), ii = tid >> 3;  // rows ii and ii + 16
-    const int ncols = min(kIC, c - j0);
-    double pa[kRT * kRT / kIT], pb[kRT * kIC / kIT];
-    auto fetch = [&](int i0, int ib, int k0) {
+    const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
+    double pa[4], pb[4];
+    auto fetch = [&](int k) {
 #pragma unroll
-        for (int q = 0; q < kRT * kRT / kIT; q++) {
-            const int idx = tid + q * kIT, kk = idx >> 5, rr = idx & 31;
-            pa[q] = rr < ib ? F[static_cast<long long>(k0 + kk) * r + i0 + rr] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < kRT * kIC / kIT; q++) {
-            const int idx = tid + q * kIT, kk = idx & 31, cc = idx >> 5;
-            pb[q] = cc < ncols ? X[(j0 + cc) * ld + k0 + kk] : 0.0;
+        for (int q = 0; q < 4; q++) {
+            const int idx = tid + 256 * q;
+            pa[q] = la(idx & 63, k + (idx >> 6));  // a warp on 32 consecutive rows of a column
+            pb[q] = lb(k + (idx & 15), idx >> 4);  // 16 consecutive rows of two columns
         }
     };
-    for (int i0 = jb0 + kRT; i0 < c; i0 += kRT) {
-        const int ib = min(kRT, c - i0);
-        double acc0 = 0.0, acc1 = 0.0;
-        fetch(i0, ib, jb0);
-        for (int k0 = jb0; k0 < i0; k0 += kRT) {
+    fetch(k0);
+    for (int k = k0; k < k1; k += kGK) {
+        __syncthreads();
 #pragma unroll
-            for (int q = 0; q < kRT * kRT / kIT; q++) {
-                const int idx = tid + q * kIT;
-                As[idx & 31][idx >> 5] = pa[q];
-            }
-#pragma unroll
-            for (int q = 0; q < kRT * kIC / kIT; q++) {
-                const int idx = tid + q * kIT;
-                Bs[idx & 31][idx >> 5] = pb[q];
-            }
-            __syncthreads();
-            if (k0 + kRT < i0) fetch(i0, ib, k0 + kRT);
-#pragma unroll 8
-            for (int kk = 0; kk < kRT; kk++) {
-                const double b = Bs[kk][jj];
-                acc0 += As[ii][kk] * b;
-                acc1 += As[ii + 16][kk] * b;
-            }
-            __syncthreads();
-        }
-        // X_IJ = -X_II T, X_II lower triangular with its zeros stored
-        Bs[ii][jj] = acc0;
-        Bs[ii + 16][jj] = acc1;
-        for (int idx = tid; idx < kRT * kRT; idx += kIT) {
-            const int rr = idx & 31, kk = idx >> 5;
-            As[rr][kk] = (rr < ib && kk < ib) ? X[(i0 + kk) * ld + i0 + rr] : 0.0;
+        for (int q = 0; q < 4; q++) {
+            const int idx = tid + 256 * q;
+            sm.A[idx >> 6][idx & 63] = pa[q];
+            sm.B[idx & 15][idx >> 4] = pb[q];
         }
         __syncthreads();
-        double x0 = 0.0, x1 = 0.0;
-#pragma unroll 8
-        for (int kk = 0; kk < kRT; kk++) {
-            const double t = Bs[kk][jj];
-            x0 += As[ii][kk] * t;
-            x1 += As[ii + 16][kk] * t;
+        if (k + kGK < k1) fetch(k + kGK);
+#pragma unroll 4
+        for (int i = 0; i < kGK; i++) {
+            double av[4], bv[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                av[q] = sm.A[i][ti + 16 * q];
+                bv[q] = sm.B[i][tj + 16 * q];
+            }
+#pragma unroll
+            for (int x = 0; x < 4; x++)
+#pragma unroll
+                for (int y = 0; y < 4; y++) acc[x][y] += av[x] * bv[y];
         }
-        if (jj < ncols) {
-            if (ii < ib) X[(j0 + jj) * ld + i0 + ii] = -x0;
-            if (ii + 16 < ib) X[(j0 + jj) * ld + i0 + ii + 16] = -x1;
-        }
-        __syncthreads();
     }
+}
+
+// X = L_JJ^{-1} from its 32 x 32 diagonal blocks, doubling the block size h:
+// with X_11 and X_22 of two neighbouring blocks known,
+//   X_21 = -X_22 (L_21 X_11),
+// two products per doubling (second = 0: T = L_21 X_11 into the front's own
+// columns, which nothing reads any more; second = 1: X_21).  Tiles: (front,
+// first row of the pair, tile row * 64, tile column * 64).  log2(c / 32)
+// doublings of dense products on a second branch of the graph, beside the
+// steps of the levels above; one block row after another, as a chain of c / 32
+// rows, took 0.76-0.87 ms.
+__global__ void __launch_bounds__(256) k_inverse(FrontArgs a, const int4* __restrict__ tiles, int h, int second)
+{
+    __shared__ GemmSmem sm;
+    const int4 tl = tiles[blockIdx.x];
+    const int s = tl.x, p1 = tl.y, p2 = p1 + h, i0 = tl.z, j0 = tl.w;
+    const int r = a.nrow[s], c = a.ncol[s], n2 = min(h, c - p2);  // rows of the second block
+    const long long ld = ld_of(r);
+    double* F = a.front + a.front_off[s];
+    double* M = a.xw + a.xw_off[s];
+    const double* Lp = a.lp + a.xw_off[s];
+    double acc[4][4] = {};
+    if (!second) {  // X_11 lower triangular: k >= column
+        gemm64(sm, acc, j0 / kGK * kGK, h,
+            [&](int i, int k) { return i0 + i < n2 && k < h ? Lp[(p1 + k) * ld + p2 + i0 + i] : 0.0; },
+            [&](int k, int j) { return k < h && j0 + j < h ? M[(p1 + j0 + j) * ld + p1 + k] : 0.0; });
+    } else {  // X_22 lower triangular: k <= row
+        gemm64(sm, acc, 0, min(n2, i0 + 64),
+            [&](int i, int k) { return i0 + i < n2 && k < n2 ? M[(p2 + k) * ld + p2 + i0 + i] : 0.0; },
+            [&](int k, int j) { return k < n2 && j0 + j < h ? F[static_cast<long long>(p1 + j0 + j) * r + p2 + k] : 0.0; });
+    }
+    const int ti = threadIdx.x & 15, tj = threadIdx.x >> 4;
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            const int i = i0 + ti + 16 * x, j = j0 + tj + 16 * y;
+            if (i >= n2 || j >= h) continue;
+            if (second) M[(p1 + j) * ld + p2 + i] = -acc[x][y];
+            else F[static_cast<long long>(p1 + j) * r + p2 + i] = acc[x][y];
+        }
+}
+
+// W = L_RJ X for every front, one 64 x 64 tile of W per CTA, written into the
+// rows below X in M.  With W the forward sweep forms a front's update
+// g = f_R - W f_J without waiting for y_J, and the backward sweep forms
+// x_J = L_JJ^{-T} y_J - W^T x_R in one step.
+__global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__ tiles)
+{
+    __shared__ GemmSmem sm;
+    const int4 tl = tiles[blockIdx.x];
+    const int s = tl.x, i0 = tl.y * 64, j0 = tl.z * 64;
+    const int r = a.nrow[s], c = a.ncol[s], m = r - c;
+    const long long ld = ld_of(r);
+    double* M = a.xw + a.xw_off[s];
+    const double* Lp = a.lp + a.xw_off[s];
+    double acc[4][4] = {};
+    gemm64(sm, acc, j0, c, [&](int i, int k) { return i0 + i < m && k < c ? Lp[k * ld + c + i0 + i] : 0.0; },
+        [&](int k, int j) { return k < c && j0 + j < c ? M[(j0 + j) * ld + k] : 0.0; });
+    const int ti = threadIdx.x & 15, tj = threadIdx.x >> 4;
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            const int i = i0 + ti + 16 * x, j = j0 + tj + 16 * y;
+            if (i < m && j < c) M[j * ld + c + i] = acc[x][y];
+        }
 }
 
 // ------------------------------------------------------------------ solves
@@ -1231,63 +1331,10 @@ __global__ void __launch_bounds__(kST) k_sub_bwd(SubArgs A)
     }
 }
 
-// W = L_RJ L_JJ^{-1} for every front, one 64 x 64 tile of W per CTA (4 x 4
-// per thread), L_RJ from the front's panel and L_JJ^{-1} (lower triangular,
-// entries above the diagonal masked) in blocks of 32, written into the rows
-// below X in M.  With W the forward sweep forms a front's update
-// g = f_R - W f_J without waiting for y_J, and the backward sweep forms
-// x_J = L_JJ^{-T} y_J - W^T x_R in one step.
-__global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__ tiles)
-{
-    const int4 tl = tiles[blockIdx.x];
-    const int s = tl.x, k0 = tl.y * 64, j0 = tl.z * 64;
-    const int r = a.nrow[s], c = a.ncol[s], m = r - c;
-    const double* F = a.front + a.front_off[s];
-    double* M = a.xw + a.xw_off[s];
-    const long long ld = ld_of(r);
-    __shared__ double As[32][64 + 1];  // As[i][k] = L_RJ[k0 + k][i0 + i]
-    __shared__ double Bs[32][64 + 1];  // Bs[i][j] = X[i0 + i][j0 + j]
-    const int tid = threadIdx.x, tk = (tid & 15) * 4, tj = (tid >> 4) * 4;
-    double acc[4][4] = {};
-    for (int i0 = (j0 / 32) * 32; i0 < c; i0 += 32) {
-        for (int idx = tid; idx < 32 * 64; idx += 256) {
-            const int i = idx >> 6, kk = idx & 63;
-            const int gi = i0 + i, gk = k0 + kk;
-            As[i][kk] = (gi < c && gk < m) ? F[static_cast<long long>(gi) * r + c + gk] : 0.0;
-            const int bi = idx & 31, bj = idx >> 5;  // consecutive threads on consecutive rows of X
-            const int hi = i0 + bi, hj = j0 + bj;
-            Bs[bi][bj] = (hi < c && hj < c && hi >= hj) ? M[hj * ld + hi] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int i = 0; i < 32; i++) {
-            double av[4], bv[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                av[q] = As[i][tk + q];
-                bv[q] = Bs[i][tj + q];
-            }
-#pragma unroll
-            for (int x = 0; x < 4; x++)
-#pragma unroll
-                for (int y = 0; y < 4; y++) acc[x][y] += av[x] * bv[y];
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int y = 0; y < 4; y++)
-#pragma unroll
-        for (int x = 0; x < 4; x++) {
-            const int gk = k0 + tk + x, gj = j0 + tj + y;
-            if (gk < m && gj < c) M[gj * ld + c + gk] = acc[x][y];
-        }
-}
-
 FrontArgs args_of(Precond& P)
 {
-    return FrontArgs { P.d_first, P.d_ncol, P.d_nrow, P.d_rows, P.d_child_ptr, P.d_child_list, P.d_relind,
-        P.d_level_list, P.d_contrib_ptr, P.d_contrib_idx, P.d_below_front, P.d_front_off, P.d_rows_off,
-        P.d_relind_off, P.d_xw_off, P.d_upd_off, P.d_front, P.d_xw, P.d_fail };
+    return FrontArgs { P.d_first, P.d_ncol, P.d_nrow, P.d_child_ptr, P.d_child_list, P.d_relind, P.d_slot, P.d_front_off,
+        P.d_rows_off, P.d_relind_off, P.d_xw_off, P.d_upd_off, P.d_slot_off, P.d_front, P.d_xw, P.d_lp, P.d_fail };
 }
 
 // the work buffers of one solve
@@ -1335,22 +1382,24 @@ void free_precond(Model& m)
     P.graphs.clear();
     if (P.factor_exec) cudaGraphExecDestroy(P.factor_exec);
     if (P.capture) cudaStreamDestroy(P.capture);
+    if (P.capture2) cudaStreamDestroy(P.capture2);
     if (P.h_flag) cudaFreeHost(P.h_flag);
-    for (int** p : { &P.d_first, &P.d_ncol, &P.d_nrow, &P.d_rows, &P.d_child_ptr, &P.d_child_list, &P.d_relind,
-             &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_panel_list, &P.d_contrib_ptr, &P.d_contrib_idx, &P.d_below_front, &P.d_parent, &P.d_cnt, &P.d_prow, &P.d_depth, &P.d_xidx, &P.d_slot })
+    for (int** p : { &P.d_first, &P.d_ncol, &P.d_nrow, &P.d_child_ptr, &P.d_child_list, &P.d_relind,
+             &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_parent, &P.d_cnt, &P.d_prow, &P.d_depth, &P.d_xidx, &P.d_slot })
         dev_free(*p);
-    for (long long** p : { &P.d_front_off, &P.d_rows_off, &P.d_relind_off, &P.d_xw_off, &P.d_upd_off, &P.d_a_pos,
+    for (long long** p : { &P.d_slot_off, &P.d_front_off, &P.d_rows_off, &P.d_relind_off, &P.d_xw_off, &P.d_upd_off, &P.d_a_pos,
              &P.d_a_src })
         dev_free(*p);
-    for (Tile** p : { &P.d_inv, &P.d_ea, &P.d_oinv }) dev_free(*p);
+    dev_free(P.d_ea);
+    dev_free(P.d_zero);
     dev_free(P.d_items);
     dev_free(P.d_item_group);
     dev_free(P.d_subs);
     dev_free(P.d_chunks);
-    dev_free(P.d_syrk);
+    dev_free(P.d_steps);
+    dev_free(P.d_invs);
     dev_free(P.d_wtiles);
-    for (double** p : { &P.d_front, &P.d_xw, &P.d_upd, &P.d_y, &P.d_t, &P.d_vals,
-             &P.d_diag_tmp })
+    for (double** p : { &P.d_front, &P.d_xw, &P.d_lp, &P.d_upd, &P.d_y, &P.d_t, &P.d_vals })
         dev_free(*p);
     delete m.precond;
     m.precond = nullptr;
@@ -1407,11 +1456,18 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     P.nlev = static_cast<int>(S.level_ptr.size()) - 1;
     const int nlev = P.nlev;
     // solve and factor schedules
-    std::vector<Tile> inv, ea, oinv;
+    std::vector<int4> ea;
+    std::vector<longlong2> zeros;
+    for (int s = 0; s < S.ns; s++) {
+        const long long n = static_cast<long long>(S.nrow[s]) * S.ncol[s], step = 16384;
+        for (long long o = 0; o < n; o += step) zeros.push_back(make_longlong2(S.front_off[s] + o, std::min(step, n - o)));
+    }
+    P.n_zero = static_cast<int>(zeros.size());
     P.ea_off.assign(1, 0);
-    std::vector<int> panel_list;
-    std::vector<int4> syrk;
+    P.w_off.assign(1, 0);
+    std::vector<int4> steps, invs, wtiles;
     P.lev_first_step.assign(1, 0);
+    P.lev_first_inv.assign(1, 0);
     for (int l = 0; l < nlev; l++) {
         int maxc = 0;
         for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
@@ -1421,43 +1477,53 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
             P.max_c = std::max(P.max_c, c);
             P.max_m = std::max(P.max_m, mm);
             maxc = std::max(maxc, c);
-            for (int o = 0; o < c; o += kRT) inv.push_back({ s, o });
-            for (int jb = 0; jb + kRT < c; jb += kRT)  // diagonal tiles with rows below them
-                for (int o = jb; o < jb + kRT; o += kIC) oinv.push_back({ s, o });
             if (S.child_ptr[s + 1] > S.child_ptr[s])
-                for (int o = 0; o < S.nrow[s]; o += kFT / 32) ea.push_back({ s, o });
+                for (int j = 0; j < S.nrow[s]; j += kEC)
+                    for (int i = j / kER * kER; i < S.nrow[s]; i += kER) ea.push_back(make_int4(s, i, j, 0));
+            for (int tk = 0; tk * 64 < mm; tk++)
+                for (int tj = 0; tj * 64 < c; tj++) wtiles.push_back(make_int4(s, tk, tj, 0));
         }
         P.ea_off.push_back(static_cast<int>(ea.size()));
+        P.w_off.push_back(static_cast<int>(wtiles.size()));
         for (int k0 = 0; k0 < maxc; k0 += kNB) {
-            Precond::Step st { l, k0, static_cast<int>(panel_list.size()), 0, static_cast<int>(syrk.size()), 0, 1 };
+            Precond::Step st { k0, static_cast<int>(steps.size()), 0 };
             for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
                 const int s = S.level_list[q];
                 const int c = S.ncol[s], r = S.nrow[s];
                 if (c <= k0) continue;
-                panel_list.push_back(s);
-                const int kb = std::min(kNB, c - k0);
-                const int m2 = r - k0 - kb;
-                st.panel_chunks = std::max(st.panel_chunks, (m2 + kFT - 1) / kFT);
-                const int nt = (m2 + kTS - 1) / kTS;
+                const int nt = (r - k0 - std::min(kNB, c - k0) + kTS - 1) / kTS;
                 for (int tj = 0; tj < nt; tj++)
-                    for (int ti = tj; ti < nt; ti++) syrk.push_back(make_int4(s, ti, tj, 0));
+                    for (int ti = tj; ti < nt; ti++)
+                        steps.push_back(make_int4(s, ti, tj, (tj == 0 ? kStoreL : 0) | (ti == 0 && c > k0 + kNB ? kNextDiag : 0)));
             }
-            st.panel_cnt = static_cast<int>(panel_list.size()) - st.panel_off;
-            st.syrk_cnt = static_cast<int>(syrk.size()) - st.syrk_off;
-            P.max_panel_cnt = std::max(P.max_panel_cnt, st.panel_cnt);
+            st.cnt = static_cast<int>(steps.size()) - st.off;
             P.steps.push_back(st);
         }
         P.lev_first_step.push_back(static_cast<int>(P.steps.size()));
+        // Doublings of the inverse, as soon as their blocks are there: the first
+        // product (L_21 X_11) after X_11's last step, the second after X_22's,
+        // in batches of kInvBatch steps.  Within a batch sizes ascend.
+        const int nsteps = (maxc + kNB - 1) / kNB;
+        for (int batch = 0; batch < nsteps; batch += kInvBatch) {
+            const int last = std::min(nsteps, batch + kInvBatch) - 1;  // step after which the batch runs
+            for (int h = kNB; h < maxc; h *= 2)
+                for (int second = 0; second < 2; second++) {
+                    Precond::Inv st { last, h, second, static_cast<int>(invs.size()), 0 };
+                    for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
+                        const int s = S.level_list[q], c = S.ncol[s];
+                        for (int p1 = 0; p1 + h < c; p1 += 2 * h) {
+                            const int ready = ((second ? std::min(c, p1 + 2 * h) : p1 + h) + kNB - 1) / kNB - 1;
+                            if (ready < batch || ready > last) continue;
+                            for (int i = 0; i < std::min(h, c - p1 - h); i += 64)
+                                for (int j = 0; j < h; j += 64) invs.push_back(make_int4(s, p1, i, j));
+                        }
+                    }
+                    st.cnt = static_cast<int>(invs.size()) - st.off;
+                    if (st.cnt > 0) P.invs.push_back(st);
+                }
+        }
+        P.lev_first_inv.push_back(static_cast<int>(P.invs.size()));
     }
-    P.n_inv_tiles = static_cast<int>(inv.size());
-    std::vector<int4> wtiles;
-    for (int s = 0; s < S.ns; s++) {
-        const int c = S.ncol[s], mm = S.nrow[s] - c;
-        for (int tk = 0; tk * 64 < mm; tk++)
-            for (int tj = 0; tj * 64 < c; tj++) wtiles.push_back(make_int4(s, tk, tj, 0));
-    }
-    P.n_wtiles = static_cast<int>(wtiles.size());
-    P.n_oinv = static_cast<int>(oinv.size());
     auto odd_h = [](int L) { return L | 1; };
     // Subtree solves: fronts on the lowest K levels are solved per subtree by
     // one CTA (k_sub_fwd / k_sub_bwd), the levels above by the dataflow
@@ -1650,20 +1716,19 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     UP(P.d_first, S.first);
     UP(P.d_ncol, S.ncol);
     UP(P.d_nrow, S.nrow);
-    UP(P.d_rows, S.rows);
     UP(P.d_child_ptr, S.child_ptr);
     UP(P.d_child_list, S.child_list);
     UP(P.d_relind, S.relind);
-    UP(P.d_level_list, S.level_list);
     UP(P.d_perm, S.perm);
     UP(P.d_front_off, S.front_off);
     UP(P.d_rows_off, S.rows_off);
     UP(P.d_relind_off, S.relind_off);
     UP(P.d_xw_off, xw_off);
+    UP(P.d_level_list, S.level_list);
     UP(P.d_slot, slot);
+    UP(P.d_slot_off, slot_off);
+    UP(P.d_zero, zeros);
     UP(P.d_upd_off, S.upd_off);
-    UP(P.d_contrib_ptr, S.contrib_ptr);
-    UP(P.d_contrib_idx, S.contrib_idx);
     UP(P.d_a_pos, S.a_pos);
     UP(P.d_a_src, S.a_src);
     UP(P.d_vals, vals);
@@ -1676,25 +1741,21 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
         UP(P.d_depth, sdepth);
         UP(P.d_xidx, xidx);
     }
-    UP(P.d_inv, inv);
-    UP(P.d_oinv, oinv);
     UP(P.d_wtiles, wtiles);
     UP(P.d_ea, ea);
-    UP(P.d_below_front, S.below_front);
-    UP(P.d_panel_list, panel_list);
-    UP(P.d_syrk, syrk);
+    UP(P.d_steps, steps);
+    UP(P.d_invs, invs);
 #undef UP
     const size_t n3 = 3 * static_cast<size_t>(std::max(S.n, 1));
     if ((st = dev_alloc(&P.d_front, static_cast<size_t>(S.front_size))) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_xw, static_cast<size_t>(std::max<long long>(xw_size, 1)))) != EFEM_OK) return st;
+    if ((st = dev_alloc(&P.d_lp, static_cast<size_t>(std::max<long long>(xw_size, 1)))) != EFEM_OK) return st;
     EFEM_CUDA(cudaMemsetAsync(P.d_xw, 0, sizeof(double) * std::max<long long>(xw_size, 1), m.stream));  // above X's diagonal, pad rows
     if ((st = dev_alloc(&P.d_upd, static_cast<size_t>(std::max<long long>(S.upd_size, 1)))) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_y, n3)) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_t, n3)) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_cnt, 4 * static_cast<size_t>(S.ns) + 2)) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_fail, 1)) != EFEM_OK) return st;
-    if ((st = dev_alloc(&P.d_diag_tmp, static_cast<size_t>(std::max(P.max_panel_cnt, 1)) * kNB * kNB)) != EFEM_OK)
-        return st;
     // persistent solve: as many CTAs as fit on the device at once
     P.solve_grid_full = std::max(1, std::min(P.n_items, P.slots));
     P.solve_grid = solve_grid_for(P);
@@ -1703,6 +1764,7 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
         EFEM_CUDA(cudaFuncSetAttribute(k_sub_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
     EFEM_CUDA(cudaStreamCreateWithFlags(&P.capture, cudaStreamNonBlocking));
+    EFEM_CUDA(cudaStreamCreateWithFlags(&P.capture2, cudaStreamNonBlocking));
     EFEM_CUDA(cudaMallocHost(&P.h_flag, sizeof(int)));
     P.ready = true;  // analysed; the numeric factor follows
     return precond_factor(m, ok, ms_factor);
@@ -1712,46 +1774,50 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
 // scatter L into the fronts, factor level by level, invert the diagonal blocks.
 // the launches of one numeric factorisation, in order, on stream st; returns
 // the number of kernels
-static long long enqueue_factor(Precond& P, cudaStream_t st)
+static long long enqueue_factor(Precond& P, cudaStream_t st, cudaStream_t st2, cudaEvent_t ev)
 {
     const Symbolic& S = P.S;
     long long n = 0;
-    cudaMemsetAsync(P.d_front, 0, sizeof(double) * S.front_size, st);
+    bool forked = false;
     cudaMemsetAsync(P.d_fail, 0, sizeof(int), st);
+    if (P.n_zero > 0) k_zero<<<P.n_zero, kFT, 0, st>>>(P.d_front, P.d_zero);
     const long long na = static_cast<long long>(S.a_pos.size());
     k_scatter_a<<<static_cast<int>(std::min<long long>(1184, (na + 255) / 256 + 1)), 256, 0, st>>>(
         P.d_front, P.d_a_pos, P.d_a_src, P.d_vals, na);
-    n++;
+    n += 2;
     FrontArgs a = args_of(P);
+    auto fork = [&]() {  // the second branch goes on from here
+        cudaEventRecord(ev, st);
+        cudaStreamWaitEvent(st2, ev, 0);
+        forked = true;
+    };
     for (int l = 0; l < P.nlev; l++) {
         const int cnt = P.ea_off[l + 1] - P.ea_off[l];
         if (cnt > 0) {
-            k_extend_add<<<cnt, kFT, 0, st>>>(a, P.d_ea + P.ea_off[l]);
+            launch_k(k_extend_add, cnt, kFT, 0, st, a, static_cast<const int4*>(P.d_ea + P.ea_off[l]));
             n++;
         }
-        for (int q = P.lev_first_step[l]; q < P.lev_first_step[l + 1]; q++) {
-            const Precond::Step& stp = P.steps[q];
-            k_panel<<<dim3(stp.panel_cnt, stp.panel_chunks), kFT, 0, st>>>(a, P.d_panel_list + stp.panel_off, stp.k0,
-                P.d_diag_tmp);
-            k_panel_store<<<stp.panel_cnt, kFT, 0, st>>>(a, P.d_panel_list + stp.panel_off, stp.k0, P.d_diag_tmp);
-            n += 2;
-            if (stp.syrk_cnt > 0) {
-                k_syrk<<<stp.syrk_cnt, kFT, 0, st>>>(a, P.d_syrk + stp.syrk_off, stp.k0);
-                n++;
-            }
+        launch_k(k_diag, S.level_ptr[l + 1] - S.level_ptr[l], kFT, 0, st, a, static_cast<const int*>(P.d_level_list + S.level_ptr[l]));
+        n++;
+        // the steps; beside them, and beside the levels above, X and W
+        int iv = P.lev_first_inv[l];
+        const int s0 = P.lev_first_step[l], s1 = P.lev_first_step[l + 1], nw = P.w_off[l + 1] - P.w_off[l];
+        for (int q = s0; q < s1; q++) {
+            if (P.steps[q].cnt > 0) launch_k(k_step, P.steps[q].cnt, kFT, 0, st, a, static_cast<const int4*>(P.d_steps + P.steps[q].off), P.steps[q].k0);
+            n++;
+            const bool more = iv < P.lev_first_inv[l + 1] && P.invs[iv].after == q - s0;
+            if (more || (q == s1 - 1 && nw > 0)) fork();
+            for (; iv < P.lev_first_inv[l + 1] && P.invs[iv].after == q - s0; iv++, n++)
+                k_inverse<<<P.invs[iv].cnt, 256, 0, st2>>>(a, P.d_invs + P.invs[iv].off, P.invs[iv].h, P.invs[iv].second);
+        }
+        if (nw > 0) {
+            k_w<<<nw, 256, 0, st2>>>(a, P.d_wtiles + P.w_off[l]);
+            n++;
         }
     }
-    if (P.n_inv_tiles > 0) {
-        k_diag_inv<<<P.n_inv_tiles, 32, 0, st>>>(a, P.d_inv);
-        n++;
-        if (P.n_oinv > 0) {
-            k_offdiag_inv<<<P.n_oinv, kIT, 0, st>>>(a, P.d_oinv);
-            n++;
-        }
-        if (P.n_wtiles > 0) {
-            k_w<<<P.n_wtiles, 256, 0, st>>>(a, P.d_wtiles);
-            n++;
-        }
+    if (forked) {
+        cudaEventRecord(ev, st2);
+        cudaStreamWaitEvent(st, ev, 0);
     }
     return n;
 }
@@ -1763,21 +1829,28 @@ static efem_status precond_factor(Model& m, int* ok, double* ms_factor)
     Precond& P = *m.precond;
     if (!P.factor_exec) {
         std::lock_guard<std::mutex> lock(capture_mutex());
-        cudaGraph_t g = nullptr;
-        EFEM_CUDA(cudaStreamBeginCapture(P.capture, cudaStreamCaptureModeThreadLocal));
-        P.factor_launches = enqueue_factor(P, P.capture);
-        const cudaError_t e = cudaStreamEndCapture(P.capture, &g);
-        if (e != cudaSuccess) {
+        // with programmatic dependent launch along the steps; a capture that refuses it is made with plain launches
+        for (int attempt = 0; attempt < 2 && !P.factor_exec; attempt++) {
+            cudaGraph_t g = nullptr;
+            cudaEvent_t ev;
+            EFEM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+            cudaError_t e = cudaStreamBeginCapture(P.capture, cudaStreamCaptureModeThreadLocal);
+            if (e == cudaSuccess) {
+                t_pdl = attempt == 0;
+                P.factor_launches = enqueue_factor(P, P.capture, P.capture2, ev);
+                t_pdl = false;
+                e = cudaStreamEndCapture(P.capture, &g);
+            }
+            cudaEventDestroy(ev);
+            if (e == cudaSuccess) e = cudaGraphInstantiate(&P.factor_exec, g, 0);
             if (g) cudaGraphDestroy(g);
-            set_error(std::string("capture of the factorisation: ") + cudaGetErrorString(e));
-            return EFEM_ERR_CUDA;
-        }
-        const cudaError_t ei = cudaGraphInstantiate(&P.factor_exec, g, 0);
-        cudaGraphDestroy(g);
-        if (ei != cudaSuccess) {
-            P.factor_exec = nullptr;
-            set_error(std::string("factorisation graph: ") + cudaGetErrorString(ei));
-            return EFEM_ERR_CUDA;
+            if (e != cudaSuccess) {
+                P.factor_exec = nullptr;
+                cudaGetLastError();
+                if (attempt == 0) continue;
+                set_error(std::string("factorisation graph: ") + cudaGetErrorString(e));
+                return EFEM_ERR_CUDA;
+            }
         }
     }
     cudaEvent_t e0, e1;

@@ -306,32 +306,6 @@ void symbolic_analysis(int n, const std::vector<int>& rowptr, const std::vector<
     }
     S.front_size = S.front_off[ns];
     S.upd_size = S.upd_off[ns];
-    // children's update-vector entries per parent row, in child order
-    {
-        std::vector<int> cnt(S.rows.size() + 1, 0);
-        for (int k = 0; k < ns; k++) {
-            if (S.parent[k] < 0) continue;
-            const long long base = S.rows_off[S.parent[k]];
-            for (long long j = S.relind_off[k]; j < S.relind_off[k + 1]; j++) cnt[base + S.relind[j] + 1]++;
-        }
-        for (size_t i = 0; i + 1 < cnt.size(); i++) cnt[i + 1] += cnt[i];
-        S.contrib_ptr = cnt;
-        S.below_front.assign(static_cast<size_t>(S.upd_size / 3), 0);
-        for (int k = 0; k < ns; k++)
-            for (long long q = S.upd_off[k] / 3; q < S.upd_off[k + 1] / 3; q++) S.below_front[q] = k;
-        S.contrib_idx.assign(cnt.back(), 0);
-        std::vector<int> fill(S.rows.size(), 0);
-        for (int s = 0; s < ns; s++)  // parents in order, children in list order
-            for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; q++) {
-                const int ch = S.child_list[q];
-                const long long base = S.rows_off[s];
-                for (long long j = S.relind_off[ch]; j < S.relind_off[ch + 1]; j++) {
-                    const long long row = base + S.relind[j];
-                    S.contrib_idx[S.contrib_ptr[row] + fill[row]++] =
-                        static_cast<int>(S.upd_off[ch] / 3 + (j - S.relind_off[ch]));
-                }
-            }
-    }
     // original entries (lower triangle) -> front positions
     for (int o = 0; o < n; o++) {
         const int j = iperm[o];

@@ -23,11 +23,6 @@ struct Symbolic {
     std::vector<long long> relind_off;
     std::vector<int> relind;           // below rows of a front -> positions in the parent's rows
     std::vector<long long> upd_off;    // (r - c) x 3 forward-solve update vector
-    // for every front row (indexed rows_off[s] + t): the update-vector entries
-    // of the children that land on it, in child order (CSR over rows)
-    std::vector<int> contrib_ptr;
-    std::vector<int> contrib_idx;      // index of a node-triple in the update array (upd_off/3 + j)
-    std::vector<int> below_front;      // for each such index, the front whose update array holds it
     std::vector<int> level_ptr, level_list;  // fronts grouped by level, leaves first
     long long front_size = 0, upd_size = 0, nnz_L = 0;
     double flops = 0;
