@@ -569,31 +569,37 @@ __global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__
 //     warps splitting the rows of one): a lane takes two consecutive rows of
 //     the four columns, so the vector in shared memory is read once for four
 //     columns; one 12-value reduction over the lanes at the end.
-//   * The matrix goes from memory to registers; only the vectors pass through
-//     shared memory, in chunks of kVC entries, so the kernel's shared memory
-//     does not depend on the fronts and every model runs 3 CTAs per SM.
-//   * All that can be had before the wait is loaded before it: the item's
-//     record, the first columns of a forward tile, the index of every row to
-//     be assembled (a dense table per front and child: consecutive threads
-//     read consecutive entries), and the backward tile's part over y.
-// What bounds it: the chain of dependent fronts (11-13 per sweep, about 5 us
-// each: notice, gather, product, publish), then the factor's bytes.  One
-// application (inside a solve, with both matrices and their transposes staged
-// through shared memory before): C3D8 beam 124 -> 113 us, C3D20R cap 330 ->
-// 192 us (281 MB, 1.5 TB/s), C3D10 finger 439 -> 241 us (340 MB, 1.4 TB/s).
+//   * The vectors pass through shared memory in chunks of kVC entries, so the
+//     kernel's shared memory does not depend on the fronts and every model
+//     runs 3 CTAs per SM.
+//   * All that can be had before the wait is fetched before it: the item's
+//     record, the first kStage values of M of every thread (staged by the
+//     thread that uses them, so no barrier stands between) and the rest of a
+//     forward tile into L2, the index of every row to be assembled (a dense
+//     table per front and child: consecutive threads read consecutive
+//     entries), and the backward tile's part over y.
+// What bounds it: the chain of dependent fronts (11-13 per sweep, 4-5 us
+// each: notice 1, gather 0.8, product 1, partial sums and store 1, publish
+// 0.5), then the factor's bytes.  One application inside a solve, against four
+// matrices staged through shared memory in 4-row tiles, and against M read
+// into registers after the wait: C3D8 beam 124, 113, now 105 us; C3D20R cap
+// 330, 192, now 182 us (281 MB, 1.5 TB/s); C3D10 finger 439, 241, now 226 us
+// (340 MB, 1.5 TB/s).  More shared memory costs more than it gives (chunks of
+// 1280 entries: cap 210 us; the index tables live in what L1 is left).
 // Every sum has a fixed order (no atomics on data): results repeat bitwise.
 enum ItemKind { kFwdTile = 0, kBwdTile = 1 };
 
-constexpr int kVC = 1024;      // vector entries (nodes) of a chunk in shared memory
+constexpr int kVC = 896;       // vector entries (nodes) of a chunk in shared memory
 constexpr int kMaxR = 256;     // most rows of a forward tile
-constexpr int kFU = 4;         // columns a forward lane loads at a time
+constexpr int kFU = 4;         // columns a forward lane loads at a time beyond the staged ones
+constexpr int kStage = 8;      // 16-byte values of M a thread stages before the wait
 // doubles of M per tile (see precond_setup).  One application, beam / cap /
 // finger, with kTileMin 1024, 2048, 4096: 115 / 192 / 242, 113 / 193 / 241,
 // 119 / 192 / 238 us; with kTileMax 4096, 6144, 10240: 114 / 196 / 243,
 // 113 / 193 / 241, 114 / 193 / 241 us.
 constexpr int kTileMin = 2048, kTileMax = 6144;
 constexpr int kRed = 8 * 64 * 3;  // doubles of the partial sums of a tile
-constexpr size_t kSolveSmem = sizeof(double) * (3 * (kVC + kMaxR) + kRed);
+constexpr size_t kSolveSmem = sizeof(double) * (3 * (kVC + kMaxR) + (kRed > 2 * kStage * kST ? kRed : 2 * kStage * kST));
 
 // device counters, one int array: [cY ns][cGin ns][exits, ns - 1 unused][cX ns][ticket][error]
 struct SolveArgs {
@@ -626,18 +632,27 @@ __device__ __forceinline__ int ld_acquire(const int* p)
 }
 
 // one thread: wait until *c >= target; false after `limit` polls (the
-// error flag is then set) or when another wait has already given up
+// error flag is then set) or when another wait has already given up.  The
+// flag is read every 16th poll only: read every time, it doubled the time
+// between two looks at the counter.
 __device__ bool wait_ge(const int* c, int target, int* err, int limit)
 {
     for (int it = 0;; it++) {
         if (ld_acquire(c) >= target) return true;
-        if (*reinterpret_cast<volatile int*>(err)) return false;
         if (it >= limit) {
             atomicExch(err, 1);
             return false;
         }
+        if ((it & 15) == 15 && *reinterpret_cast<volatile int*>(err)) return false;
         __nanosleep(64);
     }
+}
+
+// count a finished tile: its results (made visible to this thread by the
+// CTA's barrier) before the count
+__device__ __forceinline__ void signal(int* c)
+{
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(c) : "memory");
 }
 
 __device__ __forceinline__ void ld3(const double* p, double& a, double& b, double& c)
@@ -718,6 +733,13 @@ __device__ __forceinline__ void first_idx(const SolveArgs& A, const SolveItem& d
     }
 }
 
+__device__ __forceinline__ void cp16(double2* dst, const double* src)
+{
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ double2 ldm2(const double* p) { return __ldg(reinterpret_cast<const double2*>(p)); }
 
 __device__ __forceinline__ void fma6(double* acc, double2 m, const double* f)
@@ -731,6 +753,22 @@ __device__ __forceinline__ void fma6(double* acc, double2 m, const double* f)
     acc[5] += m.y * f2;
 }
 
+// two rows of four columns times z on these rows, added to the twelve sums
+__device__ __forceinline__ void fma12(double (&acc)[4][3], const double2 (&m)[4], const double* z)
+{
+    const double2* zp = reinterpret_cast<const double2*>(z);
+    const double2 za = zp[0], zc = zp[1], ze = zp[2];  // (z0 z1) (z2 z0') (z1' z2')
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        acc[q][0] += m[q].x * za.x;
+        acc[q][1] += m[q].x * za.y;
+        acc[q][2] += m[q].x * zc.x;
+        acc[q][0] += m[q].y * zc.y;
+        acc[q][1] += m[q].y * ze.x;
+        acc[q][2] += m[q].y * ze.y;
+    }
+}
+
 // twelve column sums (four columns x three components) over rows [i0, i1) of
 // the chunk that starts at row zb (even), each lane two rows every `step`
 __device__ __forceinline__ void cols_acc(double (&acc)[4][3], const double* const (&Mc)[4], const double* z, int zb,
@@ -741,17 +779,7 @@ __device__ __forceinline__ void cols_acc(double (&acc)[4][3], const double* cons
         double2 m[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) m[q] = ldm2(Mc[q] + i);
-        const double2* zp = reinterpret_cast<const double2*>(z + 3 * (i - zb));
-        const double2 za = zp[0], zc = zp[1], ze = zp[2];  // (z0 z1) (z2 z0') (z1' z2')
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            acc[q][0] += m[q].x * za.x;
-            acc[q][1] += m[q].x * za.y;
-            acc[q][2] += m[q].x * zc.x;
-            acc[q][0] += m[q].y * zc.y;
-            acc[q][1] += m[q].y * ze.x;
-            acc[q][2] += m[q].y * ze.y;
-        }
+        fma12(acc, m, z + 3 * (i - zb));
     }
 }
 
@@ -783,7 +811,8 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
     griddep_wait();
     extern __shared__ __align__(16) double sm[];
     double* vec = sm;                      // [kVC + kMaxR][3] chunk of the vector, and f on a tile's own below rows
-    double* red = sm + 3 * (kVC + kMaxR);  // partial sums
+    double* red = sm + 3 * (kVC + kMaxR);  // partial sums, once the staged values are used
+    double2* stg = reinterpret_cast<double2*>(red) + threadIdx.x;  // the thread's staged values, kST apart
     __shared__ int item_sh, ok_sh, ok2_sh;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     int* ticket = A.cnt + 4 * A.ns;
@@ -833,10 +862,13 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
             const int wk = w >> bsh, ks = (wk << (5 - lsh)) + (lane >> lsh);
             const bool act = lrow < R;
             const double* Mr = M + r0 + lrow;
-            double2 buf[kFU];
 #pragma unroll
-            for (int u = 0; u < kFU; u++)
-                buf[u] = act && ks + u * KS < kend ? ldm2(Mr + (ks + u * KS) * ld) : make_double2(0.0, 0.0);
+            for (int n = 0; n < kStage; n++)
+                if (act && ks + n * KS < kend) cp16(stg + n * kST, Mr + (ks + n * KS) * ld);
+            // the rest of a long row block at least into L2 (one lane per 64 bytes)
+            if (act && (lane & 3) == 0)
+                for (int q = ks + kStage * KS; q < kend; q += KS)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(Mr + q * ld));
             const int b0 = max(r0, c), nb = r1 - b0;  // the tile's below rows (nb <= 0: none)
             RowIdx ix[2];
             first_idx(A, d, 0, min(kend, kVC), b0, max(nb, 0), ix);
@@ -859,23 +891,28 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
                         assemble(A, d, 0, ke, b0, max(nb, 0), vec, ix);
                     }
                     __syncthreads();
-                    if (act)
-                        while (k < ke) {
-                            if (k != ks) {
+                    if (act) {
+                        if (kb == 0) {
+                            stage_wait();  // a thread reads what it staged itself
 #pragma unroll
-                                for (int u = 0; u < kFU; u++)
-                                    buf[u] = k + u * KS < ke ? ldm2(Mr + (k + u * KS) * ld) : make_double2(0.0, 0.0);
-                            }
+                            for (int n = 0; n < kStage; n++)
+                                if (ks + n * KS < ke) fma6(acc, stg[n * kST], vec + 3 * (ks + n * KS));
+                            k = ks + kStage * KS;  // (a staged column lies in the first chunk: kStage KS <= 512)
+                        }
+                        while (k < ke) {
+                            double2 buf[kFU];
+#pragma unroll
+                            for (int u = 0; u < kFU; u++)
+                                buf[u] = k + u * KS < ke ? ldm2(Mr + (k + u * KS) * ld) : make_double2(0.0, 0.0);
 #pragma unroll
                             for (int u = 0; u < kFU; u++)
                                 if (k + u * KS < ke) fma6(acc, buf[u], vec + 3 * (k + u * KS - kb));
                             k += kFU * KS;
-                            if (k >= ke) {  // the first column of the next chunk
-                                k = ke + ((ks - ke) % KS + KS) % KS;
-                                break;
-                            }
                         }
+                        if (k >= ke) k = ke + ((ks - ke) % KS + KS) % KS;  // the first column of the next chunk
+                    }
                 }
+                __syncthreads();  // the staged values make room for the partial sums
                 for (int o = 1 << lsh; o < 32; o <<= 1)
 #pragma unroll
                     for (int q = 0; q < 6; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
@@ -887,8 +924,10 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
                 __syncthreads();
                 const double* fr = vec + 3 * min(kend, kVC);
                 for (int i = tid; i < 3 * R; i += kST) {
-                    double sum = 0.0;
-                    for (int h = 0; h < nw; h++) sum += red[h * (192 << bsh) + i];
+                    double x[8];
+#pragma unroll
+                    for (int h = 0; h < 8; h++) x[h] = h < nw ? red[h * (192 << bsh) + i] : 0.0;
+                    const double sum = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
                     if (i < 3 * (c - r0))
                         A.y[3LL * (d.f0 + r0) + i] = sum;
                     else
@@ -898,9 +937,8 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
             if (tid == 0) item_sh = next;
             __syncthreads();  // the item's results are written
             if (tid == 0) {
-                __threadfence();
-                if (r0 < c) atomicAdd(A.cnt + d.s, 1);
-                if (r1 > c && d.parent >= 0) atomicAdd(A.cnt + A.ns + d.parent, 1);
+                if (r1 > c && d.parent >= 0) signal(A.cnt + A.ns + d.parent);
+                if (r0 < c) signal(A.cnt + d.s);
             }
         } else {
             // columns [r0, r1), at most 32: one quad of columns per warp, or
@@ -913,6 +951,16 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
             const double* Mc[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) Mc[q] = M + min(r0 + 4 * quad + q, r1 - 1) * ld;
+            // the first rows below the front's own, which are on the critical path
+            const int zc = c & ~1, zi = zc + 64 * h + 2 * lane, zn = min(d.r, zc + kVC);
+            if (act) {
+#pragma unroll
+                for (int n = 0; n < kStage / 4; n++)
+                    if (zi + n * step < zn) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) cp16(stg + (4 * n + q) * kST, Mc[q] + zi + n * step);
+                    }
+            }
             if (tid == 0) {
                 ok_sh = wait_ge(A.cnt + d.s, d.target + bump, err, A.spin_limit);
                 if (!ok_sh) next = atomicAdd(ticket, 1);
@@ -931,8 +979,8 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
                     if (act) cols_acc(acc, Mc, vec, zb, zb + 64 * h + 2 * lane, ze, step);
                 }
                 // below rows: -x of the ancestors, complete with the parent's
-                const int zc = c & ~1;
                 int ip[4];
+                const int io = tid < 3 * (r1 - r0) ? __ldg(pr + r0 + tid / 3) : 0;  // where the thread's result goes
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const int t = zc + tid + u * kST;
@@ -968,8 +1016,20 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
                             for (int k = 0; k < 3; k++) vec[3 * i + k] = -x[u][k];
                         }
                         __syncthreads();
-                        if (act) cols_acc(acc, Mc, vec, zb, zb + 64 * h + 2 * lane, ze, step);
+                        int i = zb + 64 * h + 2 * lane;
+                        if (act && zb == zc) {
+                            stage_wait();
+#pragma unroll
+                            for (int n = 0; n < kStage / 4; n++, i += step)
+                                if (i < ze) {
+                                    const double2 m[4] = { stg[4 * n * kST], stg[(4 * n + 1) * kST], stg[(4 * n + 2) * kST],
+                                        stg[(4 * n + 3) * kST] };
+                                    fma12(acc, m, vec + 3 * (i - zb));
+                                }
+                        }
+                        if (act) cols_acc(acc, Mc, vec, zb, i, ze, step);
                     }
+                    __syncthreads();  // the staged values make room for the partial sums
                     cols_reduce(acc);
                     if ((lane & 7) == 0) {
                         double* o = red + ((h << qsh) + quad) * 12 + 3 * (lane >> 3);
@@ -978,18 +1038,16 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
                     }
                     __syncthreads();
                     if (tid < 3 * (r1 - r0)) {
-                        double x = 0.0;
-                        for (int q = 0; q < wk; q++) x += red[(q << qsh) * 12 + tid];
-                        A.v[3LL * __ldg(pr + r0 + tid / 3) + tid % 3] = x;
+                        double x[8];
+#pragma unroll
+                        for (int q = 0; q < 8; q++) x[q] = q < wk ? red[(q << qsh) * 12 + tid] : 0.0;
+                        A.v[3LL * io + tid % 3] = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
                     }
                 }
             }
             if (tid == 0) item_sh = next;
             __syncthreads();
-            if (tid == 0) {
-                __threadfence();
-                atomicAdd(A.cnt + 3 * A.ns + d.s, 1);
-            }
+            if (tid == 0) signal(A.cnt + 3 * A.ns + d.s);
         }
     }
     // A solve that gave up leaves v partly overwritten: the last CTA to
@@ -1033,7 +1091,6 @@ __device__ __forceinline__ void stage_cols(double* dst, int lp, const double* sr
     }
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void stage_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 __device__ __forceinline__ int odd(int L) { return L | 1; }
