@@ -3,19 +3,14 @@
 // src/fe/ElementConstraint.cpp:164-205); they are built on its residual
 // (ElementConstraint.cpp:139-162, ExternalConstraint.cpp:829-959):
 //
-//   K(u) v      the directional derivative of R at u along v, computed by the
-//               residual kernels instantiated on forward-mode dual numbers
-//               (value + derivative), so the tangent is exact to rounding;
+//   K(u) v      the directional derivative of R at u along v, the residual's
+//               phases with the laws differentiated by hand (piola_tangent);
 //   K(u)^T w    the element part of K is the Hessian of the stored energy and
 //               is symmetric, so K_el^T w = K_el w; the pressure part is not
 //               (follower and directed loads are not conservative) and is
-//               transposed face by face: one dual seed per face unknown gives
-//               the column d f_face / d u_j, dotted with w on the face; an
-//               adjoint solve stores these face blocks once at its u and
-//               applies them in every Krylov iteration, and likewise the
-//               Gauss-point tangents dP/dH of the elements, so that K_el v
-//               in its iterations is C : grad v without dual numbers;
-//   dR/dtheta   the same kernels with the seed on a material constant
+//               transposed face by face, point by point;
+//   dR/dtheta   the residual on forward-mode dual numbers (value + derivative),
+//               with the seed on a material constant
 //               (C10, C01, C20, C30, D1 of one material) or on the scale of one
 //               pressure load;
 //   adjoint     K(u)^T lambda = dJ/du by restarted GMRES, right-preconditioned
@@ -27,7 +22,6 @@
 // order (a follower load's pressure value, a directed load's vector scale).
 #include <cuda_runtime.h>
 
-#include <cstdlib>
 
 #include <algorithm>
 #include <chrono>
@@ -54,7 +48,6 @@ namespace {
 constexpr int kBlock = 128;
 constexpr int kVec = 256;        // threads of the vector kernels
 constexpr int kDotBlocks = 128;  // CTAs per dot product
-constexpr size_t kStoredBytes = size_t(8) << 30;  // most device memory the stored tangents may take
 
 struct TanElemArgs {
     int n, n_free;
@@ -146,123 +139,9 @@ __global__ void __launch_bounds__(kBlock) k_elem_tangent(TanElemArgs a)
     }
 }
 
-// The Gauss-point tangents at a fixed u: C[9 m + p][e NGP + g] = dP_p / dH_m
-// (H = du/dX), one thread per (element, Gauss point, m) with the dual seed
-// on H_m; stored once per adjoint solve so that every Krylov iteration's
-// K_el v is a linear map of grad v instead of a dual-number P(F).
-template <int NEN, int NGP>
-__global__ void __launch_bounds__(kBlock) k_gp_tangent(TanElemArgs a, double* __restrict__ C)
-{
-    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const long long ng = static_cast<long long>(a.n) * NGP;
-    if (idx >= ng * 9) return;
-    const int m = static_cast<int>(idx % 9);
-    const long long eg = idx / 9;
-    const int e = static_cast<int>(eg / NGP), g = static_cast<int>(eg % NGP);
-    double A[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
-    for (int q = 0; q < NEN; q++) {
-        const int node = a.conn[static_cast<size_t>(q) * a.n + e];
-        if (node >= a.n_free) continue;
-        const double* dN = a.dN + (g * NEN + q) * 3;
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const double ui = a.u[3 * node + i];
-#pragma unroll
-            for (int k = 0; k < 3; k++) A[3 * i + k] += ui * dN[k];
-        }
-    }
-    const double* Ji = a.J0inv + (static_cast<size_t>(e) * NGP + g) * 9;
-    Dual H[9];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            H[3 * i + j] = Dual(A[3 * i] * Ji[j] + A[3 * i + 1] * Ji[3 + j] + A[3 * i + 2] * Ji[6 + j], 3 * i + j == m ? 1.0 : 0.0);
-    const MatParams<Dual> mp = a.mats[a.mat[e]];
-    Dual P[9];
-    piola(mp, H, P);
-#pragma unroll
-    for (int p = 0; p < 9; p++) C[static_cast<size_t>(9 * m + p) * ng + eg] = P[p].d;
-}
-
-// out += K_el v from the stored Gauss-point tangents: the phases of
-// k_elem_tangent with dP = C : dH, dH = grad v, in place of the dual P(F).
-template <int NEN, int NGP>
-__global__ void __launch_bounds__(kBlock) k_elem_tangent_stored(TanElemArgs a, const double* __restrict__ C)
-{
-    constexpr int EPB = tan_epb(NGP);
-    constexpr int SV = (NEN * 3) | 1, SS = 9 | 1;
-    __shared__ double s_v[EPB][SV];
-    __shared__ double s_S[EPB][NGP][SS];
-    __shared__ double s_dN[NGP][NEN][3];
-    __shared__ int s_node[EPB][NEN];
-    const int tid = threadIdx.x;
-    for (int i = tid; i < NGP * NEN * 3; i += kBlock) (&s_dN[0][0][0])[i] = a.dN[i];
-    const int e0 = blockIdx.x * EPB;
-    for (int i = tid; i < EPB * NEN; i += kBlock) {
-        const int el = i % EPB, nd = i / EPB, e = e0 + el;
-        int node = a.n_free;
-        double x[3] = { 0, 0, 0 };
-        if (e < a.n) {
-            node = a.conn[static_cast<size_t>(nd) * a.n + e];
-            if (node < a.n_free)
-#pragma unroll
-                for (int c = 0; c < 3; c++) x[c] = a.v[3 * node + c];
-        }
-        s_node[el][nd] = node;
-#pragma unroll
-        for (int c = 0; c < 3; c++) s_v[el][3 * nd + c] = x[c];
-    }
-    __syncthreads();
-    if (tid < EPB * NGP) {
-        const int el = tid / NGP, g = tid % NGP, e = e0 + el;
-        if (e < a.n) {
-            double A[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
-            for (int q = 0; q < NEN; q++)
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int k = 0; k < 3; k++) A[3 * i + k] += s_v[el][3 * q + i] * s_dN[g][q][k];
-            const double* Ji = a.J0inv + (static_cast<size_t>(e) * NGP + g) * 9;
-            double dH[9];
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) dH[3 * i + j] = A[3 * i] * Ji[j] + A[3 * i + 1] * Ji[3 + j] + A[3 * i + 2] * Ji[6 + j];
-            const size_t ng = static_cast<size_t>(a.n) * NGP, eg = static_cast<size_t>(e) * NGP + g;
-            double dP[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
-#pragma unroll
-            for (int mm = 0; mm < 9; mm++)
-#pragma unroll
-                for (int p = 0; p < 9; p++) dP[p] += C[(9 * mm + p) * ng + eg] * dH[mm];
-            const double wv = a.vol[e] * a.gw[g];
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++)
-                    s_S[el][g][3 * i + j] = wv * (dP[3 * i] * Ji[3 * j] + dP[3 * i + 1] * Ji[3 * j + 1] + dP[3 * i + 2] * Ji[3 * j + 2]);
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < EPB * NEN; i += kBlock) {
-        const int el = i % EPB, nd = i / EPB, e = e0 + el;
-        if (e >= a.n) continue;
-        const int node = s_node[el][nd];
-        if (node >= a.n_free) continue;
-        double r[3] = { 0, 0, 0 };
-        for (int g = 0; g < NGP; g++) {
-            const double* d = s_dN[g][nd];
-            const double* S = s_S[el][g];
-#pragma unroll
-            for (int c = 0; c < 3; c++) r[c] += S[3 * c] * d[0] + S[3 * c + 1] * d[1] + S[3 * c + 2] * d[2];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++) atomicAdd(a.out + 3 * node + c, r[c]);
-    }
-}
-
 struct TanFaceArgs {
     int n, n_free;
+    int gmax;                           // most points of a face in the set
     const int* __restrict__ conn;
     const int* __restrict__ table;
     const int* __restrict__ load_idx;
@@ -274,11 +153,311 @@ struct TanFaceArgs {
     const double* __restrict__ t_N;
     const double* __restrict__ t_dN;
     const double* __restrict__ u;
-    const double* __restrict__ v;       // direction (nullptr: none)
+    const double* __restrict__ v;       // direction, or the vector K^T is applied to (nullptr: none)
     const double* __restrict__ dscale;  // per pressure load: derivative of its scale (nullptr: none)
-    const double* __restrict__ w;       // transpose products: the vector K^T is applied to
     double* __restrict__ out;
 };
+
+constexpr int face_epb(int nen) { return nen >= 20 ? 8 : nen >= 8 ? 16 : 32; }
+
+template <int NEN>
+struct TanFaceSmem {
+    static constexpr int EPB = face_epb(NEN);
+    double u[EPB][(NEN * 3) | 1], v[EPB][(NEN * 3) | 1];
+    double q[EPB][(MAX_FGP * 9) | 1];  // per face point: d(cof F A0) or its norm (forward); ds/d(sum_q u_q dN_q) (transpose)
+    int node[EPB][NEN];
+    int table[EPB], ngp[EPB];
+};
+
+// out -= K_face v (transpose: K_face^T v) for one tile of faces, in the phases
+// of the face residual.  With H = du/dX at a face point and cof F = I + B(H),
+//   forward    d(cof F A0) = dB A0, dB the derivative of B along dH = dv/dX;
+//   transpose  s = lambda . (cof F A0) with lambda = sum_q w N_q (p v_q) (for a
+//              directed load lambda = (sum_q w N_q L . v_q) cof F A0 / |cof F A0|):
+//              ds/dH_ij = delta_ij (lambda . A0) - A0_i lambda_j + ([lambda]x H [A0]x^T)_ij
+//              (cof is bilinear: its derivative along E_ij contracts two permutation
+//              symbols), then back through H to the nodes.
+// In place of one pass of dual numbers over the face per unknown (3 NEN of
+// them), or of stored 3 NEN x 3 NEN blocks read in every product.
+template <int NEN>
+__device__ void tan_face_tile(const TanFaceArgs& a, int tile, TanFaceSmem<NEN>& sm, bool transpose)
+{
+    constexpr int EPB = face_epb(NEN);
+    const int tid = threadIdx.x, fb = tile * EPB;
+    if (tid < EPB) {
+        const int t = fb + tid < a.n ? a.table[fb + tid] : 0;
+        sm.table[tid] = t;
+        sm.ngp[tid] = a.t_ngp[t];
+    }
+    for (int i = tid; i < EPB * NEN; i += kBlock) {
+        const int el = i % EPB, q = i / EPB, f = fb + el;
+        int node = a.n_free;
+        double x[3] = { 0, 0, 0 }, y[3] = { 0, 0, 0 };
+        if (f < a.n) {
+            node = a.conn[static_cast<size_t>(q) * a.n + f];
+            if (node < a.n_free)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    x[c] = a.u[3 * node + c];
+                    y[c] = a.v[3 * node + c];
+                }
+        }
+        sm.node[el][q] = node;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            sm.u[el][3 * q + c] = x[c];
+            sm.v[el][3 * q + c] = y[c];
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < EPB * a.gmax; i += kBlock) {
+        const int el = i / a.gmax, g = i - el * a.gmax, f = fb + el;
+        if (f >= a.n) break;
+        if (g >= sm.ngp[el]) continue;
+        const size_t tg = static_cast<size_t>(sm.table[el]) * MAX_FGP + g;
+        const double* dN = a.t_dN + tg * NEN * 3;
+        const double* L = a.load + 4 * f;
+        const bool directed = L[0] != 0.0;
+        double Ji[9], A0[3];
+#pragma unroll
+        for (int k = 0; k < 9; k++) Ji[k] = a.J0inv[(static_cast<size_t>(f) * MAX_FGP + g) * 9 + k];
+#pragma unroll
+        for (int k = 0; k < 3; k++) A0[k] = a.A0[3 * f + k];
+        double A[9] = {}, D[9] = {}, lam[3] = {};
+#pragma unroll 2
+        for (int q = 0; q < NEN; q++) {
+            const double wn = a.t_w[sm.table[el] * MAX_FGP + g] * a.t_N[tg * NEN + q];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                lam[c] += wn * sm.v[el][3 * q + c];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    A[3 * c + k] += sm.u[el][3 * q + c] * dN[3 * q + k];
+                    if (!transpose) D[3 * c + k] += sm.v[el][3 * q + c] * dN[3 * q + k];
+                }
+            }
+        }
+        double H[9];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) H[3 * c + j] = A[3 * c] * Ji[j] + A[3 * c + 1] * Ji[3 + j] + A[3 * c + 2] * Ji[6 + j];
+        Kin<double> k;
+        kinematics(H, k);
+        double cA[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) cA[c] = A0[c] + k.B[3 * c] * A0[0] + k.B[3 * c + 1] * A0[1] + k.B[3 * c + 2] * A0[2];
+        const double nrm = ::sqrt(cA[0] * cA[0] + cA[1] * cA[1] + cA[2] * cA[2]), inrm = nrm > 0.0 ? 1.0 / nrm : 0.0;
+        double* out = sm.q[el] + 9 * g;
+        if (transpose) {
+            if (directed) {
+                const double mu = (L[1] * lam[0] + L[2] * lam[1] + L[3] * lam[2]) * inrm;
+#pragma unroll
+                for (int c = 0; c < 3; c++) lam[c] = mu * cA[c];
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; c++) lam[c] *= L[1];
+            }
+            // T = [lam]x H (rows), G = T [A0]x^T + (lam . A0) I - A0 lam^T
+            double T[9], G[9];
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                T[j] = lam[2] * H[3 + j] - lam[1] * H[6 + j];
+                T[3 + j] = lam[0] * H[6 + j] - lam[2] * H[j];
+                T[6 + j] = lam[1] * H[j] - lam[0] * H[3 + j];
+            }
+            const double la = lam[0] * A0[0] + lam[1] * A0[1] + lam[2] * A0[2];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                G[3 * c] = A0[2] * T[3 * c + 1] - A0[1] * T[3 * c + 2];
+                G[3 * c + 1] = A0[0] * T[3 * c + 2] - A0[2] * T[3 * c];
+                G[3 * c + 2] = A0[1] * T[3 * c] - A0[0] * T[3 * c + 1];
+#pragma unroll
+                for (int j = 0; j < 3; j++) G[3 * c + j] += (c == j ? la : 0.0) - A0[c] * lam[j];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int m = 0; m < 3; m++)
+                    out[3 * c + m] = G[3 * c] * Ji[3 * m] + G[3 * c + 1] * Ji[3 * m + 1] + G[3 * c + 2] * Ji[3 * m + 2];
+        } else {
+            double d[9];
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int j = 0; j < 3; j++) d[3 * c + j] = D[3 * c] * Ji[j] + D[3 * c + 1] * Ji[3 + j] + D[3 * c + 2] * Ji[6 + j];
+            double dA[3];
+            const double t = d[0] + d[4] + d[8];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const int p = 3 * ((c + 1) % 3), q = 3 * ((c + 2) % 3);
+                dA[c] = t * A0[c];
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const int x = (j + 1) % 3, y = (j + 2) % 3;
+                    dA[c] += (d[p + x] * H[q + y] + H[p + x] * d[q + y] - d[p + y] * H[q + x] - H[p + y] * d[q + x] - d[3 * j + c]) * A0[j];
+                }
+            }
+            if (directed) dA[0] = (cA[0] * dA[0] + cA[1] * dA[1] + cA[2] * dA[2]) * inrm;
+#pragma unroll
+            for (int c = 0; c < 3; c++) out[c] = dA[c];
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < EPB * NEN; i += kBlock) {
+        const int el = i % EPB, q = i / EPB, f = fb + el;
+        if (f >= a.n) continue;
+        const int node = sm.node[el][q];
+        if (node >= a.n_free) continue;
+        const int t = sm.table[el], ngp = sm.ngp[el];
+        const double* L = a.load + 4 * f;
+        double s[3] = { 0, 0, 0 };
+        for (int g = 0; g < ngp; g++) {
+            const size_t tg = static_cast<size_t>(t) * MAX_FGP + g;
+            const double* Q = sm.q[el] + 9 * g;
+            if (transpose) {
+                const double* dN = a.t_dN + (tg * NEN + q) * 3;
+                const double d0 = dN[0], d1 = dN[1], d2 = dN[2];
+#pragma unroll
+                for (int c = 0; c < 3; c++) s[c] += Q[3 * c] * d0 + Q[3 * c + 1] * d1 + Q[3 * c + 2] * d2;
+            } else {
+                const double wn = a.t_w[t * MAX_FGP + g] * a.t_N[tg * NEN + q];
+#pragma unroll
+                for (int c = 0; c < 3; c++) s[c] += wn * Q[c];
+            }
+        }
+        if (!transpose) {
+            const bool directed = L[0] != 0.0;
+            const double s0 = s[0];
+#pragma unroll
+            for (int c = 0; c < 3; c++) s[c] = directed ? L[1 + c] * s0 : L[1] * s[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) atomicAdd(a.out + 3 * node + c, -s[c]);
+    }
+}
+
+template <int NEN, int NGP>
+struct TanElemSmem {
+    static constexpr int EPB = tan_epb(NGP);
+    double u[EPB][(NEN * 3) | 1], v[EPB][(NEN * 3) | 1];  // rows of odd length: no bank conflicts over elements
+    double S[EPB][(NGP * 9) | 1];
+    double dN[NGP][(NEN * 3) | 1];
+    int node[EPB][NEN | 1];
+};
+
+// out += K_el v, the derivative of the element residual of residual.cu along
+// v, in its three phases with dP = dP/dH : dH by hand (piola_tangent) in place
+// of dual numbers; the first n_face_tiles CTAs take the faces.  Bound by
+// latency at 16 warps per SM (124 registers) and by FP64 issue.  C3D10 finger,
+// transpose product with the chamber faces: 32 us (cold), where the elements on
+// dual numbers took 77 us (240 registers, 8 warps per SM) and the faces 68 us
+// more; the products of an adjoint solve, which read stored Gauss-point
+// tangents (131 MB) and face blocks, are no slower without them.
+template <int NEN, int NGP, int MT>
+__global__ void __launch_bounds__(kBlock) k_tangent(TanElemArgs a, const MatParams<double>* __restrict__ mats,
+    TanFaceArgs fa, int n_face_tiles, int transpose)
+{
+    constexpr int EPB = tan_epb(NGP);
+    __shared__ union Smem {
+        TanElemSmem<NEN, NGP> e;
+        TanFaceSmem<NEN> f;
+        __device__ Smem() {}
+    } smem;
+    if (static_cast<int>(blockIdx.x) < n_face_tiles) {
+        tan_face_tile<NEN>(fa, blockIdx.x, smem.f, transpose != 0);
+        return;
+    }
+    auto& sm = smem.e;
+    const int tid = threadIdx.x, e0 = (static_cast<int>(blockIdx.x) - n_face_tiles) * EPB;
+    for (int i = tid; i < NGP * NEN * 3; i += kBlock) sm.dN[i / (NEN * 3)][i % (NEN * 3)] = a.dN[i];
+    for (int i = tid; i < EPB * NEN; i += kBlock) {
+        const int el = i % EPB, nd = i / EPB, e = e0 + el;
+        int node = a.n_free;
+        double x[3] = { 0, 0, 0 }, y[3] = { 0, 0, 0 };
+        if (e < a.n) {
+            node = a.conn[static_cast<size_t>(nd) * a.n + e];
+            if (node < a.n_free)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    x[c] = a.u[3 * node + c];
+                    y[c] = a.v[3 * node + c];
+                }
+        }
+        sm.node[el][nd] = node;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            sm.u[el][3 * nd + c] = x[c];
+            sm.v[el][3 * nd + c] = y[c];
+        }
+    }
+    __syncthreads();
+    if (tid < EPB * NGP) {
+        const int el = tid / NGP, g = tid % NGP, e = e0 + el;
+        if (e < a.n) {
+            const double* Jp = a.J0inv + (static_cast<size_t>(e) * NGP + g) * 9;
+            double H[9], dH[9];
+            {
+                double Ji[9], A[9] = {}, D[9] = {};
+#pragma unroll
+                for (int k = 0; k < 9; k++) Ji[k] = __ldg(Jp + k);
+#pragma unroll 2
+                for (int q = 0; q < NEN; q++)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        const double d = sm.dN[g][3 * q + k];
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            A[3 * i + k] += sm.u[el][3 * q + i] * d;
+                            D[3 * i + k] += sm.v[el][3 * q + i] * d;
+                        }
+                    }
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        H[3 * i + j] = A[3 * i] * Ji[j] + A[3 * i + 1] * Ji[3 + j] + A[3 * i + 2] * Ji[6 + j];
+                        dH[3 * i + j] = D[3 * i] * Ji[j] + D[3 * i + 1] * Ji[3 + j] + D[3 * i + 2] * Ji[6 + j];
+                    }
+            }
+            double dP[9];
+            piola_tangent<MT>(mats[__ldg(a.mat + e)], H, dH, dP);
+            const double wv = __ldg(a.vol + e) * __ldg(a.gw + g);
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const double j0 = __ldg(Jp + 3 * j), j1 = __ldg(Jp + 3 * j + 1), j2 = __ldg(Jp + 3 * j + 2);
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+                    sm.S[el][9 * g + 3 * i + j] = wv * (dP[3 * i] * j0 + dP[3 * i + 1] * j1 + dP[3 * i + 2] * j2);
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < EPB * NEN; i += kBlock) {
+        const int el = i % EPB, nd = i / EPB, e = e0 + el;
+        if (e >= a.n) continue;
+        const int node = sm.node[el][nd];
+        if (node >= a.n_free) continue;
+        double r[3] = { 0, 0, 0 };
+#pragma unroll 2
+        for (int g = 0; g < NGP; g++) {
+            const double d0 = sm.dN[g][3 * nd], d1 = sm.dN[g][3 * nd + 1], d2 = sm.dN[g][3 * nd + 2];
+            const double* S = sm.S[el] + 9 * g;
+#pragma unroll
+            for (int c = 0; c < 3; c++) r[c] += S[3 * c] * d0 + S[3 * c + 1] * d1 + S[3 * c + 2] * d2;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) atomicAdd(a.out + 3 * node + c, r[c]);
+    }
+}
+
+// faces without an element block of their kind to go with
+template <int NEN>
+__global__ void __launch_bounds__(kBlock) k_tangent_faces(TanFaceArgs a, int transpose)
+{
+    __shared__ TanFaceSmem<NEN> sm;
+    tan_face_tile<NEN>(a, blockIdx.x, sm, transpose != 0);
+}
 
 // Nodal forces f_q (all NEN nodes, dual) of face f with node displacements uu,
 // as in the face residual of residual.cu; the load value's derivative is
@@ -357,91 +536,6 @@ __global__ void __launch_bounds__(kBlock) k_face_tangent(TanFaceArgs a)
 #pragma unroll
         for (int c = 0; c < 3; c++) atomicAdd(a.out + 3 * node[q] + c, -fq[q][c].d);
     }
-}
-
-// out_j -= sum_i w_i d f_i / d u_j for every free unknown j of every face:
-// one thread per (face, local unknown), the seed on that unknown
-template <int NEN>
-__global__ void __launch_bounds__(kBlock) k_face_transpose(TanFaceArgs a)
-{
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f = idx / (3 * NEN), j = idx % (3 * NEN);
-    if (f >= a.n) return;
-    const int qj = j / 3, cj = j % 3;
-    int node[NEN];
-    Dual uu[NEN][3];
-    for (int q = 0; q < NEN; q++) {
-        node[q] = a.conn[static_cast<size_t>(q) * a.n + f];
-        const bool fr = node[q] < a.n_free;
-#pragma unroll
-        for (int c = 0; c < 3; c++) uu[q][c] = fr ? Dual(a.u[3 * node[q] + c], (q == qj && c == cj) ? 1.0 : 0.0) : Dual(0.0);
-    }
-    if (node[qj] >= a.n_free) return;
-    Dual fq[NEN][3];
-    face_forces<NEN>(a, f, uu, fq);
-    double s = 0.0;
-    for (int q = 0; q < NEN; q++) {
-        if (node[q] >= a.n_free) continue;
-#pragma unroll
-        for (int c = 0; c < 3; c++) s += a.w[3 * node[q] + c] * fq[q][c].d;
-    }
-    atomicAdd(a.out + 3 * node[qj] + cj, -s);
-}
-
-// The face tangent blocks at a fixed u: blk[f][i][j] = d f_i / d u_j over the
-// 3 NEN local unknowns (rows i of fixed nodes are 0; columns j of fixed nodes
-// are not written).  One thread per (face, local unknown j), seeded as in
-// k_face_transpose, so each block costs one set of dual passes per adjoint
-// solve instead of one per Krylov iteration.
-template <int NEN>
-__global__ void __launch_bounds__(kBlock) k_face_block(TanFaceArgs a, double* __restrict__ blk)
-{
-    constexpr int ND = 3 * NEN;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f = idx / ND, j = idx % ND;
-    if (f >= a.n) return;
-    const int qj = j / 3, cj = j % 3;
-    int node[NEN];
-    Dual uu[NEN][3];
-    for (int q = 0; q < NEN; q++) {
-        node[q] = a.conn[static_cast<size_t>(q) * a.n + f];
-        const bool fr = node[q] < a.n_free;
-#pragma unroll
-        for (int c = 0; c < 3; c++) uu[q][c] = fr ? Dual(a.u[3 * node[q] + c], (q == qj && c == cj) ? 1.0 : 0.0) : Dual(0.0);
-    }
-    if (node[qj] >= a.n_free) return;
-    Dual fq[NEN][3];
-    face_forces<NEN>(a, f, uu, fq);
-    double* b = blk + static_cast<size_t>(f) * ND * ND + j;
-    for (int q = 0; q < NEN; q++) {
-        const bool fr = node[q] < a.n_free;
-#pragma unroll
-        for (int c = 0; c < 3; c++) b[(3 * q + c) * ND] = fr ? fq[q][c].d : 0.0;
-    }
-}
-
-// out_j -= sum_i w_i blk[f][i][j]: the transpose product of k_face_transpose
-// from the stored blocks, one thread per (face, local unknown j); a warp's
-// reads of row i are consecutive in j.
-template <int NEN>
-__global__ void __launch_bounds__(kBlock) k_face_block_apply(TanFaceArgs a, const double* __restrict__ blk)
-{
-    constexpr int ND = 3 * NEN;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f = idx / ND, j = idx % ND;
-    if (f >= a.n) return;
-    const int nj = a.conn[static_cast<size_t>(j / 3) * a.n + f];
-    if (nj >= a.n_free) return;
-    const double* b = blk + static_cast<size_t>(f) * ND * ND + j;
-    double s0 = 0.0, s1 = 0.0;
-    for (int q = 0; q < NEN; q++) {
-        const int nq = a.conn[static_cast<size_t>(q) * a.n + f];
-        if (nq >= a.n_free) continue;
-        const double* wq = a.w + 3 * nq;
-        s0 += wq[0] * b[(3 * q) * ND] + wq[2] * b[(3 * q + 2) * ND];
-        s1 += wq[1] * b[(3 * q + 1) * ND];
-    }
-    atomicAdd(a.out + 3 * nj + j % 3, -(s0 + s1));
 }
 
 // ---------------------------------------------------------------- vectors
@@ -582,11 +676,6 @@ struct AdjointWS {
     int mats_seed = -2;  // the seed `mats` holds: 5 slot + k, -1 none, -2 not uploaded
     double* dscale = nullptr;
     std::vector<double> h_part;
-    // stored tangents at u, used while blocks_ready is set (inside one adjoint
-    // solve): per face set the face blocks (k_face_block), per element block
-    // the Gauss-point tangents (k_gp_tangent)
-    std::vector<double*> fblk, gpt;
-    bool blocks_ready = false;
 };
 
 void free_adjoint(Model& m)
@@ -597,8 +686,6 @@ void free_adjoint(Model& m)
         dev_free(*p);
     if (w.mats) cudaFree(w.mats);
     if (w.h_hcol) cudaFreeHost(w.h_hcol);
-    for (double*& p : w.fblk) dev_free(p);
-    for (double*& p : w.gpt) dev_free(p);
     delete m.aws;
     m.aws = nullptr;
 }
@@ -656,183 +743,102 @@ efem_status upload_dual_mats(Model& m, int slot, int k)
     return EFEM_OK;
 }
 
-// out += K_el v (dual kernels; from the stored Gauss-point tangents when
-// stored is set, which needs v and blocks_ready), or dR/dtheta with v = nullptr
-void launch_elem_tangent(Model& m, const double* u, const double* v, double* out, bool stored = false)
+// out += dR/dtheta of the elements (dual numbers, the seed in the material table)
+void launch_elem_param(Model& m, const double* u, double* out)
 {
-    for (size_t bi = 0; bi < m.blocks.size(); bi++) {
-        auto& b = m.blocks[bi];
+    for (auto& b : m.blocks) {
         if (b.n == 0) continue;
-        TanElemArgs a { b.n, m.n_free, b.conn, b.mat, b.vol, b.J0inv, b.dN, b.gw, m.aws->mats, u, v, out };
-        const double* C = stored ? m.aws->gpt[bi] : nullptr;
-        auto go = [&](auto kern, auto kern_stored, int ngp) {
-            const int epb = tan_epb(ngp);
-            if (C) kern_stored<<<(b.n + epb - 1) / epb, kBlock, 0, m.stream>>>(a, C);
-            else kern<<<(b.n + epb - 1) / epb, kBlock, 0, m.stream>>>(a);
-            m.launches++;
+        TanElemArgs a { b.n, m.n_free, b.conn, b.mat, b.vol, b.J0inv, b.dN, b.gw, m.aws->mats, u, nullptr, out };
+        const int epb = tan_epb(b.ngp), grid = (b.n + epb - 1) / epb;
+        m.launches++;
+        if (b.nen == 4 && b.ngp == 1) k_elem_tangent<4, 1><<<grid, kBlock, 0, m.stream>>>(a);
+        else if (b.nen == 10 && b.ngp == 4) k_elem_tangent<10, 4><<<grid, kBlock, 0, m.stream>>>(a);
+        else if (b.nen == 10 && b.ngp == 1) k_elem_tangent<10, 1><<<grid, kBlock, 0, m.stream>>>(a);
+        else if (b.nen == 8 && b.ngp == 8) k_elem_tangent<8, 8><<<grid, kBlock, 0, m.stream>>>(a);
+        else if (b.nen == 8 && b.ngp == 1) k_elem_tangent<8, 1><<<grid, kBlock, 0, m.stream>>>(a);
+        else if (b.nen == 20 && b.ngp == 27) k_elem_tangent<20, 27><<<grid, kBlock, 0, m.stream>>>(a);
+        else if (b.nen == 20 && b.ngp == 8) k_elem_tangent<20, 8><<<grid, kBlock, 0, m.stream>>>(a);
+    }
+}
+
+TanFaceArgs tan_face_args(const Model& m, const DevFaces& f, const double* u, const double* v, const double* dscale,
+    double* out)
+{
+    return TanFaceArgs { f.n, m.n_free, *std::max_element(f.h_ngp.begin(), f.h_ngp.end()), f.conn, f.table, f.load_idx,
+        f.A0, f.J0inv, f.load, f.t_ngp, f.t_w, f.t_N, f.t_dN, u, v, dscale, out };
+}
+
+// out -= dF/dscale
+void launch_face_param(Model& m, const double* u, const double* dscale, double* out)
+{
+    for (auto& f : m.faces) {
+        if (f.n == 0) continue;
+        const TanFaceArgs a = tan_face_args(m, f, u, nullptr, dscale, out);
+        const int grid = (f.n + kBlock - 1) / kBlock;
+        m.launches++;
+        switch (f.nen) {
+        case 4: k_face_tangent<4><<<grid, kBlock, 0, m.stream>>>(a); break;
+        case 8: k_face_tangent<8><<<grid, kBlock, 0, m.stream>>>(a); break;
+        case 10: k_face_tangent<10><<<grid, kBlock, 0, m.stream>>>(a); break;
+        case 20: k_face_tangent<20><<<grid, kBlock, 0, m.stream>>>(a); break;
+        }
+    }
+}
+
+// out += K v (transpose: K^T v): every element block's launch carries the faces of its kind
+void launch_tangent(Model& m, const double* u, const double* v, double* out, bool transpose)
+{
+    std::vector<char> done(m.faces.size(), 0);
+    for (auto& b : m.blocks) {
+        if (b.n == 0) continue;
+        TanElemArgs a { b.n, m.n_free, b.conn, b.mat, b.vol, b.J0inv, b.dN, b.gw, nullptr, u, v, out };
+        TanFaceArgs fa {};
+        int ft = 0;
+        for (size_t fs = 0; fs < m.faces.size(); fs++)
+            if (!done[fs] && m.faces[fs].n > 0 && m.faces[fs].nen == b.nen) {
+                fa = tan_face_args(m, m.faces[fs], u, v, nullptr, out);
+                ft = (fa.n + face_epb(b.nen) - 1) / face_epb(b.nen);
+                done[fs] = 1;
+            }
+        const int epb = tan_epb(b.ngp), grid = ft + (b.n + epb - 1) / epb;
+        m.launches++;
+        auto go = [&](auto nh, auto mr, auto yeoh, auto any) {
+            auto* k = b.mat_type == EFEM_NEO_HOOKEAN ? nh : b.mat_type == EFEM_MOONEY_RIVLIN ? mr : b.mat_type == EFEM_YEOH ? yeoh : any;
+            k<<<grid, kBlock, 0, m.stream>>>(a, m.d_mats, fa, ft, transpose ? 1 : 0);
         };
-#define EFEM_TAN(NEN, NGP) go(k_elem_tangent<NEN, NGP>, k_elem_tangent_stored<NEN, NGP>, NGP)
-        if (b.nen == 4 && b.ngp == 1) EFEM_TAN(4, 1);
-        else if (b.nen == 10 && b.ngp == 4) EFEM_TAN(10, 4);
-        else if (b.nen == 10 && b.ngp == 1) EFEM_TAN(10, 1);
-        else if (b.nen == 8 && b.ngp == 8) EFEM_TAN(8, 8);
-        else if (b.nen == 8 && b.ngp == 1) EFEM_TAN(8, 1);
-        else if (b.nen == 20 && b.ngp == 27) EFEM_TAN(20, 27);
-        else if (b.nen == 20 && b.ngp == 8) EFEM_TAN(20, 8);
+#define EFEM_TAN(NEN, NGP)                                                                              \
+    if (b.nen == NEN && b.ngp == NGP)                                                                   \
+        go(k_tangent<NEN, NGP, EFEM_NEO_HOOKEAN>, k_tangent<NEN, NGP, EFEM_MOONEY_RIVLIN>,              \
+            k_tangent<NEN, NGP, EFEM_YEOH>, k_tangent<NEN, NGP, -1>);
+        EFEM_TAN(4, 1)
+        EFEM_TAN(10, 4)
+        EFEM_TAN(10, 1)
+        EFEM_TAN(8, 8)
+        EFEM_TAN(8, 1)
+        EFEM_TAN(20, 27)
+        EFEM_TAN(20, 8)
 #undef EFEM_TAN
     }
-}
-
-// mode 0: out -= K_face v;  1: out -= dF/dscale;  2: out -= K_face^T w
-void launch_face_tangent(Model& m, const double* u, const double* v, const double* dscale, const double* w,
-    double* out, bool transpose)
-{
-    const AdjointWS* ws = m.aws;
     for (size_t fs = 0; fs < m.faces.size(); fs++) {
-        auto& f = m.faces[fs];
-        if (f.n == 0) continue;
-        TanFaceArgs a { f.n, m.n_free, f.conn, f.table, f.load_idx, f.A0, f.J0inv, f.load, f.t_ngp, f.t_w, f.t_N,
-            f.t_dN, u, v, dscale, w, out };
-        const int nthreads = transpose ? f.n * 3 * f.nen : f.n;
-        const int grid = (nthreads + kBlock - 1) / kBlock;
-        const double* blk = transpose && ws && ws->blocks_ready ? ws->fblk[fs] : nullptr;
+        const DevFaces& f = m.faces[fs];
+        if (done[fs] || f.n == 0) continue;
+        const TanFaceArgs a = tan_face_args(m, f, u, v, nullptr, out);
+        const int grid = (f.n + face_epb(f.nen) - 1) / face_epb(f.nen), tr = transpose ? 1 : 0;
         m.launches++;
         switch (f.nen) {
-        case 4:
-            if (blk) k_face_block_apply<4><<<grid, kBlock, 0, m.stream>>>(a, blk);
-            else if (transpose) k_face_transpose<4><<<grid, kBlock, 0, m.stream>>>(a);
-            else k_face_tangent<4><<<grid, kBlock, 0, m.stream>>>(a);
-            break;
-        case 8:
-            if (blk) k_face_block_apply<8><<<grid, kBlock, 0, m.stream>>>(a, blk);
-            else if (transpose) k_face_transpose<8><<<grid, kBlock, 0, m.stream>>>(a);
-            else k_face_tangent<8><<<grid, kBlock, 0, m.stream>>>(a);
-            break;
-        case 10:
-            if (blk) k_face_block_apply<10><<<grid, kBlock, 0, m.stream>>>(a, blk);
-            else if (transpose) k_face_transpose<10><<<grid, kBlock, 0, m.stream>>>(a);
-            else k_face_tangent<10><<<grid, kBlock, 0, m.stream>>>(a);
-            break;
-        case 20:
-            if (blk) k_face_block_apply<20><<<grid, kBlock, 0, m.stream>>>(a, blk);
-            else if (transpose) k_face_transpose<20><<<grid, kBlock, 0, m.stream>>>(a);
-            else k_face_tangent<20><<<grid, kBlock, 0, m.stream>>>(a);
-            break;
+        case 4: k_tangent_faces<4><<<grid, kBlock, 0, m.stream>>>(a, tr); break;
+        case 8: k_tangent_faces<8><<<grid, kBlock, 0, m.stream>>>(a, tr); break;
+        case 10: k_tangent_faces<10><<<grid, kBlock, 0, m.stream>>>(a, tr); break;
+        case 20: k_tangent_faces<20><<<grid, kBlock, 0, m.stream>>>(a, tr); break;
         }
     }
 }
 
-// Out of device memory for the stored tangents: free them and go on with the
-// dual-number products (blocks_ready stays unset).
-efem_status drop_stored(AdjointWS& w)
-{
-    for (double*& p : w.fblk) dev_free(p);
-    for (double*& p : w.gpt) dev_free(p);
-    w.blocks_ready = false;
-    return EFEM_OK;
-}
-
-// Device memory for stored tangents.  Running out of memory is not an error
-// (*oom is set and the caller falls back to the dual-number products); any
-// other failure is.  The environment variable EFEM_TEST_STORED_OOM=1 makes
-// every such allocation report out of memory, so that tests reach the
-// fallback without filling the GPU.
-efem_status stored_alloc(double** p, size_t n, bool* oom)
-{
-    *p = nullptr;
-    *oom = false;
-    if (n == 0) return EFEM_OK;
-    const char* force = std::getenv("EFEM_TEST_STORED_OOM");
-    if (force && force[0] == '1') {
-        *oom = true;
-        return EFEM_OK;
-    }
-    const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), n * sizeof(double));
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();  // not sticky: clear it so that later checks do not see it
-        *p = nullptr;
-        *oom = true;
-        return EFEM_OK;
-    }
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        set_error(std::string("cudaMalloc of the stored tangents: ") + cudaGetErrorString(e));
-        return EFEM_ERR_CUDA;
-    }
-    return EFEM_OK;
-}
-
-// The stored tangents at u for the Krylov iterations of one adjoint solve:
-// the face blocks of every face set and the Gauss-point tangents of every
-// element block.  Sets blocks_ready only when all of them fit in
-// kStoredBytes and in device memory; otherwise every product recomputes them
-// on dual numbers.
-efem_status build_stored_tangents(Model& m, const double* u)
-{
-    AdjointWS& w = *m.aws;
-    w.blocks_ready = false;
-    size_t total = 0;
-    for (auto& f : m.faces) total += sizeof(double) * f.n * static_cast<size_t>(9 * f.nen * f.nen);
-    for (auto& b : m.blocks) total += sizeof(double) * b.n * static_cast<size_t>(81 * b.ngp);
-    if (total == 0 || total > kStoredBytes) return EFEM_OK;
-    w.gpt.resize(m.blocks.size(), nullptr);
-    for (size_t bi = 0; bi < m.blocks.size(); bi++) {
-        auto& b = m.blocks[bi];
-        if (b.n == 0) continue;
-        const long long nthreads = 9LL * b.n * b.ngp;
-        if (!w.gpt[bi]) {
-            bool oom = false;
-            const efem_status as = stored_alloc(&w.gpt[bi], static_cast<size_t>(9 * nthreads), &oom);
-            if (as != EFEM_OK) return as;
-            if (oom) return drop_stored(w);
-        }
-        TanElemArgs a { b.n, m.n_free, b.conn, b.mat, b.vol, b.J0inv, b.dN, b.gw, w.mats, u, nullptr, nullptr };
-        const unsigned grid = static_cast<unsigned>((nthreads + kBlock - 1) / kBlock);
-        double* C = w.gpt[bi];
-        m.launches++;
-        if (b.nen == 4 && b.ngp == 1) k_gp_tangent<4, 1><<<grid, kBlock, 0, m.stream>>>(a, C);
-        else if (b.nen == 10 && b.ngp == 4) k_gp_tangent<10, 4><<<grid, kBlock, 0, m.stream>>>(a, C);
-        else if (b.nen == 10 && b.ngp == 1) k_gp_tangent<10, 1><<<grid, kBlock, 0, m.stream>>>(a, C);
-        else if (b.nen == 8 && b.ngp == 8) k_gp_tangent<8, 8><<<grid, kBlock, 0, m.stream>>>(a, C);
-        else if (b.nen == 8 && b.ngp == 1) k_gp_tangent<8, 1><<<grid, kBlock, 0, m.stream>>>(a, C);
-        else if (b.nen == 20 && b.ngp == 27) k_gp_tangent<20, 27><<<grid, kBlock, 0, m.stream>>>(a, C);
-        else if (b.nen == 20 && b.ngp == 8) k_gp_tangent<20, 8><<<grid, kBlock, 0, m.stream>>>(a, C);
-    }
-    w.fblk.resize(m.faces.size(), nullptr);
-    for (size_t fs = 0; fs < m.faces.size(); fs++) {
-        auto& f = m.faces[fs];
-        if (f.n == 0) continue;
-        if (!w.fblk[fs]) {
-            bool oom = false;
-            const efem_status as = stored_alloc(&w.fblk[fs], f.n * static_cast<size_t>(9 * f.nen * f.nen), &oom);
-            if (as != EFEM_OK) return as;
-            if (oom) return drop_stored(w);
-        }
-        TanFaceArgs a { f.n, m.n_free, f.conn, f.table, f.load_idx, f.A0, f.J0inv, f.load, f.t_ngp, f.t_w, f.t_N,
-            f.t_dN, u, nullptr, nullptr, nullptr, nullptr };
-        const int grid = (f.n * 3 * f.nen + kBlock - 1) / kBlock;
-        m.launches++;
-        switch (f.nen) {
-        case 4: k_face_block<4><<<grid, kBlock, 0, m.stream>>>(a, w.fblk[fs]); break;
-        case 8: k_face_block<8><<<grid, kBlock, 0, m.stream>>>(a, w.fblk[fs]); break;
-        case 10: k_face_block<10><<<grid, kBlock, 0, m.stream>>>(a, w.fblk[fs]); break;
-        case 20: k_face_block<20><<<grid, kBlock, 0, m.stream>>>(a, w.fblk[fs]); break;
-        }
-    }
-    EFEM_CUDA(cudaGetLastError());
-    w.blocks_ready = true;
-    return EFEM_OK;
-}
-
-// out = K(u) v  (transpose: K(u)^T v); device pointers; dual materials without seeds uploaded
+// out = K(u) v  (transpose: K(u)^T v); device pointers
 efem_status tangent(Model& m, const double* u, const double* v, double* out, bool transpose)
 {
     EFEM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 3 * m.n_free, m.stream));
-    launch_elem_tangent(m, u, v, out, m.aws->blocks_ready);
-    if (transpose)
-        launch_face_tangent(m, u, nullptr, nullptr, v, out, true);
-    else
-        launch_face_tangent(m, u, v, nullptr, nullptr, out, false);
+    launch_tangent(m, u, v, out, transpose);
     EFEM_CUDA(cudaGetLastError());
     return EFEM_OK;
 }
@@ -845,14 +851,14 @@ efem_status param_derivative(Model& m, const double* u, int k, double* out)
     if (k < 5 * nm) {
         efem_status s = upload_dual_mats(m, k / 5, k % 5);
         if (s != EFEM_OK) return s;
-        launch_elem_tangent(m, u, nullptr, out);
+        launch_elem_param(m, u, out);
         s = upload_dual_mats(m, -1, 0);
         if (s != EFEM_OK) return s;
     } else {
         std::vector<double> ds(std::max(m.n_pressure_loads, 1), 0.0);
         ds[k - 5 * nm] = 1.0;
         EFEM_CUDA(cudaMemcpyAsync(m.aws->dscale, ds.data(), sizeof(double) * ds.size(), cudaMemcpyHostToDevice, m.stream));
-        launch_face_tangent(m, u, nullptr, m.aws->dscale, nullptr, out, false);
+        launch_face_param(m, u, m.aws->dscale, out);
         // synchronise before ds goes out of scope
         EFEM_CUDA(cudaStreamSynchronize(m.stream));
     }
@@ -896,9 +902,8 @@ efem_status adjoint_gmres(Model& m, const double* u, double tol, int max_it, int
     const size_t n = w.n;
     const int R = w.restart;
     // algorithmic bytes of one Krylov iteration: the basis copy, H0, the
-    // transpose tangent (element part as an FP64 residual plus v and the zeroed
-    // output, plus the stored Gauss-point tangents; the stored face blocks or,
-    // without them, the faces' residual bytes), the norm and the scaling; plus
+    // transpose tangent (an FP64 residual plus v and the zeroed output), the
+    // norm and the scaling; plus
     // two Gram-Schmidt passes over the j + 1 basis vectors (dots: the basis and
     // w; updates: the basis, w read and written)
     const double nd = 8.0 * static_cast<double>(n);
@@ -906,14 +911,9 @@ efem_status adjoint_gmres(Model& m, const double* u, double tol, int max_it, int
     precond_info(m, &mi);
     long long rb = 0;
     double rf = 0.0;
-    residual_work(m, 8, &rb, &rf, !w.blocks_ready);
-    double fb = 0.0;
-    if (w.blocks_ready) {
-        for (auto& f : m.faces) fb += static_cast<double>(f.n) * (72.0 * f.nen * f.nen + 4.0 * f.nen);
-        for (auto& b : m.blocks) fb += static_cast<double>(b.n) * b.ngp * 81.0 * 8.0;
-    }
+    residual_work(m, 8, &rb, &rf, true);
     const double it_bytes = 2.0 * nd + 16.0 * static_cast<double>(mi.factor_nnz) + 5.0 * nd + static_cast<double>(rb) +
-        2.0 * nd + fb + 3.0 * nd;
+        2.0 * nd + 3.0 * nd;
     *bytes = 0.0;
     double bnorm = 0.0;
     efem_status s = dots(m, w.b, 1, w.b, &bnorm);
@@ -1067,9 +1067,7 @@ efem_status adjoint(Model& m, const double* d_u, const double* d_dJdu, double* d
     const int max_it = m.opts.adjoint_max_iterations > 0 ? m.opts.adjoint_max_iterations : 2000;
     int iters = 0;
     double rel = 0.0;
-    if ((s = build_stored_tangents(m, w.u)) != EFEM_OK) return s;
     s = adjoint_gmres(m, w.u, tol, max_it, &iters, &rel, &info->solve_bytes);
-    w.blocks_ready = false;  // the blocks hold K at this u only
     if (s != EFEM_OK) return s;
     info->iterations = iters;
     info->rel_residual = rel;

@@ -145,4 +145,97 @@ __device__ __forceinline__ void piola(const MatParams<T>& mp, const T* H, T* P)
     }
 }
 
+// dP = dP/dH : dH at F = I + H, the laws of piola() differentiated by hand:
+// the forward-mode dual numbers of the same expressions carry the zero
+// derivatives of every constant through each product.  Finite wherever piola()
+// is (J < 0 included: d J^{-2/3} = -2/3 J^{-2/3} dJ / J).
+template <int MT = -1>
+__device__ __forceinline__ void piola_tangent(const MatParams<double>& mp, const double* H, const double* dH, double* dP)
+{
+    const bool yeoh = MT == EFEM_YEOH || (MT < 0 && mp.type == EFEM_YEOH);
+    const bool mr = MT == EFEM_MOONEY_RIVLIN || (MT < 0 && mp.type == EFEM_MOONEY_RIVLIN);
+    Kin<double> k;
+    kinematics(H, k);
+    // dB = tr(dH) I - dH^T + d cof(H); the rows of cof are cross products of the others
+    double dB[9];
+    {
+        const double t = dH[0] + dH[4] + dH[8];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int p = 3 * ((i + 1) % 3), q = 3 * ((i + 2) % 3);
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int a = (j + 1) % 3, b = (j + 2) % 3;
+                dB[3 * i + j] = (i == j ? t : 0.0) - dH[3 * j + i] + (dH[p + a] * H[q + b] + H[p + a] * dH[q + b])
+                    - (dH[p + b] * H[q + a] + H[p + b] * dH[q + a]);
+            }
+        }
+    }
+    // d(J - 1) = cof F : dH, d(I1 - 3) = 2 F : dH
+    double dd = dH[0] + dH[4] + dH[8], da = dd;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        dd += k.B[i] * dH[i];
+        da += H[i] * dH[i];
+    }
+    da *= 2.0;
+    const double J = 1.0 + k.delta;
+    const double rc = drcbrt(J), Jm23 = rc * rc, iJ = 1.0 / J;
+    const double dJm23 = (-2.0 / 3.0) * Jm23 * iJ * dd;
+    const double cm1 = (k.a * (1.0 / 3.0) - k.delta) * iJ, c = 1.0 + cm1;
+    const double dc = (da * (1.0 / 3.0) - dd) * iJ - cm1 * iJ * dd;
+    double coef = mp.C10, dcoef = 0.0;
+    if (yeoh) {
+        const double y = J * Jm23;
+        const double t = 3.0 * (-k.delta * (y + 1.0) * Jm23 / (y * y + y + 1.0)) + k.a * Jm23;
+        const double dt = Jm23 * da + (3.0 + k.a) * dJm23;
+        coef = mp.C10 + 2.0 * mp.C20 * t + 3.0 * mp.C30 * t * t;
+        dcoef = (2.0 * mp.C20 + 6.0 * mp.C30 * t) * dt;
+    }
+    const double s1 = 2.0 * coef * Jm23, ds1 = 2.0 * (dcoef * Jm23 + coef * dJm23);
+    const double vol = 2.0 / mp.D1 * k.delta, dvol = 2.0 / mp.D1 * dd;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        const double id = (i % 4 == 0) ? 1.0 : 0.0;
+        dP[i] = ds1 * (H[i] - cm1 * id - c * k.B[i]) + s1 * (dH[i] - dc * id - dc * k.B[i] - c * dB[i])
+            + dvol * (id + k.B[i]) + vol * dB[i];
+    }
+    if (mr) {
+        double E[9], dE[9];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                E[3 * i + j] = H[3 * i + j] + H[3 * j + i] + H[i] * H[j] + H[3 + i] * H[3 + j] + H[6 + i] * H[6 + j];
+                dE[3 * i + j] = dH[3 * i + j] + dH[3 * j + i] + dH[i] * H[j] + dH[3 + i] * H[3 + j] + dH[6 + i] * H[6 + j]
+                    + H[i] * dH[j] + H[3 + i] * dH[3 + j] + H[6 + i] * dH[6 + j];
+            }
+        const double t = E[0] + E[4] + E[8], dt = dE[0] + dE[4] + dE[8];
+        double ee = 0.0, de = 0.0;
+#pragma unroll
+        for (int i = 0; i < 9; i++) {
+            ee += E[i] * E[i];
+            de += E[i] * dE[i];
+        }
+        const double i2 = 2.0 * t + 0.5 * (t * t - ee), di2 = 2.0 * dt + t * dt - de;
+        const double c2m1 = (i2 * (1.0 / 3.0) - k.delta) * iJ, c2 = 1.0 + c2m1;
+        const double dc2 = (di2 * (1.0 / 3.0) - dd) * iJ - c2m1 * iJ * dd;
+        const double s2 = mp.C01 * Jm23 * Jm23, ds2 = 2.0 * mp.C01 * Jm23 * dJm23;
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int e = 3 * i + j;
+                const double id = (i == j) ? 1.0 : 0.0;
+                const double HE = H[3 * i] * E[j] + H[3 * i + 1] * E[3 + j] + H[3 * i + 2] * E[6 + j];
+                const double dHE = dH[3 * i] * E[j] + dH[3 * i + 1] * E[3 + j] + dH[3 * i + 2] * E[6 + j] + H[3 * i] * dE[j]
+                    + H[3 * i + 1] * dE[3 + j] + H[3 * i + 2] * dE[6 + j];
+                const double q = 2.0 * (t * id - E[e] + (2.0 + t) * H[e] - HE) - 4.0 * c2m1 * id - 4.0 * c2 * k.B[e];
+                const double dq = 2.0 * (dt * id - dE[e] + dt * H[e] + (2.0 + t) * dH[e] - dHE) - 4.0 * dc2 * id
+                    - 4.0 * dc2 * k.B[e] - 4.0 * c2 * dB[e];
+                dP[e] += ds2 * q + s2 * dq;
+            }
+    }
+}
+
 }  // namespace efem

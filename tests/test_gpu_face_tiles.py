@@ -36,6 +36,26 @@ def test_residual_with_faces(etype, n, load, tmp_path):
         assert np.linalg.norm(r - ref) <= 1e-12 * np.linalg.norm(ref), threads
 
 
+@pytest.mark.parametrize("etype,n", [("C3D4", (1, 4, 4)), ("C3D4", (1, 3, 11)), ("C3D8", (1, 3, 11)), ("C3D10", (1, 2, 4)),
+                                     ("C3D10", (1, 3, 3)), ("C3D20", (2, 1, 1)), ("C3D20", (1, 3, 3))])
+@pytest.mark.parametrize("law", ["nh", "mr", "yeoh"])
+@pytest.mark.parametrize("load", ["pressure", "dpressure"])
+def test_tangent_with_faces(etype, n, law, load):
+    """K(u) v against central differences of R (truncation h^2 with h |v| about
+    1e-8 m on 1e-2 m elements, cancellation eps |R| / h: 1e-6 relative holds
+    both), and w.(K v) = (K^T w).v to rounding."""
+    case = mg.small_case(etype, law, load, n=n, size=tuple(0.01 * k for k in n))
+    m = api.Model.from_case(case)
+    u = displaced(case)
+    rng = np.random.default_rng(11)
+    v, w = rng.normal(size=u.size), rng.normal(size=u.size)
+    kv, ktw = m.hvp(u, v), m.hvp(u, w, transpose=True)
+    h = 1e-8
+    fd = (m.residual(u + h * v) - m.residual(u - h * v)) / (2 * h)
+    assert np.linalg.norm(kv - fd) <= 1e-6 * np.linalg.norm(kv)
+    assert abs(float(w @ kv) - float(ktw @ v)) <= 1e-12 * np.linalg.norm(kv) * np.linalg.norm(w)
+
+
 def test_faces_of_elements_without_a_material():
     """Two separate hexahedra, the loaded one without a material: its faces
     have no element launch to go with (the other block holds tetrahedra)."""
