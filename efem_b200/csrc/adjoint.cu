@@ -48,6 +48,7 @@ namespace {
 constexpr int kBlock = 128;
 constexpr int kVec = 256;        // threads of the vector kernels
 constexpr int kDotBlocks = 128;  // CTAs per dot product
+constexpr int kRestart = 100;    // GMRES restart length
 
 struct TanElemArgs {
     int n, n_free;
@@ -539,23 +540,34 @@ __global__ void __launch_bounds__(kBlock) k_face_tangent(TanFaceArgs a)
 }
 
 // ---------------------------------------------------------------- vectors
-// per-CTA partial sums of the dot products x_k . y (k < nk) into part[k][blockIdx.x]
+// per-CTA partial sums of the dot products x_k . y (k < nk) into
+// part[k][blockIdx.x]; a CTA takes kDotRows rows, so y is read once for them
+constexpr int kDotRows = 4;
 __global__ void __launch_bounds__(kVec) k_dots(const double* __restrict__ X, size_t ldx, int nk,
     const double* __restrict__ y, size_t n, double* __restrict__ part)
 {
-    __shared__ double sh[kVec / 32];
-    const int k = blockIdx.y;
-    const double* x = X + k * ldx;
-    double s = 0.0;
-    for (size_t i = blockIdx.x * (size_t)kVec + threadIdx.x; i < n; i += (size_t)gridDim.x * kVec) s += x[i] * y[i];
+    __shared__ double sh[kDotRows][kVec / 32];
+    const int k0 = blockIdx.y * kDotRows, rows = min(kDotRows, nk - k0);
+    const double* x = X + k0 * ldx;
+    double s[kDotRows] = {};
+#pragma unroll 2
+    for (size_t i = blockIdx.x * (size_t)kVec + threadIdx.x; i < n; i += (size_t)gridDim.x * kVec) {
+        const double yi = y[i];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+        for (int k = 0; k < kDotRows; k++)
+            if (k < rows) s[k] += x[k * ldx + i] * yi;
+    }
+#pragma unroll
+    for (int k = 0; k < kDotRows; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = s[k];
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < rows) {
         double t = 0.0;
-        for (int q = 0; q < kVec / 32; q++) t += sh[q];
-        part[static_cast<size_t>(k) * gridDim.x + blockIdx.x] = t;
+        for (int q = 0; q < kVec / 32; q++) t += sh[threadIdx.x][q];
+        part[static_cast<size_t>(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
     }
 }
 
@@ -627,23 +639,106 @@ __global__ void k_rows_reduce(const double* __restrict__ part, int nk, int nb, d
     }
 }
 
-// *out = sqrt(sum of part[0..nb))
-__global__ void k_norm_reduce(const double* __restrict__ part, int nb, double* __restrict__ out)
+// The middle of two Gram-Schmidt passes in one sweep over the basis:
+//   w += sum_k coef_k v_k  (the first pass's update, coef = -h)   and
+//   part[k] = v_k . w      (the second pass's products, with the updated w),
+// or, with Norm, the second pass's update and part = w . w beside it.
+// A CTA takes 64 entries of every vector at a time; warp q holds the rows
+// k = q mod 8 and a lane two entries, so a thread uses the values that it
+// loaded itself for both, from registers, and only the eight partial updates
+// of an entry meet in shared memory.  Bound by HBM: with 64 vectors of 240 600
+// entries (123 MB) 27 us, 4.5 TB/s.  As two updates and two products by
+// themselves (36 + 20 us each; the basis read four times) an iteration's
+// orthogonalisation took 140 us at the average 64 vectors, now 85.
+constexpr int kGsTile = 64;
+constexpr int kGsRows = 104;         // most basis vectors (kRestart + 1, rounded up to the warps)
+constexpr int kGsPer = kGsRows / 8;  // rows per warp
+constexpr int kGsBlocks = 296, kGsNormBlocks = 444;  // 2 and 3 CTAs per SM
+
+template <bool Norm>
+__global__ void __launch_bounds__(kVec, Norm ? 3 : 2) k_gs_update(double* __restrict__ w, const double* __restrict__ V, size_t ldv,
+    int nk, const double* __restrict__ coef, size_t n, double* __restrict__ part)
 {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += 32) s += part[b];
+    __shared__ double sw[2][8][kGsTile], sc[kGsRows];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < kGsRows; k += kVec) sc[k] = k < nk ? coef[k] : 0.0;
+    __syncthreads();
+    const size_t nt = (n + kGsTile - 1) / kGsTile;
+    double acc[Norm ? 1 : kGsPer] = {};
+    int b = 0;
+    for (size_t t = blockIdx.x; t < nt; t += gridDim.x, b ^= 1) {
+        const size_t i = t * kGsTile + lane;
+        const bool on0 = i < n, on1 = i + 32 < n;
+        const double* v = V + static_cast<size_t>(q) * ldv + i;
+        double x0[kGsPer], x1[kGsPer];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) *out = ::sqrt(s);
+        for (int e = 0; e < kGsPer; e++) {
+            const bool k = q + 8 * e < nk;
+            x0[e] = k && on0 ? v[8 * e * ldv] : 0.0;
+            x1[e] = k && on1 ? v[8 * e * ldv + 32] : 0.0;
+        }
+        double s0 = q == 0 && on0 ? w[i] : 0.0, s1 = q == 0 && on1 ? w[i + 32] : 0.0;
+#pragma unroll
+        for (int e = 0; e < kGsPer; e++) {
+            const double c = sc[q + 8 * e];
+            s0 += c * x0[e];
+            s1 += c * x1[e];
+        }
+        sw[b][q][lane] = s0;
+        sw[b][q][lane + 32] = s1;
+        __syncthreads();
+        double u0 = 0.0, u1 = 0.0;
+#pragma unroll
+        for (int h = 0; h < 8; h++) {
+            u0 += sw[b][h][lane];
+            u1 += sw[b][h][lane + 32];
+        }
+        if (q == 0 && on0) w[i] = u0;
+        if (q == 0 && on1) w[i + 32] = u1;
+        if constexpr (Norm) {
+            acc[0] += u0 * u0 + u1 * u1;  // the same in every warp
+        } else {
+#pragma unroll
+            for (int e = 0; e < kGsPer; e++) acc[e] += x0[e] * u0 + x1[e] * u1;
+        }
+    }
+    if constexpr (Norm) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
+    } else {
+#pragma unroll
+        for (int e = 0; e < kGsPer; e++) {
+            double s = acc[e];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0 && q + 8 * e < nk) part[static_cast<size_t>(q + 8 * e) * gridDim.x + blockIdx.x] = s;
+        }
+    }
 }
 
-// y = x / *s (0 when *s is 0)
-__global__ void __launch_bounds__(kVec) k_scale_inv(double* __restrict__ y, const double* __restrict__ x,
-    const double* __restrict__ s, size_t n)
+// *s = sqrt(sum of part[0..nb)) and y = x / *s (0 when that is 0), twice: the
+// new basis vector and the copy of it that H0 is applied to in place.  Every
+// CTA adds the partial sums for itself, in the same order.
+__global__ void __launch_bounds__(kVec) k_gs_scale(double* __restrict__ y, double* __restrict__ z,
+    const double* __restrict__ x, const double* __restrict__ part, int nb, double* __restrict__ s, size_t n)
 {
-    const double d = *s;
-    const double f = d > 0.0 ? 1.0 / d : 0.0;
-    for (size_t i = blockIdx.x * (size_t)kVec + threadIdx.x; i < n; i += (size_t)gridDim.x * kVec) y[i] = f * x[i];
+    __shared__ double sh[kVec / 32];
+    double t = 0.0;
+    for (int b = threadIdx.x; b < nb; b += kVec) t += part[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    t = 0.0;
+    for (int q = 0; q < kVec / 32; q++) t += sh[q];
+    const double d = ::sqrt(t), f = d > 0.0 ? 1.0 / d : 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *s = d;
+    for (size_t i = blockIdx.x * (size_t)kVec + threadIdx.x; i < n; i += (size_t)gridDim.x * kVec) {
+        const double v = f * x[i];
+        y[i] = v;
+        if (z) z[i] = v;
+    }
 }
 
 __global__ void __launch_bounds__(kVec) k_scale_copy(double* __restrict__ y, const double* __restrict__ x, double s, size_t n)
@@ -672,6 +767,7 @@ struct AdjointWS {
     double *part = nullptr, *coef = nullptr;
     double* hcol = nullptr;    // device: the Hessenberg column being formed
     double* h_hcol = nullptr;  // pinned host copy
+    cudaEvent_t got_col = nullptr;  // the column of the iteration is in h_hcol
     MatParams<Dual>* mats = nullptr;
     int mats_seed = -2;  // the seed `mats` holds: 5 slot + k, -1 none, -2 not uploaded
     double* dscale = nullptr;
@@ -686,13 +782,12 @@ void free_adjoint(Model& m)
         dev_free(*p);
     if (w.mats) cudaFree(w.mats);
     if (w.h_hcol) cudaFreeHost(w.h_hcol);
+    if (w.got_col) cudaEventDestroy(w.got_col);
     delete m.aws;
     m.aws = nullptr;
 }
 
 namespace {
-
-constexpr int kRestart = 100;
 
 efem_status alloc_aws(Model& m)
 {
@@ -709,10 +804,11 @@ efem_status alloc_aws(Model& m)
     if ((s = dev_alloc(&w.Z, nb)) != EFEM_OK) return s;
     for (double** p : { &w.w, &w.x, &w.b, &w.t, &w.u, &w.io })
         if ((s = dev_alloc(p, std::max<size_t>(n, 1))) != EFEM_OK) return s;
-    if ((s = dev_alloc(&w.part, static_cast<size_t>(kRestart + 1) * kDotBlocks)) != EFEM_OK) return s;
+    if ((s = dev_alloc(&w.part, static_cast<size_t>(kRestart + 1) * kGsBlocks)) != EFEM_OK) return s;
     if ((s = dev_alloc(&w.coef, static_cast<size_t>(kRestart + 1))) != EFEM_OK) return s;
     if ((s = dev_alloc(&w.hcol, static_cast<size_t>(kRestart + 2))) != EFEM_OK) return s;
     EFEM_CUDA(cudaMallocHost(&w.h_hcol, sizeof(double) * (kRestart + 2)));
+    EFEM_CUDA(cudaEventCreateWithFlags(&w.got_col, cudaEventDisableTiming));
     if ((s = dev_alloc(&w.dscale, static_cast<size_t>(std::max(m.n_pressure_loads, 1)))) != EFEM_OK) return s;
     EFEM_CUDA(cudaMalloc(&w.mats, sizeof(MatParams<Dual>) * MAX_MATS));
     w.h_part.resize(static_cast<size_t>(kRestart + 1) * kDotBlocks);
@@ -871,7 +967,7 @@ efem_status dots(Model& m, const double* X, int nk, const double* y, double* res
 {
     AdjointWS& w = *m.aws;
     const size_t n = w.n;
-    k_dots<<<dim3(kDotBlocks, nk), kVec, 0, m.stream>>>(X, n, nk, y, n, w.part);
+    k_dots<<<dim3(kDotBlocks, (nk + kDotRows - 1) / kDotRows), kVec, 0, m.stream>>>(X, n, nk, y, n, w.part);
     m.launches++;
     EFEM_CUDA(cudaMemcpyAsync(w.h_part.data(), w.part, sizeof(double) * nk * kDotBlocks, cudaMemcpyDeviceToHost, m.stream));
     EFEM_CUDA(cudaStreamSynchronize(m.stream));
@@ -928,36 +1024,42 @@ efem_status adjoint_gmres(Model& m, const double* u, double tol, int max_it, int
     EFEM_CUDA(cudaMemcpyAsync(w.t, w.b, sizeof(double) * n, cudaMemcpyDeviceToDevice, m.stream));
     int total = 0;
     while (total < max_it) {
-        // V_0 = r / beta, r = t
+        // V_0 = r / beta, r = t, and its copy for H0
         k_scale_copy<<<vec_grid(n), kVec, 0, m.stream>>>(w.V, w.t, 1.0 / beta, n);
-        m.launches++;
+        k_scale_copy<<<vec_grid(n), kVec, 0, m.stream>>>(w.Z, w.t, 1.0 / beta, n);
+        m.launches += 2;
         std::fill(g.begin(), g.end(), 0.0);
         g[0] = beta;
         int j = 0;
         bool done = false;
+        // w.w = K^T H0 V_j (Z_j: the copy of V_j, then H0 V_j)
+        auto product = [&](int jj) -> efem_status {
+            efem_status ps = precond_enqueue(m, w.Z + jj * n, m.stream);
+            if (ps != EFEM_OK) return ps;
+            m.launches += precond_launch_count(m);
+            return tangent(m, u, w.Z + jj * n, w.w, true);
+        };
+        if ((s = product(0)) != EFEM_OK) return s;
         for (; j < R && total < max_it; j++, total++) {
-            double* Zj = w.Z + j * n;
-            EFEM_CUDA(cudaMemcpyAsync(Zj, w.V + j * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, m.stream));
-            if ((s = precond_enqueue(m, Zj, m.stream)) != EFEM_OK) return s;
-            m.launches++;
-            if ((s = tangent(m, u, Zj, w.w, true)) != EFEM_OK) return s;
             *bytes += it_bytes + 2.0 * (2.0 * (j + 1) * nd + 3.0 * nd);
             // two passes of classical Gram-Schmidt, coefficients kept on the device
             // (with H0 a good preconditioner, K^T H0 v is close to the basis: the
             // first pass removes most of w in nearly every iteration, so a
             // conditional second pass would almost always run)
-            for (int pass = 0; pass < 2; pass++) {
-                k_dots<<<dim3(kDotBlocks, j + 1), kVec, 0, m.stream>>>(w.V, n, j + 1, w.w, n, w.part);
-                k_rows_reduce<<<(j + 1 + 7) / 8, 256, 0, m.stream>>>(w.part, j + 1, kDotBlocks, w.hcol, w.coef, pass);
-                launch_axpys(m.stream, w.w, w.V, n, j + 1, w.coef, n);
-                m.launches += 3;
-            }
-            k_dots<<<dim3(kDotBlocks, 1), kVec, 0, m.stream>>>(w.w, n, 1, w.w, n, w.part);
-            k_norm_reduce<<<1, 32, 0, m.stream>>>(w.part, kDotBlocks, w.hcol + j + 1);
-            k_scale_inv<<<vec_grid(n), kVec, 0, m.stream>>>(w.V + (j + 1) * n, w.w, w.hcol + j + 1, n);
-            m.launches += 3;
+            k_dots<<<dim3(kDotBlocks, (j + kDotRows) / kDotRows), kVec, 0, m.stream>>>(w.V, n, j + 1, w.w, n, w.part);
+            k_rows_reduce<<<(j + 1 + 7) / 8, 256, 0, m.stream>>>(w.part, j + 1, kDotBlocks, w.hcol, w.coef, 0);
+            k_gs_update<false><<<kGsBlocks, kVec, 0, m.stream>>>(w.w, w.V, n, j + 1, w.coef, n, w.part);
+            k_rows_reduce<<<(j + 1 + 7) / 8, 256, 0, m.stream>>>(w.part, j + 1, kGsBlocks, w.hcol, w.coef, 1);
+            k_gs_update<true><<<kGsNormBlocks, kVec, 0, m.stream>>>(w.w, w.V, n, j + 1, w.coef, n, w.part);
+            k_gs_scale<<<vec_grid(n), kVec, 0, m.stream>>>(w.V + (j + 1) * n, j + 1 < R ? w.Z + (j + 1) * n : nullptr, w.w,
+                w.part, kGsNormBlocks, w.hcol + j + 1, n);
+            m.launches += 6;
             EFEM_CUDA(cudaMemcpyAsync(w.h_hcol, w.hcol, sizeof(double) * (j + 2), cudaMemcpyDeviceToHost, m.stream));
-            EFEM_CUDA(cudaStreamSynchronize(m.stream));
+            EFEM_CUDA(cudaEventRecord(w.got_col, m.stream));
+            // the next iteration's product starts while the host reads the column
+            // (one product too many when this iteration converges)
+            if (j + 1 < R && total + 1 < max_it && (s = product(j + 1)) != EFEM_OK) return s;
+            EFEM_CUDA(cudaEventSynchronize(w.got_col));
             for (int i = 0; i <= j + 1; i++) H[static_cast<size_t>(i) * R + j] = w.h_hcol[i];
             const double hn = w.h_hcol[j + 1];
             // Givens rotations on column j

@@ -301,10 +301,9 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
     sg->ncorr = ncorr;
 }
 
-// Pass 2: q = -r - sum_j alpha_j y_j for running members (0 elsewhere); also
-// clears the triangular solve's counters for the H0 application that follows
+// Pass 2: q = -r - sum_j alpha_j y_j for running members (0 elsewhere)
 __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const double* __restrict__ r,
-    const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S, int* clear, int n_clear)
+    const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S)
 {
     const Chunk c = ch[blockIdx.x];
     const Seg* sg = S + c.seg;
@@ -318,8 +317,6 @@ __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const dou
         for (int j = 0; j < ncorr; j++) qi -= al[j] * Yh[static_cast<size_t>(j) * n + i];
         q[i] = qi;
     }
-    if (clear)
-        for (int k = blockIdx.x * kT + threadIdx.x; k < n_clear; k += gridDim.x * kT) clear[k] = 0;
 }
 
 // Pass 3: y_j . z for every slot; the member's last CTA runs the second loop
@@ -764,11 +761,8 @@ efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
             P1(1) P1(2) P1(3) P1(4) P1(5) P1(6) P1(7) P1(8)
 #undef P1
         }
-        int* clear = nullptr;
-        int n_clear = 0;
-        precond_counters(M, &clear, &n_clear);
-        kb_pass2<<<nb, kT, 0, s1>>>(U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg, clear, n_clear);
-        if ((s = precond_enqueue(M, U.q, s1, false)) != EFEM_OK) break;
+        kb_pass2<<<nb, kT, 0, s1>>>(U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg);
+        if ((s = precond_enqueue(M, U.q, s1)) != EFEM_OK) break;
         switch (U.m) {
 #define P3(K) case K: kb_pass3<K><<<nb, kT, 0, s1>>>(U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
             P3(1) P3(2) P3(3) P3(4) P3(5) P3(6) P3(7) P3(8)

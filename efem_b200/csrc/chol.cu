@@ -20,13 +20,11 @@
 //
 // Solve H0 v (3 right-hand sides interleaved per node): one persistent launch,
 // k_solve below.  Every sum is formed in a fixed order (no atomics): results
-// are deterministic.  An application by itself is replayed as one CUDA graph
-// per input vector.
+// are deterministic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <string>
 
@@ -116,15 +114,14 @@ struct Precond {
     std::vector<int> w_off;    // nlev + 1
     int4 *d_steps = nullptr, *d_invs = nullptr;  // tiles of k_step and k_inverse
     cudaStream_t capture2 = nullptr;  // second branch of the factorisation's graph
-    int* h_flag = nullptr;  // pinned: the error flag read back after an application
+    int* d_res = nullptr;   // the last application's error flag
+    int* h_flag = nullptr;  // the same in mapped host memory
     double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
            *d_vals = nullptr;
     // graph replay of the numeric factorisation (the same launches every solve)
     cudaGraphExec_t factor_exec = nullptr;
     long long factor_launches = 0;
-    // graph replay of the solve, per (input vector, work buffers)
     cudaStream_t capture = nullptr;
-    std::map<std::pair<double*, double*>, cudaGraphExec_t> graphs;
 };
 
 namespace {
@@ -618,6 +615,7 @@ struct SolveArgs {
     int spin_limit;             // polls of one wait before the solve gives up
     int test_wait;              // 1: the last item's wait target is raised by one (it can only run out)
     int n3;                     // entries of v (3 per free node)
+    int *res, *hres;            // when set: the error flag goes there (device, mapped host), and the counters are left at zero
     const int* item_group;      // batch unions: the member each item belongs to
     const int* frozen;          // batch unions: 1 for a member that no longer iterates (its items are skipped)
 };
@@ -1050,17 +1048,27 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
             if (tid == 0) signal(A.cnt + 3 * A.ns + d.s);
         }
     }
-    // A solve that gave up leaves v partly overwritten: the last CTA to
-    // leave fills it with NaN, so that a caller who cannot read the error
-    // flag (a replayed graph) still sees that the result is not valid.
+    // The last CTA to leave.  A solve that gave up leaves v partly overwritten:
+    // it is filled with NaN, so that a caller who cannot read the error flag (a
+    // replayed graph) still sees that the result is not valid.  Then the flag
+    // goes where it is read and the counters back to zero, so that no
+    // application needs a launch to clear them.
     if (tid == 0) {
         __threadfence();
-        ok_sh = atomicAdd(A.cnt + 2 * A.ns, 1) == static_cast<int>(gridDim.x) - 1 && *reinterpret_cast<volatile int*>(err);
+        ok_sh = atomicAdd(A.cnt + 2 * A.ns, 1) == static_cast<int>(gridDim.x) - 1;
+        ok2_sh = *reinterpret_cast<volatile int*>(err);
     }
     __syncthreads();
-    if (ok_sh) {
-        __threadfence();
+    if (!ok_sh) return;
+    __threadfence();
+    if (ok2_sh)
         for (int i = tid; i < A.n3; i += kST) A.v[i] = __longlong_as_double(0x7ff8000000000000LL);
+    if (A.res) {
+        for (int i = tid; i < 4 * A.ns + 2; i += kST) A.cnt[i] = 0;
+        if (tid == 0) {
+            *A.res = ok2_sh;
+            *A.hres = ok2_sh;
+        }
     }
 }
 
@@ -1411,18 +1419,19 @@ WaitCfg wait_cfg(const Model& m)
     return WaitCfg { m.opts.wait_limit > 0 ? m.opts.wait_limit : kSpinLimit, m.opts.wait_test ? 1 : 0 };
 }
 
-// enqueue one H0 application (counter reset unless the caller cleared them,
-// then the persistent solve) on stream st
+// Enqueue one H0 application on stream st.  With the model's own work buffers
+// (own) the counters are zero beforehand and left so; other buffers' are
+// cleared first and keep the error flag.
 efem_status enqueue_solve(const Precond& P, const FrontArgs& a, const SolveBufs& b, double* d_v, cudaStream_t st,
-    WaitCfg wc, bool clear = true, unsigned long long* stamp = nullptr)
+    WaitCfg wc, bool own, unsigned long long* stamp = nullptr)
 {
     const int ns = P.S.ns;
-    if (clear) EFEM_CUDA(cudaMemsetAsync(b.cnt, 0, sizeof(int) * (4 * static_cast<size_t>(ns) + 2), st));
+    if (!own) EFEM_CUDA(cudaMemsetAsync(b.cnt, 0, sizeof(int) * (4 * static_cast<size_t>(ns) + 2), st));
     const SubArgs B { a, P.d_parent, P.d_prow, P.d_perm, P.d_subs, P.d_chunks, P.d_depth, P.d_xidx, P.sub_max_r,
         P.sub_max_cols, P.sub_max_depth, P.sub_max_m, P.sub_max_c, P.sub_max_mroot, d_v, b.y, b.upd, stamp };
     if (P.n_subs > 0) k_sub_fwd<<<P.n_subs, kST, P.sub_smem_f, st>>>(B);
-    SolveArgs A { a, P.d_prow, P.d_items, P.d_slot, P.n_items, ns, d_v, b.y, b.t, b.upd, b.cnt, P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, P.d_item_group,
-        P.d_item_group ? P.d_frozen : nullptr };
+    SolveArgs A { a, P.d_prow, P.d_items, P.d_slot, P.n_items, ns, d_v, b.y, b.t, b.upd, b.cnt, P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, own ? P.d_res : nullptr, own ? P.h_flag : nullptr,
+        P.d_item_group, P.d_item_group ? P.d_frozen : nullptr };
     if (P.n_items > 0) launch_k(k_solve, P.solve_grid, kST, P.solve_smem, st, A);
     if (P.n_subs > 0) k_sub_bwd<<<P.n_subs, kST, P.sub_smem_b, st>>>(B);
     return EFEM_OK;
@@ -1435,14 +1444,12 @@ void free_precond(Model& m)
     if (!m.precond) return;
     m.epoch++;
     Precond& P = *m.precond;
-    for (auto& kv : P.graphs) cudaGraphExecDestroy(kv.second);
-    P.graphs.clear();
     if (P.factor_exec) cudaGraphExecDestroy(P.factor_exec);
     if (P.capture) cudaStreamDestroy(P.capture);
     if (P.capture2) cudaStreamDestroy(P.capture2);
     if (P.h_flag) cudaFreeHost(P.h_flag);
     for (int** p : { &P.d_first, &P.d_ncol, &P.d_nrow, &P.d_child_ptr, &P.d_child_list, &P.d_relind,
-             &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_parent, &P.d_cnt, &P.d_prow, &P.d_depth, &P.d_xidx, &P.d_slot })
+             &P.d_level_list, &P.d_perm, &P.d_fail, &P.d_parent, &P.d_cnt, &P.d_res, &P.d_prow, &P.d_depth, &P.d_xidx, &P.d_slot })
         dev_free(*p);
     for (long long** p : { &P.d_slot_off, &P.d_front_off, &P.d_rows_off, &P.d_relind_off, &P.d_xw_off, &P.d_upd_off, &P.d_a_pos,
              &P.d_a_src })
@@ -1822,7 +1829,11 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     }
     EFEM_CUDA(cudaStreamCreateWithFlags(&P.capture, cudaStreamNonBlocking));
     EFEM_CUDA(cudaStreamCreateWithFlags(&P.capture2, cudaStreamNonBlocking));
-    EFEM_CUDA(cudaMallocHost(&P.h_flag, sizeof(int)));
+    EFEM_CUDA(cudaHostAlloc(&P.h_flag, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    *P.h_flag = 0;
+    if ((st = dev_alloc(&P.d_res, 1)) != EFEM_OK) return st;
+    EFEM_CUDA(cudaMemsetAsync(P.d_res, 0, sizeof(int), m.stream));
+    EFEM_CUDA(cudaMemsetAsync(P.d_cnt, 0, sizeof(int) * (4 * static_cast<size_t>(S.ns) + 2), m.stream));
     P.ready = true;  // analysed; the numeric factor follows
     return precond_factor(m, ok, ms_factor);
 }
@@ -1933,46 +1944,10 @@ static efem_status precond_factor(Model& m, int* ok, double* ms_factor)
     return EFEM_OK;
 }
 
-// One H0 application, replayed from a CUDA graph captured (once per input
-// vector and work buffers) on the preconditioner's private stream.
-static efem_status apply_with(Model& m, double* d_v, const SolveBufs& b)
-{
-    Precond& P = *m.precond;
-    if (P.S.n == 0) return EFEM_OK;
-    const auto key = std::make_pair(d_v, b.y);
-    auto it = P.graphs.find(key);
-    if (it == P.graphs.end()) {
-        if (P.graphs.size() >= 8) {  // callers passing many distinct vectors: start over
-            EFEM_CUDA(cudaStreamSynchronize(m.stream));
-            for (auto& kv : P.graphs) cudaGraphExecDestroy(kv.second);
-            P.graphs.clear();
-        }
-        cudaGraph_t g = nullptr;
-        cudaGraphExec_t ge = nullptr;
-        std::lock_guard<std::mutex> lock(capture_mutex());
-        EFEM_CUDA(cudaStreamBeginCapture(P.capture, cudaStreamCaptureModeThreadLocal));
-        const efem_status es = enqueue_solve(P, args_of(P), b, d_v, P.capture, wait_cfg(m));
-        EFEM_CUDA(cudaStreamEndCapture(P.capture, &g));
-        if (es != EFEM_OK) {
-            cudaGraphDestroy(g);
-            return es;
-        }
-        EFEM_CUDA(cudaGraphInstantiate(&ge, g, 0));
-        cudaGraphDestroy(g);
-        it = P.graphs.emplace(key, ge).first;
-    }
-    EFEM_CUDA(cudaGraphLaunch(it->second, m.stream));
-    m.launches += 1;
-    return EFEM_OK;
-}
-
 void precond_drop_graphs(Model& m)
 {
     if (!m.precond) return;
-    if (m.on_device) cudaStreamSynchronize(m.stream);
-    for (auto& kv : m.precond->graphs) cudaGraphExecDestroy(kv.second);
-    m.precond->graphs.clear();
-    m.epoch++;  // the solver's iteration graphs hold the persistent solve's arguments too
+    m.epoch++;  // the solver's iteration graphs hold the persistent solve's arguments
 }
 
 efem_status precond_sync_grid(Model& m)
@@ -1981,9 +1956,6 @@ efem_status precond_sync_grid(Model& m)
     Precond& P = *m.precond;
     const int want = solve_grid_for(P);
     if (want == P.solve_grid) return EFEM_OK;
-    EFEM_CUDA(cudaStreamSynchronize(m.stream));
-    for (auto& kv : P.graphs) cudaGraphExecDestroy(kv.second);
-    P.graphs.clear();
     P.solve_grid = want;
     m.epoch++;  // the solver's iteration graphs hold the old grid
     return EFEM_OK;
@@ -1991,15 +1963,12 @@ efem_status precond_sync_grid(Model& m)
 
 efem_status precond_apply(Model& m, double* d_v)
 {
-    if (!m.precond || !m.precond->factored || !m.precond->ok) {
-        set_error("preconditioner not factored");
-        return EFEM_ERR_ARG;
-    }
-    Precond& P = *m.precond;
-    return apply_with(m, d_v, SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt });
+    efem_status s = precond_enqueue(m, d_v, m.stream);
+    if (s == EFEM_OK) m.launches += precond_launch_count(m);
+    return s;
 }
 
-efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, bool clear, unsigned long long* stamp)
+efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned long long* stamp)
 {
     if (!m.precond || !m.precond->factored || !m.precond->ok) {
         set_error("preconditioner not factored");
@@ -2007,8 +1976,10 @@ efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, bool cle
     }
     Precond& P = *m.precond;
     if (P.S.n == 0) return EFEM_OK;
-    return enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), clear,
-        stamp);
+    const efem_status s = enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), true, stamp);
+    if (s != EFEM_OK) return s;
+    EFEM_CUDA(cudaGetLastError());
+    return EFEM_OK;
 }
 
 efem_status precond_set_groups(Model& m, const std::vector<int>& group_of_free_node, const int* d_frozen)
@@ -2028,19 +1999,11 @@ efem_status precond_set_groups(Model& m, const std::vector<int>& group_of_free_n
     efem_status st = dev_upload(&P.d_item_group, g);
     if (st != EFEM_OK) return st;
     P.d_frozen = d_frozen;
-    for (auto& kv : P.graphs) cudaGraphExecDestroy(kv.second);  // captured solves hold the old arguments
-    P.graphs.clear();
-    m.epoch++;
+    m.epoch++;  // captured solves hold the old arguments
     return EFEM_OK;
 }
 
 bool precond_has_groups(const Model& m) { return m.precond && m.precond->d_item_group; }
-
-void precond_counters(const Model& m, int** cnt, int* n)
-{
-    *cnt = m.precond ? m.precond->d_cnt : nullptr;
-    *n = m.precond ? 4 * m.precond->S.ns + 2 : 0;
-}
 
 long long precond_launch_count(const Model& m)
 {
@@ -2048,27 +2011,19 @@ long long precond_launch_count(const Model& m)
     return (m.precond->n_items > 0 ? 1 : 0) + (m.precond->n_subs > 0 ? 2 : 0);
 }
 
-const int* precond_error_flag(const Model& m)
-{
-    return m.precond && m.precond->d_cnt ? m.precond->d_cnt + 4LL * m.precond->S.ns + 1 : nullptr;
-}
+const int* precond_error_flag(const Model& m) { return m.precond ? m.precond->d_res : nullptr; }
 
-// h_flag: where the flag is read back to (pinned memory spares the copy's staging)
-static efem_status check_solve_flag(const int* d_flag, cudaStream_t st, int* h_flag)
+static efem_status solve_gave_up()
 {
-    EFEM_CUDA(cudaMemcpyAsync(h_flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    EFEM_CUDA(cudaStreamSynchronize(st));
-    if (*h_flag) {
-        set_error("the triangular solve of the preconditioner gave up waiting for a front");
-        return EFEM_ERR_TIMEOUT;
-    }
-    return EFEM_OK;
+    set_error("the triangular solve of the preconditioner gave up waiting for a front");
+    return EFEM_ERR_TIMEOUT;
 }
 
 efem_status precond_check(Model& m)
 {
-    const int* f = precond_error_flag(m);
-    return f ? check_solve_flag(f, m.stream, m.precond->h_flag) : EFEM_OK;
+    if (!m.precond || !m.precond->h_flag) return EFEM_OK;
+    EFEM_CUDA(cudaStreamSynchronize(m.stream));
+    return *static_cast<volatile int*>(m.precond->h_flag) ? solve_gave_up() : EFEM_OK;
 }
 
 // ============================================================================
@@ -2195,9 +2150,12 @@ extern "C" efem_status efem_precond_apply_noalloc(void* model, double* d_v)
     }
     int* counters = reinterpret_cast<int*>(scratch + 2 * n3 + S.upd_size);
     const SolveBufs b { scratch, scratch + n3, scratch + 2 * n3, counters };
-    efem_status st = enqueue_solve(P, args_of(P), b, d_v, m.stream, wait_cfg(m));
+    efem_status st = enqueue_solve(P, args_of(P), b, d_v, m.stream, wait_cfg(m), false);
     if (st != EFEM_OK) return st;
     EFEM_CUDA(cudaGetLastError());
     if (capturing) return EFEM_OK;  // recorded into the caller's graph; a give-up shows as NaN in d_v
-    return check_solve_flag(counters + 4LL * S.ns + 1, m.stream, P.h_flag);
+    int flag = 0;
+    EFEM_CUDA(cudaMemcpyAsync(&flag, counters + 4LL * S.ns + 1, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
+    EFEM_CUDA(cudaStreamSynchronize(m.stream));
+    return flag ? solve_gave_up() : EFEM_OK;
 }

@@ -289,11 +289,8 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor);
 // v <- (L (x) I3)^{-1} v in place on the device (v: 3*n_free interleaved).
 efem_status precond_apply(Model& m, double* d_v);
 // The same H0 application enqueued on `stream` (for capture into a larger
-// graph); clear = false when the caller has zeroed precond_counters itself.
-// With `stamp`, the solve's first CTA stores the GPU's global timer there.
-efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, bool clear = true,
-    unsigned long long* stamp = nullptr);
-void precond_counters(const Model& m, int** cnt, int* n);  // the solve's counters, cleared before each H0 v
+// graph).  With `stamp`, the solve's first CTA stores the GPU's global timer there.
+efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned long long* stamp = nullptr);
 // Batch unions: group_of_free_node[i] = the member free node i belongs to;
 // items of member g are skipped while d_frozen[g] != 0 (a member's fronts
 // form trees of their own, so nothing else waits on them).
@@ -303,7 +300,7 @@ long long precond_launch_count(const Model& m);  // kernels per H0 application
 const int* precond_error_flag(const Model& m);   // device flag: a solve gave up waiting (nullptr before set-up)
 efem_status precond_check(Model& m);             // wait for the stream and report that flag
 void free_precond(Model& m);
-void precond_drop_graphs(Model& m);  // forget captured H0 solves (new wait limits); the factor stays
+void precond_drop_graphs(Model& m);  // captured H0 solves are out of date (new wait limits); the factor stays
 // ------------------------------------------------------------------ batches (batch.cu)
 // Solve n models as one union model (see batch.cu); EFEM_ERR_UNSUPPORTED when
 // the models cannot share one (different devices or options, gravity, an

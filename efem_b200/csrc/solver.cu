@@ -582,10 +582,9 @@ __global__ void __launch_bounds__(kThreads) k_pass3_m(const double* __restrict__
     for (int j = tid; j < ncorr; j += kThreads) S->coef[j] = scf[j];
 }
 
-// Pass 2: q = (q0 - sum_j alpha_j y_j) [/ theta when H0 = I / theta]; also
-// clears the preconditioner solve's counters for the H0 application that follows
+// Pass 2: q = (q0 - sum_j alpha_j y_j) [/ theta when H0 = I / theta]
 __global__ void __launch_bounds__(kThreads) k_pass2(double* __restrict__ q, const double* __restrict__ r,
-    const double* __restrict__ Yh, size_t n, int m, int divide_theta, const Scalars* S, int* clear, int n_clear)
+    const double* __restrict__ Yh, size_t n, int m, int divide_theta, const Scalars* S)
 {
     griddep_wait();
     __shared__ double al[kMaxHist];
@@ -600,8 +599,6 @@ __global__ void __launch_bounds__(kThreads) k_pass2(double* __restrict__ q, cons
         q[i] = divide_theta ? qi / th : qi;
     }
     griddep_launch();
-    if (clear)
-        for (int k = blockIdx.x * kThreads + threadIdx.x; k < n_clear; k += gridDim.x * kThreads) clear[k] = 0;
 }
 
 // Pass 3: y_j . z0 for every slot (grid (kRowBlocks, m)); the last CTA runs
@@ -935,12 +932,9 @@ efem_status enqueue_body(Model& m, SolverWS& w, double* x, bool use_factor, cuda
 #undef P1
     default: k_pass1<<<g1, kThreads, sm1, st>>>(x, w.xp, w.r, w.rp, w.S, w.Y, n, mm, w.sc, w.partials, w.sums);
     }
-    int* clear = nullptr;
-    int n_clear = 0;
-    if (use_factor) precond_counters(m, &clear, &n_clear);
-    launch_k(k_pass2, grid_for(n), kThreads, 0, st, w.q, w.r, w.Y, n, mm, use_factor ? 0 : 1, w.sc, clear, n_clear);
+    launch_k(k_pass2, grid_for(n), kThreads, 0, st, w.q, w.r, w.Y, n, mm, use_factor ? 0 : 1, w.sc);
     if (use_factor) {
-        efem_status s = precond_enqueue(m, w.q, st, false, &w.sc->t0_pc);
+        efem_status s = precond_enqueue(m, w.q, st, &w.sc->t0_pc);
         if (s != EFEM_OK) return s;
     }
     switch (mm) {
