@@ -22,8 +22,8 @@
 //    runs that member's small recursion, so every member follows exactly the
 //    arithmetic of a single solve.
 //  * One CUDA graph holds the iteration loop: a while node over iterations
-//    whose body holds a while node over line-search trials; each condition
-//    is set by a one-CTA kernel that reads every member's state, and both
+//    whose body holds a while node over line-search trials; both conditions
+//    are set by the CTA that ends the last member's reduction, and both
 //    loops are bounded there (kCap iterations per launch, max_line_search
 //    trials per iteration) whatever that state holds.  A member that
 //    converged (or stopped) is frozen: its x no longer moves and its
@@ -45,13 +45,15 @@
 #include <vector>
 
 #include "efem_internal.h"
+#include "reduce.cuh"
 
 namespace efem {
 
 namespace {
 
 constexpr int kT = 256;       // threads per CTA of the segmented vector kernels
-constexpr int kChunk = 2048;  // vector entries per CTA; a chunk never spans two members
+constexpr int kChunk = 512;   // vector entries per CTA; a chunk never spans two members (32 beams, us an iteration:
+                              // 172 with 512, 172 with 1024, 191 with 2048 -- too few CTAs)
 constexpr int kHist = 8;      // largest L-BFGS history of a batch
 constexpr int kCap = 64;      // iterations per launch of the iteration graph
 constexpr int kStall = 24;    // FP32 phase: iterations without halving the best ||r||_inf
@@ -78,6 +80,7 @@ struct Glob {
     int launch_iters, cap;
     int n_running;
     int pc_fail;
+    unsigned int cnt;        // members done with the current reduction
     long long body_iters;    // loop bodies run (for the launch count)
     long long trials;        // extra line-search trials run
 };
@@ -152,12 +155,45 @@ __device__ bool seg_finish(double* v, unsigned maxmask, Seg* sg, double* partial
     return true;
 }
 
+// The same for sums alone, for the passes: lane k < NV of warp 0 of the
+// member's last CTA returns with total k; *last is set there.
+template <int NV>
+__device__ __forceinline__ double seg_totals(const double (&v)[NV], Seg* sg, double* partials, double (*sh)[32], bool* last)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c0 = sg->c0, c1 = sg->c1;
+    double t = cta_sums<NV, kT / 32>(v, sh);
+    if (c1 - c0 == 1) {
+        if (threadIdx.x == 0) *last = true;
+        __syncthreads();
+        return t;
+    }
+    if (w == 0) {
+        if (lane < NV) partials[static_cast<size_t>(blockIdx.x) * NV + lane] = t;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) *last = atomicAdd(&sg->cnt, 1u) == static_cast<unsigned>(c1 - c0 - 1);
+    }
+    __syncthreads();
+    if (!*last) return 0.0;
+    __threadfence();
+    t = 0.0;
+    if (lane < NV)
+        for (int b = c0 + w; b < c1; b += kT / 32) t += __ldcg(partials + static_cast<size_t>(b) * NV + lane);
+    sh[w][lane] = t;
+    __syncthreads();
+    t = 0.0;
+    if (w == 0) {
+#pragma unroll
+        for (int q = 0; q < kT / 32; q++) t += sh[q][lane];
+        if (lane == 0) sg->cnt = 0u;
+    }
+    return t;
+}
+
 // the chunk of this CTA: member, entries [a, b)
 struct Chunk {
     int seg, a, b, pad;
 };
-
-__device__ __forceinline__ int ring(int i, int m) { return ((i % m) + m) % m; }
 
 __global__ void kb_init(Seg* S, const int* c0, const double* eps, const int* max_iter, int max_ls, int m, int nseg,
     int stall, const int* keep, int* frozen)
@@ -196,6 +232,7 @@ __global__ void kb_glob_init(Glob* G, int cap)
     G->cap = cap;
     G->n_running = 0;
     G->pc_fail = 0;
+    G->cnt = 0u;
     G->body_iters = 0;
     G->trials = 0;
 }
@@ -240,20 +277,33 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
     const double* __restrict__ r, const double* __restrict__ rp, double* __restrict__ Sh, double* __restrict__ Yh,
     size_t n, const Chunk* __restrict__ ch, Seg* S, double* partials)
 {
+    griddep_wait();
     constexpr int NV = 3 * M + 2;
+    __shared__ double sh[kT / 32][32], sG[M * M], tot[32];
+    __shared__ bool last;
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
-    const bool act = sg->state == kRun && !sg->first;
+    if (sg->state != kRun) return;  // the same in every CTA of the member: its counter stays 0
+    const bool first = sg->first;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int loc = sg->ptr % M;
     const int ncorr = sg->ncorr < M ? sg->ncorr + 1 : M;
+    if (tid < M * M) sG[tid] = sg->G[tid / M][tid % M];
+    double ys = tid < M ? sg->ys[tid] : 1.0;
     double v[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) v[k] = 0.0;
-    if (act) {
+    if (!first) {
         double* snew = Sh + static_cast<size_t>(loc) * n;
         double* ynew = Yh + static_cast<size_t>(loc) * n;
-        for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
+        for (int i = c.a + tid; i < c.b; i += kT) {
             const double si = x[i] - xp[i], ri = r[i], yi = ri - rp[i];
+            double s[M], y[M];
+#pragma unroll
+            for (int j = 0; j < M; j++) {
+                s[j] = j < ncorr && j != loc ? Sh[static_cast<size_t>(j) * n + i] : si;
+                y[j] = j < ncorr && j != loc ? Yh[static_cast<size_t>(j) * n + i] : yi;
+            }
             snew[i] = si;
             ynew[i] = yi;
             v[3 * M] += si * yi;
@@ -261,50 +311,52 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
 #pragma unroll
             for (int j = 0; j < M; j++)
                 if (j < ncorr) {
-                    const bool self = j == loc;
-                    const double sj = self ? si : Sh[static_cast<size_t>(j) * n + i];
-                    const double yj = self ? yi : Yh[static_cast<size_t>(j) * n + i];
-                    v[3 * j] += si * yj;
-                    v[3 * j + 1] += sj * yi;
-                    v[3 * j + 2] -= sj * ri;
+                    v[3 * j] += si * y[j];
+                    v[3 * j + 1] += s[j] * yi;
+                    v[3 * j + 2] -= s[j] * ri;
                 }
         }
     }
-    if (!seg_finish<NV>(v, 0u, sg, partials)) return;
-    if (threadIdx.x != 0) return;
-    if (sg->state != kRun) return;
-    if (sg->first) {  // iteration 1: d = -H0 r, no pair yet
-        sg->first = 0;
-        sg->ncorr = 0;
+    griddep_launch();
+    const double t = seg_totals<NV>(v, sg, partials, sh, &last);
+    if (!last || tid >= 32) return;
+    if (first) {  // iteration 1: d = -H0 r, no pair yet
+        if (lane == 0) {
+            sg->first = 0;
+            sg->ncorr = 0;
+        }
         return;
     }
-    const double ys = v[3 * M], yy = v[3 * M + 1];
-    for (int j = 0; j < ncorr; j++) {
-        sg->G[loc][j] = v[3 * j];
-        sg->G[j][loc] = v[3 * j + 1];
+    tot[lane] = t;
+    __syncwarp();
+    if (lane < ncorr) {
+        sG[loc * M + lane] = tot[3 * lane];
+        sG[lane * M + loc] = tot[3 * lane + 1];
     }
-    sg->G[loc][loc] = ys;
-    sg->ys[loc] = ys;
-    double al[M];
-    for (int i = 0; i < ncorr; i++) {  // newest slot first
-        const int j = ring(loc - i, M);
-        double t = v[3 * j + 2];
-        for (int q = 0; q < i; q++) {
-            const int jq = ring(loc - q, M);
-            t -= al[jq] * sg->G[j][jq];
-        }
-        al[j] = t / sg->ys[j];
+    __syncwarp();
+    if (lane == 0) sG[loc * M + loc] = tot[3 * M];
+    if (lane == loc) ys = tot[3 * M];
+    __syncwarp();
+    const double al = first_loop(lane < ncorr ? tot[3 * lane + 2] : 0.0, ys, sG, M, loc, M, ncorr);
+    if (lane < ncorr) {
+        sg->G[loc][lane] = sG[loc * M + lane];
+        sg->G[lane][loc] = sG[lane * M + loc];
+        sg->alpha[lane] = al;
     }
-    for (int j = 0; j < ncorr; j++) sg->alpha[j] = al[j];
-    sg->theta = yy / ys;
-    sg->ptr = loc + 1;
-    sg->ncorr = ncorr;
+    if (lane == 0) {
+        sg->ys[loc] = tot[3 * M];
+        sg->theta = tot[3 * M + 1] / tot[3 * M];
+        sg->ptr = loc + 1;
+        sg->ncorr = ncorr;
+    }
 }
 
 // Pass 2: q = -r - sum_j alpha_j y_j for running members (0 elsewhere)
 __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const double* __restrict__ r,
     const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S)
 {
+    griddep_wait();
+    griddep_launch();
     const Chunk c = ch[blockIdx.x];
     const Seg* sg = S + c.seg;
     __shared__ double al[kHist];
@@ -325,32 +377,29 @@ template <int M>
 __global__ void __launch_bounds__(kT) kb_pass3(const double* __restrict__ z, const double* __restrict__ Yh, size_t n,
     const Chunk* __restrict__ ch, Seg* S, double* partials)
 {
+    griddep_wait();
+    __shared__ double sh[kT / 32][32], sG[M * M];
+    __shared__ bool last;
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
-    const int ncorr = sg->state == kRun ? sg->ncorr : 0;
+    if (sg->state != kRun) return;
+    const int tid = threadIdx.x, lane = tid & 31, ncorr = sg->ncorr, ptr = sg->ptr;
+    if (tid < M * M) sG[tid] = sg->G[tid / M][tid % M];
+    const double ys = tid < M ? sg->ys[tid] : 1.0, alpha = tid < M ? sg->alpha[tid] : 0.0;
     double v[M];
 #pragma unroll
     for (int k = 0; k < M; k++) v[k] = 0.0;
-    for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
+    for (int i = c.a + tid; i < c.b; i += kT) {
         const double zi = z[i];
 #pragma unroll
         for (int j = 0; j < M; j++)
             if (j < ncorr) v[j] += Yh[static_cast<size_t>(j) * n + i] * zi;
     }
-    if (!seg_finish<M>(v, 0u, sg, partials)) return;
-    if (threadIdx.x != 0 || sg->state != kRun) return;
-    const int ptr = sg->ptr;
-    double cf[M];
-    for (int o = 0; o < ncorr; o++) {
-        const int j = ring(ptr - ncorr + o, M);
-        double t = v[j];
-        for (int p = 0; p < o; p++) {
-            const int jp = ring(ptr - ncorr + p, M);
-            t += cf[jp] * sg->G[jp][j];
-        }
-        cf[j] = sg->alpha[j] - t / sg->ys[j];
-    }
-    for (int j = 0; j < ncorr; j++) sg->coef[j] = cf[j];
+    griddep_launch();
+    const double t = seg_totals<M>(v, sg, partials, sh, &last);
+    if (!last || tid >= 32) return;
+    const double cf = second_loop(t, ys, alpha, sG, M, ptr, M, ncorr);
+    if (lane < ncorr) sg->coef[lane] = cf;
 }
 
 // Pass 4: d = z + sum_j coef_j s_j and the start of the line search of every
@@ -361,11 +410,13 @@ __global__ void __launch_bounds__(kT) kb_pass4(double* __restrict__ d, const dou
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, const Chunk* __restrict__ ch, Seg* S,
     double* partials)
 {
+    griddep_wait();
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
     const bool act = sg->state == kRun;
     const int ncorr = act ? sg->ncorr : 0;
-    __shared__ double cf[kHist];
+    __shared__ double cf[kHist], sh[kT / 32][32];
+    __shared__ bool last;
     if (threadIdx.x < kHist) cf[threadIdx.x] = static_cast<int>(threadIdx.x) < ncorr ? sg->coef[threadIdx.x] : 0.0;
     __syncthreads();
     double v[1] = { 0.0 };
@@ -383,89 +434,14 @@ __global__ void __launch_bounds__(kT) kb_pass4(double* __restrict__ d, const dou
         }
         r[i] = -fext[i];
     }
-    if (!seg_finish<1>(v, 0u, sg, partials)) return;
-    if (threadIdx.x != 0 || sg->state != kRun) return;
-    sg->dg0 = v[0];
+    griddep_launch();
+    if (!act) return;
+    const double dg0 = seg_totals<1>(v, sg, partials, sh, &last);
+    if (!last || threadIdx.x != 0) return;
+    sg->dg0 = dg0;
     sg->step = 1.0;
     sg->ls_t = 0;
     sg->trial = 1;
-}
-
-// After a trial's residual: r.d, ||r||_inf, ||x||_inf, ||x||^2 of every
-// member in its line search, which applies the reference's rule (accept when
-// |r.d| <= |r0.d|, else step x1.5 if (r.d)(r0.d) > 0, x0.5 otherwise, at
-// most max_line_search trials, LineSearchFEA.h:43-67).
-__global__ void __launch_bounds__(kT) kb_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
-    const double* __restrict__ x, const Chunk* __restrict__ ch, Seg* S, double* partials)
-{
-    const Chunk c = ch[blockIdx.x];
-    Seg* sg = S + c.seg;
-    const bool act = sg->state == kRun && sg->trial;
-    double v[4] = { 0, 0, 0, 0 };
-    if (act)
-        for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
-            const double ri = r[i], xi = x[i];
-            v[0] += ri * d[i];
-            v[1] = nan_max(v[1], fabs(ri));
-            v[2] = nan_max(v[2], fabs(xi));
-            v[3] += xi * xi;
-        }
-    if (!seg_finish<4>(v, 6u, sg, partials)) return;
-    if (threadIdx.x != 0) return;
-    if (act) {
-        sg->dg = v[0];
-        sg->rinf = v[1];
-        sg->xinf = v[2];
-        sg->x2 = v[3];
-        sg->n_res++;
-        const int t = ++sg->ls_t;
-        const bool again = !(fabs(v[0]) <= fabs(sg->dg0)) && t < sg->max_ls;
-        if (again) sg->step *= v[0] * sg->dg0 > 0 ? 1.5 : 0.5;
-        sg->trial = again ? 1 : 0;
-    }
-}
-
-// The trial loop's condition: some member wants another trial.  The loop
-// is also bounded here, whatever the members' state: after max_ls trials of
-// one iteration every line search ends.
-__global__ void __launch_bounds__(1024) kb_ls_decide(Seg* S, int nseg, int max_ls, Glob* G,
-    cudaGraphConditionalHandle h)
-{
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    const bool stop = G->ls_round + 1 >= max_ls;
-    int mine = 0;
-    for (int i = threadIdx.x; i < nseg; i += blockDim.x) {
-        Seg& s = S[i];
-        if (s.state != kRun || !s.trial) continue;
-        if (stop)
-            s.trial = 0;
-        else
-            mine = 1;
-    }
-    if (mine) atomicOr(&any, 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        G->ls_round++;
-        if (any) G->trials++;
-        cudaGraphSetConditional(h, any ? 1u : 0u);
-    }
-}
-
-// a further trial: x = xp + step d for the members still in their line search; r = -f_ext everywhere
-__global__ void __launch_bounds__(kT) kb_trial(double* __restrict__ x, const double* __restrict__ xp,
-    const double* __restrict__ d, double* __restrict__ r, const double* __restrict__ fext,
-    const Chunk* __restrict__ ch, const Seg* S)
-{
-    const Chunk c = ch[blockIdx.x];
-    const Seg* sg = S + c.seg;
-    const bool act = sg->state == kRun && sg->trial;
-    const double step = sg->step;
-    for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
-        if (act) x[i] = __fma_rn(step, d[i], xp[i]);
-        r[i] = -fext[i];
-    }
 }
 
 // End of an iteration for every running member (LBFGS.h:150-170): stop on a
@@ -473,9 +449,8 @@ __global__ void __launch_bounds__(kT) kb_trial(double* __restrict__ x, const dou
 // <= eps ||x||_inf), at the iteration limit, or (FP32 phase) when the best
 // ||r||_inf has not halved for `stall` iterations; else count the iteration.
 // Sets the iteration loop's condition: some member runs and the launch has
-// iterations left.
-__global__ void __launch_bounds__(1024) kb_decide(Seg* S, int nseg, Glob* G, const int* perr, int* frozen,
-    cudaGraphConditionalHandle h)
+// iterations left.  One CTA, all its threads.
+__device__ void iter_decide(Seg* S, int nseg, Glob* G, const int* perr, int* frozen, cudaGraphConditionalHandle h)
 {
     __shared__ int running;
     if (threadIdx.x == 0) running = 0;
@@ -517,6 +492,98 @@ __global__ void __launch_bounds__(1024) kb_decide(Seg* S, int nseg, Glob* G, con
         cudaGraphSetConditional(h, more ? 1u : 0u);
     }
 }
+
+// After a trial's residual: r.d, ||r||_inf, ||x||_inf, ||x||^2 of every
+// member in its line search, which applies the reference's rule (accept when
+// |r.d| <= |r0.d|, else step x1.5 if (r.d)(r0.d) > 0, x0.5 otherwise, at
+// most max_line_search trials, LineSearchFEA.h:43-67).  The CTA that finishes
+// the last member sets the trial loop's condition -- some member wants another
+// trial; bounded here whatever the members' state: after max_ls trials of one
+// iteration every line search ends -- and, when none does, ends the iteration.
+__global__ void __launch_bounds__(kT) kb_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
+    const double* __restrict__ x, const Chunk* __restrict__ ch, Seg* S, double* partials, int nseg, int max_ls, Glob* G,
+    const int* perr, int* frozen, cudaGraphConditionalHandle h_ls, cudaGraphConditionalHandle h_it)
+{
+    griddep_wait();
+    __shared__ int any;
+    __shared__ bool last_seg;
+    const Chunk c = ch[blockIdx.x];
+    Seg* sg = S + c.seg;
+    const bool act = sg->state == kRun && sg->trial;
+    if (act) {
+        double v[4] = { 0, 0, 0, 0 };
+        for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
+            const double ri = r[i], xi = x[i];
+            v[0] += ri * d[i];
+            v[1] = nan_max(v[1], fabs(ri));
+            v[2] = nan_max(v[2], fabs(xi));
+            v[3] += xi * xi;
+        }
+        if (!seg_finish<4>(v, 6u, sg, partials)) return;
+        if (threadIdx.x == 0) {
+            sg->dg = v[0];
+            sg->rinf = v[1];
+            sg->xinf = v[2];
+            sg->x2 = v[3];
+            sg->n_res++;
+            const int t = ++sg->ls_t;
+            const bool again = !(fabs(v[0]) <= fabs(sg->dg0)) && t < sg->max_ls;
+            if (again) sg->step *= v[0] * sg->dg0 > 0 ? 1.5 : 0.5;
+            sg->trial = again ? 1 : 0;
+        }
+    } else if (static_cast<int>(blockIdx.x) != sg->c0)
+        return;  // one CTA counts a member that takes no part
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last_seg = atomicAdd(&G->cnt, 1u) == static_cast<unsigned>(nseg - 1);
+        any = 0;
+    }
+    __syncthreads();
+    if (!last_seg) return;
+    __threadfence();
+    const bool stop = G->ls_round + 1 >= max_ls;
+    int mine = 0;
+    for (int i = threadIdx.x; i < nseg; i += blockDim.x) {
+        Seg& s = S[i];
+        if (s.state != kRun || !s.trial) continue;
+        if (stop)
+            s.trial = 0;
+        else
+            mine = 1;
+    }
+    if (mine) atomicOr(&any, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        G->cnt = 0u;
+        G->ls_round++;
+        if (any) G->trials++;
+        cudaGraphSetConditional(h_ls, any ? 1u : 0u);
+    }
+    if (!any) iter_decide(S, nseg, G, perr, frozen, h_it);
+}
+
+// a further trial: x = xp + step d for the members still in their line search; r = -f_ext everywhere
+__global__ void __launch_bounds__(kT) kb_trial(double* __restrict__ x, const double* __restrict__ xp,
+    const double* __restrict__ d, double* __restrict__ r, const double* __restrict__ fext,
+    const Chunk* __restrict__ ch, const Seg* S)
+{
+    griddep_wait();
+    griddep_launch();
+    const Chunk c = ch[blockIdx.x];
+    const Seg* sg = S + c.seg;
+    const bool act = sg->state == kRun && sg->trial;
+    const double step = sg->step;
+    for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
+        if (act) x[i] = __fma_rn(step, d[i], xp[i]);
+        r[i] = -fext[i];
+    }
+}
+
+// launch_k uses programmatic dependent launch while one of these is alive
+struct PdlScope {
+    explicit PdlScope(bool on) { t_pdl = on; }
+    ~PdlScope() { t_pdl = false; }
+};
 
 efem_status add_while_node(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t* body)
 {
@@ -560,6 +627,7 @@ struct Union {
     cudaStream_t cap[3] = { nullptr, nullptr, nullptr };
     cudaGraphExec_t loop[2] = { nullptr, nullptr };  // per element precision (FP64, FP32)
     long long loop_epoch[2] = { -1, -1 };
+    bool pdl = true;  // programmatic dependent launch in the captured loops (off if a capture refused it)
     long long per_res = 0;
     ~Union();
 };
@@ -725,13 +793,15 @@ efem_status setup_union(Union& U)
 }
 
 // the iteration graph: while (iterate) { passes, H0, first trial, residual,
-// line-search reduction; while (trial) { trial, residual, reduction }; decide }
+// line-search reduction and decisions; while (trial) { trial, residual, reduction and decisions } }
 efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
 {
     Model& M = *U.uni;
     std::lock_guard<std::mutex> lock(capture_mutex());
     cudaStream_t s0 = U.cap[0], s1 = U.cap[1], s2 = U.cap[2];
-    const int nb = U.nchunk;
+    const int nb = U.nchunk, max_ls = std::max(1, M.opts.max_linesearch);
+    const int* perr = precond_error_flag(M);
+    PdlScope pdl(U.pdl);  // the first kernel of each body graph is a plain launch
     cudaGraph_t g = nullptr;
     efem_status s = EFEM_OK;
     const long long launches = M.launches;
@@ -761,18 +831,18 @@ efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
             P1(1) P1(2) P1(3) P1(4) P1(5) P1(6) P1(7) P1(8)
 #undef P1
         }
-        kb_pass2<<<nb, kT, 0, s1>>>(U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg);
+        launch_k(kb_pass2, nb, kT, 0, s1, U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg);
         if ((s = precond_enqueue(M, U.q, s1)) != EFEM_OK) break;
         switch (U.m) {
-#define P3(K) case K: kb_pass3<K><<<nb, kT, 0, s1>>>(U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
+#define P3(K) case K: launch_k(kb_pass3<K>, nb, kT, 0, s1, U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
             P3(1) P3(2) P3(3) P3(4) P3(5) P3(6) P3(7) P3(8)
 #undef P3
         }
-        kb_pass4<<<nb, kT, 0, s1>>>(U.d, U.q, U.Sh, U.r, U.x, U.xp, U.rp, M.d_fext, U.n, U.d_chunks, U.d_seg,
+        launch_k(kb_pass4, nb, kT, 0, s1, U.d, U.q, U.Sh, U.r, U.x, U.xp, U.rp, M.d_fext, U.n, U.d_chunks, U.d_seg,
             U.partials);
         if ((s = launch_residual_on(M, U.x, U.r, s1, nullptr, false)) != EFEM_OK) break;
-        kb_ls_reduce<<<nb, kT, 0, s1>>>(U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials);
-        kb_ls_decide<<<1, 1024, 0, s1>>>(U.d_seg, U.nseg, std::max(1, M.opts.max_linesearch), U.d_glob, h_ls);
+        launch_k(kb_ls_reduce, nb, kT, 0, s1, U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials, U.nseg, max_ls, U.d_glob, perr,
+            U.d_frozen, h_ls, h_it);
         if ((s = add_while_node(s1, h_ls, &ls_body)) != EFEM_OK) break;
         if (cudaStreamBeginCaptureToGraph(s2, ls_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
@@ -780,12 +850,11 @@ efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
         }
         kb_trial<<<nb, kT, 0, s2>>>(U.x, U.xp, U.d, U.r, M.d_fext, U.d_chunks, U.d_seg);
         s = launch_residual_on(M, U.x, U.r, s2, nullptr, false);
-        kb_ls_reduce<<<nb, kT, 0, s2>>>(U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials);
-        kb_ls_decide<<<1, 1024, 0, s2>>>(U.d_seg, U.nseg, std::max(1, M.opts.max_linesearch), U.d_glob, h_ls);
+        launch_k(kb_ls_reduce, nb, kT, 0, s2, U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials, U.nseg, max_ls, U.d_glob, perr,
+            U.d_frozen, h_ls, h_it);
         cudaGraph_t tmp = nullptr;
         if (cudaStreamEndCapture(s2, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
         if (s != EFEM_OK) break;
-        kb_decide<<<1, 1024, 0, s1>>>(U.d_seg, U.nseg, U.d_glob, precond_error_flag(M), U.d_frozen, h_it);
         if (cudaStreamEndCapture(s1, &tmp) != cudaSuccess) s = EFEM_ERR_CUDA;
     } while (false);
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
@@ -852,14 +921,20 @@ efem_status run_union_phase(Union& U, int stall, const std::vector<int>& keep, l
     if (!U.loop[slot] || U.loop_epoch[slot] != M.epoch) {
         if (U.loop[slot]) cudaGraphExecDestroy(U.loop[slot]);
         U.loop[slot] = nullptr;
-        if ((s = capture_union_loop(U, &U.loop[slot])) != EFEM_OK) return s;
+        s = capture_union_loop(U, &U.loop[slot]);
+        if (s != EFEM_OK && U.pdl) {
+            cudaGetLastError();
+            U.pdl = false;  // capture again with plain launches
+            s = capture_union_loop(U, &U.loop[slot]);
+        }
+        if (s != EFEM_OK) return s;
         U.loop_epoch[slot] = M.epoch;
     }
     Glob g {};
     long long body0 = 0, trials0 = 0;
-    // per loop body: passes 1-4, H0, residual, reduction, decision; per extra trial: trial, residual, reduction
-    const long long per_body = 7 + precond_launch_count(M) + (U.per_res - 1) + 1;
-    const long long per_trial = 3 + (U.per_res - 1);
+    // per loop body: passes 1-4, H0, residual, reduction with the decisions; per extra trial: trial, residual, reduction
+    const long long per_body = 5 + precond_launch_count(M) + (U.per_res - 1);
+    const long long per_trial = 2 + (U.per_res - 1);
     for (;;) {
         EFEM_CUDA(cudaGraphLaunch(U.loop[slot], st));
         EFEM_CUDA(cudaMemcpyAsync(&g, U.d_glob, sizeof(Glob), cudaMemcpyDeviceToHost, st));

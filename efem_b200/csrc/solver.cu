@@ -43,6 +43,7 @@
 #include <map>
 
 #include "efem_internal.h"
+#include "reduce.cuh"
 
 namespace efem {
 
@@ -239,6 +240,42 @@ __global__ void k_trial(double* __restrict__ x, const double* __restrict__ xp, c
     GRID_STRIDE(i, n) x[i] = __fma_rn(step, d[i], xp[i]);
 }
 
+// End of an iteration (LBFGS.h:150-170): stop on a non-finite residual or
+// solution, on convergence (||r||_inf <= eps or <= eps ||x||_inf) or at the
+// iteration limit; otherwise count the iteration and go on, up to `cap`
+// iterations per launch.  Sets the iteration loop condition.  One thread.
+__device__ void iter_decide(Scalars* S, cudaGraphConditionalHandle h, double* hread)
+{
+    const double rinf = S->rinf, xinf = S->xinf;
+    int st = kRunning;
+    S->n_body++;
+    if (S->perr != 0.0)
+        st = kPrecondFail;
+    else if (!isfinite(rinf) || !isfinite(xinf))
+        st = kNonFinite;
+    else if (rinf <= S->eps || rinf <= S->eps * xinf)
+        st = kConverged;
+    else if (S->max_iter != 0 && S->k >= S->max_iter)
+        st = kMaxIters;
+    else if (S->stall_iters > 0 && !(rinf < 0.5 * S->best_rinf) && S->k - S->best_k >= S->stall_iters)
+        st = kStalled;
+    else {
+        if (rinf < 0.5 * S->best_rinf) {
+            S->best_rinf = rinf;
+            S->best_k = S->k;
+        }
+        S->k++;
+        if (++S->launch_iters >= S->cap) st = kCapReached;
+    }
+    S->status = st;
+    hread[kRdStatus] = st;
+    hread[kRdK] = S->k;
+    hread[kRdNExtra] = static_cast<double>(S->n_extra);
+    hread[kRdNBody] = static_cast<double>(S->n_body);
+    hread[kRdTPc] = static_cast<double>(S->t_pc);
+    cudaGraphSetConditional(h, st == kRunning ? 1u : 0u);
+}
+
 // line-search scalars: dg = r.d, rinf = ||r||_inf, xinf = ||x||_inf, x2 = ||x||^2,
 // stored in S and in the host-mapped read-back array; with a trace buffer the
 // trial also (over)writes the current iteration's record, so the record left
@@ -246,10 +283,11 @@ __global__ void k_trial(double* __restrict__ x, const double* __restrict__ xp, c
 // With `decide` (inside the device-driven line search) the last CTA also
 // applies the accept / scale rule of LineSearchFEA.h:43-67: accept when
 // |r.d| <= |r0.d|; otherwise scale the step by 1.5 (same sign) or 0.5 and try
-// again, at most max_ls trials in all; it sets the line-search loop condition.
+// again, at most max_ls trials in all; it sets the line-search loop condition
+// and, when the line search ends, the iteration loop's (iter_decide).
 __global__ void __launch_bounds__(kThreads) k_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
     const double* __restrict__ x, size_t n, Scalars* S, double* partials, const int* perr, double* hread,
-    cudaGraphConditionalHandle h, int decide)
+    cudaGraphConditionalHandle h, cudaGraphConditionalHandle h_it, int decide)
 {
     griddep_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -305,6 +343,7 @@ __global__ void __launch_bounds__(kThreads) k_ls_reduce(const double* __restrict
                 S->n_extra++;
             }
             cudaGraphSetConditional(h, again ? 1u : 0u);
+            if (!again) iter_decide(S, h_it, hread);
         }
     }
 }
@@ -412,62 +451,82 @@ __global__ void __launch_bounds__(kThreads) k_pass1(const double* __restrict__ x
     }
 }
 
-// Sums of NV values over a 1D grid in a fixed order: every CTA stores its
-// block sums; the last CTA to finish adds them up -- each thread the CTAs
-// b = t, t + kThreads, ... for all NV values at once (independent loads, a
-// couple of round trips), then a block reduction -- into out[0, NV).
-// Returns true in every thread of the last CTA.
+// ---- passes of a history of M <= 8 pairs
+//
+// Each thread reads x, xp, r, rp (or z) once for all slots and keeps the dot
+// products in registers; few CTAs, so that few partial sums are left for
+// the last CTA, whose first warp runs the recursion.  Up to kOne entries one
+// CTA does it all, and goes on with pass 2 (or 4) itself: the recursion's
+// result need not leave the CTA, and a launch is saved.  What bounds them is
+// the chain reduction - last CTA - recursion, not the vectors (17 MB of L2
+// reads on the C3D20R cap).  All passes, reductions and loop nodes of an
+// iteration: 66 -> 51 us on that cap (134k DOFs), 45 -> 31 us at 750 DOFs,
+// against five shuffles per value, 592 CTAs and a serial recursion.
+constexpr int kPT = 512;     // threads
+constexpr int kPG = 296;     // most CTAs: two per SM (one: 7 us an iteration slower on the mixed finger, 241k DOFs)
+constexpr size_t kOne = 4096;  // entries of one CTA (750 DOFs: 61.7 us an iteration against 65.0 with passes 2 and 4 apart)
+
+int pass_grid(size_t n) { return n <= kOne ? 1 : static_cast<int>(std::min<size_t>(kPG, (n + kPT - 1) / kPT)); }
+
+// Totals of NV values over the grid, in a fixed order: lane k < NV of the last
+// CTA's warp 0 returns with the total of value k; *last is set in that CTA.
 template <int NV>
-__device__ bool grid_sums(double* v, double* partials, unsigned int* counter, double* out)
+__device__ __forceinline__ double grid_totals(const double (&v)[NV], double* partials, unsigned int* counter, double (*sh)[32],
+    bool* last)
 {
-    __shared__ bool last;
-    int ops[NV];
-#pragma unroll
-    for (int k = 0; k < NV; k++) ops[k] = 0;
-    block_reduce<NV>(v, ops);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; k++) partials[blockIdx.x * NV + k] = v[k];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double t = cta_sums<NV, kPT / 32>(v, sh);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) *last = true;
+        __syncthreads();
+        return t;
+    }
+    if (w == 0) {
+        if (lane < NV) partials[blockIdx.x * NV + lane] = t;
         __threadfence();
-        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        __syncwarp();
+        if (lane == 0) *last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last) return false;
+    if (!*last) return 0.0;
     __threadfence();
-    double acc[NV];
+    t = 0.0;
+    if (lane < NV) {
+        double p[(kPG + kPT / 32 - 1) / (kPT / 32)];
 #pragma unroll
-    for (int k = 0; k < NV; k++) acc[k] = 0.0;
-    for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += kThreads) {
-        const volatile double* pb = partials + static_cast<size_t>(b) * NV;
-        double p[NV];
+        for (int e = 0; e < (kPG + kPT / 32 - 1) / (kPT / 32); e++) {
+            const int b = w + e * (kPT / 32);
+            p[e] = b < static_cast<int>(gridDim.x) ? __ldcg(partials + b * NV + lane) : 0.0;
+        }
 #pragma unroll
-        for (int k = 0; k < NV; k++) p[k] = pb[k];
-#pragma unroll
-        for (int k = 0; k < NV; k++) acc[k] += p[k];
+        for (int e = 0; e < (kPG + kPT / 32 - 1) / (kPT / 32); e++) t += p[e];
     }
-    block_reduce<NV>(acc, ops);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; k++) out[k] = acc[k];
-        *counter = 0u;
-    }
+    sh[w][lane] = t;
     __syncthreads();
-    return true;
+    t = 0.0;
+    if (w == 0) {
+#pragma unroll
+        for (int q = 0; q < kPT / 32; q++) t += sh[q][lane];
+        if (lane == 0) *counter = 0u;
+    }
+    return t;
 }
 
-// Pass 1 for a history of M <= 8 pairs on a 1D grid: each thread reads x, xp,
-// r, rp once for all slots (the 2D k_pass1 re-reads them per slot) and keeps
-// the 3M + 2 dot products in registers; the last CTA runs the same recursion.
+// Pass 1 (see the file comment) and, with one CTA, pass 2
 template <int M>
-__global__ void __launch_bounds__(kThreads) k_pass1_m(const double* __restrict__ x, const double* __restrict__ xp,
+__global__ void __launch_bounds__(kPT) k_pass1_m(const double* __restrict__ x, const double* __restrict__ xp,
     const double* __restrict__ r, const double* __restrict__ rp, double* __restrict__ Sh, double* __restrict__ Yh,
-    size_t n, Scalars* S, double* partials)
+    size_t n, Scalars* S, double* partials, double* __restrict__ q, int divide_theta)
 {
     griddep_wait();
     constexpr int NV = 3 * M + 2;
-    const int m = M;
-    const int loc = S->ptr % m;
-    const int ncorr = S->ncorr < m ? S->ncorr + 1 : m;
+    __shared__ double sh[kPT / 32][32], sG[M * M], tot[32], sal[M], sth;
+    __shared__ bool last;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int loc = S->ptr % M;
+    const int ncorr = S->ncorr < M ? S->ncorr + 1 : M;
+    if (tid < M * M) sG[tid] = S->G[tid / M][tid % M];
+    double ys = tid < M ? S->ys[tid] : 1.0;
     double v[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) v[k] = 0.0;
@@ -476,71 +535,102 @@ __global__ void __launch_bounds__(kThreads) k_pass1_m(const double* __restrict__
     GRID_STRIDE(i, n)
     {
         const double si = x[i] - xp[i], ri = r[i], yi = ri - rp[i];
+        double s[M], y[M];
+#pragma unroll
+        for (int j = 0; j < M; j++) {
+            s[j] = j < ncorr && j != loc ? Sh[j * n + i] : si;
+            y[j] = j < ncorr && j != loc ? Yh[j * n + i] : yi;
+        }
         snew[i] = si;
         ynew[i] = yi;
         v[3 * M] += si * yi;
         v[3 * M + 1] += yi * yi;
 #pragma unroll
-        for (int j = 0; j < M; j++) {
+        for (int j = 0; j < M; j++)
             if (j < ncorr) {
-                const bool self = j == loc;
-                const double sj = self ? si : Sh[j * n + i], yj = self ? yi : Yh[j * n + i];
-                v[3 * j] += si * yj;      // s_new . y_j
-                v[3 * j + 1] += sj * yi;  // s_j . y_new
-                v[3 * j + 2] -= sj * ri;  // s_j . q0
+                v[3 * j] += si * y[j];      // s_new . y_j
+                v[3 * j + 1] += s[j] * yi;  // s_j . y_new
+                v[3 * j + 2] -= s[j] * ri;  // s_j . q0
             }
-        }
     }
     griddep_launch();
-    __shared__ double tot[NV];
-    if (!grid_sums<NV>(v, partials, &S->counter[2], tot)) return;
-    extern __shared__ double dyn[];
-    double* sG = dyn;
-    double* sys = dyn + m * m;
-    double* sal = sys + m;
-    const int tid = threadIdx.x;
-    for (int q = tid; q < m * m; q += kThreads) sG[q] = S->G[q / m][q % m];
-    for (int j = tid; j < m; j += kThreads) sys[j] = S->ys[j];
-    __syncthreads();
-    const double ys = tot[3 * M], yy = tot[3 * M + 1];
-    for (int j = tid; j < ncorr; j += kThreads) {
-        sG[loc * m + j] = tot[3 * j];
-        sG[j * m + loc] = tot[3 * j + 1];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        sG[loc * m + loc] = ys;
-        sys[loc] = ys;
-        for (int i = 0; i < ncorr; i++) {  // first loop (LBFGSMat.h:106-113): newest slot first
-            const int j = ((loc - i) % m + m) % m;
-            double t = tot[3 * j + 2];
-            for (int k = 0; k < i; k++) {
-                const int jk = ((loc - k) % m + m) % m;
-                t -= sal[jk] * sG[j * m + jk];
-            }
-            sal[j] = t / sys[j];
+    const double t = grid_totals<NV>(v, partials, &S->counter[2], sh, &last);
+    if (!last) return;
+    if (tid < 32) {
+        tot[lane] = t;
+        __syncwarp();
+        if (lane < ncorr) {
+            sG[loc * M + lane] = tot[3 * lane];
+            sG[lane * M + loc] = tot[3 * lane + 1];
         }
-        S->theta = yy / ys;
-        S->ptr = loc + 1;
-        S->ncorr = ncorr;
-        S->ys[loc] = ys;
+        __syncwarp();
+        if (lane == 0) sG[loc * M + loc] = tot[3 * M];
+        if (lane == loc) ys = tot[3 * M];
+        __syncwarp();
+        const double al = first_loop(lane < ncorr ? tot[3 * lane + 2] : 0.0, ys, sG, M, loc, M, ncorr);
+        if (lane < ncorr) {
+            S->G[loc][lane] = sG[loc * M + lane];
+            S->G[lane][loc] = sG[lane * M + loc];
+            S->alpha[lane] = al;
+            sal[lane] = al;
+        }
+        if (lane == 0) {
+            sth = tot[3 * M + 1] / tot[3 * M];
+            S->theta = sth;
+            S->ptr = loc + 1;
+            S->ncorr = ncorr;
+            S->ys[loc] = tot[3 * M];
+        }
     }
+    if (gridDim.x > 1) return;
     __syncthreads();
-    for (int j = tid; j < ncorr; j += kThreads) {
-        S->G[loc][j] = sG[loc * m + j];
-        S->G[j][loc] = sG[j * m + loc];
-        S->alpha[j] = sal[j];
+    for (size_t i = tid; i < n; i += kPT) {
+        double qi = -r[i];
+        for (int j = 0; j < ncorr; j++) qi -= sal[j] * Yh[j * n + i];
+        q[i] = divide_theta ? qi / sth : qi;
     }
 }
 
-// Pass 3 for M <= 8 on a 1D grid: z read once for all slots
+// Pass 4 of entry i: d = z + sum_j coef_j s_j, the line search's start and
+// first trial; returns r . d
+__device__ __forceinline__ double pass4_entry(size_t i, double* __restrict__ d, const double* __restrict__ z,
+    const double* __restrict__ Sh, double* __restrict__ r, double* __restrict__ x, double* __restrict__ xp,
+    double* __restrict__ rp, const double* __restrict__ fext, size_t n, int ncorr, const double* cf)
+{
+    double di = z[i];
+    for (int j = 0; j < ncorr; j++) di += cf[j] * Sh[j * n + i];
+    d[i] = di;
+    const double ri = r[i], xi = x[i];
+    xp[i] = xi;
+    rp[i] = ri;
+    x[i] = xi + 1.0 * di;
+    r[i] = -fext[i];
+    return ri * di;
+}
+__device__ __forceinline__ void pass4_done(Scalars* S, double dg0)
+{
+    S->dg0 = dg0;
+    S->step = 1.0;
+    S->ls_t = 0;
+    S->tr_i++;  // the next iteration's trace record
+    S->tr_evals = 0;
+    S->t0_res = gtimer();
+}
+
+// Pass 3 and, with one CTA, pass 4
 template <int M>
-__global__ void __launch_bounds__(kThreads) k_pass3_m(const double* __restrict__ z, const double* __restrict__ Yh,
-    size_t n, Scalars* S, double* partials, int time_pc)
+__global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, const double* __restrict__ Yh,
+    size_t n, Scalars* S, double* partials, int time_pc, double* __restrict__ d, const double* __restrict__ Sh,
+    double* __restrict__ r, double* __restrict__ x, double* __restrict__ xp, double* __restrict__ rp,
+    const double* __restrict__ fext)
 {
     griddep_wait();
-    const int m = M, ncorr = S->ncorr;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && time_pc) S->t_pc += gtimer() - S->t0_pc;  // H0 just ended
+    __shared__ double sh[kPT / 32][32], sG[M * M], cf[M];
+    __shared__ bool last;
+    const int tid = threadIdx.x, lane = tid & 31, ncorr = S->ncorr, ptr = S->ptr;
+    if (blockIdx.x == 0 && tid == 0 && time_pc) S->t_pc += gtimer() - S->t0_pc;  // H0 just ended
+    if (tid < M * M) sG[tid] = S->G[tid / M][tid % M];
+    const double ys = tid < M ? S->ys[tid] : 1.0, alpha = tid < M ? S->alpha[tid] : 0.0;
     double v[M];
 #pragma unroll
     for (int k = 0; k < M; k++) v[k] = 0.0;
@@ -552,34 +642,22 @@ __global__ void __launch_bounds__(kThreads) k_pass3_m(const double* __restrict__
             if (j < ncorr) v[j] += Yh[j * n + i] * zi;
     }
     griddep_launch();
-    __shared__ double tot[M];
-    if (!grid_sums<M>(v, partials, &S->counter[3], tot)) return;
-    extern __shared__ double dyn[];
-    double* sG = dyn;
-    double* sys = dyn + m * m;
-    double* sal = sys + m;
-    double* scf = sal + m;
-    const int tid = threadIdx.x;
-    for (int q = tid; q < m * m; q += kThreads) sG[q] = S->G[q / m][q % m];
-    for (int j = tid; j < m; j += kThreads) {
-        sys[j] = S->ys[j];
-        sal[j] = S->alpha[j];
-    }
-    __syncthreads();
-    if (tid == 0) {  // second loop (LBFGSMat.h:121-128), oldest pair first
-        const int ptr = S->ptr;
-        for (int o = 0; o < ncorr; o++) {
-            const int j = ((ptr - ncorr + o) % m + m) % m;
-            double t = tot[j];
-            for (int p = 0; p < o; p++) {
-                const int jp = ((ptr - ncorr + p) % m + m) % m;
-                t += scf[jp] * sG[jp * m + j];
-            }
-            scf[j] = sal[j] - t / sys[j];
+    const double t = grid_totals<M>(v, partials, &S->counter[3], sh, &last);
+    if (!last) return;
+    if (tid < 32) {
+        const double c = second_loop(t, ys, alpha, sG, M, ptr, M, ncorr);
+        if (lane < ncorr) {
+            S->coef[lane] = c;
+            cf[lane] = c;
         }
     }
+    if (gridDim.x > 1) return;
     __syncthreads();
-    for (int j = tid; j < ncorr; j += kThreads) S->coef[j] = scf[j];
+    double w[1] = { 0.0 };
+    for (size_t i = tid; i < n; i += kPT) w[0] += pass4_entry(i, d, z, Sh, r, x, xp, rp, fext, n, ncorr, cf);
+    __syncthreads();
+    const double dg = cta_sums<1, kPT / 32>(w, sh);
+    if (tid == 0) pass4_done(S, dg);
 }
 
 // Pass 2: q = (q0 - sum_j alpha_j y_j) [/ theta when H0 = I / theta]
@@ -648,39 +726,21 @@ __global__ void __launch_bounds__(kThreads) k_pass3(const double* __restrict__ z
 // Pass 4: d = z0 + sum_j coef_j s_j, the start of the line search (r.d,
 // xp = x, rp = r, step 1) and its first trial: x = xp + 1 d, r = -f_ext for
 // the residual that follows (whose start time is stamped by the last CTA)
-__global__ void __launch_bounds__(kThreads) k_pass4(double* __restrict__ d, const double* __restrict__ z,
+__global__ void __launch_bounds__(kPT) k_pass4(double* __restrict__ d, const double* __restrict__ z,
     const double* __restrict__ Sh, double* __restrict__ r, double* __restrict__ x, double* __restrict__ xp,
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, Scalars* S, double* partials)
 {
     griddep_wait();
-    __shared__ double cf[kMaxHist];
+    __shared__ double cf[kMaxHist], sh[kPT / 32][32];
+    __shared__ bool last;
     const int ncorr = S->ncorr;
-    for (int j = threadIdx.x; j < ncorr; j += kThreads) cf[j] = S->coef[j];
+    for (int j = threadIdx.x; j < ncorr; j += kPT) cf[j] = S->coef[j];
     __syncthreads();
     double v[1] = { 0 };
-    const int ops[1] = { 0 };
-    GRID_STRIDE(i, n)
-    {
-        double di = z[i];
-        for (int j = 0; j < ncorr; j++) di += cf[j] * Sh[j * n + i];
-        d[i] = di;
-        const double ri = r[i], xi = x[i];
-        v[0] += ri * di;
-        xp[i] = xi;
-        rp[i] = ri;
-        x[i] = xi + 1.0 * di;
-        r[i] = -fext[i];
-    }
+    GRID_STRIDE(i, n) v[0] += pass4_entry(i, d, z, Sh, r, x, xp, rp, fext, n, ncorr, cf);
     griddep_launch();
-    block_reduce<1>(v, ops);
-    if (grid_finish<1>(v, ops, partials, &S->counter[1])) {
-        S->dg0 = v[0];
-        S->step = 1.0;
-        S->ls_t = 0;
-        S->tr_i++;  // the next iteration's trace record
-        S->tr_evals = 0;
-        S->t0_res = gtimer();
-    }
+    const double dg = grid_totals<1>(v, partials, &S->counter[1], sh, &last);
+    if (last && threadIdx.x == 0) pass4_done(S, dg);
 }
 
 __global__ void k_neg_copy(double* __restrict__ q, const double* __restrict__ r, size_t n)
@@ -702,44 +762,6 @@ __global__ void k_trial_dev(double* __restrict__ x, const double* __restrict__ x
         x[i] = __fma_rn(step, d[i], xp[i]);
         r[i] = -fext[i];
     }
-}
-
-// End of an iteration (LBFGS.h:150-170): stop on a non-finite residual or
-// solution, on convergence (||r||_inf <= eps or <= eps ||x||_inf) or at the
-// iteration limit; otherwise count the iteration and go on, up to `cap`
-// iterations per launch.  Sets the iteration loop condition.
-__global__ void k_iter_decide(Scalars* S, cudaGraphConditionalHandle h, double* hread)
-{
-    griddep_wait();
-    if (threadIdx.x != 0) return;
-    const double rinf = S->rinf, xinf = S->xinf;
-    int st = kRunning;
-    S->n_body++;
-    if (S->perr != 0.0)
-        st = kPrecondFail;
-    else if (!isfinite(rinf) || !isfinite(xinf))
-        st = kNonFinite;
-    else if (rinf <= S->eps || rinf <= S->eps * xinf)
-        st = kConverged;
-    else if (S->max_iter != 0 && S->k >= S->max_iter)
-        st = kMaxIters;
-    else if (S->stall_iters > 0 && !(rinf < 0.5 * S->best_rinf) && S->k - S->best_k >= S->stall_iters)
-        st = kStalled;
-    else {
-        if (rinf < 0.5 * S->best_rinf) {
-            S->best_rinf = rinf;
-            S->best_k = S->k;
-        }
-        S->k++;
-        if (++S->launch_iters >= S->cap) st = kCapReached;
-    }
-    S->status = st;
-    hread[kRdStatus] = st;
-    hread[kRdK] = S->k;
-    hread[kRdNExtra] = static_cast<double>(S->n_extra);
-    hread[kRdNBody] = static_cast<double>(S->n_body);
-    hread[kRdTPc] = static_cast<double>(S->t_pc);
-    cudaGraphSetConditional(h, st == kRunning ? 1u : 0u);
 }
 
 __global__ void k_loop_start(Scalars* S) { S->launch_iters = 0; }
@@ -901,13 +923,14 @@ double* mapped(double* h)
 // the device-driven line search (h_ls given) r was started by k_pass4 or k_trial_dev and
 // the reduction applies the accept / scale rule
 efem_status enqueue_trial_tail(Model& m, SolverWS& w, double* x, cudaStream_t st,
-    const cudaGraphConditionalHandle* h_ls = nullptr, bool init_r = true)
+    const cudaGraphConditionalHandle* h_ls = nullptr, const cudaGraphConditionalHandle* h_it = nullptr, bool init_r = true)
 {
     const size_t n = w.n;
     efem_status s = launch_residual_on(m, x, w.r, st, &w.sc->t0_res, init_r);
     if (s != EFEM_OK) return s;
     launch_k(k_ls_reduce, grid_for(n), kThreads, 0, st, w.r, w.d, x, n, w.sc, w.partials, precond_error_flag(m),
-        mapped(w.h_read), h_ls ? *h_ls : cudaGraphConditionalHandle(), h_ls ? 1 : 0);
+        mapped(w.h_read), h_ls ? *h_ls : cudaGraphConditionalHandle(),
+        h_it ? *h_it : cudaGraphConditionalHandle(), h_ls ? 1 : 0);
     return EFEM_OK;
 }
 
@@ -925,25 +948,27 @@ efem_status enqueue_body(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     const int mm = w.m;
     const dim3 g1(row_blocks(n), mm + 1), g3(row_blocks(n), mm);
     const size_t sm1 = sizeof(double) * (mm * mm + 2 * mm), sm3 = sizeof(double) * (mm * mm + 3 * mm);
-    const int G = grid_for(n);
+    const int pg = pass_grid(n), divide = use_factor ? 0 : 1;
+    const bool one = mm <= kMaxFast && pg == 1;  // passes 1 and 3 go on with 2 and 4
     switch (mm) {
-#define P1(M) case M: k_pass1_m<M><<<G, kThreads, sm1, st>>>(x, w.xp, w.r, w.rp, w.S, w.Y, n, w.sc, w.partials); break;
+#define P1(M) case M: k_pass1_m<M><<<pg, kPT, 0, st>>>(x, w.xp, w.r, w.rp, w.S, w.Y, n, w.sc, w.partials, w.q, divide); break;
         P1(1) P1(2) P1(3) P1(4) P1(5) P1(6) P1(7) P1(8)
 #undef P1
     default: k_pass1<<<g1, kThreads, sm1, st>>>(x, w.xp, w.r, w.rp, w.S, w.Y, n, mm, w.sc, w.partials, w.sums);
     }
-    launch_k(k_pass2, grid_for(n), kThreads, 0, st, w.q, w.r, w.Y, n, mm, use_factor ? 0 : 1, w.sc);
+    if (!one) launch_k(k_pass2, grid_for(n), kThreads, 0, st, w.q, w.r, w.Y, n, mm, divide, w.sc);
     if (use_factor) {
         efem_status s = precond_enqueue(m, w.q, st, &w.sc->t0_pc);
         if (s != EFEM_OK) return s;
     }
     switch (mm) {
-#define P3(M) case M: launch_k(k_pass3_m<M>, G, kThreads, sm3, st, w.q, w.Y, n, w.sc, w.partials, use_factor ? 1 : 0); break;
+#define P3(M) case M: launch_k(k_pass3_m<M>, pg, kPT, 0, st, w.q, w.Y, n, w.sc, w.partials, use_factor ? 1 : 0, w.d, w.S, \
+        w.r, x, w.xp, w.rp, m.d_fext); break;
         P3(1) P3(2) P3(3) P3(4) P3(5) P3(6) P3(7) P3(8)
 #undef P3
     default: launch_k(k_pass3, g3, kThreads, sm3, st, w.q, w.Y, n, mm, w.sc, w.partials, w.sums, use_factor ? 1 : 0);
     }
-    launch_k(k_pass4, grid_for(n), kThreads, 0, st, w.d, w.q, w.S, w.r, x, w.xp, w.rp, m.d_fext, n, w.sc, w.partials);
+    if (!one) launch_k(k_pass4, pg, kPT, 0, st, w.d, w.q, w.S, w.r, x, w.xp, w.rp, m.d_fext, n, w.sc, w.partials);
     return EFEM_OK;
 }
 
@@ -1023,17 +1048,16 @@ efem_status capture_loop(Model& m, SolverWS& w, double* x, bool use_factor, cuda
         // passes, H0 and the first trial (pass 4), its residual and the line
         // search's decision, which sets hLs; then the further trials
         s = enqueue_body(m, w, x, use_factor, s1);
-        if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s1, &h_ls, false);
+        if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s1, &h_ls, &h_iter, false);
         if (s == EFEM_OK) s = add_while(s1, h_ls, &ls_body);
         if (s == EFEM_OK && cudaStreamBeginCaptureToGraph(s2, ls_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
             s = EFEM_ERR_CUDA;
         if (s == EFEM_OK) {
             k_trial_dev<<<grid_for(w.n), kThreads, 0, s2>>>(x, w.xp, w.d, w.r, m.d_fext, w.n, w.sc);
-            s = enqueue_trial_tail(m, w, x, s2, &h_ls, false);
+            s = enqueue_trial_tail(m, w, x, s2, &h_ls, &h_iter, false);
             cudaGraph_t tmp = nullptr;
             if (cudaStreamEndCapture(s2, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
         }
-        if (s == EFEM_OK) k_iter_decide<<<1, 32, 0, s1>>>(w.sc, h_iter, mapped(w.h_read));
         cudaGraph_t tmp = nullptr;
         if (cudaStreamEndCapture(s1, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
     } while (false);
@@ -1060,7 +1084,7 @@ efem_status capture_step(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     cudaGraph_t g = nullptr;
     EFEM_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
     efem_status s = enqueue_body(m, w, x, use_factor, s0);
-    if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s0, nullptr, false);  // pass 4 started the first trial
+    if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s0, nullptr, nullptr, false);  // pass 4 started the first trial
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
     m.launches = launches;
     if (s != EFEM_OK || e != cudaSuccess) {
@@ -1120,6 +1144,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
     std::memset(info, 0, sizeof(*info));
     const long long launches0 = m.launches;
     const long long per_res = residual_launches(m);
+    const int n_passes = mm <= kMaxFast && pass_grid(n) == 1 ? 2 : 4;
     double ms_pc = 0.0;
     double rinf = 0.0, xinf = 0.0;
     int k = 1;
@@ -1262,7 +1287,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
         }
         k++;
         if (host_loop) {  // iterations 2, 3, ... one graph launch each, decisions on the host
-            const long long per_step = 4 + (ok ? precond_launch_count(m) : 0) + (per_res - 1) + 1;
+            const long long per_step = n_passes + (ok ? precond_launch_count(m) : 0) + (per_res - 1) + 1;
             double best = rinf;
             int best_k = k;
             for (;;) {
@@ -1302,9 +1327,8 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
         k_loop_params<<<1, 1, 0, st>>>(w.sc, eps, m.opts.max_iterations, std::max(1, m.opts.max_linesearch),
             kIterCap, k, stall_iters, rinf);
         m.launches++;
-        // passes, H0, trial (which starts r), residual, reductions, iteration decision
-        // passes (pass 4 starts the first trial), H0, residual, reductions, iteration decision
-        const long long per_body = 4 + (ok ? precond_launch_count(m) : 0) + (per_res - 1) + 2;
+        // passes (pass 4 starts the first trial), H0, residual, reductions with the decisions
+        const long long per_body = n_passes + (ok ? precond_launch_count(m) : 0) + (per_res - 1) + 1;
         const long long per_extra = per_res + 1;  // trial, residual, reductions
         long long n_extra = 0;
         int status = kRunning;
