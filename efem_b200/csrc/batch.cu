@@ -21,10 +21,10 @@
 //    finish a reduction adds that member's partial sums in chunk order and
 //    runs that member's small recursion, so every member follows exactly the
 //    arithmetic of a single solve.
-//  * One CUDA graph holds the iteration loop: a while node over iterations
-//    whose body holds a while node over line-search trials; both conditions
-//    are set by the CTA that ends the last member's reduction, and both
-//    loops are bounded there (kCap iterations per launch, max_line_search
+//  * One CUDA graph holds the iteration loop: a while node whose body is an
+//    iteration or a further line-search trial; its condition is set by the
+//    CTA that ends the last member's reduction, and iterations and trials
+//    are bounded there (kCap iterations per launch, max_line_search
 //    trials per iteration) whatever that state holds.  A member that
 //    converged (or stopped) is frozen: its x no longer moves and its
 //    counters stop; the loop ends when no member is running.  The host checks
@@ -77,6 +77,7 @@ struct Seg {
 
 struct Glob {
     int ls_round;            // line-search trials of the current iteration
+    int again;               // the next loop body is a further trial of some members' line searches
     int launch_iters, cap;
     int n_running;
     int pc_fail;
@@ -85,83 +86,15 @@ struct Glob {
     long long trials;        // extra line-search trials run
 };
 
-// max that keeps a NaN (fmax drops it): a non-finite residual or solution
-// must show in its infinity norm (Integrator.cpp:28-34 tests for it)
-__device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
-
-__device__ __forceinline__ double warp_sum(double v)
+// NS sums and NM maxima of a member over its chunks, in a fixed order: every
+// CTA stores its partial values; lane k of warp 0 of the member's last CTA
+// returns with total k; *last is set there.
+template <int NS, int NM = 0>
+__device__ __forceinline__ double seg_totals(const double (&v)[NS + NM], Seg* sg, double* partials, double (*sh)[32], bool* last)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = nan_max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// CTA reduction of NV values (bit k of maxmask: max, else sum); result in every thread
-template <int NV>
-__device__ void cta_reduce(double* v, unsigned maxmask)
-{
-    __shared__ double sh[NV][kT / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-        v[k] = (maxmask >> k) & 1u ? warp_max(v[k]) : warp_sum(v[k]);
-        if (lane == 0) sh[k][w] = v[k];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-        double a = 0.0;
-        for (int q = 0; q < kT / 32; q++) a = (maxmask >> k) & 1u ? nan_max(a, sh[k][q]) : a + sh[k][q];
-        v[k] = a;
-    }
-    __syncthreads();
-}
-
-// The member's sums over its chunks in chunk order: every CTA stores its NV
-// partials; the member's last CTA adds them and returns true (all its
-// threads), with the totals in v.
-template <int NV>
-__device__ bool seg_finish(double* v, unsigned maxmask, Seg* sg, double* partials)
-{
-    __shared__ bool last;
-    cta_reduce<NV>(v, maxmask);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; k++) partials[static_cast<size_t>(blockIdx.x) * NV + k] = v[k];
-        __threadfence();
-        last = atomicAdd(&sg->cnt, 1u) == static_cast<unsigned>(sg->c1 - sg->c0 - 1);
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double acc[NV];
-#pragma unroll
-    for (int k = 0; k < NV; k++) acc[k] = 0.0;
-    for (int b = sg->c0 + static_cast<int>(threadIdx.x); b < sg->c1; b += kT) {
-        const volatile double* pb = partials + static_cast<size_t>(b) * NV;
-#pragma unroll
-        for (int k = 0; k < NV; k++) acc[k] = (maxmask >> k) & 1u ? nan_max(acc[k], pb[k]) : acc[k] + pb[k];
-    }
-    cta_reduce<NV>(acc, maxmask);
-#pragma unroll
-    for (int k = 0; k < NV; k++) v[k] = acc[k];
-    if (threadIdx.x == 0) sg->cnt = 0u;
-    return true;
-}
-
-// The same for sums alone, for the passes: lane k < NV of warp 0 of the
-// member's last CTA returns with total k; *last is set there.
-template <int NV>
-__device__ __forceinline__ double seg_totals(const double (&v)[NV], Seg* sg, double* partials, double (*sh)[32], bool* last)
-{
+    constexpr int NV = NS + NM;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c0 = sg->c0, c1 = sg->c1;
-    double t = cta_sums<NV, kT / 32>(v, sh);
+    double t = cta_totals<NS, NM, kT / 32>(v, sh);
     if (c1 - c0 == 1) {
         if (threadIdx.x == 0) *last = true;
         __syncthreads();
@@ -178,13 +111,16 @@ __device__ __forceinline__ double seg_totals(const double (&v)[NV], Seg* sg, dou
     __threadfence();
     t = 0.0;
     if (lane < NV)
-        for (int b = c0 + w; b < c1; b += kT / 32) t += __ldcg(partials + static_cast<size_t>(b) * NV + lane);
+        for (int b = c0 + w; b < c1; b += kT / 32) {
+            const double p = __ldcg(partials + static_cast<size_t>(b) * NV + lane);
+            t = lane < NS ? t + p : nan_max(t, p);
+        }
     sh[w][lane] = t;
     __syncthreads();
     t = 0.0;
     if (w == 0) {
 #pragma unroll
-        for (int q = 0; q < kT / 32; q++) t += sh[q][lane];
+        for (int q = 0; q < kT / 32; q++) t = lane < NS ? t + sh[q][lane] : nan_max(t, sh[q][lane]);
         if (lane == 0) sg->cnt = 0u;
     }
     return t;
@@ -228,6 +164,7 @@ __global__ void kb_init(Seg* S, const int* c0, const double* eps, const int* max
 __global__ void kb_glob_init(Glob* G, int cap)
 {
     G->ls_round = 0;
+    G->again = 0;
     G->launch_iters = 0;
     G->cap = cap;
     G->n_running = 0;
@@ -241,6 +178,7 @@ __global__ void kb_loop_start(Glob* G)
 {
     G->launch_iters = 0;
     G->ls_round = 0;
+    G->again = 0;
 }
 
 // the initial residual's norms and the early exit (LBFGS.h:110-120) of every running member
@@ -249,21 +187,26 @@ __global__ void __launch_bounds__(kT) kb_initial(const double* __restrict__ r, c
 {
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
+    __shared__ double sh[kT / 32][32];
+    __shared__ bool last;
     double v[3] = { 0, 0, 0 };
     for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
-        v[0] = nan_max(v[0], fabs(r[i]));
-        v[1] = nan_max(v[1], fabs(x[i]));
-        v[2] += x[i] * x[i];
+        v[0] += x[i] * x[i];
+        v[1] = nan_max(v[1], fabs(r[i]));
+        v[2] = nan_max(v[2], fabs(x[i]));
     }
-    if (!seg_finish<3>(v, 3u, sg, partials) || threadIdx.x != 0) return;
-    if (sg->state != kRun) return;
-    sg->rinf = v[0];
-    sg->xinf = v[1];
-    sg->x2 = v[2];
+    const double t = seg_totals<1, 2>(v, sg, partials, sh, &last);
+    if (!last || threadIdx.x >= 32) return;
+    const double x2 = __shfl_sync(0xffffffffu, t, 0), rinf = __shfl_sync(0xffffffffu, t, 1);
+    const double xinf = __shfl_sync(0xffffffffu, t, 2);
+    if (threadIdx.x != 0 || sg->state != kRun) return;
+    sg->rinf = rinf;
+    sg->xinf = xinf;
+    sg->x2 = x2;
     sg->n_res = 1;
-    if (!isfinite(v[0]))
+    if (!isfinite(rinf))
         sg->state = kNaN;
-    else if (v[0] <= sg->eps || v[0] <= sg->eps * sqrt(v[2]))
+    else if (rinf <= sg->eps || rinf <= sg->eps * sqrt(x2))
         sg->state = kDone;
     frozen[c.seg] = sg->state != kRun;
 }
@@ -275,9 +218,10 @@ __global__ void __launch_bounds__(kT) kb_initial(const double* __restrict__ r, c
 template <int M>
 __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, const double* __restrict__ xp,
     const double* __restrict__ r, const double* __restrict__ rp, double* __restrict__ Sh, double* __restrict__ Yh,
-    size_t n, const Chunk* __restrict__ ch, Seg* S, double* partials)
+    size_t n, const Chunk* __restrict__ ch, Seg* S, double* partials, const Glob* G)
 {
     griddep_wait();
+    if (G->again) return;
     constexpr int NV = 3 * M + 2;
     __shared__ double sh[kT / 32][32], sG[M * M], tot[32];
     __shared__ bool last;
@@ -288,7 +232,7 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
     const int tid = threadIdx.x, lane = tid & 31;
     const int loc = sg->ptr % M;
     const int ncorr = sg->ncorr < M ? sg->ncorr + 1 : M;
-    if (tid < M * M) sG[tid] = sg->G[tid / M][tid % M];
+    if (tid < M * M) sG[tid] = sg->G[tid / M][tid % M] / sg->ys[tid / M];  // the new row and column follow below
     double ys = tid < M ? sg->ys[tid] : 1.0;
     double v[NV];
 #pragma unroll
@@ -329,23 +273,27 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
     }
     tot[lane] = t;
     __syncwarp();
+    const double ysn = tot[3 * M];
+    if (lane == loc) ys = ysn;
+    double u = 0.0;
     if (lane < ncorr) {
-        sG[loc * M + lane] = tot[3 * lane];
-        sG[lane * M + loc] = tot[3 * lane + 1];
+        u = tot[3 * lane + 2] / ys;
+        if (lane != loc) {
+            sG[loc * M + lane] = tot[3 * lane] / ysn;
+            sG[lane * M + loc] = tot[3 * lane + 1] / ys;
+            sg->G[loc][lane] = tot[3 * lane];
+            sg->G[lane][loc] = tot[3 * lane + 1];
+        } else {
+            sG[loc * M + loc] = 1.0;
+            sg->G[loc][loc] = ysn;
+        }
     }
     __syncwarp();
-    if (lane == 0) sG[loc * M + loc] = tot[3 * M];
-    if (lane == loc) ys = tot[3 * M];
-    __syncwarp();
-    const double al = first_loop(lane < ncorr ? tot[3 * lane + 2] : 0.0, ys, sG, M, loc, M, ncorr);
-    if (lane < ncorr) {
-        sg->G[loc][lane] = sG[loc * M + lane];
-        sg->G[lane][loc] = sG[lane * M + loc];
-        sg->alpha[lane] = al;
-    }
+    const double al = first_loop(u, sG, M, loc, M, ncorr);
+    if (lane < ncorr) sg->alpha[lane] = al;
     if (lane == 0) {
-        sg->ys[loc] = tot[3 * M];
-        sg->theta = tot[3 * M + 1] / tot[3 * M];
+        sg->ys[loc] = ysn;
+        sg->theta = tot[3 * M + 1] / ysn;
         sg->ptr = loc + 1;
         sg->ncorr = ncorr;
     }
@@ -353,10 +301,11 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
 
 // Pass 2: q = -r - sum_j alpha_j y_j for running members (0 elsewhere)
 __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const double* __restrict__ r,
-    const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S)
+    const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S, const Glob* G)
 {
     griddep_wait();
     griddep_launch();
+    if (G->again) return;
     const Chunk c = ch[blockIdx.x];
     const Seg* sg = S + c.seg;
     __shared__ double al[kHist];
@@ -375,16 +324,17 @@ __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const dou
 // (LBFGSMat.h:121-128), oldest pair first
 template <int M>
 __global__ void __launch_bounds__(kT) kb_pass3(const double* __restrict__ z, const double* __restrict__ Yh, size_t n,
-    const Chunk* __restrict__ ch, Seg* S, double* partials)
+    const Chunk* __restrict__ ch, Seg* S, double* partials, const Glob* G)
 {
     griddep_wait();
+    if (G->again) return;
     __shared__ double sh[kT / 32][32], sG[M * M];
     __shared__ bool last;
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
     if (sg->state != kRun) return;
     const int tid = threadIdx.x, lane = tid & 31, ncorr = sg->ncorr, ptr = sg->ptr;
-    if (tid < M * M) sG[tid] = sg->G[tid / M][tid % M];
+    if (tid < M * M) sG[tid] = sg->G[tid / M][tid % M] / sg->ys[tid % M];
     const double ys = tid < M ? sg->ys[tid] : 1.0, alpha = tid < M ? sg->alpha[tid] : 0.0;
     double v[M];
 #pragma unroll
@@ -398,22 +348,34 @@ __global__ void __launch_bounds__(kT) kb_pass3(const double* __restrict__ z, con
     griddep_launch();
     const double t = seg_totals<M>(v, sg, partials, sh, &last);
     if (!last || tid >= 32) return;
-    const double cf = second_loop(t, ys, alpha, sG, M, ptr, M, ncorr);
+    const double cf = second_loop(t / ys, alpha, sG, M, ptr, M, ncorr);
     if (lane < ncorr) sg->coef[lane] = cf;
 }
 
 // Pass 4: d = z + sum_j coef_j s_j and the start of the line search of every
 // running member (dg0 = r.d, xp = x, rp = r, step 1) with its first trial
-// x = xp + d; r = -f_ext everywhere for the residual that follows
+// x = xp + d; with G->again instead a further trial x = xp + step d of the
+// members still in their line search.  r = -f_ext everywhere for the residual
+// that follows.
 __global__ void __launch_bounds__(kT) kb_pass4(double* __restrict__ d, const double* __restrict__ z,
     const double* __restrict__ Sh, double* __restrict__ r, double* __restrict__ x, double* __restrict__ xp,
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, const Chunk* __restrict__ ch, Seg* S,
-    double* partials)
+    double* partials, const Glob* G)
 {
     griddep_wait();
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
     const bool act = sg->state == kRun;
+    if (G->again) {
+        griddep_launch();
+        const bool more = act && sg->trial;
+        const double step = sg->step;
+        for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
+            if (more) x[i] = __fma_rn(step, d[i], xp[i]);
+            r[i] = -fext[i];
+        }
+        return;
+    }
     const int ncorr = act ? sg->ncorr : 0;
     __shared__ double cf[kHist], sh[kT / 32][32];
     __shared__ bool last;
@@ -497,39 +459,47 @@ __device__ void iter_decide(Seg* S, int nseg, Glob* G, const int* perr, int* fro
 // member in its line search, which applies the reference's rule (accept when
 // |r.d| <= |r0.d|, else step x1.5 if (r.d)(r0.d) > 0, x0.5 otherwise, at
 // most max_line_search trials, LineSearchFEA.h:43-67).  The CTA that finishes
-// the last member sets the trial loop's condition -- some member wants another
-// trial; bounded here whatever the members' state: after max_ls trials of one
-// iteration every line search ends -- and, when none does, ends the iteration.
+// the last member decides on the loop's next body: another trial when some
+// member wants one -- bounded here whatever the members' state: after max_ls
+// trials of one iteration every line search ends -- or else the next iteration.
 __global__ void __launch_bounds__(kT) kb_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
     const double* __restrict__ x, const Chunk* __restrict__ ch, Seg* S, double* partials, int nseg, int max_ls, Glob* G,
-    const int* perr, int* frozen, cudaGraphConditionalHandle h_ls, cudaGraphConditionalHandle h_it)
+    const int* perr, int* frozen, cudaGraphConditionalHandle h)
 {
     griddep_wait();
+    __shared__ double sh[kT / 32][32];
     __shared__ int any;
-    __shared__ bool last_seg;
+    __shared__ bool last, last_seg;
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
     const bool act = sg->state == kRun && sg->trial;
     if (act) {
+        const double dg0 = sg->dg0, step = sg->step;  // before the sums, behind which they would be waited for
+        const int ls_t = sg->ls_t, sg_max = sg->max_ls, n_res = sg->n_res;
         double v[4] = { 0, 0, 0, 0 };
         for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
             const double ri = r[i], xi = x[i];
             v[0] += ri * d[i];
-            v[1] = nan_max(v[1], fabs(ri));
-            v[2] = nan_max(v[2], fabs(xi));
-            v[3] += xi * xi;
+            v[1] += xi * xi;
+            v[2] = nan_max(v[2], fabs(ri));
+            v[3] = nan_max(v[3], fabs(xi));
         }
-        if (!seg_finish<4>(v, 6u, sg, partials)) return;
-        if (threadIdx.x == 0) {
-            sg->dg = v[0];
-            sg->rinf = v[1];
-            sg->xinf = v[2];
-            sg->x2 = v[3];
-            sg->n_res++;
-            const int t = ++sg->ls_t;
-            const bool again = !(fabs(v[0]) <= fabs(sg->dg0)) && t < sg->max_ls;
-            if (again) sg->step *= v[0] * sg->dg0 > 0 ? 1.5 : 0.5;
-            sg->trial = again ? 1 : 0;
+        const double t = seg_totals<2, 2>(v, sg, partials, sh, &last);
+        if (!last) return;
+        if (threadIdx.x < 32) {
+            const double dg = __shfl_sync(0xffffffffu, t, 0), x2 = __shfl_sync(0xffffffffu, t, 1);
+            const double rinf = __shfl_sync(0xffffffffu, t, 2), xinf = __shfl_sync(0xffffffffu, t, 3);
+            if (threadIdx.x == 0) {
+                sg->dg = dg;
+                sg->rinf = rinf;
+                sg->xinf = xinf;
+                sg->x2 = x2;
+                sg->n_res = n_res + 1;
+                sg->ls_t = ls_t + 1;
+                const bool again = !(fabs(dg) <= fabs(dg0)) && ls_t + 1 < sg_max;
+                if (again) sg->step = step * (dg * dg0 > 0 ? 1.5 : 0.5);
+                sg->trial = again ? 1 : 0;
+            }
         }
     } else if (static_cast<int>(blockIdx.x) != sg->c0)
         return;  // one CTA counts a member that takes no part
@@ -556,27 +526,13 @@ __global__ void __launch_bounds__(kT) kb_ls_reduce(const double* __restrict__ r,
     if (threadIdx.x == 0) {
         G->cnt = 0u;
         G->ls_round++;
-        if (any) G->trials++;
-        cudaGraphSetConditional(h_ls, any ? 1u : 0u);
+        G->again = any;
+        if (any) {
+            G->trials++;
+            cudaGraphSetConditional(h, 1u);
+        }
     }
-    if (!any) iter_decide(S, nseg, G, perr, frozen, h_it);
-}
-
-// a further trial: x = xp + step d for the members still in their line search; r = -f_ext everywhere
-__global__ void __launch_bounds__(kT) kb_trial(double* __restrict__ x, const double* __restrict__ xp,
-    const double* __restrict__ d, double* __restrict__ r, const double* __restrict__ fext,
-    const Chunk* __restrict__ ch, const Seg* S)
-{
-    griddep_wait();
-    griddep_launch();
-    const Chunk c = ch[blockIdx.x];
-    const Seg* sg = S + c.seg;
-    const bool act = sg->state == kRun && sg->trial;
-    const double step = sg->step;
-    for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
-        if (act) x[i] = __fma_rn(step, d[i], xp[i]);
-        r[i] = -fext[i];
-    }
+    if (!any) iter_decide(S, nseg, G, perr, frozen, h);
 }
 
 // launch_k uses programmatic dependent launch while one of these is alive
@@ -624,7 +580,7 @@ struct Union {
     Glob* d_glob = nullptr;
     double *x = nullptr, *xp = nullptr, *r = nullptr, *rp = nullptr, *d = nullptr, *q = nullptr, *Sh = nullptr,
            *Yh = nullptr, *partials = nullptr;
-    cudaStream_t cap[3] = { nullptr, nullptr, nullptr };
+    cudaStream_t cap[2] = { nullptr, nullptr };
     cudaGraphExec_t loop[2] = { nullptr, nullptr };  // per element precision (FP64, FP32)
     long long loop_epoch[2] = { -1, -1 };
     bool pdl = true;  // programmatic dependent launch in the captured loops (off if a capture refused it)
@@ -792,13 +748,13 @@ efem_status setup_union(Union& U)
     return EFEM_OK;
 }
 
-// the iteration graph: while (iterate) { passes, H0, first trial, residual,
-// line-search reduction and decisions; while (trial) { trial, residual, reduction and decisions } }
+// the iteration graph: while (h) { passes, H0 and first trial, or a further
+// trial alone; residual; line-search reduction and decisions }
 efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
 {
     Model& M = *U.uni;
     std::lock_guard<std::mutex> lock(capture_mutex());
-    cudaStream_t s0 = U.cap[0], s1 = U.cap[1], s2 = U.cap[2];
+    cudaStream_t s0 = U.cap[0], s1 = U.cap[1];
     const int nb = U.nchunk, max_ls = std::max(1, M.opts.max_linesearch);
     const int* perr = precond_error_flag(M);
     PdlScope pdl(U.pdl);  // the first kernel of each body graph is a plain launch
@@ -813,48 +769,36 @@ efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
             s = EFEM_ERR_CUDA;
             break;
         }
-        cudaGraphConditionalHandle h_it, h_ls;
-        if (cudaGraphConditionalHandleCreate(&h_it, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+        cudaGraphConditionalHandle h;
+        if (cudaGraphConditionalHandleCreate(&h, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
         kb_loop_start<<<1, 1, 0, s0>>>(U.d_glob);
-        cudaGraph_t body = nullptr, ls_body = nullptr;
-        if ((s = add_while_node(s0, h_it, &body)) != EFEM_OK) break;
-        if (cudaGraphConditionalHandleCreate(&h_ls, body, 1, cudaGraphCondAssignDefault) != cudaSuccess
-            || cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaGraph_t body = nullptr;
+        if ((s = add_while_node(s0, h, &body)) != EFEM_OK) break;
+        if (cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
         switch (U.m) {
-#define P1(K) case K: kb_pass1<K><<<nb, kT, 0, s1>>>(U.x, U.xp, U.r, U.rp, U.Sh, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
+#define P1(K) case K: kb_pass1<K><<<nb, kT, 0, s1>>>(U.x, U.xp, U.r, U.rp, U.Sh, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials, U.d_glob); break;
             P1(1) P1(2) P1(3) P1(4) P1(5) P1(6) P1(7) P1(8)
 #undef P1
         }
-        launch_k(kb_pass2, nb, kT, 0, s1, U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg);
-        if ((s = precond_enqueue(M, U.q, s1)) != EFEM_OK) break;
+        launch_k(kb_pass2, nb, kT, 0, s1, U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg, U.d_glob);
+        if ((s = precond_enqueue(M, U.q, s1, nullptr, &U.d_glob->again)) != EFEM_OK) break;
         switch (U.m) {
-#define P3(K) case K: launch_k(kb_pass3<K>, nb, kT, 0, s1, U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
+#define P3(K) case K: launch_k(kb_pass3<K>, nb, kT, 0, s1, U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials, U.d_glob); break;
             P3(1) P3(2) P3(3) P3(4) P3(5) P3(6) P3(7) P3(8)
 #undef P3
         }
         launch_k(kb_pass4, nb, kT, 0, s1, U.d, U.q, U.Sh, U.r, U.x, U.xp, U.rp, M.d_fext, U.n, U.d_chunks, U.d_seg,
-            U.partials);
+            U.partials, U.d_glob);
         if ((s = launch_residual_on(M, U.x, U.r, s1, nullptr, false)) != EFEM_OK) break;
         launch_k(kb_ls_reduce, nb, kT, 0, s1, U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials, U.nseg, max_ls, U.d_glob, perr,
-            U.d_frozen, h_ls, h_it);
-        if ((s = add_while_node(s1, h_ls, &ls_body)) != EFEM_OK) break;
-        if (cudaStreamBeginCaptureToGraph(s2, ls_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-            s = EFEM_ERR_CUDA;
-            break;
-        }
-        kb_trial<<<nb, kT, 0, s2>>>(U.x, U.xp, U.d, U.r, M.d_fext, U.d_chunks, U.d_seg);
-        s = launch_residual_on(M, U.x, U.r, s2, nullptr, false);
-        launch_k(kb_ls_reduce, nb, kT, 0, s2, U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials, U.nseg, max_ls, U.d_glob, perr,
-            U.d_frozen, h_ls, h_it);
+            U.d_frozen, h);
         cudaGraph_t tmp = nullptr;
-        if (cudaStreamEndCapture(s2, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
-        if (s != EFEM_OK) break;
         if (cudaStreamEndCapture(s1, &tmp) != cudaSuccess) s = EFEM_ERR_CUDA;
     } while (false);
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
@@ -932,14 +876,13 @@ efem_status run_union_phase(Union& U, int stall, const std::vector<int>& keep, l
     }
     Glob g {};
     long long body0 = 0, trials0 = 0;
-    // per loop body: passes 1-4, H0, residual, reduction with the decisions; per extra trial: trial, residual, reduction
+    // per loop body: passes 1-4, H0, residual, reduction with the decisions (those a further trial leaves idle too)
     const long long per_body = 5 + precond_launch_count(M) + (U.per_res - 1);
-    const long long per_trial = 2 + (U.per_res - 1);
     for (;;) {
         EFEM_CUDA(cudaGraphLaunch(U.loop[slot], st));
         EFEM_CUDA(cudaMemcpyAsync(&g, U.d_glob, sizeof(Glob), cudaMemcpyDeviceToHost, st));
         EFEM_CUDA(cudaStreamSynchronize(st));
-        *launches += 1 + (g.body_iters - body0) * per_body + (g.trials - trials0) * per_trial;
+        *launches += 1 + (g.body_iters - body0 + g.trials - trials0) * per_body;
         body0 = g.body_iters;
         trials0 = g.trials;
         if (g.pc_fail) {

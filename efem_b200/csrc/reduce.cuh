@@ -39,33 +39,64 @@ __device__ __forceinline__ double cta_sums(const double (&v)[NV], double (*sh)[3
     return t;
 }
 
+// max that keeps a NaN (fmax drops it): a non-finite residual or solution
+// must show in its infinity norm (Integrator.cpp:28-34 tests for it)
+__device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
+
+// The same for NS sums followed by NM maxima of values >= 0: lane k < NS + NM
+template <int NS, int NM, int Warps>
+__device__ __forceinline__ double cta_totals(const double (&v)[NS + NM], double (*sh)[32])
+{
+    static_assert(NM == 0 || (NS <= 16 && NM <= 16), "columns of sh");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double a[NS];
+#pragma unroll
+    for (int k = 0; k < NS; k++) a[k] = v[k];
+#pragma unroll
+    for (int k = 0; k < NM; k++) {
+        double b = v[NS + k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) b = nan_max(b, __shfl_xor_sync(0xffffffffu, b, o));
+        if (lane == 0) sh[w][16 + k] = b;
+    }
+    double t = cta_sums<NS, Warps>(a, sh);
+    if (NM > 0 && w == 0 && lane >= NS && lane < NS + NM) {
+#pragma unroll
+        for (int q = 0; q < Warps; q++) t = nan_max(t, sh[q][16 + lane - NS]);
+    }
+    return t;
+}
+
 // The two-loop recursion's first loop (LBFGSMat.h:106-113) by one warp: lane k
-// holds t = s_k . q0 of slot k, ys its s_k . y_k; slots are visited newest
-// first from `loc`; G[k * ld + j] = s_k . y_j.  Returns alpha_k in lane k.
-__device__ __forceinline__ double first_loop(double t, double ys, const double* G, int ld, int loc, int m, int ncorr)
+// holds u = (s_k . q0) / ys_k of slot k and G[k * ld + j] = (s_k . y_j) / ys_k;
+// slots are visited newest first from `loc`.  Returns alpha_k in lane k.  The
+// divisions by ys_k = s_k . y_k are done beforehand, all at once: one in every
+// step of the chain made a recursion of six pairs 4.3 us.
+__device__ __forceinline__ double first_loop(double u, const double* G, int ld, int loc, int m, int ncorr)
 {
     const int lane = threadIdx.x & 31;
     double alpha = 0.0;
-    for (int i = 0; i < ncorr; i++) {
-        const int j = loc - i < 0 ? loc - i + m : loc - i;
-        const double al = __shfl_sync(0xffffffffu, t / ys, j);
+    for (int i = 0, j = loc; i < ncorr; i++, j = j == 0 ? m - 1 : j - 1) {
+        const double g = lane < ncorr ? G[lane * ld + j] : 0.0;
+        const double al = __shfl_sync(0xffffffffu, u, j);
         if (lane == j) alpha = al;
-        if (lane < ncorr) t -= al * G[lane * ld + j];
+        u -= al * g;
     }
     return alpha;
 }
 
-// The second loop (LBFGSMat.h:121-128): lane k holds t = y_k . z0 and alpha_k;
-// slots oldest first, ptr the slot after the newest.  Returns alpha - beta.
-__device__ __forceinline__ double second_loop(double t, double ys, double alpha, const double* G, int ld, int ptr, int m, int ncorr)
+// The second loop (LBFGSMat.h:121-128): lane k holds w = (y_k . z0) / ys_k and
+// alpha_k, G[j * ld + k] = (s_j . y_k) / ys_k; slots oldest first, ptr the slot
+// after the newest.  Returns alpha - beta.
+__device__ __forceinline__ double second_loop(double w, double alpha, const double* G, int ld, int ptr, int m, int ncorr)
 {
     const int lane = threadIdx.x & 31;
     double coef = 0.0;
-    for (int o = 0; o < ncorr; o++) {
-        const int j = (((ptr - ncorr + o) % m) + m) % m;
-        const double cf = __shfl_sync(0xffffffffu, alpha - t / ys, j);
+    for (int o = 0, j = (((ptr - ncorr) % m) + m) % m; o < ncorr; o++, j = j == m - 1 ? 0 : j + 1) {
+        const double g = lane < ncorr ? G[j * ld + lane] : 0.0;
+        const double cf = __shfl_sync(0xffffffffu, alpha - w, j);
         if (lane == j) coef = cf;
-        if (lane < ncorr) t += cf * G[j * ld + lane];
+        w += cf * g;
     }
     return coef;
 }

@@ -24,14 +24,14 @@
 // of the floating-point sums differs.
 //
 // Iterations run on the device.  After the first one (driven from the host),
-// a CUDA graph holds the loop: a while node over iterations whose body is the
-// four passes with H0, the residual at the first trial and the line-search
-// reductions, then a nested while node over the further trials of the line
-// search, then a one-thread kernel that applies the reference's convergence
-// and iteration-limit tests and sets the loop condition.  The accept / scale
-// rule of the line search is applied by a one-thread kernel as well.  Both
-// loops are bounded: the line search by max_linesearch, the iterations by a
-// per-launch cap, after which the host reads the state and launches the graph
+// a CUDA graph holds the loop: a while node whose body is the four passes
+// with H0, the residual at the trial and the line-search reductions, whose
+// last CTA applies the line search's accept / scale rule and the reference's
+// convergence and iteration-limit tests and sets the loop condition.  When the
+// line search wants a further trial, the passes and H0 return at once in the
+// next body and pass 4 makes the trial.  All is bounded: the line search by
+// max_linesearch, the iterations by a per-launch cap, after which the host
+// reads the state and launches the graph
 // again.  Scalars the host reads are written into mapped host memory, and the
 // time spent in the residual and in H0 is summed on the device from the GPU's
 // global timer.
@@ -73,6 +73,7 @@ struct Scalars {
     double eps, step;           // residual criterion; current line-search step
     int max_iter, max_ls, cap;  // iteration limit (0: none), trials per line search, iterations per launch
     int k, launch_iters, ls_t, status;
+    int again;                  // the next loop body is a further trial of the line search
     unsigned long long n_res, n_extra, n_body;  // residual evaluations, extra trials, device-driven iterations
     unsigned long long t0_res, t_res, t0_pc, t_pc;  // global-timer stamps and sums (ns)
     // convergence trace: record i = the state after iteration i's line search
@@ -96,16 +97,14 @@ enum { kRdDg = 0, kRdRinf, kRdXinf, kRdX2, kRdDg0, kRdPerr, kRdStatus, kRdK, kRd
 // device loop status
 enum { kRunning = 0, kConverged = 1, kMaxIters = 2, kNonFinite = 3, kPrecondFail = 4, kCapReached = 5, kStalled = 6 };
 
+// about a microsecond until the value is there: read where it can be waited for
+// behind other work
 __device__ __forceinline__ unsigned long long gtimer()
 {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-
-// max that keeps a NaN (fmax drops it): a non-finite residual or solution
-// must show in its infinity norm (Integrator.cpp:28-34 tests for it)
-__device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -240,112 +239,194 @@ __global__ void k_trial(double* __restrict__ x, const double* __restrict__ xp, c
     GRID_STRIDE(i, n) x[i] = __fma_rn(step, d[i], xp[i]);
 }
 
+// ---- reductions over the grid
+constexpr int kPT = 512;     // threads
+constexpr int kPG = 296;     // most CTAs: two per SM (one: 7 us an iteration slower on the mixed finger, 241k DOFs)
+constexpr size_t kOne = 4096;  // entries of one CTA (750 DOFs: 61.7 us an iteration against 65.0 with passes 2 and 4 apart)
+
+int pass_grid(size_t n) { return n <= kOne ? 1 : static_cast<int>(std::min<size_t>(kPG, (n + kPT - 1) / kPT)); }
+
+// Totals of NS sums and NM maxima over the grid, in a fixed order: lane k of
+// the last CTA's warp 0 returns with total k; *last is set in that CTA, all of
+// whose threads call prep() on the way (work that only that CTA needs).
+template <int NS, int NM = 0, class Prep>
+__device__ __forceinline__ double grid_totals(const double (&v)[NS + NM], double* partials, unsigned int* counter,
+    double (*sh)[32], bool* last, Prep prep)
+{
+    constexpr int NV = NS + NM;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double t = cta_totals<NS, NM, kPT / 32>(v, sh);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) *last = true;
+        prep();
+        __syncthreads();
+        return t;
+    }
+    if (w == 0) {
+        if (lane < NV) partials[blockIdx.x * NV + lane] = t;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) *last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!*last) return 0.0;
+    __threadfence();
+    t = 0.0;
+    if (lane < NV) {
+        double p[(kPG + kPT / 32 - 1) / (kPT / 32)];
+#pragma unroll
+        for (int e = 0; e < (kPG + kPT / 32 - 1) / (kPT / 32); e++) {
+            const int b = w + e * (kPT / 32);
+            p[e] = b < static_cast<int>(gridDim.x) ? __ldcg(partials + b * NV + lane) : 0.0;
+        }
+#pragma unroll
+        for (int e = 0; e < (kPG + kPT / 32 - 1) / (kPT / 32); e++) t = lane < NS ? t + p[e] : nan_max(t, p[e]);
+    }
+    prep();
+    sh[w][lane] = t;
+    __syncthreads();
+    t = 0.0;
+    if (w == 0) {
+#pragma unroll
+        for (int q = 0; q < kPT / 32; q++) t = lane < NS ? t + sh[q][lane] : nan_max(t, sh[q][lane]);
+        if (lane == 0) *counter = 0u;
+    }
+    return t;
+}
+
+// What the decisions read, loaded before the sweep: behind the sums these
+// loads would each be waited for in turn
+struct LsState {
+    double dg0, step, eps, best;
+    double* trace;
+    unsigned long long n_body;
+    int ls_t, max_ls, k, max_iter, best_k, stall, launch_iters, cap, tr_i, trace_cap, tr_evals;
+};
+
 // End of an iteration (LBFGS.h:150-170): stop on a non-finite residual or
 // solution, on convergence (||r||_inf <= eps or <= eps ||x||_inf) or at the
 // iteration limit; otherwise count the iteration and go on, up to `cap`
-// iterations per launch.  Sets the iteration loop condition.  One thread.
-__device__ void iter_decide(Scalars* S, cudaGraphConditionalHandle h, double* hread)
+// iterations per launch.  Returns the loop's status.  One thread.
+__device__ int iter_decide(Scalars* S, const LsState& L, double rinf, double xinf, int perr)
 {
-    const double rinf = S->rinf, xinf = S->xinf;
     int st = kRunning;
-    S->n_body++;
-    if (S->perr != 0.0)
+    S->n_body = L.n_body + 1;
+    if (perr)
         st = kPrecondFail;
     else if (!isfinite(rinf) || !isfinite(xinf))
         st = kNonFinite;
-    else if (rinf <= S->eps || rinf <= S->eps * xinf)
+    else if (rinf <= L.eps || rinf <= L.eps * xinf)
         st = kConverged;
-    else if (S->max_iter != 0 && S->k >= S->max_iter)
+    else if (L.max_iter != 0 && L.k >= L.max_iter)
         st = kMaxIters;
-    else if (S->stall_iters > 0 && !(rinf < 0.5 * S->best_rinf) && S->k - S->best_k >= S->stall_iters)
+    else if (L.stall > 0 && !(rinf < 0.5 * L.best) && L.k - L.best_k >= L.stall)
         st = kStalled;
     else {
-        if (rinf < 0.5 * S->best_rinf) {
+        if (rinf < 0.5 * L.best) {
             S->best_rinf = rinf;
-            S->best_k = S->k;
+            S->best_k = L.k;
         }
-        S->k++;
-        if (++S->launch_iters >= S->cap) st = kCapReached;
+        S->k = L.k + 1;
+        S->launch_iters = L.launch_iters + 1;
+        if (L.launch_iters + 1 >= L.cap) st = kCapReached;
     }
     S->status = st;
-    hread[kRdStatus] = st;
-    hread[kRdK] = S->k;
-    hread[kRdNExtra] = static_cast<double>(S->n_extra);
-    hread[kRdNBody] = static_cast<double>(S->n_body);
-    hread[kRdTPc] = static_cast<double>(S->t_pc);
-    cudaGraphSetConditional(h, st == kRunning ? 1u : 0u);
+    return st;
 }
 
 // line-search scalars: dg = r.d, rinf = ||r||_inf, xinf = ||x||_inf, x2 = ||x||^2,
-// stored in S and in the host-mapped read-back array; with a trace buffer the
+// stored in S and -- for the host's decisions, or when the device-driven loop
+// ends -- in the host-mapped read-back array (a dozen writes to host memory in
+// every iteration delayed the kernel's end: this, the loads ahead of the sweep
+// and the timer read behind other work took an iteration at 750 DOFs from 49.5
+// to 43.5 us); with a trace buffer the
 // trial also (over)writes the current iteration's record, so the record left
 // is the accepted trial's
-// With `decide` (inside the device-driven line search) the last CTA also
+// With `decide` (inside the device-driven loop) the last CTA also
 // applies the accept / scale rule of LineSearchFEA.h:43-67: accept when
 // |r.d| <= |r0.d|; otherwise scale the step by 1.5 (same sign) or 0.5 and try
-// again, at most max_ls trials in all; it sets the line-search loop condition
-// and, when the line search ends, the iteration loop's (iter_decide).
-__global__ void __launch_bounds__(kThreads) k_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
-    const double* __restrict__ x, size_t n, Scalars* S, double* partials, const int* perr, double* hread,
-    cudaGraphConditionalHandle h, cudaGraphConditionalHandle h_it, int decide)
+// again, at most max_ls trials in all; the loop's next body is that trial or,
+// when the line search ends, the next iteration (iter_decide).
+__global__ void __launch_bounds__(kPT) k_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
+    const double* __restrict__ x, size_t n, Scalars* S, double* partials, const int* perr_flag, double* hread,
+    cudaGraphConditionalHandle h, int decide)
 {
     griddep_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        S->t_res += gtimer() - S->t0_res;  // the residual just ended
-        // the loop stops unless the last CTA below decides on another trial
-        if (decide) cudaGraphSetConditional(h, 0u);
+    __shared__ double sh[kPT / 32][32];
+    __shared__ bool last;
+    LsState L = {};
+    int perr = 0;
+    unsigned long long now = 0;
+    if (threadIdx.x == 0) {
+        if (blockIdx.x == 0) {
+            now = gtimer();  // the residual just ended
+            // the loop stops unless the last CTA below decides on another body
+            if (decide) cudaGraphSetConditional(h, 0u);
+        }
+        L = LsState { S->dg0, S->step, S->eps, S->best_rinf, S->trace, S->n_body, S->ls_t, S->max_ls, S->k, S->max_iter,
+            S->best_k, S->stall_iters, S->launch_iters, S->cap, S->tr_i, S->trace_cap, S->tr_evals };
+        perr = perr_flag ? *perr_flag : 0;
     }
     double v[5] = { 0, 0, 0, 0, 0 };
-    const int ops[5] = { 0, 1, 1, 0, 0 };
     GRID_STRIDE(i, n)
     {
         const double ri = r[i], xi = x[i];
         v[0] += ri * d[i];
-        v[1] = nan_max(v[1], fabs(ri));
-        v[2] = nan_max(v[2], fabs(xi));
-        v[3] += xi * xi;
-        v[4] += ri * ri;
+        v[1] += xi * xi;
+        v[2] += ri * ri;
+        v[3] = nan_max(v[3], fabs(ri));
+        v[4] = nan_max(v[4], fabs(xi));
     }
     griddep_launch();
-    block_reduce<5>(v, ops);
-    if (grid_finish<5>(v, ops, partials, &S->counter[0])) {
-        S->dg = v[0];
-        S->rinf = v[1];
-        S->xinf = v[2];
-        S->x2 = v[3];
-        S->perr = perr ? static_cast<double>(*perr) : 0.0;
-        S->n_res++;
-        S->tr_evals++;
-        if (S->trace && S->tr_i < S->trace_cap) {
-            double* rec = S->trace + static_cast<size_t>(S->tr_i) * kTraceCols;
-            rec[0] = static_cast<double>(gtimer() - S->t_start) * 1e-9;
-            rec[1] = sqrt(v[4]);
-            rec[2] = v[1];
-            rec[3] = S->step;
-            rec[4] = static_cast<double>(S->tr_evals);
-        }
-        hread[kRdTrN] = static_cast<double>(S->tr_i + 1);
-        hread[kRdDg] = S->dg;
-        hread[kRdRinf] = S->rinf;
-        hread[kRdXinf] = S->xinf;
-        hread[kRdX2] = S->x2;
-        hread[kRdDg0] = S->dg0;
-        hread[kRdPerr] = S->perr;
-        hread[kRdNRes] = static_cast<double>(S->n_res);
-        hread[kRdTRes] = static_cast<double>(S->t_res);
-        hread[kRdTPc] = static_cast<double>(S->t_pc);
-        if (decide) {
-            const int t = ++S->ls_t;
-            const double dg = S->dg, dg0 = S->dg0;
-            const bool again = !(fabs(dg) <= fabs(dg0)) && t < S->max_ls;
-            if (again) {
-                S->step *= dg * dg0 > 0 ? 1.5 : 0.5;
-                S->n_extra++;
-            }
-            cudaGraphSetConditional(h, again ? 1u : 0u);
-            if (!again) iter_decide(S, h_it, hread);
-        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) S->t_res += now - S->t0_res;
+    const double t = grid_totals<3, 2>(v, partials, &S->counter[0], sh, &last, [] {});
+    if (!last || threadIdx.x >= 32) return;
+    const double dg = __shfl_sync(0xffffffffu, t, 0), x2 = __shfl_sync(0xffffffffu, t, 1);
+    const double r2 = __shfl_sync(0xffffffffu, t, 2), rinf = __shfl_sync(0xffffffffu, t, 3);
+    const double xinf = __shfl_sync(0xffffffffu, t, 4);
+    if (threadIdx.x != 0) return;
+    S->dg = dg;
+    S->rinf = rinf;
+    S->xinf = xinf;
+    S->x2 = x2;
+    S->perr = perr;
+    S->n_res++;
+    S->tr_evals = L.tr_evals + 1;
+    if (L.trace && L.tr_i < L.trace_cap) {
+        double* rec = L.trace + static_cast<size_t>(L.tr_i) * kTraceCols;
+        rec[0] = static_cast<double>(gtimer() - S->t_start) * 1e-9;
+        rec[1] = sqrt(r2);
+        rec[2] = rinf;
+        rec[3] = L.step;
+        rec[4] = static_cast<double>(L.tr_evals + 1);
     }
+    if (decide) {
+        S->ls_t = L.ls_t + 1;
+        const bool again = !(fabs(dg) <= fabs(L.dg0)) && L.ls_t + 1 < L.max_ls;
+        S->again = again ? 1 : 0;
+        if (again) {
+            S->step = L.step * (dg * L.dg0 > 0 ? 1.5 : 0.5);
+            S->n_extra++;
+        }
+        if (again || iter_decide(S, L, rinf, xinf, perr) == kRunning) {
+            cudaGraphSetConditional(h, 1u);
+            return;
+        }
+        hread[kRdStatus] = S->status;
+        hread[kRdK] = S->k;
+        hread[kRdNExtra] = static_cast<double>(S->n_extra);
+        hread[kRdNBody] = static_cast<double>(S->n_body);
+    }
+    hread[kRdTrN] = static_cast<double>(L.tr_i + 1);
+    hread[kRdDg] = dg;
+    hread[kRdRinf] = rinf;
+    hread[kRdXinf] = xinf;
+    hread[kRdX2] = x2;
+    hread[kRdDg0] = L.dg0;
+    hread[kRdPerr] = perr;
+    hread[kRdNRes] = static_cast<double>(S->n_res);
+    hread[kRdTRes] = static_cast<double>(*static_cast<volatile unsigned long long*>(&S->t_res));
+    hread[kRdTPc] = static_cast<double>(S->t_pc);
 }
 
 // start of the line search fused with its first trial (step 1):
@@ -383,6 +464,7 @@ __global__ void __launch_bounds__(kThreads) k_pass1(const double* __restrict__ x
     size_t n, int m, Scalars* S, double* partials, double* sums)
 {
     griddep_wait();
+    if (S->again) return;
     const int loc = S->ptr % m;
     const int ncorr = S->ncorr < m ? S->ncorr + 1 : m;  // count after the insertion; slots 0..ncorr-1 hold pairs
     const int row = blockIdx.y;
@@ -462,56 +544,6 @@ __global__ void __launch_bounds__(kThreads) k_pass1(const double* __restrict__ x
 // reads on the C3D20R cap).  All passes, reductions and loop nodes of an
 // iteration: 66 -> 51 us on that cap (134k DOFs), 45 -> 31 us at 750 DOFs,
 // against five shuffles per value, 592 CTAs and a serial recursion.
-constexpr int kPT = 512;     // threads
-constexpr int kPG = 296;     // most CTAs: two per SM (one: 7 us an iteration slower on the mixed finger, 241k DOFs)
-constexpr size_t kOne = 4096;  // entries of one CTA (750 DOFs: 61.7 us an iteration against 65.0 with passes 2 and 4 apart)
-
-int pass_grid(size_t n) { return n <= kOne ? 1 : static_cast<int>(std::min<size_t>(kPG, (n + kPT - 1) / kPT)); }
-
-// Totals of NV values over the grid, in a fixed order: lane k < NV of the last
-// CTA's warp 0 returns with the total of value k; *last is set in that CTA.
-template <int NV>
-__device__ __forceinline__ double grid_totals(const double (&v)[NV], double* partials, unsigned int* counter, double (*sh)[32],
-    bool* last)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double t = cta_sums<NV, kPT / 32>(v, sh);
-    if (gridDim.x == 1) {
-        if (threadIdx.x == 0) *last = true;
-        __syncthreads();
-        return t;
-    }
-    if (w == 0) {
-        if (lane < NV) partials[blockIdx.x * NV + lane] = t;
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) *last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!*last) return 0.0;
-    __threadfence();
-    t = 0.0;
-    if (lane < NV) {
-        double p[(kPG + kPT / 32 - 1) / (kPT / 32)];
-#pragma unroll
-        for (int e = 0; e < (kPG + kPT / 32 - 1) / (kPT / 32); e++) {
-            const int b = w + e * (kPT / 32);
-            p[e] = b < static_cast<int>(gridDim.x) ? __ldcg(partials + b * NV + lane) : 0.0;
-        }
-#pragma unroll
-        for (int e = 0; e < (kPG + kPT / 32 - 1) / (kPT / 32); e++) t += p[e];
-    }
-    sh[w][lane] = t;
-    __syncthreads();
-    t = 0.0;
-    if (w == 0) {
-#pragma unroll
-        for (int q = 0; q < kPT / 32; q++) t += sh[q][lane];
-        if (lane == 0) *counter = 0u;
-    }
-    return t;
-}
-
 // Pass 1 (see the file comment) and, with one CTA, pass 2
 template <int M>
 __global__ void __launch_bounds__(kPT) k_pass1_m(const double* __restrict__ x, const double* __restrict__ xp,
@@ -519,13 +551,16 @@ __global__ void __launch_bounds__(kPT) k_pass1_m(const double* __restrict__ x, c
     size_t n, Scalars* S, double* partials, double* __restrict__ q, int divide_theta)
 {
     griddep_wait();
+    if (S->again) return;
     constexpr int NV = 3 * M + 2;
     __shared__ double sh[kPT / 32][32], sG[M * M], tot[32], sal[M], sth;
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31;
     const int loc = S->ptr % M;
     const int ncorr = S->ncorr < M ? S->ncorr + 1 : M;
-    if (tid < M * M) sG[tid] = S->G[tid / M][tid % M];
+    const int gq = tid - (kPT - 64);  // the last two warps scale G for the recursion
+    const bool gt = gq >= 0 && gq < M * M;
+    const double g = gt ? S->G[gq / M][gq % M] : 0.0, gys = gt ? S->ys[gq / M] : 1.0;
     double ys = tid < M ? S->ys[tid] : 1.0;
     double v[NV];
 #pragma unroll
@@ -554,51 +589,67 @@ __global__ void __launch_bounds__(kPT) k_pass1_m(const double* __restrict__ x, c
             }
     }
     griddep_launch();
-    const double t = grid_totals<NV>(v, partials, &S->counter[2], sh, &last);
+    const double t = grid_totals<NV>(v, partials, &S->counter[2], sh, &last, [&] {
+        if (gt) sG[gq] = g / gys;  // the new row and column follow below
+    });
     if (!last) return;
     if (tid < 32) {
         tot[lane] = t;
         __syncwarp();
+        const double ysn = tot[3 * M];
+        if (lane == loc) ys = ysn;
+        if (lane == 31) sth = tot[3 * M + 1] / ysn;
+        double u = 0.0;
         if (lane < ncorr) {
-            sG[loc * M + lane] = tot[3 * lane];
-            sG[lane * M + loc] = tot[3 * lane + 1];
+            u = tot[3 * lane + 2] / ys;
+            if (lane != loc) {
+                sG[loc * M + lane] = tot[3 * lane] / ysn;
+                sG[lane * M + loc] = tot[3 * lane + 1] / ys;
+                S->G[loc][lane] = tot[3 * lane];
+                S->G[lane][loc] = tot[3 * lane + 1];
+            } else {
+                sG[loc * M + loc] = 1.0;
+                S->G[loc][loc] = ysn;
+            }
         }
         __syncwarp();
-        if (lane == 0) sG[loc * M + loc] = tot[3 * M];
-        if (lane == loc) ys = tot[3 * M];
-        __syncwarp();
-        const double al = first_loop(lane < ncorr ? tot[3 * lane + 2] : 0.0, ys, sG, M, loc, M, ncorr);
+        const double al = first_loop(u, sG, M, loc, M, ncorr);
         if (lane < ncorr) {
-            S->G[loc][lane] = sG[loc * M + lane];
-            S->G[lane][loc] = sG[lane * M + loc];
             S->alpha[lane] = al;
             sal[lane] = al;
         }
         if (lane == 0) {
-            sth = tot[3 * M + 1] / tot[3 * M];
             S->theta = sth;
             S->ptr = loc + 1;
             S->ncorr = ncorr;
-            S->ys[loc] = tot[3 * M];
+            S->ys[loc] = ysn;
         }
     }
     if (gridDim.x > 1) return;
     __syncthreads();
     for (size_t i = tid; i < n; i += kPT) {
         double qi = -r[i];
-        for (int j = 0; j < ncorr; j++) qi -= sal[j] * Yh[j * n + i];
+#pragma unroll
+        for (int j = 0; j < M; j++)
+            if (j < ncorr) qi -= sal[j] * Yh[j * n + i];
         q[i] = divide_theta ? qi / sth : qi;
     }
 }
 
 // Pass 4 of entry i: d = z + sum_j coef_j s_j, the line search's start and
-// first trial; returns r . d
+// first trial; returns r . d.  M: the longest history (0: any)
+template <int M>
 __device__ __forceinline__ double pass4_entry(size_t i, double* __restrict__ d, const double* __restrict__ z,
     const double* __restrict__ Sh, double* __restrict__ r, double* __restrict__ x, double* __restrict__ xp,
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, int ncorr, const double* cf)
 {
     double di = z[i];
-    for (int j = 0; j < ncorr; j++) di += cf[j] * Sh[j * n + i];
+    if constexpr (M > 0) {
+#pragma unroll
+        for (int j = 0; j < M; j++)
+            if (j < ncorr) di += cf[j] * Sh[j * n + i];
+    } else
+        for (int j = 0; j < ncorr; j++) di += cf[j] * Sh[j * n + i];
     d[i] = di;
     const double ri = r[i], xi = x[i];
     xp[i] = xi;
@@ -607,14 +658,29 @@ __device__ __forceinline__ double pass4_entry(size_t i, double* __restrict__ d, 
     r[i] = -fext[i];
     return ri * di;
 }
-__device__ __forceinline__ void pass4_done(Scalars* S, double dg0)
+__device__ __forceinline__ void pass4_done(Scalars* S, double dg0, int tr_i, unsigned long long now)
 {
     S->dg0 = dg0;
     S->step = 1.0;
     S->ls_t = 0;
-    S->tr_i++;  // the next iteration's trace record
+    S->tr_i = tr_i + 1;  // the next iteration's trace record
     S->tr_evals = 0;
-    S->t0_res = gtimer();
+    S->t0_res = now;
+}
+
+// A further trial of the device-driven line search: x = xp + step d with the
+// step held on the device, and r = -f_ext to start the residual at x (its
+// start time is stamped for the residual's timing)
+__device__ __forceinline__ void trial(const double* __restrict__ d, double* __restrict__ r, double* __restrict__ x,
+    const double* __restrict__ xp, const double* __restrict__ fext, size_t n, Scalars* S)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) S->t0_res = gtimer();
+    const double step = S->step;
+    GRID_STRIDE(i, n)
+    {
+        x[i] = __fma_rn(step, d[i], xp[i]);
+        r[i] = -fext[i];
+    }
 }
 
 // Pass 3 and, with one CTA, pass 4
@@ -628,8 +694,15 @@ __global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, c
     __shared__ double sh[kPT / 32][32], sG[M * M], cf[M];
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, ncorr = S->ncorr, ptr = S->ptr;
-    if (blockIdx.x == 0 && tid == 0 && time_pc) S->t_pc += gtimer() - S->t0_pc;  // H0 just ended
-    if (tid < M * M) sG[tid] = S->G[tid / M][tid % M];
+    if (S->again) {
+        if (gridDim.x == 1) trial(d, r, x, xp, fext, n, S);
+        return;
+    }
+    const bool timed = blockIdx.x == 0 && tid == 0 && time_pc;
+    const unsigned long long now = timed ? gtimer() : 0;  // H0 just ended
+    const int gq = tid - (kPT - 64);
+    const bool gt = gq >= 0 && gq < M * M;
+    const double g = gt ? S->G[gq / M][gq % M] : 0.0, gys = gt ? S->ys[gq % M] : 1.0;
     const double ys = tid < M ? S->ys[tid] : 1.0, alpha = tid < M ? S->alpha[tid] : 0.0;
     double v[M];
 #pragma unroll
@@ -642,10 +715,13 @@ __global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, c
             if (j < ncorr) v[j] += Yh[j * n + i] * zi;
     }
     griddep_launch();
-    const double t = grid_totals<M>(v, partials, &S->counter[3], sh, &last);
+    if (timed) S->t_pc += now - S->t0_pc;
+    const double t = grid_totals<M>(v, partials, &S->counter[3], sh, &last, [&] {
+        if (gt) sG[gq] = g / gys;
+    });
     if (!last) return;
     if (tid < 32) {
-        const double c = second_loop(t, ys, alpha, sG, M, ptr, M, ncorr);
+        const double c = second_loop(t / ys, alpha, sG, M, ptr, M, ncorr);
         if (lane < ncorr) {
             S->coef[lane] = c;
             cf[lane] = c;
@@ -654,10 +730,12 @@ __global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, c
     if (gridDim.x > 1) return;
     __syncthreads();
     double w[1] = { 0.0 };
-    for (size_t i = tid; i < n; i += kPT) w[0] += pass4_entry(i, d, z, Sh, r, x, xp, rp, fext, n, ncorr, cf);
+    for (size_t i = tid; i < n; i += kPT) w[0] += pass4_entry<M>(i, d, z, Sh, r, x, xp, rp, fext, n, ncorr, cf);
+    const unsigned long long t4 = tid == 0 ? gtimer() : 0;
+    const int tr_i = S->tr_i;
     __syncthreads();
     const double dg = cta_sums<1, kPT / 32>(w, sh);
-    if (tid == 0) pass4_done(S, dg);
+    if (tid == 0) pass4_done(S, dg, tr_i, t4);
 }
 
 // Pass 2: q = (q0 - sum_j alpha_j y_j) [/ theta when H0 = I / theta]
@@ -665,6 +743,7 @@ __global__ void __launch_bounds__(kThreads) k_pass2(double* __restrict__ q, cons
     const double* __restrict__ Yh, size_t n, int m, int divide_theta, const Scalars* S)
 {
     griddep_wait();
+    if (S->again) return;
     __shared__ double al[kMaxHist];
     const int ncorr = S->ncorr;
     for (int j = threadIdx.x; j < ncorr; j += kThreads) al[j] = S->alpha[j];
@@ -685,6 +764,7 @@ __global__ void __launch_bounds__(kThreads) k_pass3(const double* __restrict__ z
     int m, Scalars* S, double* partials, double* sums, int time_pc)
 {
     griddep_wait();
+    if (S->again) return;
     const int ncorr = S->ncorr, row = blockIdx.y;
     if (blockIdx.x == 0 && row == 0 && threadIdx.x == 0 && time_pc) S->t_pc += gtimer() - S->t0_pc;  // H0 just ended
     double v[1] = { 0 };
@@ -731,16 +811,24 @@ __global__ void __launch_bounds__(kPT) k_pass4(double* __restrict__ d, const dou
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, Scalars* S, double* partials)
 {
     griddep_wait();
+    if (S->again) {
+        trial(d, r, x, xp, fext, n, S);
+        return;
+    }
     __shared__ double cf[kMaxHist], sh[kPT / 32][32];
     __shared__ bool last;
     const int ncorr = S->ncorr;
     for (int j = threadIdx.x; j < ncorr; j += kPT) cf[j] = S->coef[j];
     __syncthreads();
     double v[1] = { 0 };
-    GRID_STRIDE(i, n) v[0] += pass4_entry(i, d, z, Sh, r, x, xp, rp, fext, n, ncorr, cf);
+    GRID_STRIDE(i, n) v[0] += pass4_entry<0>(i, d, z, Sh, r, x, xp, rp, fext, n, ncorr, cf);
     griddep_launch();
-    const double dg = grid_totals<1>(v, partials, &S->counter[1], sh, &last);
-    if (last && threadIdx.x == 0) pass4_done(S, dg);
+    const int tr_i = S->tr_i;
+    unsigned long long now = 0;
+    const double dg = grid_totals<1>(v, partials, &S->counter[1], sh, &last, [&] {
+        if (threadIdx.x == 0) now = gtimer();
+    });
+    if (last && threadIdx.x == 0) pass4_done(S, dg, tr_i, now);
 }
 
 __global__ void k_neg_copy(double* __restrict__ q, const double* __restrict__ r, size_t n)
@@ -748,23 +836,11 @@ __global__ void k_neg_copy(double* __restrict__ q, const double* __restrict__ r,
     GRID_STRIDE(i, n) q[i] = -r[i];
 }
 
-// a trial of the device-driven line search: x = xp + step d with the step
-// held on the device, and r = -f_ext to start the residual at x (its start
-// time is stamped for the residual's timing)
-__global__ void k_trial_dev(double* __restrict__ x, const double* __restrict__ xp, const double* __restrict__ d,
-    double* __restrict__ r, const double* __restrict__ fext, size_t n, Scalars* S)
+__global__ void k_loop_start(Scalars* S)
 {
-    griddep_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) S->t0_res = gtimer();
-    const double step = S->step;
-    GRID_STRIDE(i, n)
-    {
-        x[i] = __fma_rn(step, d[i], xp[i]);
-        r[i] = -fext[i];
-    }
+    S->launch_iters = 0;
+    S->again = 0;
 }
-
-__global__ void k_loop_start(Scalars* S) { S->launch_iters = 0; }
 
 // options of the device-driven loop, and the iteration number it starts at
 __global__ void k_loop_params(Scalars* S, double eps, int max_iter, int max_ls, int cap, int k, int stall_iters,
@@ -792,6 +868,7 @@ __global__ void k_solve_init(Scalars* S, double* trace, int trace_cap, int keep_
     S->t_pc = 0;
     S->n_extra = 0;
     S->n_body = 0;
+    S->again = 0;
     S->trace = trace;
     S->trace_cap = trace ? trace_cap : 0;
     S->step = 0.0;
@@ -822,7 +899,7 @@ struct SolverWS {
     int trace_cap = 0;
     int trace_n = 0;           // records the last solve produced (may exceed trace_cap)
     cudaEvent_t ev[4] = { nullptr, nullptr, nullptr, nullptr };  // solve start / end, initial H0 start / end
-    cudaStream_t capture[3] = { nullptr, nullptr, nullptr };      // outer graph, loop body, line-search body
+    cudaStream_t capture[2] = { nullptr, nullptr };               // outer graph, loop body
     struct Graphs {
         cudaGraphExec_t first = nullptr;  // iteration 1: line-search start + first trial
         cudaGraphExec_t loop = nullptr;   // iterations 2, 3, ... (device-driven)
@@ -920,17 +997,17 @@ double* mapped(double* h)
 }
 
 // the residual at the current trial x and the line-search reductions; inside
-// the device-driven line search (h_ls given) r was started by k_pass4 or k_trial_dev and
-// the reduction applies the accept / scale rule
+// the device-driven loop (h given) r was started by pass 4 and the reduction
+// applies the accept / scale rule
 efem_status enqueue_trial_tail(Model& m, SolverWS& w, double* x, cudaStream_t st,
-    const cudaGraphConditionalHandle* h_ls = nullptr, const cudaGraphConditionalHandle* h_it = nullptr, bool init_r = true)
+    const cudaGraphConditionalHandle* h = nullptr, bool init_r = true)
 {
     const size_t n = w.n;
     efem_status s = launch_residual_on(m, x, w.r, st, &w.sc->t0_res, init_r);
     if (s != EFEM_OK) return s;
-    launch_k(k_ls_reduce, grid_for(n), kThreads, 0, st, w.r, w.d, x, n, w.sc, w.partials, precond_error_flag(m),
-        mapped(w.h_read), h_ls ? *h_ls : cudaGraphConditionalHandle(),
-        h_it ? *h_it : cudaGraphConditionalHandle(), h_ls ? 1 : 0);
+    // one CTA per SM: with 296, 2.4 us an iteration slower on the finger (241k DOFs)
+    launch_k(k_ls_reduce, std::min(148, pass_grid(n)), kPT, 0, st, w.r, w.d, x, n, w.sc, w.partials, precond_error_flag(m),
+        mapped(w.h_read), h ? *h : cudaGraphConditionalHandle(), h ? 1 : 0);
     return EFEM_OK;
 }
 
@@ -958,7 +1035,7 @@ efem_status enqueue_body(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     }
     if (!one) launch_k(k_pass2, grid_for(n), kThreads, 0, st, w.q, w.r, w.Y, n, mm, divide, w.sc);
     if (use_factor) {
-        efem_status s = precond_enqueue(m, w.q, st, &w.sc->t0_pc);
+        efem_status s = precond_enqueue(m, w.q, st, &w.sc->t0_pc, &w.sc->again);
         if (s != EFEM_OK) return s;
     }
     switch (mm) {
@@ -1005,8 +1082,12 @@ efem_status add_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t
 
 // The device-driven iteration loop:
 //   k_loop_start;
-//   while (hIter) { passes + H0 + first trial; residual; reductions + decision (sets hLs);
-//                   while (hLs) { trial; residual; reductions + decision }; k_iter_decide }
+//   while (h) { passes + H0 + first trial -- or, with S->again, a further trial
+//               alone, the other kernels returning at once; residual;
+//               reductions + decisions }
+// One loop, not a loop over trials inside one over iterations: an inner while
+// node that does not run cost 1.3 us an iteration (44 to 300 us in all); a
+// further trial, of which a solve makes a handful, pays the idle launches.
 // launch_k uses programmatic dependent launch while one of these is alive
 struct PdlScope {
     explicit PdlScope(bool on) { t_pdl = on; }
@@ -1018,7 +1099,7 @@ efem_status capture_loop(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     std::lock_guard<std::mutex> lock(capture_mutex());
     PdlScope pdl(w.pdl);  // the first kernel of each body graph is a plain launch
     const long long launches = m.launches;  // capture launches nothing; replays are counted
-    cudaStream_t s0 = w.capture[0], s1 = w.capture[1], s2 = w.capture[2];
+    cudaStream_t s0 = w.capture[0], s1 = w.capture[1];
     cudaGraph_t g = nullptr;
     efem_status s = EFEM_OK;
     EFEM_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
@@ -1029,35 +1110,21 @@ efem_status capture_loop(Model& m, SolverWS& w, double* x, bool use_factor, cuda
             s = EFEM_ERR_CUDA;
             break;
         }
-        cudaGraphConditionalHandle h_iter, h_ls;
-        if (cudaGraphConditionalHandleCreate(&h_iter, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+        cudaGraphConditionalHandle h;
+        if (cudaGraphConditionalHandleCreate(&h, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
         k_loop_start<<<1, 1, 0, s0>>>(w.sc);
-        cudaGraph_t body = nullptr, ls_body = nullptr;
-        if ((s = add_while(s0, h_iter, &body)) != EFEM_OK) break;
-        if (cudaGraphConditionalHandleCreate(&h_ls, body, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
-            s = EFEM_ERR_CUDA;
-            break;
-        }
+        cudaGraph_t body = nullptr;
+        if ((s = add_while(s0, h, &body)) != EFEM_OK) break;
         if (cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
-        // passes, H0 and the first trial (pass 4), its residual and the line
-        // search's decision, which sets hLs; then the further trials
+        // passes, H0 and the trial (pass 4), its residual and the decisions
         s = enqueue_body(m, w, x, use_factor, s1);
-        if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s1, &h_ls, &h_iter, false);
-        if (s == EFEM_OK) s = add_while(s1, h_ls, &ls_body);
-        if (s == EFEM_OK && cudaStreamBeginCaptureToGraph(s2, ls_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-            s = EFEM_ERR_CUDA;
-        if (s == EFEM_OK) {
-            k_trial_dev<<<grid_for(w.n), kThreads, 0, s2>>>(x, w.xp, w.d, w.r, m.d_fext, w.n, w.sc);
-            s = enqueue_trial_tail(m, w, x, s2, &h_ls, &h_iter, false);
-            cudaGraph_t tmp = nullptr;
-            if (cudaStreamEndCapture(s2, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
-        }
+        if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s1, &h, false);
         cudaGraph_t tmp = nullptr;
         if (cudaStreamEndCapture(s1, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
     } while (false);
@@ -1084,7 +1151,7 @@ efem_status capture_step(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     cudaGraph_t g = nullptr;
     EFEM_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
     efem_status s = enqueue_body(m, w, x, use_factor, s0);
-    if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s0, nullptr, nullptr, false);  // pass 4 started the first trial
+    if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s0, nullptr, false);  // pass 4 started the first trial
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
     m.launches = launches;
     if (s != EFEM_OK || e != cudaSuccess) {
@@ -1329,7 +1396,6 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
         m.launches++;
         // passes (pass 4 starts the first trial), H0, residual, reductions with the decisions
         const long long per_body = n_passes + (ok ? precond_launch_count(m) : 0) + (per_res - 1) + 1;
-        const long long per_extra = per_res + 1;  // trial, residual, reductions
         long long n_extra = 0;
         int status = kRunning;
         for (;;) {
@@ -1337,7 +1403,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
             EFEM_CUDA(cudaStreamSynchronize(st));
             status = static_cast<int>(hr[kRdStatus]);
             const long long nb = static_cast<long long>(hr[kRdNBody]), ne = static_cast<long long>(hr[kRdNExtra]);
-            m.launches += 1 + (nb - n_body) * per_body + (ne - n_extra) * per_extra;
+            m.launches += 1 + (nb - n_body + ne - n_extra) * per_body;
             n_body = nb;
             n_extra = ne;
             if (status != kCapReached) break;
