@@ -7,7 +7,8 @@
 //                            (src/fe/ExternalConstraint.cpp:829-959)
 //   nodal forces             r starts from -f_ext (:149-167)
 //
-// Element kernel: one CTA processes EPB elements in three phases.
+// Element kernel (k_elem_thread replaces it for FP32 C3D20 with 27 points where
+// it is faster): one CTA processes EPB elements in three phases.
 //   1. stage: threads (element, node) load conn (SoA, coalesced over elements)
 //      and gather u, relative to the element's first node, into shared memory;
 //   2. Gauss point: thread (element, gp) forms H = (u . dN) J0^{-1}, P(I+H) and
@@ -23,6 +24,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstdlib>
 #include <vector>
 
 #include "efem_internal.h"
@@ -391,6 +393,197 @@ __global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a, FaceArgs<T
     griddep_launch();
 }
 
+// The FP32 kernel of 20 nodes and 27 points: G threads per element, in
+// different warps, share its Gauss points.  k_elem_residual reads 6
+// shared-memory words per 9 multiply-adds of phase 2 and 12 per 9 of phase 3
+// (79% of the memory pipe with 27 points); here a node's u is one 16-byte word
+// of the thread's own column, dN a broadcast (every lane of a warp is at the
+// same point) and the forces are added up in registers.  J0^{-1} of the next
+// point is fetched by the warp for its 32 elements, coalesced, while this one
+// is worked on.  60 sums leave 16 warps an SM, so issue (57%) and not memory
+// bounds it; 128 registers, as 144 leave 12.  The residual of 60 625 elements
+// 131 -> 105 us (G = 1: 5 us more).  For 4 to 10 nodes, 8 points of 20, and in FP64,
+// where the sums do not fit or are few, k_elem_residual was as fast or faster
+// (FP32: C3D8 25.0 against 25.8, C3D10 32.4 against 34.1, C3D20R 28.0 against
+// 30.8 us), and small blocks want its many threads: the autotuner decides.
+constexpr int kTB = 64;    // threads
+constexpr int kSplit = 2;  // threads per element
+
+template <typename T>
+constexpr bool has_thread_kernel(int nen, int ngp) { return sizeof(T) == 4 && nen == 20 && ngp == 27; }
+
+// three values of a row of four
+__device__ __forceinline__ void load3(const float* p, float& a, float& b, float& c)
+{
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a = v.x;
+    b = v.y;
+    c = v.z;
+}
+
+template <int NEN, int NGP, int MT, int G>
+__global__ void __launch_bounds__(kTB, 8) k_elem_thread(ElemArgs<float> a, FaceArgs<float> fa, int n_face_tiles)
+{
+    griddep_wait();
+    using T = float;
+    constexpr int E = kTB / G;  // elements
+    __shared__ union Smem {
+        struct {
+            alignas(16) T dN[NGP * NEN * 4];
+            alignas(16) T w[4 * NEN * kTB];  // u [NEN][E][4]; for G > 1 at the end the sums [G][3 NEN][E]
+            T J[kTB / 32][32 * 9];           // a warp's J0^{-1} at its Gauss point
+        } e;
+        FaceSmem<NEN, T, face_epb<NEN, kTB>()> f;
+        __device__ Smem() {}
+    } smem;
+    if (static_cast<int>(blockIdx.x) < n_face_tiles) {
+        face_tile<NEN, T, kTB>(fa, blockIdx.x, smem.f);
+        griddep_launch();
+        return;
+    }
+    T* su = smem.e.w;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int part = w % G, grp = w / G, el = grp * 32 + lane;
+    const int e0 = (static_cast<int>(blockIdx.x) - n_face_tiles) * E, e = e0 + el, ew = e0 + grp * 32;
+    if (a.frozen) {  // a batch union: skip the CTA when every member it covers has stopped iterating
+        const int e1 = min(a.n, e0 + E) - 1;
+        bool act = false;
+        for (int g = __ldg(a.egroup + e0); g <= __ldg(a.egroup + e1); g++) act = act || !a.frozen[g];
+        if (!act) {
+            griddep_launch();
+            return;
+        }
+    }
+    T* sJ = smem.e.J[w];
+    T jn[9];
+    const T* J0 = a.J0inv + static_cast<size_t>(ew) * NGP * 9;
+    const int jmax = min(a.n - ew, 32) * (NGP * 9);
+    int jo[9];  // the lane's offsets in the warp's J0^{-1} at point 0 (past jmax: no element)
+#pragma unroll
+    for (int k = 0; k < 9; k++) jo[k] = (k * 32 + lane) / 9 * (NGP * 9) + (k * 32 + lane) % 9;
+    auto fetch = [&](int g) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) jn[k] = jo[k] < jmax ? __ldg(J0 + jo[k] + g * 9) : T(0);
+    };
+    fetch(part);
+    for (int i = tid; i < NGP * NEN * 3; i += kTB) smem.e.dN[i / 3 * 4 + i % 3] = a.dN[i];
+    // displacements relative to the element's first node, formed in FP64 (as in k_elem_residual)
+    const int ec = min(e, a.n - 1);
+    {
+        const int n0 = __ldg(a.conn + ec);
+        double z0 = 0.0, z1 = 0.0, z2 = 0.0;
+        if (n0 < a.n_free) {
+            z0 = __ldg(a.u + 3 * n0);
+            z1 = __ldg(a.u + 3 * n0 + 1);
+            z2 = __ldg(a.u + 3 * n0 + 2);
+        }
+#pragma unroll
+        for (int q = part; q < NEN; q += G) {
+            const int node = __ldg(a.conn + static_cast<size_t>(q) * a.n + ec);
+            double w0 = 0.0, w1 = 0.0, w2 = 0.0;
+            if (node < a.n_free) {
+                w0 = __ldg(a.u + 3 * node);
+                w1 = __ldg(a.u + 3 * node + 1);
+                w2 = __ldg(a.u + 3 * node + 2);
+            }
+            *reinterpret_cast<float4*>(su + (q * E + el) * 4)
+                = make_float4(static_cast<T>(w0 - z0), static_cast<T>(w1 - z1), static_cast<T>(w2 - z2), 0.0f);
+        }
+    }
+    const MatParams<T>* mp = a.mats + __ldg(a.mat + ec);
+    const T vol = __ldg(a.vol + ec);
+    T f[3 * NEN];
+#pragma unroll
+    for (int k = 0; k < 3 * NEN; k++) f[k] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int g = part; g < NGP; g += G) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) sJ[k * 32 + lane] = jn[k];
+        __syncwarp();
+        if (g + G < NGP) fetch(g + G);
+        const T* d = smem.e.dN + g * (NEN * 4);
+        T A[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) A[k] = 0;
+#pragma unroll
+        for (int q = 0; q < NEN; q++) {
+            T u0, u1, u2, d0, d1, d2;
+            load3(su + (q * E + el) * 4, u0, u1, u2);
+            load3(d + 4 * q, d0, d1, d2);
+            A[0] += u0 * d0; A[1] += u0 * d1; A[2] += u0 * d2;
+            A[3] += u1 * d0; A[4] += u1 * d1; A[5] += u1 * d2;
+            A[6] += u2 * d0; A[7] += u2 * d1; A[8] += u2 * d2;
+        }
+        T H[9], P[9];
+        const T* Jp = sJ + 9 * lane;
+        {
+            T Ji[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) Ji[k] = Jp[k];
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+                    H[3 * i + j] = A[3 * i] * Ji[j] + A[3 * i + 1] * Ji[3 + j] + A[3 * i + 2] * Ji[6 + j];
+        }
+        piola<T, MT>(*mp, H, P);
+        const T wv = vol * __ldg(a.gw + g);
+        T S[9];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const T j0 = Jp[3 * j], j1 = Jp[3 * j + 1], j2 = Jp[3 * j + 2];
+#pragma unroll
+            for (int i = 0; i < 3; i++) S[3 * i + j] = wv * (P[3 * i] * j0 + P[3 * i + 1] * j1 + P[3 * i + 2] * j2);
+        }
+#pragma unroll
+        for (int q = 0; q < NEN; q++) {
+            T d0, d1, d2;
+            load3(d + 4 * q, d0, d1, d2);
+#pragma unroll
+            for (int i = 0; i < 3; i++) f[3 * q + i] += S[3 * i] * d0 + S[3 * i + 1] * d1 + S[3 * i + 2] * d2;
+        }
+        __syncwarp();
+    }
+    auto scatter = [&](int q, T f0, T f1, T f2) {
+        const int node = __ldg(a.conn + static_cast<size_t>(q) * a.n + e);
+        if (node >= a.n_free) return;
+        if (a.contrib) {
+            const size_t sl = a.slot0 + static_cast<size_t>(q) * a.n + e;
+            a.contrib[sl] = static_cast<double>(f0);
+            a.contrib[a.n_slots + sl] = static_cast<double>(f1);
+            a.contrib[2 * a.n_slots + sl] = static_cast<double>(f2);
+        } else {
+            atomicAdd(a.r + 3 * node, static_cast<double>(f0));
+            atomicAdd(a.r + 3 * node + 1, static_cast<double>(f1));
+            atomicAdd(a.r + 3 * node + 2, static_cast<double>(f2));
+        }
+    };
+    if constexpr (G == 1) {
+        if (e < a.n) {
+#pragma unroll
+            for (int q = 0; q < NEN; q++) scatter(q, f[3 * q], f[3 * q + 1], f[3 * q + 2]);
+        }
+    } else {
+        __syncthreads();  // u is no longer read
+#pragma unroll
+        for (int k = 0; k < 3 * NEN; k++) su[(part * 3 * NEN + k) * E + el] = f[k];
+        __syncthreads();
+        if (e < a.n)
+            for (int q = part; q < NEN; q += G) {
+                T s[3];
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    s[i] = su[(3 * q + i) * E + el];
+#pragma unroll
+                    for (int p = 1; p < G; p++) s[i] += su[(p * 3 * NEN + 3 * q + i) * E + el];
+                }
+                scatter(q, s[0], s[1], s[2]);
+            }
+    }
+    griddep_launch();
+}
+
 // Deterministic scatter, second half: free node i adds its contributions in
 // ascending slot order, r_i += sum_k contrib[gidx[k]], one thread per node
 __global__ void __launch_bounds__(kBlock) k_gather(int n_free, const int* __restrict__ gptr,
@@ -424,13 +617,28 @@ void launch_elem_blk(const ElemArgs<T>& a, const FaceArgs<T>& fa, int mt, cudaSt
     }
 }
 
+template <int NEN, int NGP>
+void launch_elem_thread(const ElemArgs<float>& a, const FaceArgs<float>& fa, int mt, cudaStream_t st)
+{
+    constexpr int E = kTB / kSplit, FPB = face_epb<NEN, kTB>();
+    const int ft = (fa.n + FPB - 1) / FPB, grid = ft + (a.n + E - 1) / E;
+    switch (mt) {
+    case EFEM_NEO_HOOKEAN: launch_k(k_elem_thread<NEN, NGP, EFEM_NEO_HOOKEAN, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
+    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_thread<NEN, NGP, EFEM_MOONEY_RIVLIN, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
+    case EFEM_YEOH: launch_k(k_elem_thread<NEN, NGP, EFEM_YEOH, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
+    default: launch_k(k_elem_thread<NEN, NGP, -1, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
+    }
+}
+
 template <int NEN, int NGP, typename T>
 void launch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, const T* J0, const T* dN, const T* gw,
     int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc, const int* frozen,
-    const FaceArgs<T>& fa)
+    const FaceArgs<T>& fa, bool split)
 {
     ElemArgs<T> a { b.n, n_free, b.conn, b.mat, vol, J0, dN, gw, mats, u, r, sc.contrib, sc.n_slots, sc.slot0,
         b.egroup, b.egroup ? frozen : nullptr };
+    if constexpr (has_thread_kernel<T>(NEN, NGP))
+        if (split) return launch_elem_thread<NEN, NGP>(a, fa, b.mat_type, st);
     if (threads == 64) launch_elem_blk<NEN, NGP, T, 64>(a, fa, b.mat_type, st);
     else if (threads == 256) launch_elem_blk<NEN, NGP, T, 256>(a, fa, b.mat_type, st);
     else launch_elem_blk<NEN, NGP, T, 128>(a, fa, b.mat_type, st);
@@ -440,11 +648,11 @@ void launch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, cons
 template <typename T>
 void dispatch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, const T* J0, const T* dN, const T* gw,
     int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc = Scatter(),
-    const int* frozen = nullptr, const FaceArgs<T>& fa = FaceArgs<T> {})
+    const int* frozen = nullptr, const FaceArgs<T>& fa = FaceArgs<T> {}, bool split = false)
 {
 #define CASE(NEN, NGP)                                                                                 \
     if (b.nen == NEN && b.ngp == NGP) {                                                                \
-        launch_elem<NEN, NGP, T>(b, mats, vol, J0, dN, gw, n_free, u, r, st, threads, sc, frozen, fa); \
+        launch_elem<NEN, NGP, T>(b, mats, vol, J0, dN, gw, n_free, u, r, st, threads, sc, frozen, fa, split); \
         return;                                                                                        \
     }
     CASE(4, 1)
@@ -490,9 +698,10 @@ int block_of_faces(const Model& m, const DevFaces& f)
 }  // namespace
 
 // Autotuner of the element kernels' CTA size: for every element block and
-// both precisions, time the 64-, 128- and 256-thread variants (2 warm-up and
-// 5 timed launches each, CUDA events on the model's stream, at u = 0: the
-// kernels' work does not depend on the values) and keep the fastest.
+// both precisions, time the 64-, 128- and 256-thread variants and, where there
+// is one, k_elem_thread (2 warm-up and 5 timed launches each, CUDA events on
+// the model's stream, at u = 0: the kernels' work does not depend on the
+// values) and keep the fastest (EFEM_TEST_ELEM_SPLIT: k_elem_thread).
 // opts.elem_threads = 64 / 128 / 256 forces one variant instead; so does
 // deterministic mode (128 unless forced), so that every model and every solve
 // runs the same instantiation and the results repeat bitwise whatever the
@@ -510,29 +719,36 @@ efem_status tune_element_blocks(Model& m)
         for (int prec = 0; prec < 2; prec++) {
             if (forced == 64 || forced == 128 || forced == 256) {
                 b.threads[prec] = forced;
+                b.split[prec] = false;
                 continue;
             }
             if (b.n == 0) {
                 b.threads[prec] = 128;
+                b.split[prec] = false;
                 continue;
             }
             float best = 1e30f;
-            for (int t : { 64, 128, 256 }) {
+            for (int t : { 64, 128, 256, -kTB }) {  // negative: k_elem_thread
+                if (t < 0 && !(prec == 1 && has_thread_kernel<float>(b.nen, b.ngp))) continue;
+                const int threads = std::abs(t);
+                const bool split = t < 0;
                 for (int rep = 0; rep < 7; rep++) {
                     if (rep == 2) EFEM_CUDA(cudaEventRecord(e0, m.stream));
                     if (prec == 1)
                         dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, m.d_u, m.d_r,
-                            m.stream, t);
+                            m.stream, threads, Scatter(), nullptr, FaceArgs<float> {}, split);
                     else
-                        dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, m.d_u, m.d_r, m.stream, t);
+                        dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, m.d_u, m.d_r, m.stream,
+                            threads, Scatter(), nullptr, FaceArgs<double> {}, split);
                 }
                 EFEM_CUDA(cudaEventRecord(e1, m.stream));
                 EFEM_CUDA(cudaEventSynchronize(e1));
                 float ms = 0.f;
                 EFEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best) {
+                if (ms < best || (split && std::getenv("EFEM_TEST_ELEM_SPLIT"))) {
                     best = ms;
-                    b.threads[prec] = t;
+                    b.threads[prec] = threads;
+                    b.split[prec] = split;
                 }
             }
         }
@@ -595,10 +811,10 @@ efem_status launch_residual_on(Model& m, const double* d_u, double* d_r, cudaStr
             if (f.n > 0 && block_of_faces(m, f) == static_cast<int>(bi)) with = &f;
         if (mixed)
             dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, d_u, d_r, stream,
-                b.threads[1], sc, m.d_frozen_groups, with ? faces_of(*with, 0.0f) : FaceArgs<float> {});
+                b.threads[1], sc, m.d_frozen_groups, with ? faces_of(*with, 0.0f) : FaceArgs<float> {}, b.split[1]);
         else
             dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, d_u, d_r, stream, b.threads[0], sc,
-                m.d_frozen_groups, with ? faces_of(*with, 0.0) : FaceArgs<double> {});
+                m.d_frozen_groups, with ? faces_of(*with, 0.0) : FaceArgs<double> {}, b.split[0]);
     }
     for (auto& f : m.faces) {
         if (f.n == 0 || block_of_faces(m, f) >= 0) continue;
