@@ -21,10 +21,10 @@
 //    finish a reduction adds that member's partial sums in chunk order and
 //    runs that member's small recursion, so every member follows exactly the
 //    arithmetic of a single solve.
-//  * One CUDA graph holds the iteration loop: a while node whose body is an
-//    iteration or a further line-search trial; its condition is set by the
-//    CTA that ends the last member's reduction, and iterations and trials
-//    are bounded there (kCap iterations per launch, max_line_search
+//  * One CUDA graph holds the iteration loop: a while node over iterations
+//    whose body holds a while node over line-search trials; both conditions
+//    are set by the CTA that ends the last member's reduction, and both
+//    loops are bounded there (kCap iterations per launch, max_line_search
 //    trials per iteration) whatever that state holds.  A member that
 //    converged (or stopped) is frozen: its x no longer moves and its
 //    counters stop; the loop ends when no member is running.  The host checks
@@ -77,7 +77,6 @@ struct Seg {
 
 struct Glob {
     int ls_round;            // line-search trials of the current iteration
-    int again;               // the next loop body is a further trial of some members' line searches
     int launch_iters, cap;
     int n_running;
     int pc_fail;
@@ -164,7 +163,6 @@ __global__ void kb_init(Seg* S, const int* c0, const double* eps, const int* max
 __global__ void kb_glob_init(Glob* G, int cap)
 {
     G->ls_round = 0;
-    G->again = 0;
     G->launch_iters = 0;
     G->cap = cap;
     G->n_running = 0;
@@ -178,7 +176,6 @@ __global__ void kb_loop_start(Glob* G)
 {
     G->launch_iters = 0;
     G->ls_round = 0;
-    G->again = 0;
 }
 
 // the initial residual's norms and the early exit (LBFGS.h:110-120) of every running member
@@ -218,10 +215,9 @@ __global__ void __launch_bounds__(kT) kb_initial(const double* __restrict__ r, c
 template <int M>
 __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, const double* __restrict__ xp,
     const double* __restrict__ r, const double* __restrict__ rp, double* __restrict__ Sh, double* __restrict__ Yh,
-    size_t n, const Chunk* __restrict__ ch, Seg* S, double* partials, const Glob* G)
+    size_t n, const Chunk* __restrict__ ch, Seg* S, double* partials)
 {
     griddep_wait();
-    if (G->again) return;
     constexpr int NV = 3 * M + 2;
     __shared__ double sh[kT / 32][32], sG[M * M], tot[32];
     __shared__ bool last;
@@ -301,11 +297,10 @@ __global__ void __launch_bounds__(kT) kb_pass1(const double* __restrict__ x, con
 
 // Pass 2: q = -r - sum_j alpha_j y_j for running members (0 elsewhere)
 __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const double* __restrict__ r,
-    const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S, const Glob* G)
+    const double* __restrict__ Yh, size_t n, const Chunk* __restrict__ ch, const Seg* S)
 {
     griddep_wait();
     griddep_launch();
-    if (G->again) return;
     const Chunk c = ch[blockIdx.x];
     const Seg* sg = S + c.seg;
     __shared__ double al[kHist];
@@ -324,10 +319,9 @@ __global__ void __launch_bounds__(kT) kb_pass2(double* __restrict__ q, const dou
 // (LBFGSMat.h:121-128), oldest pair first
 template <int M>
 __global__ void __launch_bounds__(kT) kb_pass3(const double* __restrict__ z, const double* __restrict__ Yh, size_t n,
-    const Chunk* __restrict__ ch, Seg* S, double* partials, const Glob* G)
+    const Chunk* __restrict__ ch, Seg* S, double* partials)
 {
     griddep_wait();
-    if (G->again) return;
     __shared__ double sh[kT / 32][32], sG[M * M];
     __shared__ bool last;
     const Chunk c = ch[blockIdx.x];
@@ -354,28 +348,16 @@ __global__ void __launch_bounds__(kT) kb_pass3(const double* __restrict__ z, con
 
 // Pass 4: d = z + sum_j coef_j s_j and the start of the line search of every
 // running member (dg0 = r.d, xp = x, rp = r, step 1) with its first trial
-// x = xp + d; with G->again instead a further trial x = xp + step d of the
-// members still in their line search.  r = -f_ext everywhere for the residual
-// that follows.
+// x = xp + d; r = -f_ext everywhere for the residual that follows
 __global__ void __launch_bounds__(kT) kb_pass4(double* __restrict__ d, const double* __restrict__ z,
     const double* __restrict__ Sh, double* __restrict__ r, double* __restrict__ x, double* __restrict__ xp,
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, const Chunk* __restrict__ ch, Seg* S,
-    double* partials, const Glob* G)
+    double* partials)
 {
     griddep_wait();
     const Chunk c = ch[blockIdx.x];
     Seg* sg = S + c.seg;
     const bool act = sg->state == kRun;
-    if (G->again) {
-        griddep_launch();
-        const bool more = act && sg->trial;
-        const double step = sg->step;
-        for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
-            if (more) x[i] = __fma_rn(step, d[i], xp[i]);
-            r[i] = -fext[i];
-        }
-        return;
-    }
     const int ncorr = act ? sg->ncorr : 0;
     __shared__ double cf[kHist], sh[kT / 32][32];
     __shared__ bool last;
@@ -459,12 +441,12 @@ __device__ void iter_decide(Seg* S, int nseg, Glob* G, const int* perr, int* fro
 // member in its line search, which applies the reference's rule (accept when
 // |r.d| <= |r0.d|, else step x1.5 if (r.d)(r0.d) > 0, x0.5 otherwise, at
 // most max_line_search trials, LineSearchFEA.h:43-67).  The CTA that finishes
-// the last member decides on the loop's next body: another trial when some
-// member wants one -- bounded here whatever the members' state: after max_ls
-// trials of one iteration every line search ends -- or else the next iteration.
+// the last member sets the trial loop's condition -- some member wants another
+// trial; bounded here whatever the members' state: after max_ls trials of one
+// iteration every line search ends -- and, when none does, ends the iteration.
 __global__ void __launch_bounds__(kT) kb_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
     const double* __restrict__ x, const Chunk* __restrict__ ch, Seg* S, double* partials, int nseg, int max_ls, Glob* G,
-    const int* perr, int* frozen, cudaGraphConditionalHandle h)
+    const int* perr, int* frozen, cudaGraphConditionalHandle h_ls, cudaGraphConditionalHandle h_it)
 {
     griddep_wait();
     __shared__ double sh[kT / 32][32];
@@ -526,13 +508,27 @@ __global__ void __launch_bounds__(kT) kb_ls_reduce(const double* __restrict__ r,
     if (threadIdx.x == 0) {
         G->cnt = 0u;
         G->ls_round++;
-        G->again = any;
-        if (any) {
-            G->trials++;
-            cudaGraphSetConditional(h, 1u);
-        }
+        if (any) G->trials++;
+        cudaGraphSetConditional(h_ls, any ? 1u : 0u);
     }
-    if (!any) iter_decide(S, nseg, G, perr, frozen, h);
+    if (!any) iter_decide(S, nseg, G, perr, frozen, h_it);
+}
+
+// a further trial: x = xp + step d for the members still in their line search; r = -f_ext everywhere
+__global__ void __launch_bounds__(kT) kb_trial(double* __restrict__ x, const double* __restrict__ xp,
+    const double* __restrict__ d, double* __restrict__ r, const double* __restrict__ fext,
+    const Chunk* __restrict__ ch, const Seg* S)
+{
+    griddep_wait();
+    griddep_launch();
+    const Chunk c = ch[blockIdx.x];
+    const Seg* sg = S + c.seg;
+    const bool act = sg->state == kRun && sg->trial;
+    const double step = sg->step;
+    for (int i = c.a + threadIdx.x; i < c.b; i += kT) {
+        if (act) x[i] = __fma_rn(step, d[i], xp[i]);
+        r[i] = -fext[i];
+    }
 }
 
 // launch_k uses programmatic dependent launch while one of these is alive
@@ -580,7 +576,7 @@ struct Union {
     Glob* d_glob = nullptr;
     double *x = nullptr, *xp = nullptr, *r = nullptr, *rp = nullptr, *d = nullptr, *q = nullptr, *Sh = nullptr,
            *Yh = nullptr, *partials = nullptr;
-    cudaStream_t cap[2] = { nullptr, nullptr };
+    cudaStream_t cap[3] = { nullptr, nullptr, nullptr };
     cudaGraphExec_t loop[2] = { nullptr, nullptr };  // per element precision (FP64, FP32)
     long long loop_epoch[2] = { -1, -1 };
     bool pdl = true;  // programmatic dependent launch in the captured loops (off if a capture refused it)
@@ -748,13 +744,13 @@ efem_status setup_union(Union& U)
     return EFEM_OK;
 }
 
-// the iteration graph: while (h) { passes, H0 and first trial, or a further
-// trial alone; residual; line-search reduction and decisions }
+// the iteration graph: while (iterate) { passes, H0, first trial, residual,
+// line-search reduction and decisions; while (trial) { trial, residual, reduction and decisions } }
 efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
 {
     Model& M = *U.uni;
     std::lock_guard<std::mutex> lock(capture_mutex());
-    cudaStream_t s0 = U.cap[0], s1 = U.cap[1];
+    cudaStream_t s0 = U.cap[0], s1 = U.cap[1], s2 = U.cap[2];
     const int nb = U.nchunk, max_ls = std::max(1, M.opts.max_linesearch);
     const int* perr = precond_error_flag(M);
     PdlScope pdl(U.pdl);  // the first kernel of each body graph is a plain launch
@@ -769,36 +765,48 @@ efem_status capture_union_loop(Union& U, cudaGraphExec_t* out)
             s = EFEM_ERR_CUDA;
             break;
         }
-        cudaGraphConditionalHandle h;
-        if (cudaGraphConditionalHandleCreate(&h, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+        cudaGraphConditionalHandle h_it, h_ls;
+        if (cudaGraphConditionalHandleCreate(&h_it, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
         kb_loop_start<<<1, 1, 0, s0>>>(U.d_glob);
-        cudaGraph_t body = nullptr;
-        if ((s = add_while_node(s0, h, &body)) != EFEM_OK) break;
-        if (cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaGraph_t body = nullptr, ls_body = nullptr;
+        if ((s = add_while_node(s0, h_it, &body)) != EFEM_OK) break;
+        if (cudaGraphConditionalHandleCreate(&h_ls, body, 1, cudaGraphCondAssignDefault) != cudaSuccess
+            || cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
         switch (U.m) {
-#define P1(K) case K: kb_pass1<K><<<nb, kT, 0, s1>>>(U.x, U.xp, U.r, U.rp, U.Sh, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials, U.d_glob); break;
+#define P1(K) case K: kb_pass1<K><<<nb, kT, 0, s1>>>(U.x, U.xp, U.r, U.rp, U.Sh, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
             P1(1) P1(2) P1(3) P1(4) P1(5) P1(6) P1(7) P1(8)
 #undef P1
         }
-        launch_k(kb_pass2, nb, kT, 0, s1, U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg, U.d_glob);
-        if ((s = precond_enqueue(M, U.q, s1, nullptr, &U.d_glob->again)) != EFEM_OK) break;
+        launch_k(kb_pass2, nb, kT, 0, s1, U.q, U.r, U.Yh, U.n, U.d_chunks, U.d_seg);
+        if ((s = precond_enqueue(M, U.q, s1)) != EFEM_OK) break;
         switch (U.m) {
-#define P3(K) case K: launch_k(kb_pass3<K>, nb, kT, 0, s1, U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials, U.d_glob); break;
+#define P3(K) case K: launch_k(kb_pass3<K>, nb, kT, 0, s1, U.q, U.Yh, U.n, U.d_chunks, U.d_seg, U.partials); break;
             P3(1) P3(2) P3(3) P3(4) P3(5) P3(6) P3(7) P3(8)
 #undef P3
         }
         launch_k(kb_pass4, nb, kT, 0, s1, U.d, U.q, U.Sh, U.r, U.x, U.xp, U.rp, M.d_fext, U.n, U.d_chunks, U.d_seg,
-            U.partials, U.d_glob);
+            U.partials);
         if ((s = launch_residual_on(M, U.x, U.r, s1, nullptr, false)) != EFEM_OK) break;
         launch_k(kb_ls_reduce, nb, kT, 0, s1, U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials, U.nseg, max_ls, U.d_glob, perr,
-            U.d_frozen, h);
+            U.d_frozen, h_ls, h_it);
+        if ((s = add_while_node(s1, h_ls, &ls_body)) != EFEM_OK) break;
+        if (cudaStreamBeginCaptureToGraph(s2, ls_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+            s = EFEM_ERR_CUDA;
+            break;
+        }
+        kb_trial<<<nb, kT, 0, s2>>>(U.x, U.xp, U.d, U.r, M.d_fext, U.d_chunks, U.d_seg);
+        s = launch_residual_on(M, U.x, U.r, s2, nullptr, false);
+        launch_k(kb_ls_reduce, nb, kT, 0, s2, U.r, U.d, U.x, U.d_chunks, U.d_seg, U.partials, U.nseg, max_ls, U.d_glob, perr,
+            U.d_frozen, h_ls, h_it);
         cudaGraph_t tmp = nullptr;
+        if (cudaStreamEndCapture(s2, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
+        if (s != EFEM_OK) break;
         if (cudaStreamEndCapture(s1, &tmp) != cudaSuccess) s = EFEM_ERR_CUDA;
     } while (false);
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
@@ -876,13 +884,14 @@ efem_status run_union_phase(Union& U, int stall, const std::vector<int>& keep, l
     }
     Glob g {};
     long long body0 = 0, trials0 = 0;
-    // per loop body: passes 1-4, H0, residual, reduction with the decisions (those a further trial leaves idle too)
+    // per loop body: passes 1-4, H0, residual, reduction with the decisions; per extra trial: trial, residual, reduction
     const long long per_body = 5 + precond_launch_count(M) + (U.per_res - 1);
+    const long long per_trial = 2 + (U.per_res - 1);
     for (;;) {
         EFEM_CUDA(cudaGraphLaunch(U.loop[slot], st));
         EFEM_CUDA(cudaMemcpyAsync(&g, U.d_glob, sizeof(Glob), cudaMemcpyDeviceToHost, st));
         EFEM_CUDA(cudaStreamSynchronize(st));
-        *launches += 1 + (g.body_iters - body0 + g.trials - trials0) * per_body;
+        *launches += 1 + (g.body_iters - body0) * per_body + (g.trials - trials0) * per_trial;
         body0 = g.body_iters;
         trials0 = g.trials;
         if (g.pc_fail) {

@@ -618,7 +618,6 @@ struct SolveArgs {
     int *res, *hres;            // when set: the error flag goes there (device, mapped host), and the counters are left at zero
     const int* item_group;      // batch unions: the member each item belongs to
     const int* frozen;          // batch unions: 1 for a member that no longer iterates (its items are skipped)
-    const int* skip;            // when set and nonzero: this launch does nothing (a body that is a line-search trial)
 };
 
 constexpr int kSpinLimit = 1 << 22;  // default polls of one wait (about half a second)
@@ -808,7 +807,6 @@ __device__ __forceinline__ void cols_reduce(double (&acc)[4][3])
 __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
 {
     griddep_wait();
-    if (A.skip && __ldcg(A.skip)) return;
     extern __shared__ __align__(16) double sm[];
     double* vec = sm;                      // [kVC + kMaxR][3] chunk of the vector, and f on a tile's own below rows
     double* red = sm + 3 * (kVC + kMaxR);  // partial sums, once the staged values are used
@@ -1215,7 +1213,6 @@ struct SubArgs {
     double* y;
     double* upd;
     unsigned long long* stamp;
-    const int* skip;
 };
 
 __device__ __forceinline__ void sub_stage(const SubArgs& A, const SubChunk& ch, double* dst)
@@ -1241,7 +1238,6 @@ __device__ __forceinline__ void sub_stage(const SubArgs& A, const SubChunk& ch, 
 // subtree root, written to the update array.
 __global__ void __launch_bounds__(kST) k_sub_fwd(SubArgs A)
 {
-    if (A.skip && __ldcg(A.skip)) return;
     extern __shared__ double sm[];
     double* buf[2] = { sm, sm + kSubStage };
     double* bsub = sm + 2 * kSubStage;          // [ncols][3] right-hand side on the subtree's columns
@@ -1332,7 +1328,6 @@ __global__ void __launch_bounds__(kST) k_sub_fwd(SubArgs A)
 // x_J = L_JJ^{-T} y_J - W^T x_R, x_R from the CTA's own copy of the solution.
 __global__ void __launch_bounds__(kST) k_sub_bwd(SubArgs A)
 {
-    if (A.skip && __ldcg(A.skip)) return;
     extern __shared__ double sm[];
     double* buf[2] = { sm, sm + kSubStage };
     double* ysub = sm + 2 * kSubStage;        // [ncols][3]
@@ -1428,15 +1423,15 @@ WaitCfg wait_cfg(const Model& m)
 // (own) the counters are zero beforehand and left so; other buffers' are
 // cleared first and keep the error flag.
 efem_status enqueue_solve(const Precond& P, const FrontArgs& a, const SolveBufs& b, double* d_v, cudaStream_t st,
-    WaitCfg wc, bool own, unsigned long long* stamp = nullptr, const int* skip = nullptr)
+    WaitCfg wc, bool own, unsigned long long* stamp = nullptr)
 {
     const int ns = P.S.ns;
     if (!own) EFEM_CUDA(cudaMemsetAsync(b.cnt, 0, sizeof(int) * (4 * static_cast<size_t>(ns) + 2), st));
     const SubArgs B { a, P.d_parent, P.d_prow, P.d_perm, P.d_subs, P.d_chunks, P.d_depth, P.d_xidx, P.sub_max_r,
-        P.sub_max_cols, P.sub_max_depth, P.sub_max_m, P.sub_max_c, P.sub_max_mroot, d_v, b.y, b.upd, stamp, skip };
+        P.sub_max_cols, P.sub_max_depth, P.sub_max_m, P.sub_max_c, P.sub_max_mroot, d_v, b.y, b.upd, stamp };
     if (P.n_subs > 0) k_sub_fwd<<<P.n_subs, kST, P.sub_smem_f, st>>>(B);
     SolveArgs A { a, P.d_prow, P.d_items, P.d_slot, P.n_items, ns, d_v, b.y, b.t, b.upd, b.cnt, P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, own ? P.d_res : nullptr, own ? P.h_flag : nullptr,
-        P.d_item_group, P.d_item_group ? P.d_frozen : nullptr, skip };
+        P.d_item_group, P.d_item_group ? P.d_frozen : nullptr };
     if (P.n_items > 0) launch_k(k_solve, P.solve_grid, kST, P.solve_smem, st, A);
     if (P.n_subs > 0) k_sub_bwd<<<P.n_subs, kST, P.sub_smem_b, st>>>(B);
     return EFEM_OK;
@@ -1973,7 +1968,7 @@ efem_status precond_apply(Model& m, double* d_v)
     return s;
 }
 
-efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned long long* stamp, const int* skip)
+efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned long long* stamp)
 {
     if (!m.precond || !m.precond->factored || !m.precond->ok) {
         set_error("preconditioner not factored");
@@ -1981,7 +1976,7 @@ efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned
     }
     Precond& P = *m.precond;
     if (P.S.n == 0) return EFEM_OK;
-    const efem_status s = enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), true, stamp, skip);
+    const efem_status s = enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), true, stamp);
     if (s != EFEM_OK) return s;
     EFEM_CUDA(cudaGetLastError());
     return EFEM_OK;

@@ -291,8 +291,7 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor);
 efem_status precond_apply(Model& m, double* d_v);
 // The same H0 application enqueued on `stream` (for capture into a larger
 // graph).  With `stamp`, the solve's first CTA stores the GPU's global timer there.
-efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned long long* stamp = nullptr,
-    const int* skip = nullptr);
+efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned long long* stamp = nullptr);
 // Batch unions: group_of_free_node[i] = the member free node i belongs to;
 // items of member g are skipped while d_frozen[g] != 0 (a member's fronts
 // form trees of their own, so nothing else waits on them).

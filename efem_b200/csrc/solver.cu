@@ -24,14 +24,14 @@
 // of the floating-point sums differs.
 //
 // Iterations run on the device.  After the first one (driven from the host),
-// a CUDA graph holds the loop: a while node whose body is the four passes
-// with H0, the residual at the trial and the line-search reductions, whose
-// last CTA applies the line search's accept / scale rule and the reference's
-// convergence and iteration-limit tests and sets the loop condition.  When the
-// line search wants a further trial, the passes and H0 return at once in the
-// next body and pass 4 makes the trial.  All is bounded: the line search by
-// max_linesearch, the iterations by a per-launch cap, after which the host
-// reads the state and launches the graph
+// a CUDA graph holds the loop: a while node over iterations whose body is the
+// four passes with H0, the residual at the first trial and the line-search
+// reductions, then a nested while node over the further trials.  The last CTA
+// of the reductions applies the line search's accept / scale rule and the
+// reference's convergence and iteration-limit tests and sets the loop
+// conditions.  Both loops are bounded: the line search by max_linesearch, the
+// iterations by a per-launch cap, after which the host reads the state and
+// launches the graph
 // again.  Scalars the host reads are written into mapped host memory, and the
 // time spent in the residual and in H0 is summed on the device from the GPU's
 // global timer.
@@ -73,7 +73,6 @@ struct Scalars {
     double eps, step;           // residual criterion; current line-search step
     int max_iter, max_ls, cap;  // iteration limit (0: none), trials per line search, iterations per launch
     int k, launch_iters, ls_t, status;
-    int again;                  // the next loop body is a further trial of the line search
     unsigned long long n_res, n_extra, n_body;  // residual evaluations, extra trials, device-driven iterations
     unsigned long long t0_res, t_res, t0_pc, t_pc;  // global-timer stamps and sums (ns)
     // convergence trace: record i = the state after iteration i's line search
@@ -338,18 +337,18 @@ __device__ int iter_decide(Scalars* S, const LsState& L, double rinf, double xin
 // stored in S and -- for the host's decisions, or when the device-driven loop
 // ends -- in the host-mapped read-back array (a dozen writes to host memory in
 // every iteration delayed the kernel's end: this, the loads ahead of the sweep
-// and the timer read behind other work took an iteration at 750 DOFs from 49.5
-// to 43.5 us); with a trace buffer the
+// and the timer read behind other work took an iteration at 750 DOFs from 51
+// to 45 us); with a trace buffer the
 // trial also (over)writes the current iteration's record, so the record left
 // is the accepted trial's
 // With `decide` (inside the device-driven loop) the last CTA also
 // applies the accept / scale rule of LineSearchFEA.h:43-67: accept when
 // |r.d| <= |r0.d|; otherwise scale the step by 1.5 (same sign) or 0.5 and try
-// again, at most max_ls trials in all; the loop's next body is that trial or,
-// when the line search ends, the next iteration (iter_decide).
+// again, at most max_ls trials in all; it sets the line-search loop condition
+// and, when the line search ends, the iteration loop's (iter_decide).
 __global__ void __launch_bounds__(kPT) k_ls_reduce(const double* __restrict__ r, const double* __restrict__ d,
     const double* __restrict__ x, size_t n, Scalars* S, double* partials, const int* perr_flag, double* hread,
-    cudaGraphConditionalHandle h, int decide)
+    cudaGraphConditionalHandle h_ls, cudaGraphConditionalHandle h_it, int decide)
 {
     griddep_wait();
     __shared__ double sh[kPT / 32][32];
@@ -360,8 +359,8 @@ __global__ void __launch_bounds__(kPT) k_ls_reduce(const double* __restrict__ r,
     if (threadIdx.x == 0) {
         if (blockIdx.x == 0) {
             now = gtimer();  // the residual just ended
-            // the loop stops unless the last CTA below decides on another body
-            if (decide) cudaGraphSetConditional(h, 0u);
+            // the line-search loop stops unless the last CTA below decides on another trial
+            if (decide) cudaGraphSetConditional(h_ls, 0u);
         }
         L = LsState { S->dg0, S->step, S->eps, S->best_rinf, S->trace, S->n_body, S->ls_t, S->max_ls, S->k, S->max_iter,
             S->best_k, S->stall_iters, S->launch_iters, S->cap, S->tr_i, S->trace_cap, S->tr_evals };
@@ -403,15 +402,15 @@ __global__ void __launch_bounds__(kPT) k_ls_reduce(const double* __restrict__ r,
     if (decide) {
         S->ls_t = L.ls_t + 1;
         const bool again = !(fabs(dg) <= fabs(L.dg0)) && L.ls_t + 1 < L.max_ls;
-        S->again = again ? 1 : 0;
         if (again) {
             S->step = L.step * (dg * L.dg0 > 0 ? 1.5 : 0.5);
             S->n_extra++;
-        }
-        if (again || iter_decide(S, L, rinf, xinf, perr) == kRunning) {
-            cudaGraphSetConditional(h, 1u);
+            cudaGraphSetConditional(h_ls, 1u);
             return;
         }
+        const bool more = iter_decide(S, L, rinf, xinf, perr) == kRunning;
+        cudaGraphSetConditional(h_it, more ? 1u : 0u);
+        if (more) return;
         hread[kRdStatus] = S->status;
         hread[kRdK] = S->k;
         hread[kRdNExtra] = static_cast<double>(S->n_extra);
@@ -464,7 +463,6 @@ __global__ void __launch_bounds__(kThreads) k_pass1(const double* __restrict__ x
     size_t n, int m, Scalars* S, double* partials, double* sums)
 {
     griddep_wait();
-    if (S->again) return;
     const int loc = S->ptr % m;
     const int ncorr = S->ncorr < m ? S->ncorr + 1 : m;  // count after the insertion; slots 0..ncorr-1 hold pairs
     const int row = blockIdx.y;
@@ -551,16 +549,14 @@ __global__ void __launch_bounds__(kPT) k_pass1_m(const double* __restrict__ x, c
     size_t n, Scalars* S, double* partials, double* __restrict__ q, int divide_theta)
 {
     griddep_wait();
-    if (S->again) return;
     constexpr int NV = 3 * M + 2;
-    __shared__ double sh[kPT / 32][32], sG[M * M], tot[32], sal[M], sth;
+    __shared__ double sh[kPT / 32][32], sG[M * M], sys[M], tot[32], sal[M], sth;
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31;
     const int loc = S->ptr % M;
     const int ncorr = S->ncorr < M ? S->ncorr + 1 : M;
-    const int gq = tid - (kPT - 64);  // the last two warps scale G for the recursion
-    const bool gt = gq >= 0 && gq < M * M;
-    const double g = gt ? S->G[gq / M][gq % M] : 0.0, gys = gt ? S->ys[gq / M] : 1.0;
+    if (tid < M * M) sG[tid] = S->G[tid / M][tid % M];
+    if (tid < M) sys[tid] = S->ys[tid];
     double ys = tid < M ? S->ys[tid] : 1.0;
     double v[NV];
 #pragma unroll
@@ -590,7 +586,9 @@ __global__ void __launch_bounds__(kPT) k_pass1_m(const double* __restrict__ x, c
     }
     griddep_launch();
     const double t = grid_totals<NV>(v, partials, &S->counter[2], sh, &last, [&] {
-        if (gt) sG[gq] = g / gys;  // the new row and column follow below
+        // the last two warps scale G for the recursion; the new row and column follow below
+        const int k = tid - (kPT - 64);
+        if (k >= 0 && k < M * M) sG[k] /= sys[k / M];
     });
     if (!last) return;
     if (tid < 32) {
@@ -668,21 +666,6 @@ __device__ __forceinline__ void pass4_done(Scalars* S, double dg0, int tr_i, uns
     S->t0_res = now;
 }
 
-// A further trial of the device-driven line search: x = xp + step d with the
-// step held on the device, and r = -f_ext to start the residual at x (its
-// start time is stamped for the residual's timing)
-__device__ __forceinline__ void trial(const double* __restrict__ d, double* __restrict__ r, double* __restrict__ x,
-    const double* __restrict__ xp, const double* __restrict__ fext, size_t n, Scalars* S)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) S->t0_res = gtimer();
-    const double step = S->step;
-    GRID_STRIDE(i, n)
-    {
-        x[i] = __fma_rn(step, d[i], xp[i]);
-        r[i] = -fext[i];
-    }
-}
-
 // Pass 3 and, with one CTA, pass 4
 template <int M>
 __global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, const double* __restrict__ Yh,
@@ -691,18 +674,13 @@ __global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, c
     const double* __restrict__ fext)
 {
     griddep_wait();
-    __shared__ double sh[kPT / 32][32], sG[M * M], cf[M];
+    __shared__ double sh[kPT / 32][32], sG[M * M], sys[M], cf[M];
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, ncorr = S->ncorr, ptr = S->ptr;
-    if (S->again) {
-        if (gridDim.x == 1) trial(d, r, x, xp, fext, n, S);
-        return;
-    }
     const bool timed = blockIdx.x == 0 && tid == 0 && time_pc;
     const unsigned long long now = timed ? gtimer() : 0;  // H0 just ended
-    const int gq = tid - (kPT - 64);
-    const bool gt = gq >= 0 && gq < M * M;
-    const double g = gt ? S->G[gq / M][gq % M] : 0.0, gys = gt ? S->ys[gq % M] : 1.0;
+    if (tid < M * M) sG[tid] = S->G[tid / M][tid % M];
+    if (tid < M) sys[tid] = S->ys[tid];
     const double ys = tid < M ? S->ys[tid] : 1.0, alpha = tid < M ? S->alpha[tid] : 0.0;
     double v[M];
 #pragma unroll
@@ -717,7 +695,8 @@ __global__ void __launch_bounds__(kPT) k_pass3_m(const double* __restrict__ z, c
     griddep_launch();
     if (timed) S->t_pc += now - S->t0_pc;
     const double t = grid_totals<M>(v, partials, &S->counter[3], sh, &last, [&] {
-        if (gt) sG[gq] = g / gys;
+        const int k = tid - (kPT - 64);
+        if (k >= 0 && k < M * M) sG[k] /= sys[k % M];
     });
     if (!last) return;
     if (tid < 32) {
@@ -743,7 +722,6 @@ __global__ void __launch_bounds__(kThreads) k_pass2(double* __restrict__ q, cons
     const double* __restrict__ Yh, size_t n, int m, int divide_theta, const Scalars* S)
 {
     griddep_wait();
-    if (S->again) return;
     __shared__ double al[kMaxHist];
     const int ncorr = S->ncorr;
     for (int j = threadIdx.x; j < ncorr; j += kThreads) al[j] = S->alpha[j];
@@ -764,7 +742,6 @@ __global__ void __launch_bounds__(kThreads) k_pass3(const double* __restrict__ z
     int m, Scalars* S, double* partials, double* sums, int time_pc)
 {
     griddep_wait();
-    if (S->again) return;
     const int ncorr = S->ncorr, row = blockIdx.y;
     if (blockIdx.x == 0 && row == 0 && threadIdx.x == 0 && time_pc) S->t_pc += gtimer() - S->t0_pc;  // H0 just ended
     double v[1] = { 0 };
@@ -811,10 +788,6 @@ __global__ void __launch_bounds__(kPT) k_pass4(double* __restrict__ d, const dou
     double* __restrict__ rp, const double* __restrict__ fext, size_t n, Scalars* S, double* partials)
 {
     griddep_wait();
-    if (S->again) {
-        trial(d, r, x, xp, fext, n, S);
-        return;
-    }
     __shared__ double cf[kMaxHist], sh[kPT / 32][32];
     __shared__ bool last;
     const int ncorr = S->ncorr;
@@ -836,11 +809,25 @@ __global__ void k_neg_copy(double* __restrict__ q, const double* __restrict__ r,
     GRID_STRIDE(i, n) q[i] = -r[i];
 }
 
-__global__ void k_loop_start(Scalars* S)
+// a trial of the device-driven line search: x = xp + step d with the step
+// held on the device, and r = -f_ext to start the residual at x (its start
+// time is stamped for the residual's timing)
+__global__ void k_trial_dev(double* __restrict__ x, const double* __restrict__ xp, const double* __restrict__ d,
+    double* __restrict__ r, const double* __restrict__ fext, size_t n, Scalars* S)
 {
-    S->launch_iters = 0;
-    S->again = 0;
+    griddep_wait();
+    const bool timed = blockIdx.x == 0 && threadIdx.x == 0;
+    const unsigned long long now = timed ? gtimer() : 0;
+    const double step = S->step;
+    GRID_STRIDE(i, n)
+    {
+        x[i] = __fma_rn(step, d[i], xp[i]);
+        r[i] = -fext[i];
+    }
+    if (timed) S->t0_res = now;
 }
+
+__global__ void k_loop_start(Scalars* S) { S->launch_iters = 0; }
 
 // options of the device-driven loop, and the iteration number it starts at
 __global__ void k_loop_params(Scalars* S, double eps, int max_iter, int max_ls, int cap, int k, int stall_iters,
@@ -868,7 +855,6 @@ __global__ void k_solve_init(Scalars* S, double* trace, int trace_cap, int keep_
     S->t_pc = 0;
     S->n_extra = 0;
     S->n_body = 0;
-    S->again = 0;
     S->trace = trace;
     S->trace_cap = trace ? trace_cap : 0;
     S->step = 0.0;
@@ -899,7 +885,7 @@ struct SolverWS {
     int trace_cap = 0;
     int trace_n = 0;           // records the last solve produced (may exceed trace_cap)
     cudaEvent_t ev[4] = { nullptr, nullptr, nullptr, nullptr };  // solve start / end, initial H0 start / end
-    cudaStream_t capture[2] = { nullptr, nullptr };               // outer graph, loop body
+    cudaStream_t capture[3] = { nullptr, nullptr, nullptr };      // outer graph, loop body, line-search body
     struct Graphs {
         cudaGraphExec_t first = nullptr;  // iteration 1: line-search start + first trial
         cudaGraphExec_t loop = nullptr;   // iterations 2, 3, ... (device-driven)
@@ -997,17 +983,18 @@ double* mapped(double* h)
 }
 
 // the residual at the current trial x and the line-search reductions; inside
-// the device-driven loop (h given) r was started by pass 4 and the reduction
-// applies the accept / scale rule
+// the device-driven loop (h_ls given) r was started by pass 4 or k_trial_dev and
+// the reduction applies the accept / scale rule
 efem_status enqueue_trial_tail(Model& m, SolverWS& w, double* x, cudaStream_t st,
-    const cudaGraphConditionalHandle* h = nullptr, bool init_r = true)
+    const cudaGraphConditionalHandle* h_ls = nullptr, const cudaGraphConditionalHandle* h_it = nullptr, bool init_r = true)
 {
     const size_t n = w.n;
     efem_status s = launch_residual_on(m, x, w.r, st, &w.sc->t0_res, init_r);
     if (s != EFEM_OK) return s;
     // one CTA per SM: with 296, 2.4 us an iteration slower on the finger (241k DOFs)
     launch_k(k_ls_reduce, std::min(148, pass_grid(n)), kPT, 0, st, w.r, w.d, x, n, w.sc, w.partials, precond_error_flag(m),
-        mapped(w.h_read), h ? *h : cudaGraphConditionalHandle(), h ? 1 : 0);
+        mapped(w.h_read), h_ls ? *h_ls : cudaGraphConditionalHandle(),
+        h_it ? *h_it : cudaGraphConditionalHandle(), h_ls ? 1 : 0);
     return EFEM_OK;
 }
 
@@ -1035,7 +1022,7 @@ efem_status enqueue_body(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     }
     if (!one) launch_k(k_pass2, grid_for(n), kThreads, 0, st, w.q, w.r, w.Y, n, mm, divide, w.sc);
     if (use_factor) {
-        efem_status s = precond_enqueue(m, w.q, st, &w.sc->t0_pc, &w.sc->again);
+        efem_status s = precond_enqueue(m, w.q, st, &w.sc->t0_pc);
         if (s != EFEM_OK) return s;
     }
     switch (mm) {
@@ -1082,12 +1069,11 @@ efem_status add_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t
 
 // The device-driven iteration loop:
 //   k_loop_start;
-//   while (h) { passes + H0 + first trial -- or, with S->again, a further trial
-//               alone, the other kernels returning at once; residual;
-//               reductions + decisions }
-// One loop, not a loop over trials inside one over iterations: an inner while
-// node that does not run cost 1.3 us an iteration (44 to 300 us in all); a
-// further trial, of which a solve makes a handful, pays the idle launches.
+//   while (hIter) { passes + H0 + first trial; residual; reductions + decisions;
+//                   while (hLs) { trial; residual; reductions + decisions } }
+// The inner node costs 1.3 us an iteration even when it does not run; a single
+// loop whose passes and H0 return at once in a further trial made a solve with
+// ten trials an iteration (the C3D8 beam from u = 0) 12% slower.
 // launch_k uses programmatic dependent launch while one of these is alive
 struct PdlScope {
     explicit PdlScope(bool on) { t_pdl = on; }
@@ -1099,7 +1085,7 @@ efem_status capture_loop(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     std::lock_guard<std::mutex> lock(capture_mutex());
     PdlScope pdl(w.pdl);  // the first kernel of each body graph is a plain launch
     const long long launches = m.launches;  // capture launches nothing; replays are counted
-    cudaStream_t s0 = w.capture[0], s1 = w.capture[1];
+    cudaStream_t s0 = w.capture[0], s1 = w.capture[1], s2 = w.capture[2];
     cudaGraph_t g = nullptr;
     efem_status s = EFEM_OK;
     EFEM_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
@@ -1110,21 +1096,35 @@ efem_status capture_loop(Model& m, SolverWS& w, double* x, bool use_factor, cuda
             s = EFEM_ERR_CUDA;
             break;
         }
-        cudaGraphConditionalHandle h;
-        if (cudaGraphConditionalHandleCreate(&h, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+        cudaGraphConditionalHandle h_iter, h_ls;
+        if (cudaGraphConditionalHandleCreate(&h_iter, outer, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
         k_loop_start<<<1, 1, 0, s0>>>(w.sc);
-        cudaGraph_t body = nullptr;
-        if ((s = add_while(s0, h, &body)) != EFEM_OK) break;
+        cudaGraph_t body = nullptr, ls_body = nullptr;
+        if ((s = add_while(s0, h_iter, &body)) != EFEM_OK) break;
+        if (cudaGraphConditionalHandleCreate(&h_ls, body, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+            s = EFEM_ERR_CUDA;
+            break;
+        }
         if (cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             s = EFEM_ERR_CUDA;
             break;
         }
-        // passes, H0 and the trial (pass 4), its residual and the decisions
+        // passes, H0 and the first trial (pass 4), its residual and the
+        // decisions, which set hLs; then the further trials
         s = enqueue_body(m, w, x, use_factor, s1);
-        if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s1, &h, false);
+        if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s1, &h_ls, &h_iter, false);
+        if (s == EFEM_OK) s = add_while(s1, h_ls, &ls_body);
+        if (s == EFEM_OK && cudaStreamBeginCaptureToGraph(s2, ls_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+            s = EFEM_ERR_CUDA;
+        if (s == EFEM_OK) {
+            k_trial_dev<<<grid_for(w.n), kThreads, 0, s2>>>(x, w.xp, w.d, w.r, m.d_fext, w.n, w.sc);
+            s = enqueue_trial_tail(m, w, x, s2, &h_ls, &h_iter, false);
+            cudaGraph_t tmp = nullptr;
+            if (cudaStreamEndCapture(s2, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
+        }
         cudaGraph_t tmp = nullptr;
         if (cudaStreamEndCapture(s1, &tmp) != cudaSuccess && s == EFEM_OK) s = EFEM_ERR_CUDA;
     } while (false);
@@ -1151,7 +1151,7 @@ efem_status capture_step(Model& m, SolverWS& w, double* x, bool use_factor, cuda
     cudaGraph_t g = nullptr;
     EFEM_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
     efem_status s = enqueue_body(m, w, x, use_factor, s0);
-    if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s0, nullptr, false);  // pass 4 started the first trial
+    if (s == EFEM_OK) s = enqueue_trial_tail(m, w, x, s0, nullptr, nullptr, false);  // pass 4 started the first trial
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
     m.launches = launches;
     if (s != EFEM_OK || e != cudaSuccess) {
@@ -1396,6 +1396,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
         m.launches++;
         // passes (pass 4 starts the first trial), H0, residual, reductions with the decisions
         const long long per_body = n_passes + (ok ? precond_launch_count(m) : 0) + (per_res - 1) + 1;
+        const long long per_extra = per_res + 1;  // trial, residual, reductions
         long long n_extra = 0;
         int status = kRunning;
         for (;;) {
@@ -1403,7 +1404,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
             EFEM_CUDA(cudaStreamSynchronize(st));
             status = static_cast<int>(hr[kRdStatus]);
             const long long nb = static_cast<long long>(hr[kRdNBody]), ne = static_cast<long long>(hr[kRdNExtra]);
-            m.launches += 1 + (nb - n_body + ne - n_extra) * per_body;
+            m.launches += 1 + (nb - n_body) * per_body + (ne - n_extra) * per_extra;
             n_body = nb;
             n_extra = ne;
             if (status != kCapReached) break;
