@@ -1077,7 +1077,9 @@ efem_status adjoint_gmres(Model& m, const double* u, double tol, int max_it, int
             g[j + 1] = -sn[j] * g[j];
             g[j] = cs[j] * g[j];
             *relres = std::fabs(g[j + 1]) / bnorm;
-            if (*relres <= tol || hn == 0.0) {
+            // not finite (an H0 application that gave up leaves NaN, or u or dJ/du
+            // hold one): nothing that follows could become finite again
+            if (*relres <= tol || hn == 0.0 || !std::isfinite(*relres) || !std::isfinite(hn)) {
                 j++;
                 total++;
                 done = true;

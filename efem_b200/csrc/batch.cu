@@ -894,10 +894,7 @@ efem_status run_union_phase(Union& U, int stall, const std::vector<int>& keep, l
         *launches += 1 + (g.body_iters - body0) * per_body + (g.trials - trials0) * per_trial;
         body0 = g.body_iters;
         trials0 = g.trials;
-        if (g.pc_fail) {
-            set_error("the triangular solve of the preconditioner gave up waiting for a front");
-            return EFEM_ERR_TIMEOUT;
-        }
+        if (g.pc_fail) return precond_gave_up(M);
         if (g.n_running == 0) break;
     }
     return EFEM_OK;

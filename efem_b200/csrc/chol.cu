@@ -115,7 +115,7 @@ struct Precond {
     int4 *d_steps = nullptr, *d_invs = nullptr;  // tiles of k_step and k_inverse
     cudaStream_t capture2 = nullptr;  // second branch of the factorisation's graph
     int* d_res = nullptr;   // the last application's error flag
-    int* h_flag = nullptr;  // the same in mapped host memory
+    int* h_flag = nullptr;  // mapped host memory: set by any application that gave up, cleared by the host
     double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
            *d_vals = nullptr;
     // graph replay of the numeric factorisation (the same launches every solve)
@@ -615,7 +615,8 @@ struct SolveArgs {
     int spin_limit;             // polls of one wait before the solve gives up
     int test_wait;              // 1: the last item's wait target is raised by one (it can only run out)
     int n3;                     // entries of v (3 per free node)
-    int *res, *hres;            // when set: the error flag goes there (device, mapped host), and the counters are left at zero
+    int *res, *hres;            // when set: this application's error flag, and a mapped host flag that stays set until the
+                                // host clears it; the counters are left at zero
     const int* item_group;      // batch unions: the member each item belongs to
     const int* frozen;          // batch unions: 1 for a member that no longer iterates (its items are skipped)
 };
@@ -1067,7 +1068,7 @@ __global__ void __launch_bounds__(kST, 3) k_solve(SolveArgs A)
         for (int i = tid; i < 4 * A.ns + 2; i += kST) A.cnt[i] = 0;
         if (tid == 0) {
             *A.res = ok2_sh;
-            *A.hres = ok2_sh;
+            if (ok2_sh) *A.hres = 1;  // never cleared here: applications queued behind a failed one must not hide it
         }
     }
 }
@@ -1977,6 +1978,7 @@ efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned
     Precond& P = *m.precond;
     if (P.S.n == 0) return EFEM_OK;
     const efem_status s = enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), true, stamp);
+    if (m.opts.wait_test == 2) m.opts.wait_test = 0;  // that was the one application
     if (s != EFEM_OK) return s;
     EFEM_CUDA(cudaGetLastError());
     return EFEM_OK;
@@ -2013,8 +2015,9 @@ long long precond_launch_count(const Model& m)
 
 const int* precond_error_flag(const Model& m) { return m.precond ? m.precond->d_res : nullptr; }
 
-static efem_status solve_gave_up()
+efem_status precond_gave_up(Model& m)
 {
+    if (m.precond && m.precond->h_flag) *static_cast<volatile int*>(m.precond->h_flag) = 0;
     set_error("the triangular solve of the preconditioner gave up waiting for a front");
     return EFEM_ERR_TIMEOUT;
 }
@@ -2023,7 +2026,7 @@ efem_status precond_check(Model& m)
 {
     if (!m.precond || !m.precond->h_flag) return EFEM_OK;
     EFEM_CUDA(cudaStreamSynchronize(m.stream));
-    return *static_cast<volatile int*>(m.precond->h_flag) ? solve_gave_up() : EFEM_OK;
+    return *static_cast<volatile int*>(m.precond->h_flag) ? precond_gave_up(m) : EFEM_OK;
 }
 
 // ============================================================================
@@ -2157,5 +2160,5 @@ extern "C" efem_status efem_precond_apply_noalloc(void* model, double* d_v)
     int flag = 0;
     EFEM_CUDA(cudaMemcpyAsync(&flag, counters + 4LL * S.ns + 1, sizeof(int), cudaMemcpyDeviceToHost, m.stream));
     EFEM_CUDA(cudaStreamSynchronize(m.stream));
-    return flag ? solve_gave_up() : EFEM_OK;
+    return flag ? precond_gave_up(m) : EFEM_OK;
 }

@@ -299,7 +299,8 @@ efem_status precond_set_groups(Model& m, const std::vector<int>& group_of_free_n
 bool precond_has_groups(const Model& m);
 long long precond_launch_count(const Model& m);  // kernels per H0 application
 const int* precond_error_flag(const Model& m);   // device flag: a solve gave up waiting (nullptr before set-up)
-efem_status precond_check(Model& m);             // wait for the stream and report that flag
+efem_status precond_check(Model& m);             // wait for the stream; EFEM_ERR_TIMEOUT if any application since the last check gave up
+efem_status precond_gave_up(Model& m);           // EFEM_ERR_TIMEOUT with its message, the host's flag cleared (stream idle)
 void free_precond(Model& m);
 void precond_drop_graphs(Model& m);  // captured H0 solves are out of date (new wait limits); the factor stays
 // ------------------------------------------------------------------ batches (batch.cu)

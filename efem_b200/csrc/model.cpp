@@ -955,7 +955,7 @@ efem_status efem_set_options(void* model, const efem_options* o)
     if (!o || o->m <= 0 || o->max_linesearch <= 0 || o->max_iterations < 0 || o->residual_criterion < 0
         || (o->precision != EFEM_FP64 && o->precision != EFEM_MIXED) || (o->integration != 0 && o->integration != 1)
         || o->trace < 0 || (o->line_search != 0 && o->line_search != 1) || o->wait_limit < 0
-        || (o->wait_test != 0 && o->wait_test != 1)) {
+        || o->wait_test < 0 || o->wait_test > 2) {
         efem::set_error("invalid options (NLSolverParam::check_param rules)");
         return EFEM_ERR_ARG;
     }

@@ -1362,10 +1362,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
                 EFEM_CUDA(cudaStreamSynchronize(st));
                 m.launches += per_step;
                 if (ok) info->n_precond_applies++;
-                if (hr[kRdPerr] != 0.0) {
-                    set_error("the triangular solve of the preconditioner gave up waiting for a front");
-                    return EFEM_ERR_TIMEOUT;
-                }
+                if (hr[kRdPerr] != 0.0) return precond_gave_up(m);
                 if ((s = line_search()) != EFEM_OK) return s;
                 rinf = hr[kRdRinf];
                 xinf = hr[kRdXinf];
@@ -1416,10 +1413,7 @@ efem_status run_solve_phase(Model& m, double* x, efem_solve_info* info, bool ref
             info->n_precond_applies += static_cast<int>(n_body);
             ms_pc += hr[kRdTPc] * 1e-6;
         }
-        if (status == kPrecondFail) {
-            set_error("the triangular solve of the preconditioner gave up waiting for a front");
-            return EFEM_ERR_TIMEOUT;
-        }
+        if (status == kPrecondFail) return precond_gave_up(m);
         if (status == kNonFinite) goto nan_exit;
         if (status == kConverged) converged = true;
         if (status == kMaxIters) info->flags |= EFEM_SOLVE_MAX_ITERS;

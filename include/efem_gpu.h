@@ -134,7 +134,9 @@ typedef struct {
                                  (2^22 polls, about half a second) */
     int wait_test;            /* test aid, 0 = off: 1 makes one wait of every H0 application wait for
                                  a count that no work item produces, so it runs out after wait_limit
-                                 polls -- the timeout path without a GPU fault */
+                                 polls -- the timeout path without a GPU fault; 2: of the next H0
+                                 application alone (efem_precond_apply, efem_adjoint or the first of
+                                 efem_solve), and the option is 0 again */
 } efem_options;
 
 enum {

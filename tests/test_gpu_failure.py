@@ -13,7 +13,9 @@ device wait -- none faults, traps or hangs the GPU.
   application wait for a count that no work item produces, and
   options.wait_limit bounds it to a few hundred polls.  The call returns
   EFEM_ERR_TIMEOUT, the output holds NaN, and the next call with the test
-  aid off succeeds with the right result in the same CUDA context.
+  aid off succeeds with the right result in the same CUDA context.  With
+  wait_test = 2 only the first application of a call gives up; the adjoint,
+  which queues further ones behind it, reports it all the same.
 """
 import ctypes
 import json
@@ -82,3 +84,23 @@ def test_wait_that_runs_out_reports_timeout_and_the_gpu_stays_usable(tmp_path):
     u, info = m.solve()
     assert info["flags"] & api.SOLVE_CONVERGED and info["r_inf"] <= 1e-6
     assert rel(u, d["u_solve"]) <= 1e-6, rel(u, d["u_solve"])
+
+
+def test_adjoint_reports_the_one_application_that_gave_up(tmp_path):
+    cfg, d = write_golden_case(golden_files("case_C3D20_nh_pressure.npz")[0], tmp_path)
+    m = api.Model.from_json(cfg)
+    u, _ = m.solve()
+    g = np.zeros(m.n_dof)
+    g[-1] = 1.0
+    want, _, info = m.adjoint(u, g)
+    assert info["iterations"] > 3  # further applications are queued behind the first
+    m.set_options(wait_test=2, wait_limit=200)
+    with pytest.raises(api.EfemError) as e:
+        m.adjoint(u, g)
+    assert e.value.status == api.ERR_TIMEOUT and "gave up" in api.last_error()
+    # the test aid is used up, and neither the next application nor the next gradient sees the old failure
+    m.set_options(wait_limit=0)
+    assert np.all(np.isfinite(m.precond_apply(g)))
+    got, _, info = m.adjoint(u, g)
+    assert info["flags"] & api.SOLVE_CONVERGED
+    assert rel(got, want) <= 1e-7  # two GMRES solves to 1e-8
