@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include "efem_internal.h"
@@ -254,22 +255,34 @@ struct ElemSmem {
     int node[EPB][NEN | 1];
 };
 
-// MT: the block's one material law, or -1 when its elements mix laws.  The
-// first n_face_tiles CTAs take the pressure faces of the block's kind.
-template <int NEN, int NGP, typename T, int BLK, int MT>
+struct NoFaces {};
+template <int NEN, typename T, int BLK, bool Faces>
+using FaceSmemIf = std::conditional_t<Faces, FaceSmem<NEN, T, face_epb<NEN, BLK>()>, NoFaces>;
+
+// MT: the block's one material law, or -1 when its elements mix laws.  With
+// Faces the first n_face_tiles CTAs take the pressure faces of the block's
+// kind.  Blocks without faces have a kernel without them: a kernel's registers
+// are the larger of the two parts', and the faces' cost the neo-Hookean FP64
+// elements a third of their warps (C3D8 64 -> 92 registers; the residual of
+// 119 700 elements 53.0 -> 57.0 us, of 105 000 C3D10 tetrahedra 37.5 -> 39.7).
+// With faces the one launch is the faster one all the same (57.5 against 64.9
+// and 40.3 against 49.5 us for two).
+template <int NEN, int NGP, typename T, int BLK, int MT, bool Faces>
 __global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a, FaceArgs<T> fa, int n_face_tiles)
 {
     griddep_wait();
     constexpr int EPB = elems_per_cta<NGP, BLK>();
     __shared__ union Smem {
         ElemSmem<NEN, NGP, T, EPB> e;
-        FaceSmem<NEN, T, face_epb<NEN, BLK>()> f;
+        FaceSmemIf<NEN, T, BLK, Faces> f;
         __device__ Smem() {}
     } smem;
-    if (static_cast<int>(blockIdx.x) < n_face_tiles) {
-        face_tile<NEN, T, BLK>(fa, blockIdx.x, smem.f);
-        griddep_launch();
-        return;
+    if constexpr (Faces) {
+        if (static_cast<int>(blockIdx.x) < n_face_tiles) {
+            face_tile<NEN, T, BLK>(fa, blockIdx.x, smem.f);
+            griddep_launch();
+            return;
+        }
     }
     auto& s_u = smem.e.u;
     auto& s_S = smem.e.S;
@@ -277,7 +290,7 @@ __global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a, FaceArgs<T
     auto& s_node = smem.e.node;
 
     const int tid = threadIdx.x;
-    const int e0 = (static_cast<int>(blockIdx.x) - n_face_tiles) * EPB;
+    const int e0 = (static_cast<int>(blockIdx.x) - (Faces ? n_face_tiles : 0)) * EPB;
     if (a.frozen) {  // a batch union: skip the CTA when every member it covers has stopped iterating
         const int e1 = min(a.n, e0 + EPB) - 1;
         bool act = false;
@@ -604,17 +617,26 @@ __global__ void __launch_bounds__(kBlock) k_gather(int n_free, const int* __rest
     r[3 * i + 2] = s2;
 }
 
+template <int NEN, int NGP, typename T, int BLK, bool Faces>
+void launch_elem_law(const ElemArgs<T>& a, const FaceArgs<T>& fa, int ft, int mt, cudaStream_t st)
+{
+    constexpr int EPB = elems_per_cta<NGP, BLK>();
+    const int grid = ft + (a.n + EPB - 1) / EPB;
+    switch (mt) {
+    case EFEM_NEO_HOOKEAN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_NEO_HOOKEAN, Faces>, grid, BLK, 0, st, a, fa, ft); break;
+    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_MOONEY_RIVLIN, Faces>, grid, BLK, 0, st, a, fa, ft); break;
+    case EFEM_YEOH: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_YEOH, Faces>, grid, BLK, 0, st, a, fa, ft); break;
+    default: launch_k(k_elem_residual<NEN, NGP, T, BLK, -1, Faces>, grid, BLK, 0, st, a, fa, ft); break;
+    }
+}
+
 template <int NEN, int NGP, typename T, int BLK>
 void launch_elem_blk(const ElemArgs<T>& a, const FaceArgs<T>& fa, int mt, cudaStream_t st)
 {
-    constexpr int EPB = elems_per_cta<NGP, BLK>(), FPB = face_epb<NEN, BLK>();
-    const int ft = (fa.n + FPB - 1) / FPB, grid = ft + (a.n + EPB - 1) / EPB;
-    switch (mt) {
-    case EFEM_NEO_HOOKEAN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_NEO_HOOKEAN>, grid, BLK, 0, st, a, fa, ft); break;
-    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_MOONEY_RIVLIN>, grid, BLK, 0, st, a, fa, ft); break;
-    case EFEM_YEOH: launch_k(k_elem_residual<NEN, NGP, T, BLK, EFEM_YEOH>, grid, BLK, 0, st, a, fa, ft); break;
-    default: launch_k(k_elem_residual<NEN, NGP, T, BLK, -1>, grid, BLK, 0, st, a, fa, ft); break;
-    }
+    constexpr int FPB = face_epb<NEN, BLK>();
+    const int ft = (fa.n + FPB - 1) / FPB;
+    if (ft > 0) launch_elem_law<NEN, NGP, T, BLK, true>(a, fa, ft, mt, st);
+    else launch_elem_law<NEN, NGP, T, BLK, false>(a, fa, 0, mt, st);
 }
 
 template <int NEN, int NGP>
@@ -695,13 +717,34 @@ int block_of_faces(const Model& m, const DevFaces& f)
     return -1;
 }
 
+// arguments of face set f, in the element kernels' precision
+template <typename T>
+FaceArgs<T> face_args_of(const Model& m, const DevFaces& f, const double* u, double* r, bool det)
+{
+    Scatter sc;
+    if (det) sc = Scatter { m.d_contrib, m.n_slots, f.slot0 };
+    if constexpr (sizeof(T) == 4)
+        return face_args<float>(f, f.J0inv_f, f.t_w_f, f.t_N_f, f.t_dN_f, m.n_free, u, r, sc);
+    else
+        return face_args<double>(f, f.J0inv, f.t_w, f.t_N, f.t_dN, m.n_free, u, r, sc);
+}
+
+// the faces that go with element block bi (n = 0: none)
+template <typename T>
+FaceArgs<T> faces_with(const Model& m, size_t bi, const double* u, double* r, bool det)
+{
+    for (auto& f : m.faces)
+        if (f.n > 0 && block_of_faces(m, f) == static_cast<int>(bi)) return face_args_of<T>(m, f, u, r, det);
+    return FaceArgs<T> {};
+}
+
 }  // namespace
 
 // Autotuner of the element kernels' CTA size: for every element block and
 // both precisions, time the 64-, 128- and 256-thread variants and, where there
-// is one, k_elem_thread (2 warm-up and 5 timed launches each, CUDA events on
-// the model's stream, at u = 0: the kernels' work does not depend on the
-// values) and keep the fastest (EFEM_TEST_ELEM_SPLIT: k_elem_thread).
+// is one, k_elem_thread (2 warm-up and 5 timed launches each, with the faces
+// that go along, CUDA events on the model's stream, at u = 0: the kernels' work
+// does not depend on the values) and keep the fastest (EFEM_TEST_ELEM_SPLIT: k_elem_thread).
 // opts.elem_threads = 64 / 128 / 256 forces one variant instead; so does
 // deterministic mode (128 unless forced), so that every model and every solve
 // runs the same instantiation and the results repeat bitwise whatever the
@@ -715,7 +758,8 @@ efem_status tune_element_blocks(Model& m)
     cudaEvent_t e0, e1;
     EFEM_CUDA(cudaEventCreate(&e0));
     EFEM_CUDA(cudaEventCreate(&e1));
-    for (auto& b : m.blocks) {
+    for (size_t bi = 0; bi < m.blocks.size(); bi++) {
+        DevBlock& b = m.blocks[bi];
         for (int prec = 0; prec < 2; prec++) {
             if (forced == 64 || forced == 128 || forced == 256) {
                 b.threads[prec] = forced;
@@ -736,10 +780,10 @@ efem_status tune_element_blocks(Model& m)
                     if (rep == 2) EFEM_CUDA(cudaEventRecord(e0, m.stream));
                     if (prec == 1)
                         dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, m.d_u, m.d_r,
-                            m.stream, threads, Scatter(), nullptr, FaceArgs<float> {}, split);
+                            m.stream, threads, Scatter(), nullptr, faces_with<float>(m, bi, m.d_u, m.d_r, false), split);
                     else
                         dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, m.d_u, m.d_r, m.stream,
-                            threads, Scatter(), nullptr, FaceArgs<double> {}, split);
+                            threads, Scatter(), nullptr, faces_with<double>(m, bi, m.d_u, m.d_r, false), split);
                 }
                 EFEM_CUDA(cudaEventRecord(e1, m.stream));
                 EFEM_CUDA(cudaEventSynchronize(e1));
@@ -791,38 +835,26 @@ efem_status launch_residual_on(Model& m, const double* d_u, double* d_r, cudaStr
         set_error("deterministic scatter requested but its tables are not built");
         return EFEM_ERR_ARG;
     }
-    auto faces_of = [&](const DevFaces& f, auto tag) {
-        using T = decltype(tag);
-        Scatter sc;
-        if (det) sc = Scatter { m.d_contrib, m.n_slots, f.slot0 };
-        if constexpr (sizeof(T) == 4)
-            return face_args<float>(f, f.J0inv_f, f.t_w_f, f.t_N_f, f.t_dN_f, m.n_free, d_u, d_r, sc);
-        else
-            return face_args<double>(f, f.J0inv, f.t_w, f.t_N, f.t_dN, m.n_free, d_u, d_r, sc);
-    };
     for (size_t bi = 0; bi < m.blocks.size(); bi++) {
         const DevBlock& b = m.blocks[bi];
         if (b.n == 0) continue;
         m.launches++;
         Scatter sc;
         if (det) sc = Scatter { m.d_contrib, m.n_slots, b.slot0 };
-        const DevFaces* with = nullptr;
-        for (auto& f : m.faces)
-            if (f.n > 0 && block_of_faces(m, f) == static_cast<int>(bi)) with = &f;
         if (mixed)
             dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, d_u, d_r, stream,
-                b.threads[1], sc, m.d_frozen_groups, with ? faces_of(*with, 0.0f) : FaceArgs<float> {}, b.split[1]);
+                b.threads[1], sc, m.d_frozen_groups, faces_with<float>(m, bi, d_u, d_r, det), b.split[1]);
         else
             dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, d_u, d_r, stream, b.threads[0], sc,
-                m.d_frozen_groups, with ? faces_of(*with, 0.0) : FaceArgs<double> {}, b.split[0]);
+                m.d_frozen_groups, faces_with<double>(m, bi, d_u, d_r, det), b.split[0]);
     }
     for (auto& f : m.faces) {
         if (f.n == 0 || block_of_faces(m, f) >= 0) continue;
         m.launches++;
         if (mixed)
-            dispatch_face<float>(f.nen, faces_of(f, 0.0f), stream);
+            dispatch_face<float>(f.nen, face_args_of<float>(m, f, d_u, d_r, det), stream);
         else
-            dispatch_face<double>(f.nen, faces_of(f, 0.0), stream);
+            dispatch_face<double>(f.nen, face_args_of<double>(m, f, d_u, d_r, det), stream);
     }
     if (det) {
         launch_k(k_gather, (m.n_free + kBlock - 1) / kBlock, kBlock, 0, stream, m.n_free, m.d_gptr, m.d_gidx,
