@@ -67,7 +67,7 @@ constexpr int MAX_MATS = 16;
 struct DevBlock {
     int kind = 0, nen = 0, ngp = 0, n = 0;
     int threads[2] = { 128, 128 };  // element-kernel CTA size per precision (FP64, FP32), from the autotuner
-    bool split[2] = { false, false };  // k_elem_thread instead of k_elem_residual, from the autotuner too
+    int per_sm[2] = { 0, 0 };  // not 0: k_elem_thread, at most this many CTAs per SM, instead of k_elem_residual (autotuner)
     int mat_type = -1;            // the one material law of every element, or -1 when they mix laws
     size_t slot0 = 0;             // deterministic scatter: first contribution slot, slot = slot0 + a * n + e
     int* conn = nullptr;          // [nen][n]

@@ -413,14 +413,20 @@ __global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a, FaceArgs<T
 // of the thread's own column, dN a broadcast (every lane of a warp is at the
 // same point) and the forces are added up in registers.  J0^{-1} of the next
 // point is fetched by the warp for its 32 elements, coalesced, while this one
-// is worked on.  60 sums leave 16 warps an SM, so issue (57%) and not memory
-// bounds it; 128 registers, as 144 leave 12.  The residual of 60 625 elements
-// 131 -> 105 us (G = 1: 5 us more).  For 4 to 10 nodes, 8 points of 20, and in FP64,
+// is worked on.  What bounds it is latency at 16 warps an SM: 8 CTAs by 128
+// registers (60 sums) and by shared memory; and the last wave, for which 7 CTAs
+// an SM are sometimes the better number, so the autotuner times both (`pad`).
+// One residual in a solve, neo-Hookean, with 8 and 7: 36 864 elements 53 and
+// 64 us, 60 625 elements 84 and 82, 70 713 elements 96 and 105.
+// A direct call on 60 625 elements went from 131 to 105 us (G = 1: 5 us more).  For 4 to 10 nodes, 8 points of 20, and in FP64,
 // where the sums do not fit or are few, k_elem_residual was as fast or faster
 // (FP32: C3D8 25.0 against 25.8, C3D10 32.4 against 34.1, C3D20R 28.0 against
 // 30.8 us), and small blocks want its many threads: the autotuner decides.
 constexpr int kTB = 64;    // threads
 constexpr int kSplit = 2;  // threads per element
+constexpr int kPerSM = 8;  // CTAs per SM
+constexpr size_t kPadSmem = 2048;  // dynamic shared memory that leaves room for 7
+constexpr size_t kSmemSM = 233472, kSmemCTA = 1024;  // shared memory of an SM, and what the system takes of it per CTA
 
 template <typename T>
 constexpr bool has_thread_kernel(int nen, int ngp) { return sizeof(T) == 4 && nen == 20 && ngp == 27; }
@@ -435,7 +441,7 @@ __device__ __forceinline__ void load3(const float* p, float& a, float& b, float&
 }
 
 template <int NEN, int NGP, int MT, int G>
-__global__ void __launch_bounds__(kTB, 8) k_elem_thread(ElemArgs<float> a, FaceArgs<float> fa, int n_face_tiles)
+__global__ void __launch_bounds__(kTB, kPerSM) k_elem_thread(ElemArgs<float> a, FaceArgs<float> fa, int n_face_tiles)
 {
     griddep_wait();
     using T = float;
@@ -443,12 +449,14 @@ __global__ void __launch_bounds__(kTB, 8) k_elem_thread(ElemArgs<float> a, FaceA
     __shared__ union Smem {
         struct {
             alignas(16) T dN[NGP * NEN * 4];
-            alignas(16) T w[4 * NEN * kTB];  // u [NEN][E][4]; for G > 1 at the end the sums [G][3 NEN][E]
+            alignas(16) T w[4 * NEN * E > 3 * NEN * G * E ? 4 * NEN * E : 3 * NEN * G * E];  // u [NEN][E][4]; at the end the sums [G][3 NEN][E]
             T J[kTB / 32][32 * 9];           // a warp's J0^{-1} at its Gauss point
         } e;
         FaceSmem<NEN, T, face_epb<NEN, kTB>()> f;
         __device__ Smem() {}
     } smem;
+    static_assert(kPerSM * (sizeof(Smem) + kSmemCTA) <= kSmemSM, "kPerSM CTAs on an SM");
+    static_assert(kPerSM * (sizeof(Smem) + kSmemCTA + kPadSmem) > kSmemSM, "one less with the pad");
     if (static_cast<int>(blockIdx.x) < n_face_tiles) {
         face_tile<NEN, T, kTB>(fa, blockIdx.x, smem.f);
         griddep_launch();
@@ -640,27 +648,28 @@ void launch_elem_blk(const ElemArgs<T>& a, const FaceArgs<T>& fa, int mt, cudaSt
 }
 
 template <int NEN, int NGP>
-void launch_elem_thread(const ElemArgs<float>& a, const FaceArgs<float>& fa, int mt, cudaStream_t st)
+void launch_elem_thread(const ElemArgs<float>& a, const FaceArgs<float>& fa, int mt, cudaStream_t st, int per_sm)
 {
+    const size_t pad = per_sm < kPerSM ? kPadSmem : 0;
     constexpr int E = kTB / kSplit, FPB = face_epb<NEN, kTB>();
     const int ft = (fa.n + FPB - 1) / FPB, grid = ft + (a.n + E - 1) / E;
     switch (mt) {
-    case EFEM_NEO_HOOKEAN: launch_k(k_elem_thread<NEN, NGP, EFEM_NEO_HOOKEAN, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
-    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_thread<NEN, NGP, EFEM_MOONEY_RIVLIN, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
-    case EFEM_YEOH: launch_k(k_elem_thread<NEN, NGP, EFEM_YEOH, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
-    default: launch_k(k_elem_thread<NEN, NGP, -1, kSplit>, grid, kTB, 0, st, a, fa, ft); break;
+    case EFEM_NEO_HOOKEAN: launch_k(k_elem_thread<NEN, NGP, EFEM_NEO_HOOKEAN, kSplit>, grid, kTB, pad, st, a, fa, ft); break;
+    case EFEM_MOONEY_RIVLIN: launch_k(k_elem_thread<NEN, NGP, EFEM_MOONEY_RIVLIN, kSplit>, grid, kTB, pad, st, a, fa, ft); break;
+    case EFEM_YEOH: launch_k(k_elem_thread<NEN, NGP, EFEM_YEOH, kSplit>, grid, kTB, pad, st, a, fa, ft); break;
+    default: launch_k(k_elem_thread<NEN, NGP, -1, kSplit>, grid, kTB, pad, st, a, fa, ft); break;
     }
 }
 
 template <int NEN, int NGP, typename T>
 void launch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, const T* J0, const T* dN, const T* gw,
     int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc, const int* frozen,
-    const FaceArgs<T>& fa, bool split)
+    const FaceArgs<T>& fa, int per_sm)
 {
     ElemArgs<T> a { b.n, n_free, b.conn, b.mat, vol, J0, dN, gw, mats, u, r, sc.contrib, sc.n_slots, sc.slot0,
         b.egroup, b.egroup ? frozen : nullptr };
     if constexpr (has_thread_kernel<T>(NEN, NGP))
-        if (split) return launch_elem_thread<NEN, NGP>(a, fa, b.mat_type, st);
+        if (per_sm) return launch_elem_thread<NEN, NGP>(a, fa, b.mat_type, st, per_sm);
     if (threads == 64) launch_elem_blk<NEN, NGP, T, 64>(a, fa, b.mat_type, st);
     else if (threads == 256) launch_elem_blk<NEN, NGP, T, 256>(a, fa, b.mat_type, st);
     else launch_elem_blk<NEN, NGP, T, 128>(a, fa, b.mat_type, st);
@@ -670,11 +679,11 @@ void launch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, cons
 template <typename T>
 void dispatch_elem(const DevBlock& b, const MatParams<T>* mats, const T* vol, const T* J0, const T* dN, const T* gw,
     int n_free, const double* u, double* r, cudaStream_t st, int threads, const Scatter& sc = Scatter(),
-    const int* frozen = nullptr, const FaceArgs<T>& fa = FaceArgs<T> {}, bool split = false)
+    const int* frozen = nullptr, const FaceArgs<T>& fa = FaceArgs<T> {}, int per_sm = 0)
 {
 #define CASE(NEN, NGP)                                                                                 \
     if (b.nen == NEN && b.ngp == NGP) {                                                                \
-        launch_elem<NEN, NGP, T>(b, mats, vol, J0, dN, gw, n_free, u, r, st, threads, sc, frozen, fa, split); \
+        launch_elem<NEN, NGP, T>(b, mats, vol, J0, dN, gw, n_free, u, r, st, threads, sc, frozen, fa, per_sm); \
         return;                                                                                        \
     }
     CASE(4, 1)
@@ -742,7 +751,7 @@ FaceArgs<T> faces_with(const Model& m, size_t bi, const double* u, double* r, bo
 
 // Autotuner of the element kernels' CTA size: for every element block and
 // both precisions, time the 64-, 128- and 256-thread variants and, where there
-// is one, k_elem_thread (2 warm-up and 5 timed launches each, with the faces
+// is one, k_elem_thread with 8 and 7 CTAs per SM (2 warm-up and 5 timed launches each, with the faces
 // that go along, CUDA events on the model's stream, at u = 0: the kernels' work
 // does not depend on the values) and keep the fastest (EFEM_TEST_ELEM_SPLIT: k_elem_thread).
 // opts.elem_threads = 64 / 128 / 256 forces one variant instead; so does
@@ -763,36 +772,35 @@ efem_status tune_element_blocks(Model& m)
         for (int prec = 0; prec < 2; prec++) {
             if (forced == 64 || forced == 128 || forced == 256) {
                 b.threads[prec] = forced;
-                b.split[prec] = false;
+                b.per_sm[prec] = 0;
                 continue;
             }
             if (b.n == 0) {
                 b.threads[prec] = 128;
-                b.split[prec] = false;
+                b.per_sm[prec] = 0;
                 continue;
             }
             float best = 1e30f;
-            for (int t : { 64, 128, 256, -kTB }) {  // negative: k_elem_thread
+            for (int t : { 64, 128, 256, -kPerSM, 1 - kPerSM }) {  // negative: k_elem_thread, CTAs per SM
                 if (t < 0 && !(prec == 1 && has_thread_kernel<float>(b.nen, b.ngp))) continue;
-                const int threads = std::abs(t);
-                const bool split = t < 0;
+                const int threads = t < 0 ? kTB : t, per_sm = t < 0 ? -t : 0;
                 for (int rep = 0; rep < 7; rep++) {
                     if (rep == 2) EFEM_CUDA(cudaEventRecord(e0, m.stream));
                     if (prec == 1)
                         dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, m.d_u, m.d_r,
-                            m.stream, threads, Scatter(), nullptr, faces_with<float>(m, bi, m.d_u, m.d_r, false), split);
+                            m.stream, threads, Scatter(), nullptr, faces_with<float>(m, bi, m.d_u, m.d_r, false), per_sm);
                     else
                         dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, m.d_u, m.d_r, m.stream,
-                            threads, Scatter(), nullptr, faces_with<double>(m, bi, m.d_u, m.d_r, false), split);
+                            threads, Scatter(), nullptr, faces_with<double>(m, bi, m.d_u, m.d_r, false), per_sm);
                 }
                 EFEM_CUDA(cudaEventRecord(e1, m.stream));
                 EFEM_CUDA(cudaEventSynchronize(e1));
                 float ms = 0.f;
                 EFEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best || (split && std::getenv("EFEM_TEST_ELEM_SPLIT"))) {
+                if (ms < best || (per_sm && std::getenv("EFEM_TEST_ELEM_SPLIT"))) {
                     best = ms;
                     b.threads[prec] = threads;
-                    b.split[prec] = split;
+                    b.per_sm[prec] = per_sm;
                 }
             }
         }
@@ -843,10 +851,10 @@ efem_status launch_residual_on(Model& m, const double* d_u, double* d_r, cudaStr
         if (det) sc = Scatter { m.d_contrib, m.n_slots, b.slot0 };
         if (mixed)
             dispatch_elem<float>(b, m.d_mats_f, b.vol_f, b.J0inv_f, b.dN_f, b.gw_f, m.n_free, d_u, d_r, stream,
-                b.threads[1], sc, m.d_frozen_groups, faces_with<float>(m, bi, d_u, d_r, det), b.split[1]);
+                b.threads[1], sc, m.d_frozen_groups, faces_with<float>(m, bi, d_u, d_r, det), b.per_sm[1]);
         else
             dispatch_elem<double>(b, m.d_mats, b.vol, b.J0inv, b.dN, b.gw, m.n_free, d_u, d_r, stream, b.threads[0], sc,
-                m.d_frozen_groups, faces_with<double>(m, bi, d_u, d_r, det), b.split[0]);
+                m.d_frozen_groups, faces_with<double>(m, bi, d_u, d_r, det), b.per_sm[0]);
     }
     for (auto& f : m.faces) {
         if (f.n == 0 || block_of_faces(m, f) >= 0) continue;

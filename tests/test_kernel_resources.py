@@ -41,3 +41,12 @@ def test_blocks_without_faces_do_not_pay_for_them(kernels):
     for (nen, ngp, t, threads, law, faces), regs in elem.items():
         if not faces and threads == 128 and law == 0:
             assert SM_REGISTERS // (128 * regs) >= (6 if t == "d" else 9), (nen, ngp, t, regs)
+
+
+def test_register_summing_kernel_fits_eight_times(kernels):
+    """k_elem_thread: 128 registers and the shared memory for eight CTAs of 64
+    threads (16 warps) on an SM of 228 KB, 1 KB of which each CTA takes besides."""
+    found = [v for k, v in kernels.items() if "k_elem_thread" in k]
+    assert len(found) == 4
+    for regs, smem in found:
+        assert SM_REGISTERS // (64 * regs) >= 8 and 233472 // (smem + 1024) >= 8, (regs, smem)
