@@ -24,7 +24,6 @@
 
 #include <algorithm>
 #include <climits>
-#include <cstdlib>
 #include <type_traits>
 #include <vector>
 
@@ -753,15 +752,17 @@ FaceArgs<T> faces_with(const Model& m, size_t bi, const double* u, double* r, bo
 // both precisions, time the 64-, 128- and 256-thread variants and, where there
 // is one, k_elem_thread with 8 and 7 CTAs per SM (2 warm-up and 5 timed launches each, with the faces
 // that go along, CUDA events on the model's stream, at u = 0: the kernels' work
-// does not depend on the values) and keep the fastest (EFEM_TEST_ELEM_SPLIT: k_elem_thread).
-// opts.elem_threads = 64 / 128 / 256 forces one variant instead; so does
+// does not depend on the values) and keep the fastest.
+// opts.elem_threads = 64 / 128 / 256 forces one variant instead, and 1 forces
+// k_elem_thread where there is one (the rest as with 0); so does
 // deterministic mode (128 unless forced), so that every model and every solve
 // runs the same instantiation and the results repeat bitwise whatever the
 // timings.
 int element_tune_key(const Model& m) { return m.opts.elem_threads | (m.opts.deterministic ? 0x400 : 0); }
 efem_status tune_element_blocks(Model& m)
 {
-    const int forced = m.opts.elem_threads ? m.opts.elem_threads : (m.opts.deterministic ? 128 : 0);
+    const bool want_thread = m.opts.elem_threads == 1;
+    const int forced = m.opts.elem_threads && !want_thread ? m.opts.elem_threads : (m.opts.deterministic ? 128 : 0);
     const size_t n = 3 * static_cast<size_t>(std::max(m.n_free, 1));
     EFEM_CUDA(cudaMemsetAsync(m.d_u, 0, n * sizeof(double), m.stream));
     cudaEvent_t e0, e1;
@@ -770,6 +771,12 @@ efem_status tune_element_blocks(Model& m)
     for (size_t bi = 0; bi < m.blocks.size(); bi++) {
         DevBlock& b = m.blocks[bi];
         for (int prec = 0; prec < 2; prec++) {
+            const bool has_thread = prec == 1 && has_thread_kernel<float>(b.nen, b.ngp);
+            if (want_thread && has_thread) {
+                b.threads[prec] = kTB;
+                b.per_sm[prec] = kPerSM;
+                continue;
+            }
             if (forced == 64 || forced == 128 || forced == 256) {
                 b.threads[prec] = forced;
                 b.per_sm[prec] = 0;
@@ -782,7 +789,7 @@ efem_status tune_element_blocks(Model& m)
             }
             float best = 1e30f;
             for (int t : { 64, 128, 256, -kPerSM, 1 - kPerSM }) {  // negative: k_elem_thread, CTAs per SM
-                if (t < 0 && !(prec == 1 && has_thread_kernel<float>(b.nen, b.ngp))) continue;
+                if (t < 0 && !has_thread) continue;
                 const int threads = t < 0 ? kTB : t, per_sm = t < 0 ? -t : 0;
                 for (int rep = 0; rep < 7; rep++) {
                     if (rep == 2) EFEM_CUDA(cudaEventRecord(e0, m.stream));
@@ -797,7 +804,7 @@ efem_status tune_element_blocks(Model& m)
                 EFEM_CUDA(cudaEventSynchronize(e1));
                 float ms = 0.f;
                 EFEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best || (per_sm && std::getenv("EFEM_TEST_ELEM_SPLIT"))) {
+                if (ms < best) {
                     best = ms;
                     b.threads[prec] = threads;
                     b.per_sm[prec] = per_sm;

@@ -115,7 +115,9 @@ typedef struct {
     double adjoint_tolerance; /* relative residual of the adjoint solve (default 1e-8) */
     int adjoint_max_iterations; /* GMRES iteration limit of the adjoint solve (default 2000) */
     int elem_threads;         /* element-kernel CTA size: 0 = chosen per element block by the autotuner
-                                 at set-up (64, 128 or 256 threads, timed); 64 / 128 / 256 = forced */
+                                 at set-up (64, 128 or 256 threads, timed); 64 / 128 / 256 = forced;
+                                 1 = as 0, but FP32 elements of 20 nodes and 27 points take the kernel
+                                 that sums the forces in registers, without being timed */
     int consistent_inertia;   /* gravity loads: 1 consistent mass, 0 lumped (analysis "consistent_inertia",
                                  src/io/Config.cpp:63-65) */
     int trace;                /* > 0: keep a convergence trace of up to this many records per solve
