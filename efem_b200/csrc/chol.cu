@@ -73,7 +73,7 @@ struct Precond {
     bool factored = false;  // numeric factor present
     bool ok = false;        // factor is positive definite
     double ms_factor = 0;
-    int max_r = 0, max_c = 0, max_m = 0, nlev = 0;
+    int nlev = 0;
     // solve schedule: the persistent kernel's items, launch shape
     int n_items = 0, solve_grid = 1, solve_grid_full = 1, slots = 1;
     size_t solve_smem = 0;
@@ -116,8 +116,7 @@ struct Precond {
     cudaStream_t capture2 = nullptr;  // second branch of the factorisation's graph
     int* d_res = nullptr;   // the last application's error flag
     int* h_flag = nullptr;  // mapped host memory: set by any application that gave up, cleared by the host
-    double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_t = nullptr,
-           *d_vals = nullptr;
+    double *d_front = nullptr, *d_upd = nullptr, *d_y = nullptr, *d_vals = nullptr;
     // graph replay of the numeric factorisation (the same launches every solve)
     cudaGraphExec_t factor_exec = nullptr;
     long long factor_launches = 0;
@@ -608,7 +607,6 @@ struct SolveArgs {
     int n_items, ns;
     double* v;
     double* y;
-    double* t;
     double* upd;
     int* cnt;
     unsigned long long* stamp;  // when set: global timer at the start of the solve
@@ -1406,7 +1404,6 @@ FrontArgs args_of(Precond& P)
 // the work buffers of one solve
 struct SolveBufs {
     double* y;    // forward result, 3 per node
-    double* t;    // backward intermediate, 3 per node
     double* upd;  // fronts' update vectors
     int* cnt;     // completion counters, ticket, error flag (4 ns + 2)
 };
@@ -1431,7 +1428,8 @@ efem_status enqueue_solve(const Precond& P, const FrontArgs& a, const SolveBufs&
     const SubArgs B { a, P.d_parent, P.d_prow, P.d_perm, P.d_subs, P.d_chunks, P.d_depth, P.d_xidx, P.sub_max_r,
         P.sub_max_cols, P.sub_max_depth, P.sub_max_m, P.sub_max_c, P.sub_max_mroot, d_v, b.y, b.upd, stamp };
     if (P.n_subs > 0) k_sub_fwd<<<P.n_subs, kST, P.sub_smem_f, st>>>(B);
-    SolveArgs A { a, P.d_prow, P.d_items, P.d_slot, P.n_items, ns, d_v, b.y, b.t, b.upd, b.cnt, P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, own ? P.d_res : nullptr, own ? P.h_flag : nullptr,
+    SolveArgs A { a, P.d_prow, P.d_items, P.d_slot, P.n_items, ns, d_v, b.y, b.upd, b.cnt,
+        P.n_subs > 0 ? nullptr : stamp, wc.limit, wc.test, 3 * P.S.n, own ? P.d_res : nullptr, own ? P.h_flag : nullptr,
         P.d_item_group, P.d_item_group ? P.d_frozen : nullptr };
     if (P.n_items > 0) launch_k(k_solve, P.solve_grid, kST, P.solve_smem, st, A);
     if (P.n_subs > 0) k_sub_bwd<<<P.n_subs, kST, P.sub_smem_b, st>>>(B);
@@ -1464,7 +1462,7 @@ void free_precond(Model& m)
     dev_free(P.d_steps);
     dev_free(P.d_invs);
     dev_free(P.d_wtiles);
-    for (double** p : { &P.d_front, &P.d_xw, &P.d_lp, &P.d_upd, &P.d_y, &P.d_t, &P.d_vals })
+    for (double** p : { &P.d_front, &P.d_xw, &P.d_lp, &P.d_upd, &P.d_y, &P.d_vals })
         dev_free(*p);
     delete m.precond;
     m.precond = nullptr;
@@ -1538,9 +1536,6 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
         for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; q++) {
             const int s = S.level_list[q];
             const int c = S.ncol[s], mm = S.nrow[s] - c;
-            P.max_r = std::max(P.max_r, S.nrow[s]);
-            P.max_c = std::max(P.max_c, c);
-            P.max_m = std::max(P.max_m, mm);
             maxc = std::max(maxc, c);
             if (S.child_ptr[s + 1] > S.child_ptr[s])
                 for (int j = 0; j < S.nrow[s]; j += kEC)
@@ -1818,7 +1813,6 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     EFEM_CUDA(cudaMemsetAsync(P.d_xw, 0, sizeof(double) * std::max<long long>(xw_size, 1), m.stream));  // above X's diagonal, pad rows
     if ((st = dev_alloc(&P.d_upd, static_cast<size_t>(std::max<long long>(S.upd_size, 1)))) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_y, n3)) != EFEM_OK) return st;
-    if ((st = dev_alloc(&P.d_t, n3)) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_cnt, 4 * static_cast<size_t>(S.ns) + 2)) != EFEM_OK) return st;
     if ((st = dev_alloc(&P.d_fail, 1)) != EFEM_OK) return st;
     // persistent solve: as many CTAs as fit on the device at once
@@ -1977,7 +1971,7 @@ efem_status precond_enqueue(Model& m, double* d_v, cudaStream_t stream, unsigned
     }
     Precond& P = *m.precond;
     if (P.S.n == 0) return EFEM_OK;
-    const efem_status s = enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_t, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), true, stamp);
+    const efem_status s = enqueue_solve(P, args_of(P), SolveBufs { P.d_y, P.d_upd, P.d_cnt }, d_v, stream, wait_cfg(m), true, stamp);
     if (m.opts.wait_test == 2) m.opts.wait_test = 0;  // that was the one application
     if (s != EFEM_OK) return s;
     EFEM_CUDA(cudaGetLastError());
@@ -2039,14 +2033,16 @@ efem_status precond_check(Model& m)
 // control loops that forbid the implicit device synchronisation an allocation
 // can cause.  For them efem_precond_apply_noalloc runs the same forward and
 // backward sweeps as efem_precond_apply, but its working memory (the forward
-// and backward intermediates, 3 per free node each, the fronts' update
-// vectors, and the solve's completion counters) lives in the fixed array
-// below instead of buffers owned by the model.
+// result, 3 per free node, the fronts' update vectors, and the solve's
+// completion counters) lives in the fixed array below instead of buffers owned
+// by the model.
 //
 // Limits and sharing:
 //   * the array holds kNoAllocDoubles doubles (16 MiB); a model that needs
-//     more (6 * free nodes + its update-vector length + 2 * fronts + 1) is
-//     rejected;
+//     more than that by the interface's formula (6 * free nodes + its
+//     update-vector length + 2 * fronts + 1) is rejected.  The sweeps use
+//     half of the formula's first term; which models are refused is part of
+//     the interface and stays;
 //   * every GPU that loads this library keeps the array until the process
 //     exits;
 //   * all calls share the array and it keeps the last call's contents; the
@@ -2091,7 +2087,7 @@ extern "C" efem_status efem_precond_apply_noalloc(void* model, double* d_v)
         return EFEM_ERR_ARG;
     }
     Model& m = *static_cast<Model*>(model);
-    // two vectors of 3 per free node are the least any model needs: refuse
+    // by the interface's formula 6 per free node are the least any model needs: refuse
     // models that cannot fit before asking for anything else
     if (6 * static_cast<size_t>(m.n_free) > kNoAllocDoubles) {
         set_error("model needs at least " + std::to_string(6 * static_cast<size_t>(m.n_free))
@@ -2151,8 +2147,8 @@ extern "C" efem_status efem_precond_apply_noalloc(void* model, double* d_v)
             return EFEM_ERR_ARG;
         }
     }
-    int* counters = reinterpret_cast<int*>(scratch + 2 * n3 + S.upd_size);
-    const SolveBufs b { scratch, scratch + n3, scratch + 2 * n3, counters };
+    int* counters = reinterpret_cast<int*>(scratch + n3 + S.upd_size);
+    const SolveBufs b { scratch, scratch + n3, counters };
     efem_status st = enqueue_solve(P, args_of(P), b, d_v, m.stream, wait_cfg(m), false);
     if (st != EFEM_OK) return st;
     EFEM_CUDA(cudaGetLastError());
