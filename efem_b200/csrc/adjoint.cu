@@ -58,16 +58,17 @@ struct TanElemArgs {
     const double* __restrict__ J0inv;
     const double* __restrict__ dN;
     const double* __restrict__ gw;
-    const MatParams<Dual>* __restrict__ mats;
+    const MatParams<Dual>* __restrict__ mats;  // k_elem_tangent: one constant seeded
     const double* __restrict__ u;
-    const double* __restrict__ v;   // direction (nullptr: none)
+    const double* __restrict__ v;   // direction (k_tangent)
     double* __restrict__ out;       // += derivative of r
 };
 
-// elements per CTA of the tangent kernel (dual numbers double the shared memory)
+// elements per CTA of the tangent kernels (two values per unknown in shared memory)
 __host__ __device__ constexpr int tan_epb(int ngp) { return (kBlock / ngp) < 1 ? 1 : ((kBlock / ngp) > 32 ? 32 : kBlock / ngp); }
 
-// The element residual of residual.cu on dual numbers: out += d r_el.
+// The element residual of residual.cu on dual numbers, the seed on a material
+// constant: out += d r_el / d theta.
 template <int NEN, int NGP>
 __global__ void __launch_bounds__(kBlock) k_elem_tangent(TanElemArgs a)
 {
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(kBlock) k_elem_tangent(TanElemArgs a)
             node = a.conn[static_cast<size_t>(nd) * a.n + e];
             if (node < a.n_free)
 #pragma unroll
-                for (int c = 0; c < 3; c++) x[c] = Dual(a.u[3 * node + c], a.v ? a.v[3 * node + c] : 0.0);
+                for (int c = 0; c < 3; c++) x[c] = Dual(a.u[3 * node + c]);
         }
         s_node[el][nd] = node;
 #pragma unroll
@@ -154,8 +155,8 @@ struct TanFaceArgs {
     const double* __restrict__ t_N;
     const double* __restrict__ t_dN;
     const double* __restrict__ u;
-    const double* __restrict__ v;       // direction, or the vector K^T is applied to (nullptr: none)
-    const double* __restrict__ dscale;  // per pressure load: derivative of its scale (nullptr: none)
+    const double* __restrict__ v;       // tangent: direction, or the vector K^T is applied to
+    const double* __restrict__ dscale;  // k_face_tangent: per pressure load, the derivative of its scale
     double* __restrict__ out;
 };
 
@@ -470,7 +471,7 @@ __device__ void face_forces(const TanFaceArgs& a, int f, const Dual (*uu)[3], Du
     const int ngp = a.t_ngp[t];
     const double* L = a.load + 4 * f;
     const bool directed = L[0] != 0.0;
-    const double ds = a.dscale ? a.dscale[a.load_idx[f]] : 0.0;
+    const double ds = a.dscale[a.load_idx[f]];
     Dual cA[MAX_FGP][3];
     for (int g = 0; g < ngp; g++) {
         const double* dN = a.t_dN + (static_cast<size_t>(t) * MAX_FGP + g) * NEN * 3;
@@ -515,7 +516,7 @@ __device__ void face_forces(const TanFaceArgs& a, int f, const Dual (*uu)[3], Du
     }
 }
 
-// out -= d f (the face part of R is -f): K_face v, or dR/dscale
+// out -= d f / d scale (the face part of R is -f)
 template <int NEN>
 __global__ void __launch_bounds__(kBlock) k_face_tangent(TanFaceArgs a)
 {
@@ -527,8 +528,7 @@ __global__ void __launch_bounds__(kBlock) k_face_tangent(TanFaceArgs a)
         node[q] = a.conn[static_cast<size_t>(q) * a.n + f];
         const bool fr = node[q] < a.n_free;
 #pragma unroll
-        for (int c = 0; c < 3; c++)
-            uu[q][c] = fr ? Dual(a.u[3 * node[q] + c], a.v ? a.v[3 * node[q] + c] : 0.0) : Dual(0.0);
+        for (int c = 0; c < 3; c++) uu[q][c] = Dual(fr ? a.u[3 * node[q] + c] : 0.0);
     }
     Dual fq[NEN][3];
     face_forces<NEN>(a, f, uu, fq);
@@ -769,7 +769,6 @@ struct AdjointWS {
     double* h_hcol = nullptr;  // pinned host copy
     cudaEvent_t got_col = nullptr;  // the column of the iteration is in h_hcol
     MatParams<Dual>* mats = nullptr;
-    int mats_seed = -2;  // the seed `mats` holds: 5 slot + k, -1 none, -2 not uploaded
     double* dscale = nullptr;
     std::vector<double> h_part;
 };
@@ -816,13 +815,9 @@ efem_status alloc_aws(Model& m)
 }
 
 // material table on dual numbers; seed (slot, k) puts derivative 1 on constant
-// k (0 C10, 1 C01, 2 C20, 3 C30, 4 D1) of material slot `slot` (-1: none)
+// k (0 C10, 1 C01, 2 C20, 3 C30, 4 D1) of material slot `slot`
 efem_status upload_dual_mats(Model& m, int slot, int k)
 {
-    // the table depends on the seed alone (a model's materials are fixed)
-    const int seed = slot < 0 ? -1 : 5 * slot + k;
-    if (m.aws->mats_seed == seed) return EFEM_OK;
-    m.aws->mats_seed = -2;
     std::vector<MatParams<Dual>> h(std::max<size_t>(m.materials_used.size(), 1));
     for (size_t i = 0; i < m.materials_used.size(); i++) {
         const HostMaterial& hm = m.materials_used[i];
@@ -835,7 +830,6 @@ efem_status upload_dual_mats(Model& m, int slot, int k)
         h[i].D1 = Dual(hm.D1, s && k == 4 ? 1.0 : 0.0);
     }
     EFEM_CUDA(cudaMemcpyAsync(m.aws->mats, h.data(), sizeof(MatParams<Dual>) * h.size(), cudaMemcpyHostToDevice, m.stream));
-    m.aws->mats_seed = seed;
     return EFEM_OK;
 }
 
@@ -948,8 +942,6 @@ efem_status param_derivative(Model& m, const double* u, int k, double* out)
         efem_status s = upload_dual_mats(m, k / 5, k % 5);
         if (s != EFEM_OK) return s;
         launch_elem_param(m, u, out);
-        s = upload_dual_mats(m, -1, 0);
-        if (s != EFEM_OK) return s;
     } else {
         std::vector<double> ds(std::max(m.n_pressure_loads, 1), 0.0);
         ds[k - 5 * nm] = 1.0;
@@ -1132,7 +1124,6 @@ efem_status hvp(Model& m, const double* d_u, const double* d_v, double* d_out, b
 {
     efem_status s = alloc_aws(m);
     if (s != EFEM_OK) return s;
-    if ((s = upload_dual_mats(m, -1, 0)) != EFEM_OK) return s;
     return tangent(m, d_u, d_v, d_out, transpose);
 }
 
@@ -1164,7 +1155,6 @@ efem_status adjoint(Model& m, const double* d_u, const double* d_dJdu, double* d
         set_error("approximate Jacobian is not positive definite (no preconditioner for the adjoint solve)");
         return EFEM_ERR_NAN;
     }
-    if ((s = upload_dual_mats(m, -1, 0)) != EFEM_OK) return s;
     EFEM_CUDA(cudaMemcpyAsync(w.u, d_u, sizeof(double) * n, cudaMemcpyDeviceToDevice, m.stream));
     EFEM_CUDA(cudaMemcpyAsync(w.b, d_dJdu, sizeof(double) * n, cudaMemcpyDeviceToDevice, m.stream));
     const double tol = m.opts.adjoint_tolerance > 0 ? m.opts.adjoint_tolerance : 1e-8;

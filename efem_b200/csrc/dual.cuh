@@ -1,8 +1,8 @@
 // Forward-mode dual numbers (value + one directional derivative) for the
-// tangent kernels.  Instantiating the material and kinematics templates of
-// mechanics.cuh on Dual gives, in one pass, P(F) and its derivative along a
-// chosen direction: a displacement increment (the true tangent K(u) v) or a
-// material constant (dR/dtheta).
+// parameter derivatives.  Instantiating the material and kinematics templates
+// of mechanics.cuh on Dual gives, in one pass, P(F) and its derivative with
+// respect to a material constant, or a face's forces and theirs with respect to
+// the load's scale (dR/dtheta).
 #pragma once
 #include <cuda_runtime.h>
 
