@@ -41,10 +41,25 @@ def test_residual_with_faces(etype, n, load, tmp_path):
 @pytest.mark.parametrize("law", ["nh", "mr", "yeoh"])
 @pytest.mark.parametrize("load", ["pressure", "dpressure"])
 def test_tangent_with_faces(etype, n, law, load):
+    check_tangent(mg.small_case(etype, law, load, n=n, size=tuple(0.01 * k for k in n)))
+
+
+@pytest.mark.parametrize("etype,n", [("C3D4", (2, 2, 3)), ("C3D8", (3, 3, 3)), ("C3D10", (2, 2, 2)), ("C3D20", (3, 2, 2))])
+@pytest.mark.parametrize("load", ["pressure", "dpressure", "force"])
+def test_tangent_of_mixed_laws(etype, n, load):
+    """Three laws in one element block: the law is chosen at run time."""
+    case = mg.small_case(etype, "nh", load, n=n, size=tuple(0.01 * k for k in n))
+    case.materials = [mg.mat_nh(), mg.mat_mr(C10=57000.0, C01=57000.0), mg.mat_yeoh(C10=114000.0, C20=16000.0, C30=16000.0)]
+    for i, mat in enumerate(case.materials):
+        mat["id"] = i + 1
+    case.mesh.mat = 1 + np.arange(case.mesh.conn.shape[0]) % 3
+    check_tangent(case)
+
+
+def check_tangent(case):
     """K(u) v against central differences of R (truncation h^2 with h |v| about
     1e-8 m on 1e-2 m elements, cancellation eps |R| / h: 1e-6 relative holds
     both), and w.(K v) = (K^T w).v to rounding."""
-    case = mg.small_case(etype, law, load, n=n, size=tuple(0.01 * k for k in n))
     m = api.Model.from_case(case)
     u = displaced(case)
     rng = np.random.default_rng(11)

@@ -1,7 +1,8 @@
 """The L-BFGS vector kernels at the sizes where they can go wrong -- fewer
 entries than a warp, one CTA's last and the grid's first size (4096 entries),
 histories that wrap, the general kernels' history of 9 -- against the same
-iteration written with numpy on the library's own r(u) and H0 v."""
+iteration written with numpy on the library's own r(u) and H0 v; and a batch's,
+whose members are cut into chunks of 512 entries."""
 import numpy as np
 import pytest
 
@@ -63,3 +64,24 @@ def test_iterations_match_numpy(n, load, hist):
     assert info["niter"] == ITERS and info["n_residual_evals"] == evals and (evals > ITERS + 1) == (load == -10.0)
     # both sides round alike but for the order of sums: eps times the condition (up to 1e6 on the slender bar)
     assert np.linalg.norm(u - ref) <= 1e-9 * np.linalg.norm(ref)
+
+
+# 12, 510 and 513 (one chunk and two), 1020 and 1026 (two and three) DOFs; some
+# members take further line-search trials while the others wait
+@pytest.mark.parametrize("hist", [1, 3, 8])
+def test_batch_iterations_match_numpy(hist):
+    members = [((1, 1, 1), -2e-3), ((17, 4, 1), -2e-3), ((19, 2, 2), -2e-3), ((2, 1, 1), -10.0), ((34, 4, 1), -2e-3),
+               ((38, 2, 2), -2e-3), ((8, 4, 4), -10.0)]
+    o = options(hist)
+    ms = [api.Model.from_case(case(n, load), o) for n, load in members]
+    assert [m.n_dof for m in ms] == [12, 510, 513, 24, 1020, 1026, 600]
+    us, infos = api.batch_solve(ms)
+    trials = set()
+    for m, u, info, (n, _) in zip(ms, us, infos, members):
+        assert info["flags"] & api.SOLVE_BATCHED
+        ref, evals = lbfgs(m, o)
+        assert info["niter"] == ITERS and info["n_residual_evals"] == evals, n
+        # the members lie apart in the union, so their J0 round to about 1e-14 instead of 1e-16
+        assert np.linalg.norm(u - ref) <= 1e-8 * np.linalg.norm(ref), n
+        trials.add(evals > ITERS + 1)
+    assert trials == {False, True}
