@@ -653,7 +653,7 @@ __global__ void k_rows_reduce(const double* __restrict__ part, int nk, int nb, d
 constexpr int kGsTile = 64;
 constexpr int kGsRows = 104;         // most basis vectors (kRestart + 1, rounded up to the warps)
 constexpr int kGsPer = kGsRows / 8;  // rows per warp
-constexpr int kGsBlocks = 296, kGsNormBlocks = 444;  // 2 and 3 CTAs per SM
+constexpr int kGsBlocks = 2 * kSMs, kGsNormBlocks = 3 * kSMs;
 
 template <bool Norm>
 __global__ void __launch_bounds__(kVec, Norm ? 3 : 2) k_gs_update(double* __restrict__ w, const double* __restrict__ V, size_t ldv,
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(kVec) k_scale_copy(double* __restrict__ y, con
     for (size_t i = blockIdx.x * (size_t)kVec + threadIdx.x; i < n; i += (size_t)gridDim.x * kVec) y[i] = s * x[i];
 }
 
-int vec_grid(size_t n) { return static_cast<int>(std::min<size_t>(592, std::max<size_t>(1, (n + kVec - 1) / kVec))); }
+int vec_grid(size_t n) { return static_cast<int>(std::min<size_t>(4 * kSMs, std::max<size_t>(1, (n + kVec - 1) / kVec))); }
 
 // y += sum_k c_k X_k (rows of stride ldx): the 16-byte form when the layout allows
 void launch_axpys(cudaStream_t st, double* y, const double* X, size_t ldx, int nk, const double* c, size_t n)

@@ -1845,7 +1845,7 @@ static long long enqueue_factor(Precond& P, cudaStream_t st, cudaStream_t st2, c
     cudaMemsetAsync(P.d_fail, 0, sizeof(int), st);
     if (P.n_zero > 0) k_zero<<<P.n_zero, kFT, 0, st>>>(P.d_front, P.d_zero);
     const long long na = static_cast<long long>(S.a_pos.size());
-    k_scatter_a<<<static_cast<int>(std::min<long long>(1184, (na + 255) / 256 + 1)), 256, 0, st>>>(
+    k_scatter_a<<<static_cast<int>(std::min<long long>(8 * kSMs, (na + 255) / 256 + 1)), 256, 0, st>>>(
         P.d_front, P.d_a_pos, P.d_a_src, P.d_vals, na);
     n += 2;
     FrontArgs a = args_of(P);

@@ -63,6 +63,7 @@ struct MatParams {
 };
 
 constexpr int MAX_MATS = 16;
+constexpr int kSMs = 148;  // SMs of a B200: sizes grids of loops over any number of CTAs, nothing depends on it
 
 struct DevBlock {
     int kind = 0, nen = 0, ngp = 0, n = 0;

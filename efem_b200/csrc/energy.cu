@@ -116,7 +116,7 @@ efem_status total_potential(Model& m, const double* d_u, double* pi)
     const size_t n = 3 * static_cast<size_t>(m.n_free);
     double w = 0.0;
     if (n > 0) {
-        const int grid = static_cast<int>(std::min<size_t>(296, (n + kBlock - 1) / kBlock));
+        const int grid = static_cast<int>(std::min<size_t>(2 * kSMs, (n + kBlock - 1) / kBlock));
         double* part = nullptr;
         EFEM_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(double) * grid, m.stream));
         k_dot_part<<<grid, kBlock, 0, m.stream>>>(m.d_fext, d_u, n, part);

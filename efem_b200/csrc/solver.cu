@@ -52,7 +52,7 @@ thread_local bool t_pdl = false;
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMaxBlocks = 592;  // 4 x 148 SMs
+constexpr int kMaxBlocks = 4 * kSMs;
 constexpr int kMaxHist = 64;
 constexpr int kRowBlocks = 128;  // CTAs per history slot in the dot-product passes (m > kMaxFast)
 constexpr int kMaxFast = 8;      // history lengths with the 1D-grid passes k_pass1_m / k_pass3_m
@@ -240,8 +240,12 @@ __global__ void k_trial(double* __restrict__ x, const double* __restrict__ xp, c
 
 // ---- reductions over the grid
 constexpr int kPT = 512;     // threads
-constexpr int kPG = 296;     // most CTAs: two per SM (one: 7 us an iteration slower on the mixed finger, 241k DOFs)
-constexpr size_t kOne = 4096;  // entries of one CTA (750 DOFs: 61.7 us an iteration against 65.0 with passes 2 and 4 apart)
+constexpr int kPG = 2 * kSMs;  // most CTAs (one per SM: 7 us an iteration slower on the mixed finger, 241k DOFs)
+// Entries up to which one CTA makes the passes.  Microseconds an iteration with
+// one CTA and with the grid, C3D8 boxes of 600, 1470, 2916, 3900, 4200, 5808
+// DOFs: 46.5 / 59.8, 55.4 / 65.3, 69.2 / 73.4, 77.1 / 75.5, 78.4 / 76.8,
+// 90.5 / 82.1
+constexpr size_t kOne = 3584;
 
 int pass_grid(size_t n) { return n <= kOne ? 1 : static_cast<int>(std::min<size_t>(kPG, (n + kPT - 1) / kPT)); }
 
@@ -992,7 +996,7 @@ efem_status enqueue_trial_tail(Model& m, SolverWS& w, double* x, cudaStream_t st
     efem_status s = launch_residual_on(m, x, w.r, st, &w.sc->t0_res, init_r);
     if (s != EFEM_OK) return s;
     // one CTA per SM: with 296, 2.4 us an iteration slower on the finger (241k DOFs)
-    launch_k(k_ls_reduce, std::min(148, pass_grid(n)), kPT, 0, st, w.r, w.d, x, n, w.sc, w.partials, precond_error_flag(m),
+    launch_k(k_ls_reduce, std::min(kSMs, pass_grid(n)), kPT, 0, st, w.r, w.d, x, n, w.sc, w.partials, precond_error_flag(m),
         mapped(w.h_read), h_ls ? *h_ls : cudaGraphConditionalHandle(),
         h_it ? *h_it : cudaGraphConditionalHandle(), h_ls ? 1 : 0);
     return EFEM_OK;
@@ -1067,6 +1071,12 @@ efem_status add_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t
     return EFEM_OK;
 }
 
+// launch_k uses programmatic dependent launch while one of these is alive
+struct PdlScope {
+    explicit PdlScope(bool on) { t_pdl = on; }
+    ~PdlScope() { t_pdl = false; }
+};
+
 // The device-driven iteration loop:
 //   k_loop_start;
 //   while (hIter) { passes + H0 + first trial; residual; reductions + decisions;
@@ -1074,12 +1084,6 @@ efem_status add_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t
 // The inner node costs 1.3 us an iteration even when it does not run; a single
 // loop whose passes and H0 return at once in a further trial made a solve with
 // ten trials an iteration (the C3D8 beam from u = 0) 12% slower.
-// launch_k uses programmatic dependent launch while one of these is alive
-struct PdlScope {
-    explicit PdlScope(bool on) { t_pdl = on; }
-    ~PdlScope() { t_pdl = false; }
-};
-
 efem_status capture_loop(Model& m, SolverWS& w, double* x, bool use_factor, cudaGraphExec_t* out)
 {
     std::lock_guard<std::mutex> lock(capture_mutex());

@@ -1,5 +1,5 @@
 """The L-BFGS vector kernels at the sizes where they can go wrong -- fewer
-entries than a warp, one CTA's last and the grid's first size (4096 entries),
+entries than a warp, one CTA's last and the grid's first size (3584 entries),
 histories that wrap, the general kernels' history of 9 -- against the same
 iteration written with numpy on the library's own r(u) and H0 v; and a batch's,
 whose members are cut into chunks of 512 entries."""
@@ -52,8 +52,9 @@ def lbfgs(m, o):
     return x, evals
 
 
-# 12, 24, 4056, 4092, 4104 and 17 424 DOFs; the load of -10 takes further line-search trials
-@pytest.mark.parametrize("n,load", [((1, 1, 1), -2e-3), ((2, 1, 1), -10.0), ((8, 12, 12), -2e-3), ((341, 1, 1), -2e-3),
+# 12, 24, 3570, 3588, 4056, 4092, 4104 and 17 424 DOFs; the load of -10 takes further line-search trials
+@pytest.mark.parametrize("n,load", [((1, 1, 1), -2e-3), ((2, 1, 1), -10.0), ((14, 16, 4), -2e-3),
+                                    ((13, 22, 3), -2e-3), ((8, 12, 12), -2e-3), ((341, 1, 1), -2e-3),
                                     ((8, 18, 8), -2e-3), ((24, 21, 10), -10.0)])
 @pytest.mark.parametrize("hist", [1, 3, 8, 9])
 def test_iterations_match_numpy(n, load, hist):
