@@ -351,7 +351,9 @@ struct TanElemSmem {
 // out += K_el v, the derivative of the element residual of residual.cu along
 // v, in its three phases with dP = dP/dH : dH by hand (piola_tangent) in place
 // of dual numbers; the first n_face_tiles CTAs take the faces.  Bound by
-// latency at 16 warps per SM (124 registers) and by FP64 issue.  C3D10 finger,
+// latency: 16 warps per SM with the neo-Hookean and Yeoh laws (124 to 126
+// registers; issue slots 29% busy, a third of the stalls on loads), 12 with
+// Mooney-Rivlin and in blocks of mixed laws (164 to 168).  C3D10 Yeoh finger,
 // transpose product with the chamber faces: 32 us (cold), where the elements on
 // dual numbers took 77 us (240 registers, 8 warps per SM) and the faces 68 us
 // more; the products of an adjoint solve, which read stored Gauss-point
@@ -646,8 +648,9 @@ __global__ void k_rows_reduce(const double* __restrict__ part, int nk, int nb, d
 // A CTA takes 64 entries of every vector at a time; warp q holds the rows
 // k = q mod 8 and a lane two entries, so a thread uses the values that it
 // loaded itself for both, from registers, and only the eight partial updates
-// of an entry meet in shared memory.  Bound by HBM: with 64 vectors of 240 600
-// entries (123 MB) 27 us, 4.5 TB/s.  As two updates and two products by
+// of an entry meet in shared memory.  With 64 vectors of 240 600 entries
+// (123 MB) 27 us, 4.5 TB/s: bound by the loads in flight (16 warps an SM of 122
+// registers, 45% of the stalls on loads) below HBM's rate.  As two updates and two products by
 // themselves (36 + 20 us each; the basis read four times) an iteration's
 // orthogonalisation took 140 us at the average 64 vectors, now 85.
 constexpr int kGsTile = 64;

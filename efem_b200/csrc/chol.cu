@@ -574,9 +574,13 @@ __global__ void __launch_bounds__(256) k_w(FrontArgs a, const int4* __restrict__
 //     forward tile into L2, the index of every row to be assembled (a dense
 //     table per front and child: consecutive threads read consecutive
 //     entries), and the backward tile's part over y.
-// What bounds it: the chain of dependent fronts (11-13 per sweep, 4-5 us
-// each: notice 1, gather 0.8, product 1, partial sums and store 1, publish
-// 0.5), then the factor's bytes.  One application inside a solve, against four
+// What bounds it: on the beam and at the top of every tree the chain of
+// dependent fronts (11-13 per sweep, 4-5 us each: notice 1, gather 0.8, product
+// 1, partial sums and store 1, publish 0.5); on the cap and the finger below the
+// top, where a level has about as many items as there are CTAs and the children
+// are long done, the latencies of one item after another in its CTA (2 us from
+// taking an item to being ready with nothing to wait for: record, indices,
+// counter; gather 0.8-1, product 2-5, sums and publishing 2); not the bytes.  One application inside a solve, against four
 // matrices staged through shared memory in 4-row tiles, and against M read
 // into registers after the wait: C3D8 beam 124, 113, now 105 us; C3D20R cap
 // 330, 192, now 182 us (281 MB, 1.5 TB/s); C3D10 finger 439, 241, now 226 us
@@ -1590,8 +1594,8 @@ efem_status precond_setup(Model& m, bool refactor, int* ok, double* ms_factor)
     // k_solve.  opts.solve_subtree_levels = K asks for them (K is lowered
     // until the subtrees fit in shared memory); the default (-1) is K = 0.
     // Measured on the 20 480-element C3D8 beam (11 levels), one H0
-    // application inside the solve costs 274 us per iteration with K = 0 and
-    // 290, 322, 361, 450 us with K = 1, 2, 3, 4: a subtree CTA streams its
+    // application inside the solve costs 106 us with K = 0 and 125, 152, 186,
+    // 283 us with K = 1, 2, 3, 4: a subtree CTA streams its
     // factor rows one 32 KB chunk ahead, about 20 GB/s, and works through its
     // fronts one after another, which is slower than the notification steps
     // of the levels it replaces.

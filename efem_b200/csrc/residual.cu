@@ -412,9 +412,10 @@ __global__ void __launch_bounds__(BLK) k_elem_residual(ElemArgs<T> a, FaceArgs<T
 // of the thread's own column, dN a broadcast (every lane of a warp is at the
 // same point) and the forces are added up in registers.  J0^{-1} of the next
 // point is fetched by the warp for its 32 elements, coalesced, while this one
-// is worked on.  What bounds it is latency at 16 warps an SM: 8 CTAs by 128
-// registers (60 sums) and by shared memory; and the last wave, for which 7 CTAs
-// an SM are sometimes the better number, so the autotuner times both (`pad`).
+// is worked on.  What bounds it: issue slots 57% busy and no warp ready in
+// the other cycles at 16 warps an SM (8 CTAs by 128 registers, 60 of them sums,
+// and by shared memory); and the last wave, for which 7 CTAs an SM are sometimes
+// the better number, so the autotuner times both (`pad`).
 // One residual in a solve, neo-Hookean, with 8 and 7: 36 864 elements 53 and
 // 64 us, 60 625 elements 84 and 82, 70 713 elements 96 and 105.
 // A direct call on 60 625 elements went from 131 to 105 us (G = 1: 5 us more).  For 4 to 10 nodes, 8 points of 20, and in FP64,

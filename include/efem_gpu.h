@@ -293,8 +293,8 @@ efem_status efem_solve_trace(void* model, double* out, int capacity, int* n_reco
  * with derivatives, for gradient-based design and fitting.  Vectors follow
  * efem_options.device_ptrs like efem_residual. */
 
-/* Kv = K(u) v, the true tangent dR/du at u applied to v (forward-mode
- * derivative of the residual, exact to rounding). */
+/* Kv = K(u) v, the true tangent dR/du at u applied to v (the residual's
+ * expressions differentiated by hand, exact to rounding). */
 efem_status efem_hvp(void* model, const double* u, const double* v, double* Kv);
 
 /* KTw = K(u)^T w.  The element part of K is symmetric; the pressure part is
